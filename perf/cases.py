@@ -164,7 +164,8 @@ def prepare(case, seed):
         kq, vq = _quantizers(c)
         lens = torch.from_numpy(_lens(c, seed).astype(np.int32)).to(DEV)
         q = _normal(g, dt, b, c["hq"], c["lq"], d)
-        s["call"] = P.PackedAttention(q, _rows(c, kq, g, b, c["lk"] + 4), _rows(c, vq, g, b, c["lk"] + 4), lens, kq, vq, s["cfg"])
+        s.update(q=q, k=_rows(c, kq, g, b, c["lk"] + 4), v=_rows(c, vq, g, b, c["lk"] + 4), kq=kq, vq=vq)
+        s["call"] = P.PackedAttention(q, s["k"], s["v"], lens, kq, vq, s["cfg"])
     elif c["kind"] == "blocks":
         kq, vq = _quantizers(c)
         left, blocks = c["lk"], []
@@ -172,7 +173,8 @@ def prepare(case, seed):
             blocks.append(P.KvBlockRef(_rows(c, kq, g, b, c["page"]), _rows(c, vq, g, b, c["page"]), min(left, c["page"])))
             left -= c["page"]
         lens = torch.from_numpy(_lens(c, seed).astype(np.int32)).to(DEV)
-        s["call"] = P.PackedBlocksAttention(_normal(g, dt, b, c["hq"], c["lq"], d), blocks, kq, vq, s["cfg"], kv_len=lens)
+        s.update(q=_normal(g, dt, b, c["hq"], c["lq"], d), blocks=blocks, kq=kq, vq=vq)
+        s["call"] = P.PackedBlocksAttention(s["q"], blocks, kq, vq, s["cfg"], kv_len=lens)
     elif c["kind"] == "append":
         s["kq"], s["vq"] = _quantizers(c)
         s["q"] = _normal(g, dt, b, c["lq"], c["hq"], d)
@@ -255,3 +257,76 @@ def tolerance(case):
     else:
         rel = 3.7e-3 if case["kind"] in ("step", "packed", "blocks") else 1.7e-3
     return {"rel": rel, "differ": 0.0}
+
+
+E2M1 = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0, -0.0, -0.5, -1.0, -1.5, -2.0, -3.0, -4.0, -6.0], dtype=torch.float64)
+
+
+def _decoded(rows, fmt, quantizer):
+    """Packed rows (..., words) as 64-bit values, rotated back."""
+    d = quantizer.dim
+    by = rows.contiguous().view(torch.uint8)
+    width = d if fmt in ("fp8", "mxfp8") else d // 2
+    scale = by[..., 4 * (rows.shape[-1] - 2):4 * (rows.shape[-1] - 1)].contiguous().view(torch.float32).double()
+    e4m3 = lambda x: x.contiguous().view(torch.float8_e4m3fn).to(torch.float64)
+    codes = by[..., :width]
+    if fmt in ("fp8", "mxfp8"):
+        x = e4m3(codes)
+    else:
+        table = quantizer.tab[:16].double() if fmt == "turbo4" else E2M1.to(DEV)
+        x = table[torch.stack([codes & 15, codes >> 4], -1).long()].flatten(-2)
+    if fmt in ("mxfp4", "mxfp8"):
+        x = x * torch.exp2(by[..., width:width + d // 32].double() - 127).repeat_interleave(32, -1)
+    elif fmt == "nvfp4":
+        x = x * e4m3(by[..., width:width + d // 16]).repeat_interleave(16, -1)
+    x = x * scale
+    if quantizer.signs is not None:  # y = H (signs x) / sqrt(d), and H / sqrt(d) is its own inverse
+        h = torch.ones(1, 1, dtype=torch.float64, device=DEV)
+        while h.shape[0] < d:
+            h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+        x = (x @ h) * (d ** -0.5) * quantizer.signs.double()
+    return x
+
+
+def _attend(q, k, v, causal):
+    """q (hq, lq, d) over k, v (hkv, lk, d) in 64 bits, masks aligned at the bottom right, a kv head and some rows at a time."""
+    hq, lq, d = q.shape
+    hkv, lk, _ = k.shape
+    out = torch.empty(q.shape, dtype=torch.float64, device=DEV)
+    step = max(1, (1 << 27) // (lk * (hq // hkv)))
+    for h in range(hkv):
+        heads = slice(h * (hq // hkv), (h + 1) * (hq // hkv))
+        for at in range(0, lq, step):
+            s = (q[heads, at:at + step].double() @ k[h].double().T) * d ** -0.5
+            if causal:
+                n = torch.arange(at, at + s.shape[1], device=DEV)[:, None] + lk - lq
+                s.masked_fill_(torch.arange(lk, device=DEV)[None] > n, -torch.inf)
+            out[heads, at:at + step] = torch.softmax(s, -1) @ v[h].double()
+    return out
+
+
+def exact(case, seed):
+    """What `run` returns in 64 bits; packed rows have no such value (they are compared as whole numbers)."""
+    c, s = case, prepare(case, seed)
+    if c["kind"] == "codec":
+        return None, _decoded(s["quantizer"].quantize(s["x"]).data, c["fmt"], s["quantizer"]).view(s["x"].shape)
+    if c["kind"] == "varlen":
+        cu = s["cu"].tolist()
+        parts = [[t[i:j].transpose(0, 1) for t in (s["q"], s["k"], s["v"])] for i, j in zip(cu, cu[1:])]
+        return torch.cat([_attend(*p, c["causal"]).transpose(0, 1) for p in parts])
+    if c["kind"] in ("dense", "append"):
+        rows = zip(*(t.transpose(1, 2) for t in (s["q"], s["k"], s["v"])))
+        out = torch.stack([_attend(*r, c.get("causal", True)).transpose(0, 1) for r in rows])
+        return (out, None, None) if c["kind"] == "append" else out
+    if c["kind"] in ("step", "chunk"):
+        _, k, v = run(s)
+        lens, kq, vq, q = [s["cache"].len] * c["b"], s["cache"].kq, s["cache"].vq, s["q"]
+    else:
+        q, kq, vq = s["q"], s["kq"], s["vq"]
+        if c["kind"] == "blocks":
+            k, v = (torch.cat([getattr(x, n)[:, :, :x.rows] for x in s["blocks"]], 2) for n in ("k", "v"))
+        else:
+            k, v = s["k"], s["v"]
+        lens = torch.from_numpy(_lens(c, seed)).tolist()
+    out = torch.stack([_attend(q[i], _decoded(k[i, :, :n], c["fmt"], kq), _decoded(v[i, :, :n], c["fmt"], vq), True) for i, n in enumerate(lens)])
+    return (out, None, None) if c["kind"] in ("step", "chunk") else out
