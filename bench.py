@@ -841,7 +841,7 @@ def prefill_leg(env, steps, warmup):
             "e2e": {"value": flops / (e2e_ms * 1e-3) / 1e12, "unit": "TFLOP/s", "ms_per_step": e2e_ms,
                     "h2d_bytes_per_step": int(sum(t.numel() for t in sets[0])) * 2 * world, "d2h_bytes_per_step": int(out_host.numel()) * 2 * world},
             "gpu_launches": steps * 2 * world,  # the attention kernel and the quantize-on-append kernel (K and V in one grid)
-            "roofline": {"bound": "tensor", "kernel": "fa_prefill_sm100_kernel2 (attention alone)", "achieved": achieved,
+            "roofline": {"bound": "tensor", "kernel": "fa_prefill_tma_kernel (attention alone)", "achieved": achieved,
                          "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "peak_source": kind + (f" x {world} GPUs" if world > 1 else ""),
                          "frac_of_sustained": achieved / (pk["bf16_tflops_sustained"] * world) if "bf16_tflops_sustained" in pk else None,
                          # dram read + write of one launch at B = 1 (50.4 + 3.0 MB, part of q / k / v still in L2 from the

@@ -1,7 +1,12 @@
-// Prefill attention tiles on the 5th generation tensor cores (tcgen05, accumulators in tensor memory).
+// Prefill attention tiles on the 5th generation tensor cores (tcgen05, accumulators in tensor memory), f16 or bf16. Query
+// rows are packed (row = token * group + head in group, so the heads that share a kv head also share every K / V tile).
+// Three kernels:
+//   fa_prefill_tma_kernel<64 | 128>  head dims up to 128, any tensors that tensor maps describe (groups of a power of two):
+//              256 rows per work item, tiles by tensor copies. Everything usual runs here.
+//   fa_prefill_sm100_kernel2         head dim 128, 1024 rows and more that no map describes: 16-byte chunk copies.
+//   fa_prefill_sm100_kernel          the same from 512 rows on: 128 rows per block.
 //
-// One block = 128 packed query rows (row = token * group + head in group, so the heads that share a
-// kv head also share every K / V tile) of one (batch entry, kv head), head dim 128, f16 or bf16.
+// fa_prefill_sm100_kernel: one block = 128 packed query rows of one (batch entry, kv head), head dim 128.
 //   warps 0-3  softmax: thread = row. Reads its row of S from tensor memory, keeps the running
 //              maximum and sum in registers, writes P (16-bit pairs) back to tensor memory and, when the
 //              maximum moved by more than 2^8, rescales its row of O in tensor memory.
@@ -246,25 +251,6 @@ __device__ __forceinline__ void pf_exp32(const uint32_t (&s)[32], uint64_t sc2, 
         pr[i] = pf_pack2<BF16>(a0, a1);
     }
 }
-template <bool BF16>
-__device__ __forceinline__ void pf_exp64(const uint32_t (&sa)[32], const uint32_t (&sb)[32], uint64_t sc2, uint64_t nm2, uint64_t &acc_a,
-                                         uint64_t &acc_b, uint32_t (&pr)[32]) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        float a0, a1, b0, b1;
-        upk2(ffma2(pk2(u2f(sa[2 * i]), u2f(sa[2 * i + 1])), sc2, nm2), a0, a1);
-        upk2(ffma2(pk2(u2f(sb[2 * i]), u2f(sb[2 * i + 1])), sc2, nm2), b0, b1);
-        a0 = fast_exp2(a0);
-        a1 = fast_exp2(a1);
-        b0 = fast_exp2(b0);
-        b1 = fast_exp2(b1);
-        acc_a = fadd2(acc_a, pk2(a0, a1));
-        acc_b = fadd2(acc_b, pk2(b0, b1));
-        pr[i] = pf_pack2<BF16>(a0, a1);
-        pr[16 + i] = pf_pack2<BF16>(b0, b1);
-    }
-}
-
 // bounded wait that also ends when another role gave up; false = give up
 __device__ __forceinline__ bool pf_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
     for (uint32_t i = 0; i < (1u << 20); ++i) {
@@ -584,12 +570,8 @@ constexpr int B_KF = 0, B_VF = P2_STAGES, B_KE = 2 * P2_STAGES, B_VE = 3 * P2_ST
               B_X = B_DRAIN + 1,  // per group: both halves of the rows have published their maxima (or sums)
               B_Q = B_X + 2;      // the Q tile has landed
 
-// TMA: K / V tiles arrive through two tensor copies each (boxes of 64 head-dim elements x 128 keys, 128-byte swizzle)
-// that one lane issues, instead of 8192 16-byte cp.async chunks per tile from the whole loader warp.
-template <bool BF16, bool TMA>
-__global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const FaParams p, const __grid_constant__ CUtensorMap tm_k,
-                                                                           const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_q,
-                                                                           const uint32_t tm_order) {
+template <bool BF16>
+__global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const FaParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + P2_SM_BAR);
@@ -598,7 +580,6 @@ __global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const 
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + P2_SM_BAR + 192);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + P2_SM_BAR + 200);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool q_tma = TMA && (tm_order >> 16) != 0;  // the Q tile comes by tensor copies too (bit 16)
 
     const uint32_t hk = blockIdx.y, b = blockIdx.z, G = p.group;
     uint32_t lq = p.lq, lk = p.lk;
@@ -632,8 +613,8 @@ __global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const 
 
     if (tid == 0) {
         for (int i = 0; i < P2_STAGES; ++i) {
-            mbar_init(&bars[B_KF + i], TMA ? 1 : 32);
-            mbar_init(&bars[B_VF + i], TMA ? 1 : 32);
+            mbar_init(&bars[B_KF + i], 32);
+            mbar_init(&bars[B_VF + i], 32);
             mbar_init(&bars[B_KE + i], 1);
             mbar_init(&bars[B_VE + i], 1);
         }
@@ -645,7 +626,7 @@ __global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const 
         mbar_init(&bars[B_X + 1], 256);
         mbar_init(&bars[B_O], 1);
         mbar_init(&bars[B_DRAIN], 1);
-        mbar_init(&bars[B_Q], q_tma ? 1 : P2_THREADS);
+        mbar_init(&bars[B_Q], P2_THREADS);
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -659,7 +640,7 @@ __global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const 
     // Q: 256 rows x 16 chunks (two K-major operands of 128 rows). Nobody waits for it here: every thread leaves an
     // asynchronous arrival on the Q barrier, which the issuing thread waits for before its first product, so the first
     // K / V tiles load at the same time.
-    for (int idx = tid; idx < P2_ROWS * 16 && !q_tma; idx += P2_THREADS) {
+    for (int idx = tid; idx < P2_ROWS * 16; idx += P2_THREADS) {
         const int blk = idx >> 5, l = idx & 31;
         const int grp = blk >> 2, kc = (blk & 3) * 4 + (l >> 3), rr = grp * 8 + (l & 7);
         const uint32_t r = row0 + rr;
@@ -668,53 +649,10 @@ __global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const 
         const uint64_t off = (p.varlen ? (q0 + i) * p.q_ss : b * p.q_sb + i * p.q_ss) + h * p.q_sh;
         pf_cp16(sbase + P2_SM_Q + grp * 2048 + kc * 128 + (rr & 7) * 16, qb + off * 2 + kc * 16, ok);
     }
-    if (!q_tma) asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar0 + 8 * B_Q) : "memory");
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar0 + 8 * B_Q) : "memory");
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == P2_LOADER && TMA) {
-        // ================================================================ loader (tensor copies)
-        // coordinates: the head-dim element, then kv head, key and batch entry in the order of their strides (tm_order: two
-        // bits each for the places of head, key and batch entry; K in bits 0-5, V in bits 8-13); keys past the end of the
-        // tensor read as zeros
-        if (lane == 0) {
-            auto load = [&](const CUtensorMap *map, uint32_t ord, uint32_t dst, int j0, uint32_t bar) {
-                const uint32_t ph = ord & 3u, pk = (ord >> 2) & 3u;
-                const int c1 = ph == 0 ? (int)hk : (pk == 0 ? j0 : (int)b), c2 = ph == 1 ? (int)hk : (pk == 1 ? j0 : (int)b),
-                          c3 = ph == 2 ? (int)hk : (pk == 2 ? j0 : (int)b);
-                tma_load_4d(dst, map, 0, c1, c2, c3, bar);
-                tma_load_4d(dst + P2_KT_BYTES / 2, map, 64, c1, c2, c3, bar);
-            };
-            bool ok = true;
-            int issued_k = 0, issued_v = 0;
-            if (q_tma && ntiles > 0) {
-                // Q: coordinates (element, head in group, kv head, token, batch entry); a box is 64 elements of all heads
-                // of the group for 256 / G tokens = 256 packed rows (row = token * G + head), one box per half of the
-                // head dim: [half][row tile of 128][row][128 bytes, swizzled]
-                mbar_expect_tx(&bars[B_Q], 2 * PF_Q_BYTES);
-                tma_load_5d(sbase + P2_SM_Q, &tm_q, 0, 0, (int)hk, (int)(row0 / G), (int)b, bar0 + 8 * B_Q);
-                tma_load_5d(sbase + P2_SM_Q + PF_Q_BYTES, &tm_q, 64, 0, (int)hk, (int)(row0 / G), (int)b, bar0 + 8 * B_Q);
-            }
-            for (int t = 0; t < ntiles; ++t) {
-                const int st = t % P2_STAGES, j0 = (int)(t_lo + (long long)t * P2_BN);
-                if (t >= P2_STAGES && !(ok = pf_wait(bar0 + 8 * (B_KE + st), ((t / P2_STAGES) - 1) & 1, abort_flag))) break;
-                const uint32_t dk = sbase + P2_SM_K + st * P2_KT_BYTES, dv = sbase + P2_SM_V + st * P2_VT_BYTES;
-                mbar_expect_tx(&bars[B_KF + st], P2_KT_BYTES);
-                load(&tm_k, tm_order & 0x3fu, dk, j0, bar0 + 8 * (B_KF + st));
-                issued_k = t + 1;
-                if (t >= P2_STAGES && !(ok = pf_wait(bar0 + 8 * (B_VE + st), ((t / P2_STAGES) - 1) & 1, abort_flag))) break;
-                mbar_expect_tx(&bars[B_VF + st], P2_VT_BYTES);
-                load(&tm_v, (tm_order >> 8) & 0x3fu, dv, j0, bar0 + 8 * (B_VF + st));
-                issued_v = t + 1;
-            }
-            if (!ok) {
-                // gave up: the copies already issued must land before the block may leave (bounded)
-                *abort_flag = 1;
-                if (q_tma) pf_wait_landed(bar0 + 8 * B_Q, 0);
-                for (int t = max(issued_k - P2_STAGES, 0); t < issued_k; ++t) pf_wait_landed(bar0 + 8 * (B_KF + t % P2_STAGES), (t / P2_STAGES) & 1);
-                for (int t = max(issued_v - P2_STAGES, 0); t < issued_v; ++t) pf_wait_landed(bar0 + 8 * (B_VF + t % P2_STAGES), (t / P2_STAGES) & 1);
-            }
-        }
-    } else if (warp == P2_LOADER) {
+    if (warp == P2_LOADER) {
         // ================================================================ loader (16-byte chunks)
         // Per lane constants: the lane's row and chunk inside a step of 32 chunks (K: 8 rows x 4 chunks of one
         // core-matrix row group; V: 16 keys x 2 chunks), so that a copy costs an add or two besides itself.
@@ -799,18 +737,14 @@ __global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const 
                 const uint32_t ks_ = sbase + P2_SM_K + (t % P2_STAGES) * P2_KT_BYTES, qs_ = sbase + P2_SM_Q + g * PF_Q_BYTES;
 #pragma unroll
                 for (int ks = 0; ks < PF_D / 16; ++ks)
-                    tc_mma_ss(tmem + p2_s_col(g),
-                              q_tma ? tc_desc_sw128(sbase + P2_SM_Q + (ks >> 2) * PF_Q_BYTES + g * (PF_Q_BYTES / 2) + (ks & 3) * 32, 16, 1024)
-                                    : tc_desc(qs_ + ks * 256, 128, 2048),
-                              TMA ? tc_desc_sw128(ks_ + (ks >> 2) * (P2_KT_BYTES / 2) + (ks & 3) * 32, 16, 1024) : tc_desc(ks_ + ks * 256, 128, 2048), IQK,
-                              ks > 0 ? 1u : 0u);
+                    tc_mma_ss(tmem + p2_s_col(g), tc_desc(qs_ + ks * 256, 128, 2048), tc_desc(ks_ + ks * 256, 128, 2048), IQK, ks > 0 ? 1u : 0u);
                 tc_commit(bar0 + 8 * (B_S + g));
             };
             auto issue_pv = [&](int g, int t) {  // O_g += P_g(t) V(t)
                 const uint32_t vs = sbase + P2_SM_V + (t % P2_STAGES) * P2_VT_BYTES;
 #pragma unroll
                 for (int ks = 0; ks < P2_BN / 16; ++ks)
-                    tc_mma_ts(tmem + p2_o_col(g), tmem + p2_s_col(g) + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8), TMA ? tc_desc_sw128(vs + ks * 2048, P2_VT_BYTES / 2, 1024) : tc_desc(vs + ks * 256, 128, 2048), IPV,
+                    tc_mma_ts(tmem + p2_o_col(g), tmem + p2_s_col(g) + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8), tc_desc(vs + ks * 256, 128, 2048), IPV,
                               (t > 0 || ks > 0) ? 1u : 0u);  // P of keys 0-63 / 64-127 sits in the first columns of each half of S
             };
             if (ntiles > 0) {
@@ -1016,19 +950,643 @@ __global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const 
 }
 
 
-bool fa_prefill_sm100_supported(const FaParams &p, bool kv16) {
-    if (!kv16 || p.kv_kind != 0 || p.d != PF_D || p.n_splits != 1) return false;
-    if (p.q_dtype != B200_F16 && p.q_dtype != B200_BF16) return false;
-    if (p.softcap > 0.0f || p.alibi != nullptr) return false;
-    if (!(p.scale * p.kd > 0.0f)) return false;  // the row maximum is taken before the scale is applied
-    if ((uint64_t)p.lq * p.group < 4 * PF_BM) return false;  // short chunks and decode stay on the mma.sync kernel
-    // 16-byte chunks of q rows
-    if ((reinterpret_cast<uintptr_t>(p.q) & 15) || ((p.q_sb | p.q_ss | p.q_sh) & 7)) return false;
-    static const bool off = [] { const char *e = diag_env("B200_FA_NO_TCGEN05"); return e && *e == '1'; }();
-    return !off;
+// ---------------------------------------------------------------------------------------------
+// fa_prefill_tma_kernel: everything by tensor copies, one softmax thread per row, head dims up to 128.
+//   256 packed rows per work item in two groups of 128 (A: warps 0-3, B: warps 4-7, thread = row, the row's 128 scores of
+//   a key tile in registers), warp 8 loads, warps 9 and 10 issue the products of one group each, warp 11 owns the tensor
+//   memory: S_A 128, S_B 128 (P_g over the first 64 columns of S_g), O_A HD, O_B HD columns.
+// What bounds it: the exponentials (16 per cycle and SM) and, at head dim 128, the products take the same 2 048 cycles per
+// tile of 256 x 128 scores; at head dim 64 the exponentials alone do. Hence
+//   * one thread per row: the scores are read from tensor memory once, and no maximum crosses a barrier (two threads per
+//     row read them twice and met at a barrier in every tile);
+//   * the groups' exponentials take turns (head dim 128), so that one group's run under the other's products;
+//   * P is handed over in two parts, so the products of the first 96 keys run under the exponentials of the others;
+//   * one issuing thread per group: the groups' chains (scores, softmax, products) only meet at the shared stages;
+//   * a block goes on to other blocks' items (cluster launch control): the next item's Q and first tiles load and its first
+//     scores are formed while the last one's rows leave, and no SM waits for a heavy item that came last.
+// Measured (us, causal unless said; before: two threads per row, a block per item; head dims other than 128 on mma.sync,
+// sequences of different lengths by 16-byte chunks): B 4, 4096 tokens, 32 / 8 heads of 128: 690 -> 502 (1 094 TFLOP/s); B 1,
+// 16 384 tokens: 2 031 -> 1 785 (1 232); 8 x 1000 tokens, 16 heads of 64, no mask: 416 -> 77; 4 x 4096, 16 heads of 64: 1 410 ->
+// 220; 2 x 2048, 16 / 4 heads of 96: 417 -> 48; 12 sequences of 100-2960: 654 -> 354. At 16 384 tokens a tile of 256 x 128 takes
+// 3 100 cycles (the power limit holds the clock near 1.55 GHz), of which a group spends 1 500 in its exponentials and 1 250
+// waiting for its next scores: eight 128 x 128 x 16 products with both operands in shared memory take 840 cycles, not 512.
+// Taken back: a polynomial for some of the exponentials (on the multiply-add pipe; degree 5, f32 accurate) made every size
+// slower, 531 -> 545 at 2 of 16 pairs, -> 635 at 6.
+// A group skips the key tiles that none of its rows sees.
+// ---------------------------------------------------------------------------------------------
+constexpr int P3_THREADS = 384, P3_ROWS = 256, P3_BN = 128, P3_LOADER = 8, P3_ISSUER = 9, P3_OWNER = 11;
+template <int HD>
+struct P3 {
+    static constexpr int HALVES = HD / 64, STAGES = HD == 128 ? 2 : 4;
+    static constexpr uint32_t Q_HALF = P3_ROWS * 128, Q_BYTES = HALVES * Q_HALF;          // [half][row][128 bytes, swizzled]
+    static constexpr uint32_t T_HALF = P3_BN * 128, T_BYTES = HALVES * T_HALF;             // a K or V tile, likewise
+    static constexpr uint32_t SM_K = Q_BYTES, SM_V = SM_K + STAGES * T_BYTES, SM_OUT = SM_V + STAGES * T_BYTES, SM_BAR = SM_OUT + 8 * 4096, SMEM = SM_BAR + 512;
+    // barriers
+    static constexpr int KF = 0, VF = STAGES, KE = 2 * STAGES, VE = 3 * STAGES, QF = 4 * STAGES, QE = QF + 1, S = QE + 1, P0 = S + 2, P1 = P0 + 2, O = P1 + 2,
+                         DRAIN = O + 2, TK = DRAIN + 2, SR = TK + 8, PV = SR + 2, VT = PV + 2, IF = VT + STAGES, IE = IF + 2, CL = IE + 2, GO = CL + 1, COUNT = GO + 1;
+    // Head dim 64 leaves tensor memory for P beside S: the next scores are formed as soon as the last ones are in registers.
+    // At 128 P lies over the first columns of S, and the next scores follow the products that read it.
+    static constexpr bool EARLY = HD == 64;
+    static constexpr bool TURNS = !EARLY;  // the groups' exponentials take turns (see the softmax warps)
+    __host__ __device__ static constexpr uint32_t p_col(int g) { return EARLY ? 384u + 64u * g : 128u * g; }
+    static_assert(COUNT * 8 <= 464, "barriers");  // then the answer (464), item numbers (480), tensor memory (496), give-up flag (504)
+};
+
+// The grid's work: items = (batch entries x kv heads) x row tiles. The pairs are taken `hpc` at a time (their keys and
+// values stay in L2 together), inside such a chunk the row tiles with the most keys first.
+struct P3Grid {
+    uint32_t tiles, pairs, hpc, items;
+    uint32_t group_log2;  // query heads per kv head (a power of two)
+    uint32_t tm_order;  // places of head, key and batch entry in the maps (two bits each): K in bits 0-5, V in bits 8-13
+};
+
+struct P3Item {
+    uint32_t b, hk, row0, R, gl;
+    uint64_t q0, k0;
+    int lq, lk;
+    int t_lo, t_hi;  // the keys that some row of the item sees
+    int ntiles;
+};
+// the keys [lo, hi) that row r sees
+__device__ __forceinline__ void p3_range(const FaParams &p, const P3Item &it, uint32_t r, int &lo, int &hi) {
+    const int pos = (int)(r >> it.gl) + it.lk - it.lq;
+    lo = p.wl >= 0 && pos > p.wl ? min(pos - p.wl, it.lk) : 0;
+    hi = p.wr >= 0 && pos < it.lk - p.wr - 1 ? pos + p.wr + 1 : it.lk;
+    hi = max(hi, lo);
+}
+// work item n; false when it has no rows
+__device__ __forceinline__ bool p3_item(const FaParams &p, const P3Grid &gr, uint32_t n, P3Item &it) {
+    const uint32_t per = gr.hpc * gr.tiles, chunk = n / per, first = chunk * gr.hpc, width = min(gr.hpc, gr.pairs - first), m = n - chunk * per;
+    const uint32_t rank = m / width, pair = first + (m - rank * width);
+    it.b = pair / p.hkv;
+    it.hk = pair - it.b * p.hkv;
+    it.row0 = (gr.tiles - 1 - rank) * P3_ROWS;
+    it.gl = gr.group_log2;
+    it.lq = (int)p.lq;
+    it.lk = (int)p.lk;
+    it.q0 = (uint64_t)it.b * p.lq;
+    it.k0 = 0;
+    if (p.varlen) {
+        it.q0 = p.cu_q[it.b];
+        it.lq = (int)(p.cu_q[it.b + 1] - p.cu_q[it.b]);
+        it.k0 = p.cu_k[it.b];
+        it.lk = (int)(p.cu_k[it.b + 1] - p.cu_k[it.b]);
+    }
+    it.R = (uint32_t)it.lq << it.gl;
+    if (it.row0 >= it.R) return false;
+    int tmp;
+    p3_range(p, it, it.row0, it.t_lo, tmp);
+    p3_range(p, it, min(it.row0 + P3_ROWS, it.R) - 1, tmp, it.t_hi);
+    it.t_hi = max(it.t_hi, it.t_lo);
+    it.ntiles = (it.t_hi - it.t_lo + P3_BN - 1) / P3_BN;
+    return true;
+}
+// the key tiles [t0, t1) of the item that some row of group g sees (empty: t0 == t1)
+__device__ __forceinline__ void p3_group(const FaParams &p, const P3Item &it, int g, int &t0, int &t1) {
+    t0 = t1 = 0;
+    const uint32_t first = it.row0 + g * PF_BM;
+    if (first >= it.R || it.ntiles == 0) return;
+    int lo, hi, tmp;
+    p3_range(p, it, first, lo, tmp);
+    p3_range(p, it, min(first + PF_BM, it.R) - 1, tmp, hi);
+    if (hi <= lo) return;
+    t0 = (lo - it.t_lo) / P3_BN;
+    t1 = (hi - it.t_lo + P3_BN - 1) / P3_BN;
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+    return e != 0;
+}
+// tcgen05.wait::ld that also carries the loaded registers, so that nothing that uses them moves in front of it
+__device__ __forceinline__ void tc_wait_ld_for(uint32_t (&r)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
+                   "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]),
+                   "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]),
+                   "+r"(r[31])
+                 :
+                 : "memory");
+}
+// a whole warp waits, and goes on or gives up together
+__device__ __forceinline__ bool p3_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, pf_wait(bar, parity, abort_flag));
+}
+// Asks for a block of the grid that has not started yet (cluster launch control): the answer, 16 bytes, lands in shared memory
+// and is counted on `bar`.
+__device__ __forceinline__ void clc_try_cancel(uint32_t answer, uint32_t bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar) : "memory");
+}
+// the x index of the block that was given to this one, or -1 when none was left
+__device__ __forceinline__ int clc_answer(uint32_t answer) {
+    uint32_t given, x = 0;
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b128 a;\n ld.shared.b128 a, [%2];\n clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n"
+        " selp.u32 %1, 1, 0, p;\n @p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, a;\n}"
+        : "+r"(x), "=r"(given)
+        : "r"(answer)
+        : "memory");
+    return given ? (int)x : -1;
 }
 
-// ---- tensor maps of K / V for the tensor-copy loader -------------------------------------------------------------------
+template <int HD, bool BF16>
+__global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaParams p, const __grid_constant__ CUtensorMap tm_k,
+                                                                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_q,
+                                                                       const P3Grid gr) {
+    using C = P3<HD>;
+    constexpr int NS = C::STAGES;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const uint32_t sbase = smem_u32(smem), bar0 = sbase + C::SM_BAR;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + C::SM_BAR);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + C::SM_BAR + 496);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + C::SM_BAR + 504);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (*reinterpret_cast<volatile int *>(&g_wait_failed)) return;
+    if (tid == 0) {
+        for (int i = 0; i < NS; ++i) {
+            mbar_init(&bars[C::KF + i], 1);
+            mbar_init(&bars[C::VF + i], 1);
+            mbar_init(&bars[C::KE + i], 2);
+            mbar_init(&bars[C::VE + i], 2);
+            mbar_init(&bars[C::VT + i], 1);
+        }
+        mbar_init(&bars[C::QF], 1);
+        mbar_init(&bars[C::QE], 2);
+        for (int g = 0; g < 2; ++g) {
+            mbar_init(&bars[C::S + g], 1);
+            mbar_init(&bars[C::P0 + g], 4);
+            mbar_init(&bars[C::P1 + g], 4);
+            mbar_init(&bars[C::O + g], 1);
+            mbar_init(&bars[C::DRAIN + g], 1);
+            mbar_init(&bars[C::SR + g], 4);
+            mbar_init(&bars[C::PV + g], 1);
+        }
+        for (int i = 0; i < 8; ++i) mbar_init(&bars[C::TK + i], 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars[C::IF + i], 1);
+            mbar_init(&bars[C::IE + i], 11);  // loader, two issuers, eight softmax warps
+        }
+        mbar_init(&bars[C::CL], 1);
+        mbar_init(&bars[C::GO], 1);
+        *abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == P3_OWNER) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    bool ok = true;
+    volatile int *items = reinterpret_cast<volatile int *>(smem + C::SM_BAR + 480);
+    // the block's k-th work item, as the owner warp announces it; false: there is none (or a wait has run out)
+    auto next_item = [&](int k, int &n) {
+        if (!ok || !(ok = p3_wait(bar0 + 8 * (C::IF + (k & 1)), (k >> 1) & 1, abort_flag))) return false;
+        n = items[k & 1];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[C::IE + (k & 1)]);
+        return n >= 0;
+    };
+
+    if (warp >= 8) {
+        // 128 threads x 56 + 256 x 224 = the launch's 384 x 168 registers
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == P3_LOADER) {
+            // ============================================================ loader
+            uint32_t kv = 0, nq = 0;  // key tiles and Q tiles so far
+            const uint64_t k_total = p.varlen ? p.cu_k[p.b] : 0;
+            const char *kbase = reinterpret_cast<const char *>(p.k), *vbase = reinterpret_cast<const char *>(p.v);
+            for (int k = 0, n; next_item(k, n); ++k) {
+                P3Item it;
+                p3_item(p, gr, n, it);
+                if (it.ntiles == 0) {
+                    if (lane == 0) mbar_arrive(&bars[C::GO]);
+                    continue;
+                }
+                auto load = [&](const CUtensorMap *map, uint32_t ord, uint32_t dst, int j, uint32_t bar) {
+                    const uint32_t ph = ord & 3u, pk = (ord >> 2) & 3u;
+                    const int bb = p.varlen ? 0 : (int)it.b;
+                    const int c1 = ph == 0 ? (int)it.hk : (pk == 0 ? j : bb), c2 = ph == 1 ? (int)it.hk : (pk == 1 ? j : bb),
+                              c3 = ph == 2 ? (int)it.hk : (pk == 2 ? j : bb);
+                    for (int hf = 0; hf < C::HALVES; ++hf) tma_load_4d(dst + hf * C::T_HALF, map, 64 * hf, c1, c2, c3, bar);
+                };
+                if (nq > 0 && !(ok = p3_wait(bar0 + 8 * C::QE, (nq - 1) & 1, abort_flag))) break;
+                if (lane == 0) {
+                    // Q: coordinates (element, head in group, kv head, token, batch entry); a box is 64 elements of all heads of
+                    // the group for 256 / G tokens = 256 packed rows (row = token * G + head)
+                    mbar_expect_tx(&bars[C::QF], C::Q_BYTES);
+                    const int tok = (int)((p.varlen ? it.q0 : 0) + (it.row0 >> it.gl));
+                    for (int hf = 0; hf < C::HALVES; ++hf)
+                        tma_load_5d(sbase + hf * C::Q_HALF, &tm_q, 64 * hf, 0, (int)it.hk, tok, p.varlen ? 0 : (int)it.b, bar0 + 8 * C::QF);
+                }
+                __syncwarp();
+                ++nq;
+                for (int t = 0; t < it.ntiles; ++t, ++kv) {
+                    const int st = kv % NS, j0 = it.t_lo + t * P3_BN;
+                    const uint32_t ph = ((kv / NS) - 1) & 1, dk = sbase + C::SM_K + st * C::T_BYTES, dv = sbase + C::SM_V + st * C::T_BYTES;
+                    if (p.varlen && it.k0 + j0 + P3_BN > k_total) {
+                        // the end of the last sequence: its rows alone, by 16-byte chunks in the layout of the tensor copies
+                        if (kv >= NS && !(ok = p3_wait(bar0 + 8 * (C::KE + st), ph, abort_flag) && p3_wait(bar0 + 8 * (C::VE + st), ph, abort_flag))) break;
+                        const char *kr = kbase + ((it.k0 + j0) * p.k_ss + it.hk * p.k_sh) * 2, *vr = vbase + ((it.k0 + j0) * p.v_ss + it.hk * p.v_sh) * 2;
+                        const int rows = it.t_hi - j0;
+                        for (int idx = lane; idx < P3_BN * HD / 8; idx += 32) {
+                            const int row = idx / (HD / 8), ch = idx % (HD / 8);
+                            const bool in = row < rows && (uint32_t)ch * 8 < p.d;
+                            const uint32_t at = (ch >> 3) * C::T_HALF + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
+                            pf_cp16(dk + at, in ? kr + (uint64_t)row * p.k_ss * 2 + ch * 16 : kr, in);
+                            pf_cp16(dv + at, in ? vr + (uint64_t)row * p.v_ss * 2 + ch * 16 : vr, in);
+                        }
+                        asm volatile("cp.async.commit_group;" ::: "memory");
+                        asm volatile("cp.async.wait_group 0;" ::: "memory");
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) {
+                            mbar_arrive(&bars[C::KF + st]);
+                            mbar_arrive(&bars[C::VF + st]);
+                        }
+                        continue;
+                    }
+                    if (kv >= NS && !(ok = p3_wait(bar0 + 8 * (C::KE + st), ph, abort_flag))) break;
+                    if (lane == 0) {
+                        mbar_expect_tx(&bars[C::KF + st], C::T_BYTES);
+                        load(&tm_k, gr.tm_order & 0x3fu, dk, (int)it.k0 + j0, bar0 + 8 * (C::KF + st));
+                    }
+                    __syncwarp();
+                    if (kv >= NS && !(ok = p3_wait(bar0 + 8 * (C::VE + st), ph, abort_flag))) {
+                        if (lane == 0) pf_wait_landed(bar0 + 8 * (C::KF + st), (kv / NS) & 1);
+                        break;
+                    }
+                    if (lane == 0) {
+                        // past the end of the item's keys lie other sequences' rows: the owner warp clears them first
+                        const int full = p.varlen && j0 + P3_BN > it.t_hi ? C::VT + st : C::VF + st;
+                        mbar_expect_tx(&bars[full], C::T_BYTES);
+                        load(&tm_v, (gr.tm_order >> 8) & 0x3fu, dv, (int)it.k0 + j0, bar0 + 8 * full);
+                    }
+                    __syncwarp();
+                }
+                if (lane == 0) mbar_arrive(&bars[C::GO]);
+            }
+            if (!ok) {
+                // gave up: the copies already issued must land before the block may leave (bounded)
+                *abort_flag = 1;
+                if (lane == 0) {
+                    if (nq > 0) pf_wait_landed(bar0 + 8 * C::QF, (nq - 1) & 1);
+                    for (uint32_t t = kv > NS ? kv - NS : 0; t < kv; ++t) {
+                        pf_wait_landed(bar0 + 8 * (C::KF + t % NS), (t / NS) & 1);
+                        if (!p.varlen) pf_wait_landed(bar0 + 8 * (C::VF + t % NS), (t / NS) & 1);
+                    }
+                    if (p.varlen)  // a V tile may land on the tail's barrier: a pause that outlasts any copy
+                        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+                }
+            }
+        } else if (warp == P3_OWNER) {
+            // ============================================================ work items; rows behind the keys of an item (varlen)
+            // The grid has a block per item. A block starts with its own and then takes over blocks that have not started
+            // (heaviest first), so that late items go where there is time; items without rows end here. It asks when the last
+            // tile of an item has been requested: the answer comes while the tiles in flight are worked on (asked for at an item's
+            // start, the early blocks claim too much: 181 against 142 us for 512 items of 1 to 32 tiles).
+            const uint64_t k_total = p.varlen ? p.cu_k[p.b] : 0;
+            uint32_t kv = 0, asked = 0, parity = 0;  // parity: of each stage's tail barrier, a bit each
+            P3Item it, ahead;
+            int n = (int)blockIdx.x;
+            auto take = [&](P3Item &x) {  // the next block's item, if there is one with rows
+                for (;;) {
+                    if (lane == 0) {
+                        mbar_expect_tx(&bars[C::CL], 16);
+                        clc_try_cancel(sbase + C::SM_BAR + 464, bar0 + 8 * C::CL);
+                    }
+                    __syncwarp();
+                    if (!(ok = p3_wait(bar0 + 8 * C::CL, asked++ & 1, abort_flag))) {
+                        if (lane == 0) pf_wait_landed(bar0 + 8 * C::CL, (asked - 1) & 1);
+                        n = -1;
+                        return;
+                    }
+                    n = clc_answer(sbase + C::SM_BAR + 464);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read before the next answer is written
+                    __syncwarp();
+                    if (n < 0 || p3_item(p, gr, (uint32_t)n, x)) return;
+                }
+            };
+            auto announce = [&](int k) {
+                if (k >= 2 && !(ok = ok && p3_wait(bar0 + 8 * (C::IE + (k & 1)), ((k >> 1) - 1) & 1, abort_flag))) return;
+                if (lane == 0) {
+                    items[k & 1] = n;
+                    mbar_arrive(&bars[C::IF + (k & 1)]);
+                }
+                __syncwarp();
+            };
+            if (!p3_item(p, gr, (uint32_t)n, it)) take(it);
+            announce(0);
+            for (int k = 1; ok && n >= 0; ++k, it = ahead) {
+                if (!(ok = p3_wait(bar0 + 8 * C::GO, (k - 1) & 1, abort_flag))) break;
+                take(ahead);
+                announce(k);
+                if (!ok || !p.varlen || it.ntiles == 0) continue;
+                kv += it.ntiles;
+                const int st = (kv - 1) % NS, j0 = it.t_lo + (it.ntiles - 1) * P3_BN;
+                if (j0 + P3_BN <= it.t_hi || it.k0 + j0 + P3_BN > k_total) continue;
+                // The tile reaches into the next sequence (or into keys that no row of the item sees). Their weights are zero,
+                // but zero times an infinity is not: the rows are cleared before V is announced.
+                if (!(ok = p3_wait(bar0 + 8 * (C::VT + st), (parity >> st) & 1, abort_flag))) break;
+                parity ^= 1u << st;
+                for (int idx = (it.t_hi - j0) * 8 + lane; idx < P3_BN * 8; idx += 32)
+#pragma unroll
+                    for (int hf = 0; hf < C::HALVES; ++hf)
+                        *reinterpret_cast<uint4 *>(smem + C::SM_V + st * C::T_BYTES + hf * C::T_HALF + idx * 16) = make_uint4(0, 0, 0, 0);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars[C::VF + st]);
+            }
+            if (!ok) *abort_flag = 1;
+        } else {
+            // ============================================================ matrix products of group g
+            const int g = warp - P3_ISSUER;
+            constexpr uint32_t IQK = tc_idesc(BF16, false, PF_BM, P3_BN), IPV = tc_idesc(BF16, true, PF_BM, HD);
+            const uint32_t s_t = tmem + 128u * g, p_t = tmem + C::p_col(g), o_t = tmem + 256u + (uint32_t)HD * g;
+            const int nks = (int)(p.d + 15) / 16;  // steps of 16 along the head dim that hold anything
+            const uint64_t q_desc = tc_desc_sw128(sbase + g * (C::Q_HALF / 2), 16, 1024);
+            uint32_t kv = 0, nq = 0, sc = 0;
+            // S_g = Q_g K^T of the tile in stage st
+            auto scores = [&](int st, bool last) {
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t k_desc = tc_desc_sw128(sbase + C::SM_K + st * C::T_BYTES, 16, 1024);
+#pragma unroll
+                    for (int ks = 0; ks < HD / 16; ++ks)
+                        if (ks < nks)
+                            tc_mma_ss(s_t, q_desc + (uint64_t)(((ks >> 2) * C::Q_HALF + (ks & 3) * 32) >> 4),
+                                      k_desc + (uint64_t)(((ks >> 2) * C::T_HALF + (ks & 3) * 32) >> 4), IQK, ks > 0 ? 1u : 0u);
+                    tc_commit(bar0 + 8 * (C::S + g));
+                    tc_commit(bar0 + 8 * (C::KE + st));
+                    if (last) tc_commit(bar0 + 8 * C::QE);
+                }
+                __syncwarp();
+            };
+            for (int k = 0, n; next_item(k, n); ++k) {
+                P3Item it;
+                p3_item(p, gr, n, it);
+                if (it.ntiles == 0) continue;
+                int t0, t1;
+                p3_group(p, it, g, t0, t1);
+                if (!(ok = p3_wait(bar0 + 8 * C::QF, nq & 1, abort_flag))) break;
+                ++nq;
+                if (t0 == t1 && elect_one()) mbar_arrive(&bars[C::QE]);
+                __syncwarp();
+                for (int t = 0; t < it.ntiles; ++t, ++kv) {
+                    const int st = kv % NS;
+                    const uint32_t ph = (kv / NS) & 1;
+                    if (t < t0 || t >= t1) {  // a tile that only the other group needs
+                        if (!(ok = p3_wait(bar0 + 8 * (C::KF + st), ph, abort_flag))) break;
+                        if (elect_one()) mbar_arrive(&bars[C::KE + st]);
+                        __syncwarp();
+                        if (!(ok = p3_wait(bar0 + 8 * (C::VF + st), ph, abort_flag))) break;
+                        if (elect_one()) mbar_arrive(&bars[C::VE + st]);
+                        __syncwarp();
+                        continue;
+                    }
+                    // S_g(t): behind O_g += P_g V(t - 1), which reads P out of S_g's columns, or (EARLY) one tile ahead
+                    if (!C::EARLY || t == t0) {
+                        if (!(ok = p3_wait(bar0 + 8 * (C::KF + st), ph, abort_flag))) break;
+                        scores(st, t == t1 - 1);
+                    }
+                    if (C::EARLY && t + 1 < t1) {
+                        const int sn = (kv + 1) % NS;
+                        ok = p3_wait(bar0 + 8 * (C::SR + g), sc & 1, abort_flag) && p3_wait(bar0 + 8 * (C::KF + sn), ((kv + 1) / NS) & 1, abort_flag);
+                        if (!ok) break;
+                        scores(sn, t + 1 == t1 - 1);
+                    }
+                    ok = p3_wait(bar0 + 8 * (C::VF + st), ph, abort_flag) && p3_wait(bar0 + 8 * (C::P0 + g), sc & 1, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t v_desc = tc_desc_sw128(sbase + C::SM_V + st * C::T_BYTES, C::T_HALF, 1024);
+                    if (elect_one()) {  // O_g += P_g(t) V(t): the first 96 keys while the others' exponentials run
+#pragma unroll
+                        for (int ks = 0; ks < 6; ++ks) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, (t > t0 || ks > 0) ? 1u : 0u);
+                    }
+                    __syncwarp();
+                    if (!(ok = p3_wait(bar0 + 8 * (C::P1 + g), sc & 1, abort_flag))) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+#pragma unroll
+                        for (int ks = 6; ks < 8; ++ks) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, 1u);
+                        tc_commit(bar0 + 8 * (C::VE + st));
+                        if (C::EARLY) tc_commit(bar0 + 8 * (C::PV + g));
+                        if (t == t1 - 1) tc_commit(bar0 + 8 * (C::O + g));
+                    }
+                    __syncwarp();
+                    ++sc;
+                }
+            }
+            if (!ok) {
+                *abort_flag = 1;
+                // let the products already issued finish before the tensor memory goes
+                if (elect_one()) {
+                    tc_commit(bar0 + 8 * (C::DRAIN + g));
+                    pf_wait_landed(bar0 + 8 * (C::DRAIN + g), 0);
+                }
+                __syncwarp();
+            }
+        }
+    } else {
+        // ================================================================ softmax, thread = row
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        const int g = warp >> 2, w4 = warp & 3;
+        const uint32_t lane_base = tmem + ((uint32_t)(w4 * 32) << 16), s_col = lane_base + 128u * g, p_col = lane_base + C::p_col(g), o_col = lane_base + 256u + (uint32_t)HD * g;
+        const float sl2 = p.scale * p.kd * PF_LOG2E;
+        uint32_t sc = 0, oc = 0, tk = 0;
+        P3Item it;
+        int n, t0, t1, r_lo, r_hi, lomax, himin;
+        // work item k: the group's key tiles, the row's keys and the tightest bounds over the group's rows, from the item's
+        // first key on
+        auto begin = [&](int k) {
+            if (!next_item(k, n)) return false;
+            p3_item(p, gr, (uint32_t)n, it);
+            p3_group(p, it, g, t0, t1);
+            const uint32_t g_row0 = it.row0 + g * PF_BM, r = g_row0 + w4 * 32 + lane;
+            r_lo = r_hi = lomax = 0, himin = -1;
+            if (t1 > t0) {
+                int lo, hi, tmp;
+                if (r < it.R) {
+                    p3_range(p, it, r, lo, hi);
+                    r_lo = lo - it.t_lo;
+                    r_hi = hi - it.t_lo;
+                }
+                p3_range(p, it, min(g_row0 + PF_BM, it.R) - 1, lo, tmp);
+                p3_range(p, it, g_row0, tmp, hi);
+                lomax = lo - it.t_lo;
+                himin = g_row0 + PF_BM > it.R ? -1 : hi - it.t_lo;
+            }
+            return true;
+        };
+        bool more = begin(0);
+        for (int k = 1; more && ok; ++k) {
+            float mref = -INFINITY, l = 0.0f;
+            for (int t = 0; t < it.ntiles; ++t) {
+                const bool mine = t >= t0 && t < t1;
+                // The groups' exponentials take turns, A(0) B(0) A(1) B(1) ... (warp w4 of A and warp w4 of B share an SM
+                // quadrant): left alone, both groups end up computing exponentials at the same time, at half the rate each, and
+                // waiting for their products at the same time. Not where the scores come early: there nobody waits.
+                auto my_turn = [&]() { return g == 0 ? (tk == 0 || p3_wait(bar0 + 8 * (C::TK + w4), (tk - 1) & 1, abort_flag)) : p3_wait(bar0 + 8 * (C::TK + 4 + w4), tk & 1, abort_flag); };
+                auto pass_turn = [&]() { if (lane == 0) mbar_arrive(&bars[C::TK + (g ^ 1) * 4 + w4]); };
+                if (!mine) {
+                    if (C::TURNS) {
+                        if (!(ok = my_turn())) break;
+                        pass_turn();
+                        ++tk;
+                    }
+                    continue;
+                }
+                if (!(ok = p3_wait(bar0 + 8 * (C::S + g), sc & 1, abort_flag))) break;
+                tc_fence_after();
+                uint32_t s0[32], s1[32], s2[32], s3[32];
+                tc_ld32(s_col, s0);
+                tc_ld32(s_col + 32, s1);
+                tc_wait_ld_for(s0);
+                tc_wait_ld_for(s1);
+                tc_ld32(s_col + 64, s2);
+                tc_ld32(s_col + 96, s3);
+                const int j0 = t * P3_BN;  // from the item's first key
+                const bool full = j0 >= lomax && j0 + P3_BN <= himin;
+                const int lo_rel = r_lo - j0, hi_rel = r_hi - j0;
+                if (!full) {
+                    pf_mask32(s0, 0, lo_rel, hi_rel);
+                    pf_mask32(s1, 32, lo_rel, hi_rel);
+                }
+                const float mx01 = pf_max64(s0, s1);
+                tc_wait_ld_for(s2);
+                tc_wait_ld_for(s3);
+                if (C::EARLY) {  // the scores are in registers: the next ones may come
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars[C::SR + g]);
+                }
+                if (!full) {
+                    pf_mask32(s2, 64, lo_rel, hi_rel);
+                    pf_mask32(s3, 96, lo_rel, hi_rel);
+                }
+                const float mx = fmaxf(mx01, pf_max64(s2, s3)) * sl2;  // sl2 > 0: the maximum commutes with the scale
+                bool need = false;
+                if (t == t0) mref = mx;
+                else need = mx > mref + PF_SLACK;
+                // O_g += P_g V(t - 1) has read P and written O (where the scores do not come early, their barrier says that)
+                auto products_done = [&]() {
+                    if (!C::EARLY || t == t0) return true;
+                    const bool done = p3_wait(bar0 + 8 * (C::PV + g), (sc - 1) & 1, abort_flag);
+                    tc_fence_after();
+                    return done;
+                };
+                if (__any_sync(0xffffffffu, need)) {
+                    // rows whose maximum moved: O goes to the new reference
+                    const float f = need ? fast_exp2(mref - mx) : 1.0f;
+                    if (need) mref = mx;
+                    l *= f;
+                    ok = products_done();
+                    if (!ok) break;
+#pragma unroll 1
+                    for (int ch = 0; ch < HD / 32; ++ch) {
+                        uint32_t o[32];
+                        tc_ld32(o_col + 32 * ch, o);
+                        tc_wait_ld_for(o);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = f2u(u2f(o[i]) * f);
+                        tc_st32(o_col + 32 * ch, o);
+                    }
+                }
+                const float ms = mref == -INFINITY ? 0.0f : mref;
+                const uint64_t sc2 = pk2(sl2, sl2), nm2 = pk2(-ms, -ms);
+                uint64_t acc_a = pk2(0.0f, 0.0f), acc_b = acc_a;
+                uint32_t pr[16];
+                if (C::TURNS) ok = my_turn();
+                if (!ok) break;
+                pf_exp32<BF16>(s0, sc2, nm2, acc_a, pr);
+                ok = products_done();
+                if (!ok) break;
+                tc_st16(p_col, pr);
+                pf_exp32<BF16>(s1, sc2, nm2, acc_b, pr);
+                tc_st16(p_col + 16, pr);
+                pf_exp32<BF16>(s2, sc2, nm2, acc_a, pr);
+                tc_st16(p_col + 32, pr);
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars[C::P0 + g]);
+                pf_exp32<BF16>(s3, sc2, nm2, acc_b, pr);
+                tc_st16(p_col + 48, pr);
+                if (C::TURNS) pass_turn();
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars[C::P1 + g]);
+                ++sc;
+                ++tk;
+                float a0, a1, b0, b1;
+                upk2(acc_a, a0, a1);
+                upk2(acc_b, b0, b1);
+                l += (a0 + a1) + (b0 + b1);
+            }
+            if (!ok) break;
+            // the next item's figures while the last products run
+            const P3Item cur = it;
+            const bool any = t1 > t0;
+            more = begin(k);
+            if (!ok) break;
+            if (any) {
+                if (!(ok = p3_wait(bar0 + 8 * (C::O + g), oc & 1, abort_flag))) break;
+                ++oc;
+                tc_fence_after();
+            }
+            // ---- the row of the output: O / l, or zeros
+            const float inv = l > 0.0f ? p.vd / l : 0.0f;
+            // 64 elements of the warp's 32 rows at a time through shared memory, so that eight lanes write 128 bytes of a row
+            // (a lane that writes its own row leaves every store in 32 lines)
+            uint8_t *const stage = smem + C::SM_OUT + warp * 4096;
+#pragma unroll 1
+            for (int hf = 0; hf < C::HALVES; ++hf) {
+#pragma unroll
+                for (int ch = 0; ch < 2; ++ch) {
+                    uint32_t o[32];
+                    if (any) {
+                        tc_ld32(o_col + 64 * hf + 32 * ch, o);
+                        tc_wait_ld_for(o);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = 0u;
+                    }
+#pragma unroll
+                    for (int v4 = 0; v4 < 4; ++v4) {
+                        uint4 w;
+                        w.x = pf_pack2<BF16>(u2f(o[8 * v4]) * inv, u2f(o[8 * v4 + 1]) * inv);
+                        w.y = pf_pack2<BF16>(u2f(o[8 * v4 + 2]) * inv, u2f(o[8 * v4 + 3]) * inv);
+                        w.z = pf_pack2<BF16>(u2f(o[8 * v4 + 4]) * inv, u2f(o[8 * v4 + 5]) * inv);
+                        w.w = pf_pack2<BF16>(u2f(o[8 * v4 + 6]) * inv, u2f(o[8 * v4 + 7]) * inv);
+                        *reinterpret_cast<uint4 *>(stage + lane * 128 + (((ch * 4 + v4) ^ (lane & 7)) << 4)) = w;
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t row = i * 4 + (lane >> 3), c8 = lane & 7, rr = cur.row0 + g * PF_BM + w4 * 32 + row;
+                    const uint4 w = *reinterpret_cast<const uint4 *>(stage + row * 128 + ((c8 ^ (row & 7)) << 4));
+                    const uint64_t orow = (cur.q0 + (rr >> cur.gl)) * p.hq + (cur.hk << cur.gl) + (rr & ((1u << cur.gl) - 1));
+                    if (rr < cur.R && 64 * hf + 8 * c8 < p.d)
+                        *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p.o) + orow * p.d + 64 * hf + 8 * c8) = w;
+                }
+                __syncwarp();
+            }
+            tc_fence_before();  // O has been read before the next item's first P is announced
+        }
+        if (!ok) *abort_flag = 1;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == P3_OWNER) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    if (tid == 0 && *abort_flag) atomicExch(&g_wait_failed, 1);
+}
+
+// ---- tensor maps -------------------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                   const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static EncodeTiledFn encode_tiled_fn() {
@@ -1040,14 +1598,15 @@ static EncodeTiledFn encode_tiled_fn() {
     }();
     return fn;
 }
-// A (batch, kv head, key, 128) tensor of 16-bit elements with element strides s_b, s_h, s_s and contiguous head dim as
-// a rank-4 map: head dim first, the other three in ascending order of stride (entries of extent 1 last). Boxes of
-// 64 x 128 keys, 128-byte swizzle. `order` gets the places of head, key and batch (two bits each). False when the tensor
-// cannot be described (alignment, strides) or the driver refuses.
-static bool make_kv_map(CUtensorMap *m, uint32_t *order, const void *base, bool bf16, uint64_t nb, uint64_t hkv, uint64_t lk, uint64_t s_b, uint64_t s_h,
-                        uint64_t s_s) {
-    const EncodeTiledFn enc = encode_tiled_fn();
-    if (!enc || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
+// What a map says of K or V: a (batch, kv head, key, d) tensor of 16-bit elements with element strides s_b, s_h, s_s and
+// contiguous head dim, rank 4: head dim first, the other three in ascending order of stride (entries of extent 1 last).
+// `order` gets the places of head, key and batch (two bits each). False when no map can describe the tensor.
+struct KvDims {
+    uint64_t size[3], stride[3];
+    uint32_t order;
+};
+static bool kv_dims(KvDims *m, const void *base, uint64_t nb, uint64_t hkv, uint64_t lk, uint64_t d_, uint64_t s_b, uint64_t s_h, uint64_t s_s) {
+    if (reinterpret_cast<uintptr_t>(base) & 15) return false;
     struct Dim {
         uint64_t size, stride;
         int role;
@@ -1056,86 +1615,152 @@ static bool make_kv_map(CUtensorMap *m, uint32_t *order, const void *base, bool 
         if ((a.size == 1) != (c.size == 1)) return c.size == 1;  // entries of extent 1 go last
         return a.size > 1 && a.stride < c.stride;
     });
-    uint64_t prev = PF_D * 2;
+    uint64_t prev = d_ * 2;
+    m->order = 0;
     for (int i = 0; i < 3; ++i) {
-        if (d[i].size == 1) d[i].stride = prev;  // any legal value: the coordinate is always 0
-        if ((d[i].stride & 15) || d[i].stride < prev || d[i].stride >= (1ull << 40) || d[i].size > (1ull << 31)) return false;
-        prev = d[i].stride * d[i].size;
+        if (d[i].size == 0) return false;
+        if (d[i].size == 1) {
+            d[i].stride = (d_ * 2 + 15) / 16 * 16;  // any legal value: the coordinate is always 0
+        } else {
+            if ((d[i].stride & 15) || d[i].stride < prev || d[i].stride >= (1ull << 40) || d[i].size > (1ull << 31)) return false;
+            prev += d[i].stride * (d[i].size - 1);
+        }
+        m->size[i] = d[i].size;
+        m->stride[i] = d[i].stride;
+        m->order |= (uint32_t)i << (2 * d[i].role);
     }
-    uint32_t ord = 0;
-    for (int i = 0; i < 3; ++i) ord |= (uint32_t)i << (2 * d[i].role);
-    const cuuint64_t dims[4] = {(cuuint64_t)PF_D, d[0].size, d[1].size, d[2].size};
-    const cuuint64_t strides[3] = {d[0].stride, d[1].stride, d[2].stride};
+    return true;
+}
+// boxes of 64 elements x 128 keys, 128-byte swizzle; elements past the head dim and keys past the end read as zeros
+static bool make_kv_map(CUtensorMap *m, const KvDims &k, const void *base, bool bf16, uint64_t d) {
+    const cuuint64_t dims[4] = {(cuuint64_t)d, k.size[0], k.size[1], k.size[2]};
+    const cuuint64_t strides[3] = {k.stride[0], k.stride[1], k.stride[2]};
     cuuint32_t box[4] = {64, 1, 1, 1};
-    box[1 + ((ord >> 2) & 3u)] = P2_BN;
+    box[1 + ((k.order >> 2) & 3u)] = P3_BN;
     const cuuint32_t estr[4] = {1, 1, 1, 1};
-    const CUresult r = enc(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    *order = ord;
-    return r == CUDA_SUCCESS;
+    const EncodeTiledFn enc = encode_tiled_fn();
+    return enc && enc(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The (batch, token, head, 128) query tensor as a rank-5 map (element, head in group, kv head, token, batch entry) whose
-// box of 64 x G x 1 x 256 / G lands as 256 packed rows (row = token * G + head in group).
-static bool make_q_map(CUtensorMap *m, const FaParams &p, bool bf16) {
-    const EncodeTiledFn enc = encode_tiled_fn();
-    const uint64_t G = p.group;
-    if (!enc || G == 0 || G > 256 || (G & (G - 1)) || (reinterpret_cast<uintptr_t>(p.q) & 15)) return false;
-    const cuuint64_t dims[5] = {(cuuint64_t)PF_D, G, p.hkv, p.lq, p.b};
-    cuuint64_t strides[4] = {p.q_sh * 2, G * p.q_sh * 2, p.q_ss * 2, p.q_sb * 2};
-    if (G == 1) strides[0] = PF_D * 2;
+// The (batch, token, head, d) query tensor as a rank-5 map (element, head in group, kv head, token, batch entry) whose box of
+// 64 x G x 1 x 256 / G lands as 256 packed rows (row = token * G + head in group). Sequences of different lengths: one
+// batch entry of all tokens.
+static bool q_strides(const FaParams &p, cuuint64_t (&strides)[4]) {
+    const uint64_t G = p.group, row = (uint64_t)p.d * 2;
+    if (G == 0 || G > 256 || (G & (G - 1)) || (reinterpret_cast<uintptr_t>(p.q) & 15)) return false;
+    strides[0] = p.q_sh * 2;
+    strides[1] = G * p.q_sh * 2;
+    strides[2] = p.q_ss * 2;
+    strides[3] = p.q_sb * 2;
+    if (G == 1) strides[0] = (row + 15) / 16 * 16;
     if (p.hkv == 1) strides[1] = strides[0] * G;
-    if (p.b == 1) strides[3] = strides[2] * p.lq;
+    if (p.varlen || p.b == 1) strides[3] = strides[2];
+    if (!p.varlen && p.lq == 1) strides[2] = strides[1];
     for (int i = 0; i < 4; ++i)
-        if ((strides[i] & 15) || strides[i] < PF_D * 2 || strides[i] >= (1ull << 40)) return false;
-    const cuuint32_t box[5] = {64, (cuuint32_t)G, 1, (cuuint32_t)(P2_ROWS / G), 1};
+        if ((strides[i] & 15) || strides[i] < row || strides[i] >= (1ull << 40)) return false;
+    return true;
+}
+static bool make_q_map(CUtensorMap *m, const FaParams &p, bool bf16) {
+    cuuint64_t strides[4];
+    if (!q_strides(p, strides)) return false;
+    const uint64_t G = p.group;
+    const cuuint64_t dims[5] = {(cuuint64_t)p.d, G, p.hkv, p.varlen ? p.rows_total / p.hq : p.lq, p.varlen ? 1u : p.b};
+    const cuuint32_t box[5] = {64, (cuuint32_t)G, 1, (cuuint32_t)(P3_ROWS / G), 1};
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    return enc(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void *>(p.q), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const EncodeTiledFn enc = encode_tiled_fn();
+    return enc && enc(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void *>(p.q), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// K and V of a call as maps see them. Sequences of different lengths are one batch entry of keys without an end: the kernel
+// copies by tensor map only tiles that lie inside a sequence.
+static bool kv_dims_of(const FaParams &p, KvDims *k, KvDims *v) {
+    const uint64_t nb = p.varlen ? 1 : p.b, n = p.varlen ? (1ull << 31) : p.lk;
+    return kv_dims(k, p.k, nb, p.hkv, n, p.d, p.k_sb, p.k_sh, p.k_ss) && kv_dims(v, p.v, nb, p.hkv, n, p.d, p.v_sb, p.v_sh, p.v_ss);
+}
+
+enum { PF_NONE = 0, PF_ROWS128, PF_ROWS256, PF_TMA };
+constexpr uint64_t P3_MIN_ROWS = 512;  // two items' worth of rows per kv head; below, 64-row tiles spread over more SMs
+static int fa_prefill_route(const FaParams &p, bool kv16) {
+    if (!kv16 || p.kv_kind != 0 || p.n_splits != 1) return PF_NONE;
+    if (p.q_dtype != B200_F16 && p.q_dtype != B200_BF16) return PF_NONE;
+    if (p.softcap > 0.0f || p.alibi != nullptr) return PF_NONE;
+    if (!(p.scale * p.kd > 0.0f)) return PF_NONE;  // the row maximum is taken before the scale is applied
+    static const bool off = [] { const char *e = diag_env("B200_FA_NO_TCGEN05"); return e && *e == '1'; }();
+    if (off) return PF_NONE;
+    const uint64_t rows = (uint64_t)p.lq * p.group;
+    KvDims k, v;
+    cuuint64_t qs[4];
+    static const bool no_tma = [] { const char *e = diag_env("B200_FA_NO_TMA"); return e && *e == '1'; }();
+    if (!no_tma && rows >= P3_MIN_ROWS && p.d <= 128 && (reinterpret_cast<uintptr_t>(p.o) & 15) == 0 && p.lk < (1u << 31) && rows < (1ull << 31) &&
+        (rows + P3_ROWS - 1) / P3_ROWS * p.b * p.hkv < (1ull << 31) && q_strides(p, qs) &&
+        kv_dims_of(p, &k, &v))
+        return PF_TMA;
+    // tensors that no map describes: 16-byte chunks, head dim 128
+    if (p.d != PF_D || rows < 4 * PF_BM) return PF_NONE;  // short chunks and decode stay on the mma.sync kernel
+    if ((reinterpret_cast<uintptr_t>(p.q) & 15) || ((p.q_sb | p.q_ss | p.q_sh) & 7)) return PF_NONE;
+    static const long force = [] { const char *e = diag_env("B200_FA_TC_ROWS"); return e ? atol(e) : 0l; }();  // 128 or 256: tile height
+    if (force == 128) return PF_ROWS128;
+    if (force == 256) return PF_ROWS256;
+    // 256-row blocks halve the K / V traffic per product and overlap softmax with products inside the block; they
+    // need enough blocks to fill the device
+    return rows >= 1024 ? PF_ROWS256 : PF_ROWS128;
+}
+bool fa_prefill_sm100_supported(const FaParams &p, bool kv16) { return fa_prefill_route(p, kv16) != PF_NONE; }
+
+// shared memory opt-in, once per kernel, thread and device
+template <typename K>
+static int pf_opt_in(K kern, uint32_t bytes, bool (&done)[16]) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 16 && !done[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return set_error(B200_ERR_LAUNCH, "flash_attn (tcgen05 tiles): shared memory opt-in: %s", cudaGetErrorString(e));
+        done[dev] = true;
+    }
+    return B200_OK;
+}
+
+template <int HD, bool BF16>
+static int fa_prefill_tma_launch(const FaParams &p, cudaStream_t stream) {
+    static thread_local bool done[16] = {};
+    const int rc = pf_opt_in(fa_prefill_tma_kernel<HD, BF16>, P3<HD>::SMEM, done);
+    if (rc) return rc;
+    KvDims k, v;
+    CUtensorMap tm_k, tm_v, tm_q;
+    if (!kv_dims_of(p, &k, &v) || !make_kv_map(&tm_k, k, p.k, BF16, p.d) || !make_kv_map(&tm_v, v, p.v, BF16, p.d) || !make_q_map(&tm_q, p, BF16))
+        return set_error(B200_ERR_LAUNCH, "flash_attn (tcgen05 tiles): the driver refuses a tensor map");
+    P3Grid gr;
+    const uint64_t rows = (uint64_t)p.lq * p.group, pair_bytes = std::max<uint64_t>((uint64_t)p.lk * p.d * 4, 1);
+    gr.tiles = (uint32_t)((rows + P3_ROWS - 1) / P3_ROWS);
+    gr.pairs = p.b * p.hkv;
+    gr.hpc = (uint32_t)std::min<uint64_t>(std::max<uint64_t>((64ull << 20) / pair_bytes, 1), gr.pairs);
+    gr.items = gr.tiles * gr.pairs;
+    gr.group_log2 = 0;
+    while ((1u << gr.group_log2) < p.group) ++gr.group_log2;
+    gr.tm_order = k.order | (v.order << 8);
+    fa_prefill_tma_kernel<HD, BF16><<<gr.items, P3_THREADS, P3<HD>::SMEM, stream>>>(p, tm_k, tm_v, tm_q, gr);
+    return check_launch("flash_attn (tcgen05 tiles)");
 }
 
 int fa_prefill_sm100_launch(const FaParams &p, bool bf16, cudaStream_t stream) {
-    static thread_local bool done[16][2] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 16 && !done[dev][bf16]) {
-        cudaError_t e = bf16 ? cudaFuncSetAttribute(fa_prefill_sm100_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM)
-                             : cudaFuncSetAttribute(fa_prefill_sm100_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PF_SMEM);
-        if (e == cudaSuccess)
-            e = bf16 ? cudaFuncSetAttribute(fa_prefill_sm100_kernel2<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2_SMEM)
-                     : cudaFuncSetAttribute(fa_prefill_sm100_kernel2<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2_SMEM);
-        if (e == cudaSuccess)
-            e = bf16 ? cudaFuncSetAttribute(fa_prefill_sm100_kernel2<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2_SMEM)
-                     : cudaFuncSetAttribute(fa_prefill_sm100_kernel2<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2_SMEM);
-        if (e != cudaSuccess) return set_error(B200_ERR_LAUNCH, "flash_attn (tcgen05 tiles): shared memory opt-in: %s", cudaGetErrorString(e));
-        done[dev][bf16] = true;
+    const int route = fa_prefill_route(p, p.kv_kind == 0);
+    if (route == PF_TMA) {
+        if (p.d <= 64) return bf16 ? fa_prefill_tma_launch<64, true>(p, stream) : fa_prefill_tma_launch<64, false>(p, stream);
+        return bf16 ? fa_prefill_tma_launch<128, true>(p, stream) : fa_prefill_tma_launch<128, false>(p, stream);
     }
     const uint64_t rows = (uint64_t)p.lq * p.group;
-    static const long force = [] { const char *e = diag_env("B200_FA_TC_ROWS"); return e ? atol(e) : 0l; }();  // 128 or 256: tile height
-    // 256-row blocks halve the K / V traffic per product and overlap softmax with products inside the block; they
-    // need enough blocks to fill the device
-    bool two = rows >= 1024;
-    if (force == 128) two = false;
-    if (force == 256) two = true;
-    if (two) {
+    static thread_local bool done[2][2][16] = {};
+    if (route == PF_ROWS256) {
+        const int rc = bf16 ? pf_opt_in(fa_prefill_sm100_kernel2<true>, P2_SMEM, done[0][1]) : pf_opt_in(fa_prefill_sm100_kernel2<false>, P2_SMEM, done[0][0]);
+        if (rc) return rc;
         const dim3 grid((unsigned)((rows + P2_ROWS - 1) / P2_ROWS), p.hkv, p.b);
-        // K / V through tensor copies when the tensors can be described by a map (fixed-length batches, 16-byte aligned
-        // strides); otherwise 16-byte chunks
-        static const bool no_tma = [] { const char *e = diag_env("B200_FA_NO_TMA"); return e && *e == '1'; }();
-        static const bool no_qtma = [] { const char *e = diag_env("B200_FA_NO_QTMA"); return e && *e == '1'; }();
-        CUtensorMap tm_k, tm_v, tm_q;
-        uint32_t ok_ = 0, ov_ = 0;
-        const bool tma = !no_tma && !p.varlen && make_kv_map(&tm_k, &ok_, p.k, bf16, p.b, p.hkv, p.lk, p.k_sb, p.k_sh, p.k_ss) &&
-                         make_kv_map(&tm_v, &ov_, p.v, bf16, p.b, p.hkv, p.lk, p.v_sb, p.v_sh, p.v_ss);
-        const bool qtma = tma && !no_qtma && make_q_map(&tm_q, p, bf16);
-        const uint32_t order = ok_ | (ov_ << 8) | (qtma ? 1u << 16 : 0u);
-        if (!tma) memset(&tm_k, 0, sizeof(tm_k)), memset(&tm_v, 0, sizeof(tm_v));
-        if (!qtma) memset(&tm_q, 0, sizeof(tm_q));
-        if (tma && bf16) fa_prefill_sm100_kernel2<true, true><<<grid, P2_THREADS, P2_SMEM, stream>>>(p, tm_k, tm_v, tm_q, order);
-        else if (tma) fa_prefill_sm100_kernel2<false, true><<<grid, P2_THREADS, P2_SMEM, stream>>>(p, tm_k, tm_v, tm_q, order);
-        else if (bf16) fa_prefill_sm100_kernel2<true, false><<<grid, P2_THREADS, P2_SMEM, stream>>>(p, tm_k, tm_v, tm_q, order);
-        else fa_prefill_sm100_kernel2<false, false><<<grid, P2_THREADS, P2_SMEM, stream>>>(p, tm_k, tm_v, tm_q, order);
+        if (bf16) fa_prefill_sm100_kernel2<true><<<grid, P2_THREADS, P2_SMEM, stream>>>(p);
+        else fa_prefill_sm100_kernel2<false><<<grid, P2_THREADS, P2_SMEM, stream>>>(p);
     } else {
+        const int rc = bf16 ? pf_opt_in(fa_prefill_sm100_kernel<true>, PF_SMEM, done[1][1]) : pf_opt_in(fa_prefill_sm100_kernel<false>, PF_SMEM, done[1][0]);
+        if (rc) return rc;
         const dim3 grid((unsigned)((rows + PF_BM - 1) / PF_BM), p.hkv, p.b);
         if (bf16) fa_prefill_sm100_kernel<true><<<grid, PF_THREADS, PF_SMEM, stream>>>(p);
         else fa_prefill_sm100_kernel<false><<<grid, PF_THREADS, PF_SMEM, stream>>>(p);

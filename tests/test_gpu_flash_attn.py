@@ -374,6 +374,51 @@ def test_prefill_append_from_two_host_threads(P, oracle):
     assert P._abi.lib().b200_device_wait_status() == 0
 
 
+def _plain(q, k, v, scale, wl, wr):
+    """(lq, hq, d) over (lk, hkv, d) in 64 bits, plain torch; zeros for rows without a key."""
+    lq, lk, g = q.shape[0], k.shape[0], q.shape[1] // k.shape[1]
+    kk, vv = (t.double().transpose(0, 1).repeat_interleave(g, 0) for t in (k, v))
+    s = (q.double().transpose(0, 1) @ kk.transpose(1, 2)) * scale
+    pos, j = torch.arange(lq, device=q.device)[:, None] + lk - lq, torch.arange(lk, device=q.device)[None]
+    hidden = torch.zeros((lq, lk), dtype=torch.bool, device=q.device)
+    if wl >= 0:
+        hidden |= j < pos - wl
+    if wr >= 0:
+        hidden |= j > pos + wr
+    return (torch.softmax(s.masked_fill(hidden, -torch.inf), -1).nan_to_num(0.0) @ vv).transpose(0, 1)
+
+
+# the edges of the tensor-copy tiles (256 packed rows in groups of 128, key tiles of 128, head dims up to 64 and up to 128), and
+# the forms beside them: groups that are no power of two (16-byte chunks), more work items than SMs, a group without rows
+@pytest.mark.parametrize("lq,lk,b,hq,hkv,d,wl,wr", [
+    (512, 127, 1, 1, 1, 64, -1, -1), (128, 128, 1, 4, 1, 128, -1, 0), (513, 129, 2, 2, 2, 72, -1, -1), (600, 600, 1, 2, 2, 8, -1, 0),
+    (1025, 1025, 1, 1, 1, 64, -1, 0), (900, 300, 1, 4, 1, 128, -1, 0), (700, 1300, 2, 4, 2, 128, 129, 3), (700, 1300, 1, 2, 2, 64, 300, 0),
+    (520, 520, 10, 16, 16, 64, -1, 0), (520, 520, 10, 16, 16, 128, -1, 0), (300, 300, 1, 6, 2, 128, -1, 0), (300, 300, 1, 256, 1, 40, -1, 0)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_tensor_copy_tiles_at_their_edges(P, lq, lk, b, hq, hkv, d, wl, wr, dt):
+    g = torch.Generator(device="cuda:0").manual_seed(lq + lk)
+    q, k, v = (torch.randn((b, n, h, d), generator=g, device="cuda:0", dtype=dt) for n, h in ((lq, hq), (lk, hkv), (lk, hkv)))
+    q[:, ::3] *= 6  # rows whose maximum moves a lot
+    out = P.flash_attn.flash_attn_with_config(q, k, v, cfg_of(P, d, wl, wr))
+    want = torch.stack([_plain(*x, 1.0 / np.sqrt(d), wl, wr) for x in zip(q, k, v)])
+    # output and weights are each rounded to the type once: half an ulp each, 2^-9 (2^-12), at most; their sum in the 2-norm
+    assert (out.double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dt] * want.norm()
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (2, 2, 64), (4, 4, 96)])
+def test_varlen_rows_beside_infinities(P, hq, hkv, d):
+    """The last key tile of a sequence reaches into the next one: what is there, infinities and NaN included, has no part in it."""
+    lens = [700, 600, 1, 513]
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda:0")
+    g = torch.Generator(device="cuda:0").manual_seed(d)
+    q, k, v = (torch.randn((sum(lens), h, d), generator=g, device="cuda:0", dtype=torch.bfloat16) for h in (hq, hkv, hkv))
+    k[700:1300], v[700:1300] = float("inf"), float("nan")
+    out = P.flash_attn.flash_attn_varlen(q, k, v, cu, cu, 700, 700, 1.0 / np.sqrt(d), True)
+    for a, e in ((0, 700), (1300, 1301), (1301, 1814)):
+        want = _plain(q[a:e], k[a:e], v[a:e], 1.0 / np.sqrt(d), -1, 0)
+        assert (out[a:e].double() - want).norm() <= 2.0 ** -8 * want.norm()
+
+
 def test_argument_errors(P):
     A = P._abi
     F = P.flash_attn
