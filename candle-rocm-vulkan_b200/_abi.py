@@ -65,6 +65,12 @@ class KvAppendArgs(C.Structure):
                 ("flags", C.c_uint32), ("pad", C.c_uint32)]
 
 
+class KvUnpackArgs(C.Structure):
+    _fields_ = [("k_cache", C.c_void_p), ("v_cache", C.c_void_p), ("k_cache_strides", u64x3), ("v_cache_strides", u64x3),
+                ("k", C.c_void_p), ("v", C.c_void_p), ("b", C.c_uint32), ("hkv", C.c_uint32), ("t", C.c_uint32), ("d", C.c_uint32),
+                ("dtype", C.c_int32), ("pad", C.c_uint32), ("kq", QuantSide), ("vq", QuantSide)]
+
+
 class Page(C.Structure):
     _fields_ = [("k", C.c_void_p), ("v", C.c_void_p), ("rows", C.c_uint32), ("k_cap", C.c_uint32),
                 ("v_cap", C.c_uint32), ("pad", C.c_uint32)]
@@ -109,7 +115,7 @@ class FaArgs(C.Structure):
 SYMBOLS = [
     "b200_row_layout", "b200_codebook", "b200_hadamard_signs", "b200_qjl_matrix", "b200_row_group", "b200_split_count_grouped",
     "b200_tq_residual", "b200_tq_signs", "b200_rotation_matrix", "b200_tq_rotate_dense",
-    "b200_describe", "b200_last_error", "b200_tq_rotate", "b200_tq_quantize", "b200_tq_dequantize", "b200_kv_append",
+    "b200_describe", "b200_last_error", "b200_tq_rotate", "b200_tq_quantize", "b200_tq_dequantize", "b200_kv_append", "b200_kv_unpack",
     "b200_tq_attention_workspace_bytes", "b200_tq_attention", "b200_tq_attention_static", "b200_tq_attention_gather",
     "b200_flash_attn_workspace_bytes", "b200_flash_attn_paged_workspace_bytes", "b200_flash_attn_paged",
     "b200_flash_attn", "b200_fa_prefill_append", "b200_device_wait_status", "b200_device_wait_check",
@@ -151,6 +157,7 @@ def lib():
         l.b200_tq_quantize.argtypes = [C.POINTER(TqQuantArgs), C.c_void_p]
         l.b200_tq_dequantize.argtypes = [C.POINTER(TqDequantArgs), C.c_void_p]
         l.b200_kv_append.argtypes = [C.POINTER(KvAppendArgs), C.c_void_p]
+        l.b200_kv_unpack.argtypes = [C.POINTER(KvUnpackArgs), C.c_void_p]
         l.b200_tq_attention_workspace_bytes.argtypes = [C.POINTER(TqAttnArgs)]
         l.b200_tq_attention_workspace_bytes.restype = C.c_size_t
         l.b200_tq_attention.argtypes = [C.POINTER(TqAttnArgs), C.c_void_p]

@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(QW * 32) quant_rows_kernel(const QuantParams p
 }
 
 // ---------------------------------------------------------------------------------------------
-// Rows of 128 elements in the block-scaled formats. Eight lanes share a row (four rows per warp): lane l of the eight owns
+// Rows of 128 elements. Eight lanes share a row (four rows per warp): lane l of the eight owns
 // elements 16 l .. 16 l + 15 (two or four 16-byte loads), which is exactly one NVFP4 scale block and half an MX block, so the
 // block arithmetic runs once per 16 elements, the row maximum is three shuffles, and a lane's codes are already the 8 or
 // 16 bytes of the row that it stores. The codes come from the hardware conversions (cvt.rn.satfinite.e2m1x2 /
@@ -343,6 +343,12 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
     const int lane = threadIdx.x & 31, l8 = lane & 7;
     const uint32_t rows = p.nb * p.nh * p.nt;
     const uint32_t mode = sp.mode;
+    // codebook formats: the boundaries between neighbouring codes, ascending; 15 words in 15 banks, so no two lanes collide
+    __shared__ float bound[16];
+    if (mode <= B200_TURBO_PROD) {
+        if (threadIdx.x < 16) bound[threadIdx.x] = threadIdx.x < (1u << sp.cb) - 1u ? sp.tab[16 + threadIdx.x] : 0.0f;
+        __syncthreads();
+    }
     after_prev_begin(p);
     for (uint32_t base = (blockIdx.x * Q128_WARPS + (threadIdx.x >> 5)) * Q128_RPW; base < rows; base += gridDim.x * Q128_WARPS * Q128_RPW) {
         bool live = base + (lane >> 3) < rows;  // a row past the end repeats the last one and stores nothing
@@ -393,6 +399,52 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
             for (int k = 0; k < 16; ++k) x[k] *= s;
         }
 
+        if (mode <= B200_TURBO_PROD) {
+            // Sum of squares in the order of the reference's 128 lanes (red[t] += red[t + s], s = 64 ... 1): index bits 6, 5, 4
+            // are the row's lanes, and each step leaves half of the residues with either lane (residue bit 3 with lane bit 2,
+            // and so on); bits 3, 2, 1 then lie across the lanes, bit 0 in the register.
+            float v[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = __fmul_rn(x[k], x[k]);
+#pragma unroll
+            for (int o = 4, n = 8; o > 0; o >>= 1, n >>= 1) {
+                const bool up = l8 & o;
+#pragma unroll
+                for (int k = 0; k < n; ++k) {
+                    const float keep = up ? v[k + n] : v[k], give = up ? v[k] : v[k + n];
+                    v[k] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, o));
+                }
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
+                v[1] = __fadd_rn(v[1], __shfl_xor_sync(0xffffffffu, v[1], o));
+            }
+            const float norm = __fsqrt_rn(__fadd_rn(v[0], v[1]));
+            const float inv = norm > 0.0f ? __fdiv_rn(1.0f, norm) : 0.0f;
+            const uint32_t cb = sp.cb;
+            uint64_t w = 0;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                // the number of boundaries that u reaches: they ascend, so by halves (a NaN reaches none)
+                const float u = __fmul_rn(x[k], inv);
+                uint32_t idx = 0;
+                for (uint32_t st = 1u << (cb - 1); st; st >>= 1) idx += u >= bound[idx + st - 1] ? st : 0u;
+                w |= (uint64_t)idx << (k * cb);
+            }
+            if (live) {
+                if (cb == 4) {
+                    orow[2 * l8] = (uint32_t)w, orow[2 * l8 + 1] = (uint32_t)(w >> 32);
+                } else {
+                    uint16_t *dst = reinterpret_cast<uint16_t *>(orow) + l8 * cb;  // 16 codes of cb bits
+                    for (uint32_t i = 0; i < cb; ++i) dst[i] = (uint16_t)(w >> (16 * i));
+                }
+                for (int i = l8; i < sp.aux_words; i += 8) orow[sp.code_words + i] = 0u;
+                if (l8 < 2) orow[sp.code_words + sp.aux_words + l8] = l8 ? 0u : f2u(norm);
+            }
+            continue;
+        }
+
         // the lane's maximum; a NaN survives only if all sixteen are NaNs (fmaxf drops a NaN operand). z is a NaN when
         // the lane holds a NaN or an infinity.
         float bm = fabsf(x[0]), z = x[0] * 0.0f;
@@ -423,7 +475,7 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
                 *reinterpret_cast<uint2 *>(orow + 2 * l8) = make_uint2(w[0], w[1]);
                 reinterpret_cast<uint8_t *>(orow + 16)[l8] = (uint8_t)scode;
             }
-        } else if (mode == B200_FP8) {
+        } else if (mode == B200_FP8_ROW) {
             cw = 32;
             float am = fmaxf(0.0f, bm);
             am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
@@ -496,6 +548,118 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint32_t *__res
             // prod rows: the QJL coefficient of element j (candle-core/kernels/turbo_quant_impl.h:219-222)
             const float c = __fdiv_rn(__fmul_rn(__fmul_rn(u2f(r[rsc_off]), u2f(r[rsc_off + 1])), 1.2533141f), (float)D);
             zs[idx] = ((r[code_words + (j >> 5)] >> (j & 31u)) & 1u) ? c : -c;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Packed rows back to values in one pass: decode, rotate back, cast, store. LPR lanes share a row, each with 16 consecutive
+// elements (as in quant_rows128_kernel); grid.y: keys, values. Bound by memory: 65 528 rows of 72 bytes to bf16 move 21 MB.
+// The chain it stands for (dequant_rows_kernel, hadamard_rows_kernel, a cast; in f32, with a copy in front when the rows
+// are not back to back) moves ten times the bytes in three or four launches. Values are the chain's, bit for bit: the same
+// roundings in the same order, butterflies from index bit 0 up. Measured: keys and values of 8192 x 8 cached MXFP8 rows, rotated, for a chunk of 1024 query tokens: the
+// call 414 -> 173 us (141 of them the attention); 65 528 TurboQuant-4 rows packed and unpacked 250 -> 56 us (with the codebook
+// formats in quant_rows128_kernel, and each row packed once instead of twice).
+// ---------------------------------------------------------------------------------------------
+struct UnpackSide {
+    const uint32_t *src;
+    void *dst;  // contiguous (batch entry, head, row, element)
+    const float *tab, *signs;
+    uint64_t s_b, s_h, s_t;  // words
+    int32_t mode, cb, code_words, rsc_off, rot;
+};
+struct UnpackParams {
+    UnpackSide side[2];
+    uint32_t nb, nh, nt;
+    uint32_t nt_mul, nt_shr, nh_mul, nh_shr;
+};
+constexpr int UP_WARPS = 8;
+
+template <int LPR, int DT>
+__global__ void __launch_bounds__(UP_WARPS * 32) unpack_rows_kernel(const UnpackParams p) {
+    constexpr int RPW = 32 / LPR, D = LPR * 16;
+    const UnpackSide &sp = p.side[blockIdx.y];
+    const int lane = threadIdx.x & 31, ll = lane % LPR;
+    const uint32_t rows = p.nb * p.nh * p.nt, mode = sp.mode, cb = sp.cb;
+    __shared__ float tab[16];
+    if (mode <= B200_TURBO_PROD) {
+        if (threadIdx.x < 16) tab[threadIdx.x] = sp.tab[threadIdx.x];
+        __syncthreads();
+    }
+    for (uint32_t base = (blockIdx.x * UP_WARPS + (threadIdx.x >> 5)) * RPW; base < rows; base += gridDim.x * UP_WARPS * RPW) {
+        const bool live = base + lane / LPR < rows;  // a row past the end repeats the last one and stores nothing
+        const uint32_t row = live ? base + lane / LPR : rows - 1;
+        const uint32_t bh = fastdiv(row, p.nt_mul, p.nt_shr), t = row - bh * p.nt, b = fastdiv(bh, p.nh_mul, p.nh_shr), h = bh - b * p.nh;
+        const uint32_t *r = sp.src + b * sp.s_b + h * sp.s_h + t * sp.s_t;
+        const float rsc0 = u2f(__ldg(r + sp.rsc_off));
+        const uint8_t *aux = reinterpret_cast<const uint8_t *>(r + sp.code_words);
+        float x[16];
+        if (cb == 8) {
+            const float sc = mode == B200_MXFP8 ? e8m0_to_f(__ldg(aux + ll / 2)) : 1.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t w = __ldg(r + 4 * ll + i);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float e = e4m3_to_f((w >> (8 * k)) & 0xffu);
+                    x[4 * i + k] = __fmul_rn(rsc0, mode == B200_MXFP8 ? __fmul_rn(e, sc) : e);
+                }
+            }
+        } else {
+            // 16 codes of cb bits from bit 16 cb ll on: a word, or two
+            const uint32_t bit0 = 16u * cb * ll, sh = bit0 & 31u;
+            uint64_t w = __ldg(r + (bit0 >> 5));
+            if (sh + 16u * cb > 32u) w |= (uint64_t)__ldg(r + (bit0 >> 5) + 1) << 32;
+            w >>= sh;
+            const uint32_t mask = (1u << cb) - 1u;
+            if (mode <= B200_TURBO_PROD) {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) x[k] = __fmul_rn(rsc0, tab[(uint32_t)(w >> (k * cb)) & mask]);
+            } else {
+                const float sc = mode == B200_MXFP4 ? e8m0_to_f(__ldg(aux + ll / 2)) : e4m3_to_f(__ldg(aux + ll));
+#pragma unroll
+                for (int k = 0; k < 16; ++k) x[k] = __fmul_rn(rsc0, __fmul_rn(fp4_to_f((uint32_t)(w >> (4 * k)) & 15u), sc));
+            }
+        }
+        if (sp.rot == B200_ROT_HADAMARD) {
+            // x = diag(s) H y / sqrt(D)
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    if (!(k & o)) {
+                        const float a = x[k], c = x[k | o];
+                        x[k] = __fadd_rn(a, c);
+                        x[k | o] = __fsub_rn(a, c);
+                    }
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < LPR; o <<= 1) {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const float y = __shfl_xor_sync(0xffffffffu, x[k], o);
+                    x[k] = (lane & o) ? __fsub_rn(y, x[k]) : __fadd_rn(x[k], y);
+                }
+            }
+            const float s = 1.0f / sqrtf((float)D);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) x[k] = __fmul_rn(__fmul_rn(x[k], s), __ldg(sp.signs + 16 * ll + k));
+        }
+        if (!live) continue;
+        char *dst = reinterpret_cast<char *>(sp.dst) + ((uint64_t)row * D + 16 * ll) * dtype_size(DT);
+        if (DT == B200_F32) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) reinterpret_cast<float4 *>(dst)[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+        } else {
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (DT == B200_BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(x[2 * i + 1]), "f"(x[2 * i]));
+                else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(x[2 * i + 1]), "f"(x[2 * i]));
+            }
+            reinterpret_cast<uint4 *>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            reinterpret_cast<uint4 *>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
     }
 }
@@ -630,14 +794,13 @@ static void fastdiv_init(uint32_t d, uint32_t &mul, uint32_t &shr) {
     mul = (uint32_t)((((one << (32 + shr)) + d - 1) / d) - (one << 32));
 }
 
-// rows of 128 block-scaled elements whose source rows can be read as 16-byte vectors
+// rows of 128 elements whose source rows can be read as 16-byte vectors
 static bool rows128_takes(const QuantParams &p, int sides) {
     static const bool off = diag_env("B200_QUANT_GENERIC") != nullptr;
     if (off || p.d != 128 || (uint64_t)p.nb * p.nh * p.nt >= 0x7fffff00ull) return false;
     const uint64_t vec = p.src_dtype == B200_F32 ? 3 : 7;  // elements per 16 bytes - 1
     for (int s = 0; s < sides; ++s) {
         const QuantSideParams &sp = p.side[s];
-        if (sp.mode != B200_MXFP4 && sp.mode != B200_NVFP4 && sp.mode != B200_MXFP8 && sp.mode != B200_FP8) return false;
         if (((uintptr_t)sp.src & 15) || (sp.s_b & vec) || (sp.s_h & vec) || (sp.s_t & vec)) return false;
         if (sp.rot == B200_ROT_HADAMARD && ((uintptr_t)sp.signs & 15)) return false;
         // NVFP4 code words are stored in pairs
@@ -788,6 +951,70 @@ extern "C" int b200_tq_dequantize(const B200TqDequantArgs *a, b200_stream_t stre
     dequant_rows_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a->data, a->tab, a->out, a->rows, a->dim, stride, a->mode,
                                                                l.code_bits, l.code_words, l.rsc_offset, a->zs);
     return check_launch("tq_dequantize");
+}
+
+template <int LPR>
+static int launch_unpack(const UnpackParams &p, int sides, int dt, cudaStream_t stream) {
+    const uint64_t rows = (uint64_t)p.nb * p.nh * p.nt, per_block = UP_WARPS * (32 / LPR);
+    // what is resident at once (eight blocks per SM), shared by the sides; more rows per block beyond that
+    const unsigned most = 148u * 8u / sides, gx = (unsigned)std::min<uint64_t>((rows + per_block - 1) / per_block, most);
+    const dim3 grid(gx, sides);
+    if (dt == B200_F32) unpack_rows_kernel<LPR, B200_F32><<<grid, UP_WARPS * 32, 0, stream>>>(p);
+    else if (dt == B200_F16) unpack_rows_kernel<LPR, B200_F16><<<grid, UP_WARPS * 32, 0, stream>>>(p);
+    else unpack_rows_kernel<LPR, B200_BF16><<<grid, UP_WARPS * 32, 0, stream>>>(p);
+    return check_launch("kv_unpack");
+}
+
+extern "C" int b200_kv_unpack(const B200KvUnpackArgs *a, b200_stream_t stream) {
+    if (!a) return set_error(B200_ERR_BAD_ARG, "kv_unpack: null args");
+    if (a->dtype != B200_F32 && a->dtype != B200_F16 && a->dtype != B200_BF16)
+        return set_error(B200_ERR_BAD_ARG, "kv_unpack: output dtype must be f32, f16 or bf16");
+    const uint64_t rows = (uint64_t)a->b * a->hkv * a->t;
+    if (rows == 0) return B200_OK;
+    const int sides = a->v_cache || a->v ? 2 : 1;
+    const void *srcs[2] = {a->k_cache, a->v_cache};
+    void *dsts[2] = {a->k, a->v};
+    const uint64_t *ss[2] = {a->k_cache_strides, a->v_cache_strides};
+    const B200QuantSide *qs[2] = {&a->kq, &a->vq};
+    UnpackParams p;
+    memset(&p, 0, sizeof(p));
+    for (int s = 0; s < sides; ++s) {
+        if (!srcs[s] || !dsts[s]) return set_error(B200_ERR_BAD_ARG, "kv_unpack: null pointer");
+        if (reinterpret_cast<uintptr_t>(dsts[s]) & 15) return set_error(B200_ERR_BAD_ARG, "kv_unpack: outputs must be 16-byte aligned");
+        QuantSideParams q;
+        const int rc = fill_side(q, *qs[s], a->d);
+        if (rc) return rc;
+        if (q.mode == B200_TURBO_PROD) return set_error(B200_ERR_UNSUPPORTED_SHAPE, "kv_unpack: prod rows need their sketch (b200_tq_dequantize)");
+        if (ss[s][2] < (uint64_t)q.row_words) return set_error(B200_ERR_BAD_ARG, "kv_unpack: row stride below the row size");
+        UnpackSide &u = p.side[s];
+        u.src = reinterpret_cast<const uint32_t *>(srcs[s]);
+        u.dst = dsts[s];
+        u.tab = q.tab;
+        u.signs = q.signs;
+        u.s_b = ss[s][0];
+        u.s_h = ss[s][1];
+        u.s_t = ss[s][2];
+        u.mode = q.mode;
+        u.cb = q.cb;
+        u.code_words = q.code_words;
+        u.rsc_off = q.code_words + q.aux_words;
+        u.rot = q.rot;
+    }
+    if (rows >= 0x7fffff00ull) return set_error(B200_ERR_UNSUPPORTED_SHAPE, "kv_unpack: more than 2^31 rows");
+    p.nb = a->b;
+    p.nh = a->hkv;
+    p.nt = a->t;
+    fastdiv_init(p.nt, p.nt_mul, p.nt_shr);
+    fastdiv_init(p.nh, p.nh_mul, p.nh_shr);
+    cudaStream_t st = (cudaStream_t)stream;
+    switch (a->d) {
+    case 32: return launch_unpack<2>(p, sides, a->dtype, st);
+    case 64: return launch_unpack<4>(p, sides, a->dtype, st);
+    case 128: return launch_unpack<8>(p, sides, a->dtype, st);
+    case 256: return launch_unpack<16>(p, sides, a->dtype, st);
+    case 512: return launch_unpack<32>(p, sides, a->dtype, st);
+    }
+    return set_error(B200_ERR_UNSUPPORTED_SHAPE, "kv_unpack: head dim %u (powers of two from 32 to 512)", a->d);
 }
 
 extern "C" int b200_tq_residual(const B200TqResidArgs *a, b200_stream_t stream) {

@@ -232,8 +232,12 @@ class TurboQuantizer:
             return self.quantize_rotated_rows(x)
         if self.rotation == "dense":
             return self.quantize_rotated_rows(self.rotate(x))
+        # the fused rotation comes with the append, which takes two tensors: one half of the rows each (an odd number of
+        # rows: both write the same bytes of the middle one)
+        x = x.view(1, 1, rows, d)
         out = torch.empty((1, 1, rows, self.layout.row_words), dtype=torch.int32, device=x.device)
-        _kv_append(x.view(1, 1, rows, d), x.view(1, 1, rows, d), out, out.clone(), self, self, 0)
+        half = (rows + 1) // 2
+        _kv_append(x[:, :, :half], x[:, :, rows - half:], out[:, :, :half], out[:, :, rows - half:], self, self, 0)
         return out.view(rows, self.layout.row_words)
 
     def dequantize_rows(self, data: torch.Tensor) -> torch.Tensor:
@@ -259,7 +263,15 @@ class TurboQuantizer:
         return QuantizedTensor(self.quantize_rows(x.reshape(-1, d)), x.shape, x.dtype)
 
     def dequantize(self, q: QuantizedTensor) -> torch.Tensor:
+        if self.unpacks(q.dtype) and q.data.dim() == 2 and q.data.shape[1] == self.layout.row_words and q.data.is_cuda:
+            data = q.data.contiguous()
+            return _kv_unpack(data.view(1, 1, *data.shape), None, self, None, data.shape[0], q.dtype)[0].reshape(q.shape)
         return self.dequantize_rows(q.data).reshape(q.shape).to(q.dtype)
+
+    def unpacks(self, dtype) -> bool:
+        """Whether b200_kv_unpack reads these rows (decode, rotation back and cast in one launch) into `dtype`."""
+        return self.dim in (32, 64, 128, 256, 512) and self.qjl is None and self.rotation != "dense" and dtype in (
+            torch.float32, torch.float16, torch.bfloat16)
 
 
 def _kv_append(k, v, k_cache, v_cache, kq: TurboQuantizer, vq: TurboQuantizer, pos, pos_add: int = 0, status=None, after_prev: bool = False):
@@ -288,6 +300,18 @@ def _kv_append(k, v, k_cache, v_cache, kq: TurboQuantizer, vq: TurboQuantizer, p
         # B200_KV_AFTER_PREV: the stream's previous kernel neither reads the rows written here nor writes k, v or pos
         A.KV_AFTER_PREV if after_prev else 0, 0)
     A.check(A.lib().b200_kv_append(C.byref(args), _stream(k.device)))
+
+
+def _kv_unpack(k_rows, v_rows, kq: TurboQuantizer, vq: Optional[TurboQuantizer], t: int, dtype):
+    """b200_kv_unpack: the first `t` rows of (b, hkv, cap, words) caches as (b, hkv, t, d) tensors; `v_rows` may be None."""
+    b, h = k_rows.shape[:2]
+    k = torch.empty((b, h, t, kq.dim), dtype=dtype, device=k_rows.device)
+    v = torch.empty_like(k) if v_rows is not None else None
+    args = A.KvUnpackArgs(k_rows.data_ptr(), v_rows.data_ptr() if v is not None else None, A.u64x3(*k_rows.stride()[:3]),
+                          A.u64x3(*v_rows.stride()[:3]) if v is not None else A.u64x3(), k.data_ptr(), v.data_ptr() if v is not None else None,
+                          b, h, t, kq.dim, _dtype_id(k), 0, kq.side(), (vq or kq).side())
+    A.check(A.lib().b200_kv_unpack(C.byref(args), _stream(k.device)))
+    return k, v
 
 
 _WORKSPACES = {}
@@ -665,6 +689,8 @@ class TurboKvCache:
             return None
         b, h, _, _ = self.k.shape
         dt = self.dtype or torch.float32
+        if self.kq.unpacks(dt) and self.vq.unpacks(dt):
+            return _kv_unpack(self.k, self.v, self.kq, self.vq, self.len, dt)
         deq = lambda q, x: q.dequantize_rows(x[:, :, : self.len].reshape(b * h * self.len, -1)).reshape(
             b, h, self.len, self.dim).to(dt)
         return deq(self.kq, self.k), deq(self.vq, self.v)

@@ -235,6 +235,23 @@ typedef struct B200KvAppendArgs {
 #define B200_KV_AFTER_PREV 1u
 int b200_kv_append(const B200KvAppendArgs *args, b200_stream_t stream);
 
+/* The way back: the rows [0, t) of the packed caches (b, hkv, cap, words) as contiguous (b, hkv, t, d) tensors in `dtype`,
+ * rotation undone, in one launch. Replaces TurboKvCache::keys_values (candle-nn/src/turbo_quant.rs:947-966: slices made
+ * contiguous, tq_dequant to f32, matmul with the rotation, to_dtype); the values are those of that chain, bit for bit.
+ * v_cache = v = NULL: only k. Head dims 32, 64, 128, 256, 512; prod rows and other head dims return
+ * B200_ERR_UNSUPPORTED_SHAPE (b200_tq_dequantize serves them). Outputs 16-byte aligned. */
+typedef struct B200KvUnpackArgs {
+    const uint32_t *k_cache, *v_cache;
+    uint64_t k_cache_strides[3]; /* (batch, head, row) in words */
+    uint64_t v_cache_strides[3];
+    void *k, *v;
+    uint32_t b, hkv, t, d;
+    int32_t dtype;               /* B200_F32, B200_F16 or B200_BF16 */
+    uint32_t pad;
+    B200QuantSide kq, vq;
+} B200KvUnpackArgs;
+int b200_kv_unpack(const B200KvUnpackArgs *args, b200_stream_t stream);
+
 /* ---- paged rows --------------------------------------------------------------------------------- */
 /* One block of a paged cache, device memory. Block i holds `rows` valid keys; k / v point at its
  * (batch 0, kv head 0, row 0); head stride = k_cap (v_cap) rows, batch stride = hkv head strides.

@@ -147,6 +147,24 @@ pub struct B200KvAppendArgs {
 }
 
 #[repr(C)]
+pub struct B200KvUnpackArgs {
+    pub k_cache: *const u32,
+    pub v_cache: *const u32,
+    pub k_cache_strides: [u64; 3],
+    pub v_cache_strides: [u64; 3],
+    pub k: *mut c_void,
+    pub v: *mut c_void,
+    pub b: u32,
+    pub hkv: u32,
+    pub t: u32,
+    pub d: u32,
+    pub dtype: i32,
+    pub pad: u32,
+    pub kq: B200QuantSide,
+    pub vq: B200QuantSide,
+}
+
+#[repr(C)]
 #[derive(Clone, Copy)]
 pub struct B200Page {
     pub k: *const c_void,
@@ -274,6 +292,7 @@ extern "C" {
     pub fn b200_tq_rotate_dense(input: *const f32, out: *mut f32, pi: *const f32, rows: u64, dim: u32, inverse: c_int,
                                 stream: b200_stream_t) -> c_int;
     pub fn b200_kv_append(args: *const B200KvAppendArgs, stream: b200_stream_t) -> c_int;
+    pub fn b200_kv_unpack(args: *const B200KvUnpackArgs, stream: b200_stream_t) -> c_int;
 
     // attention over packed rows (CudaStorage::tq_attention / tq_attention_paged)
     pub fn b200_tq_attention_workspace_bytes(args: *const B200TqAttnArgs) -> usize;

@@ -252,3 +252,44 @@ def test_prod_rows_bit_exact_with_reference_kernels(P, oracle, golden, bits, dim
             + oracle.dequantize_qjl(g[key + "_rows"], dim, bits) @ oracle.qjl_matrix(dim, MG.PROD_SEED))
     got = qz.dequantize_rows(rows_dev(g[key + "_rows"])).cpu().numpy()
     assert np.allclose(got, want, atol=2e-5 * max(1.0, float(np.abs(want).max())), rtol=1e-5)
+
+
+@pytest.mark.parametrize("dim", [32, 64, 128, 256, 512])
+@pytest.mark.parametrize("name", ["fp8", "mxfp8", "mxfp4", "nvfp4", "turbo4", "turbo3", "turbo2", "turbo1"])
+def test_unpack_equals_the_chain(name, dim):
+    """b200_kv_unpack (decode, rotation back, cast, one launch) against dequantize + rotate + cast, bit for bit: every type,
+    rotation, row counts at the edges of a warp's rows, caches with spare rows."""
+    P = pkg()
+    f = P.QuantFormat.parse(name)
+    g = torch.Generator(device="cuda:0").manual_seed(dim)
+    for rot in ("none", "hadamard"):
+        for n, h, t, dt in ((1, 1, 1, torch.float32), (2, 3, 37, torch.bfloat16), (1, 2, 16, torch.float16)):
+            kq, vq = P.TurboQuantizer(f, dim, rot, 42, "cuda:0"), P.TurboQuantizer(f, dim, rot, 44, "cuda:0")
+            cache = P.TurboKvCache(f, f, dim, rot, 42, t + 5, "cuda:0")
+            x, y = (torch.randn((n, h, t, dim), generator=g, device="cuda:0", dtype=dt) for _ in range(2))
+            x[..., 3] *= 50
+            cache.append(x, y)
+            for got, rows, q in zip(cache.keys_values(), (cache.k, cache.v), (kq, vq)):
+                want = q.dequantize_rows(rows[:, :, :t].reshape(-1, rows.shape[-1])).view(x.shape).to(dt)
+                assert torch.equal(got, want), (rot, t, dt)
+            packed = kq.quantize(x)
+            assert torch.equal(packed.data.view(n, h, t, -1), cache.k[:, :, :t])
+            assert torch.equal(kq.dequantize(packed), kq.dequantize_rows(packed.data).view(x.shape).to(dt))
+
+
+@pytest.mark.parametrize("name", ["turbo4", "turbo3", "turbo2", "turbo1", "prod5", "prod2"])
+def test_codebook_rows_of_128_on_both_kernels(name):
+    """Rows of 128 whose source can be read in vectors against the same rows read from an odd address (the kernel for every
+    length, itself checked against the oracle): the same bytes, zero rows, infinities and NaN included."""
+    P = pkg()
+    q = P.TurboQuantizer(P.QuantFormat.parse(name), 128, "none", 42, "cuda:0")
+    x = torch.randn((133, 128), generator=torch.Generator(device="cuda:0").manual_seed(1), device="cuda:0")
+    x[5] = 0.0
+    x[6, 9], x[7, 100], x[8, 0] = float("inf"), float("nan"), -float("inf")
+    x[9] *= 1e-30
+    x[10] *= 1e30
+    for dt in (torch.float32, torch.bfloat16, torch.float16):
+        a = x.to(dt)
+        odd = torch.empty(a.numel() + 1, dtype=dt, device="cuda:0")[1:].view(a.shape)
+        odd.copy_(a)
+        assert torch.equal(q.quantize_rotated_rows(a), q.quantize_rotated_rows(odd)), dt
