@@ -446,26 +446,43 @@ __global__ void __launch_bounds__(FA_WARPS * 32) fa_dense_kernel(const FaParams 
     }
 }
 
-// candle-core/kernels/flash_attn_impl.h:445-473
+// candle-core/kernels/flash_attn_impl.h:445-473. One warp per row: a lane has the weights of splits lane and lane + 32 (there are
+// 64 at most), and four neighbouring elements of the sums, four splits' loads on their way at a time. Launched as a
+// programmatic dependent of the kernel that writes the partial results, whose end it waits for.
 __global__ void __launch_bounds__(128) fa_combine_kernel(const float *__restrict__ part_o, const float *__restrict__ part_lse,
                                                         void *__restrict__ o, int o_dtype, uint64_t rows, uint32_t D, uint32_t n_splits) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (uint64_t row = (uint64_t)blockIdx.x * 4 + warp; row < rows; row += (uint64_t)gridDim.x * 4) {
-        float mx = -INFINITY;
-        for (uint32_t s = 0; s < n_splits; ++s) mx = fmaxf(mx, part_lse[(uint64_t)s * rows + row]);
-        float wsum = 0.0f;
-        for (uint32_t s = 0; s < n_splits; ++s) {
-            const float e = part_lse[(uint64_t)s * rows + row];
-            wsum += e == -INFINITY ? 0.0f : expf(e - mx);
-        }
-        for (uint32_t d = lane; d < D; d += 32) {
-            float acc = 0.0f;
-            for (uint32_t s = 0; s < n_splits; ++s) {
-                const float e = part_lse[(uint64_t)s * rows + row];
-                const float w = e == -INFINITY ? 0.0f : expf(e - mx);
-                if (w != 0.0f) acc += w * part_o[((uint64_t)s * rows + row) * D + d];
+        float e0 = (uint32_t)lane < n_splits ? part_lse[(uint64_t)lane * rows + row] : -INFINITY;
+        float e1 = (uint32_t)lane + 32 < n_splits ? part_lse[(uint64_t)(lane + 32) * rows + row] : -INFINITY;
+        float mx = fmaxf(e0, e1);
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, k));
+        e0 = e0 == -INFINITY ? 0.0f : expf(e0 - mx);
+        e1 = e1 == -INFINITY ? 0.0f : expf(e1 - mx);
+        float wsum = e0 + e1;
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, k);
+        for (uint32_t d0 = 0; d0 < D; d0 += 128) {
+            const uint32_t d = d0 + 4 * lane;
+            float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (uint32_t s0 = 0; s0 < n_splits; s0 += 4) {
+                float4 v[4];
+                float w[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t s = s0 + k;
+                    w[k] = __shfl_sync(0xffffffffu, s < 32 ? e0 : e1, s & 31u);
+                    if (s >= n_splits || d >= D) w[k] = 0.0f;
+                    v[k] = w[k] != 0.0f ? *reinterpret_cast<const float4 *>(part_o + ((uint64_t)s * rows + row) * D + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) a[0] += w[k] * v[k].x, a[1] += w[k] * v[k].y, a[2] += w[k] * v[k].z, a[3] += w[k] * v[k].w;
             }
-            store_elem_rt(o, row * D + d, wsum > 0.0f ? acc / wsum : 0.0f, o_dtype);
+            if (d < D)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) store_elem_rt(o, row * D + d + k, wsum > 0.0f ? a[k] / wsum : 0.0f, o_dtype);
         }
     }
 }
@@ -475,6 +492,7 @@ struct FaPlan {
     dim3 grid;
     size_t smem, ws_bytes, off_lse;
     bool bf16;  // mma operand type
+    bool decode_tma;  // fa_decode_tma_kernel takes the call
 };
 
 // keys before every block of a paged call, and their total behind them: one block of threads, a running sum over
@@ -548,14 +566,15 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false) {
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint64_t ctas = (uint64_t)row_tiles * a->hkv * std::max<uint32_t>(a->b, 1);
+    pl.decode_tma = fa_decode_tma_takes(p, paged);
     uint32_t splits = 1;
     if (ctas < 2ull * sms && a->lk > 2 * FA_BN) {
         const uint64_t by_occ = (2ull * sms + ctas - 1) / ctas, by_keys = (a->lk + 4 * FA_BN - 1) / (4 * FA_BN);
         splits = (uint32_t)std::min<uint64_t>(std::min(by_occ, by_keys), 64);
     } else if (rows <= 16 && a->lk >= 16 * FA_BN) {
         // decode with enough blocks to fill the device: up to four key splits where they make the blocks a better fit to
-        // whole waves of resident blocks (four per SM up to head dim 64, three up to 128, one at 256)
-        const uint64_t resident = (uint64_t)sms * (a->d > 128 ? 1 : (a->d > 64 ? 3 : 4));
+        // whole waves of resident blocks (fa_decode_tma_kernel: two per SM; fa_dense_kernel: four up to head dim 64, three up to 128, one at 256)
+        const uint64_t resident = (uint64_t)sms * (pl.decode_tma ? 2 : (a->d > 128 ? 1 : (a->d > 64 ? 3 : 4)));
         double best = 0.0;
         for (uint32_t sp = 1; sp <= 4; ++sp) {
             const uint64_t n = ctas * sp, waves = (n + resident - 1) / resident;
@@ -578,6 +597,22 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false) {
     return B200_OK;
 }
 
+static int fa_combine_launch(const FaPlan &pl, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min<uint64_t>((pl.p.rows_total + 3) / 4, 148ull * 16));
+    cfg.blockDim = dim3(128);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fa_combine_kernel, (const float *)pl.p.part_o, (const float *)pl.p.part_lse, pl.p.o, (int)pl.p.q_dtype,
+                                             pl.p.rows_total, pl.p.d, pl.p.n_splits);
+    if (e != cudaSuccess) return set_error(B200_ERR_LAUNCH, "fa_combine: %s", cudaGetErrorString(e));
+    return check_launch("fa_combine");
+}
+
 template <int HD, bool BF16, bool DEC>
 static int fa_launch_as(const FaPlan &pl, cudaStream_t stream) {
     auto kern = fa_dense_kernel<HD, BF16, DEC>;
@@ -595,9 +630,7 @@ static int fa_launch_as(const FaPlan &pl, cudaStream_t stream) {
     int rc = check_launch("flash_attn");
     if (rc) return rc;
     if (pl.p.n_splits > 1) {
-        const unsigned gx = (unsigned)std::min<uint64_t>((pl.p.rows_total + 3) / 4, 148ull * 16);
-        fa_combine_kernel<<<gx, 128, 0, stream>>>(pl.p.part_o, pl.p.part_lse, pl.p.o, pl.p.q_dtype, pl.p.rows_total, pl.p.d, pl.p.n_splits);
-        rc = check_launch("fa_combine");
+        rc = fa_combine_launch(pl, stream);
     }
     return rc;
 }
@@ -636,6 +669,10 @@ extern "C" int b200_flash_attn(const B200FaArgs *a, b200_stream_t stream_) {
     const bool bf = pl.bf16;
     // long prefill chunks: tiles on the tcgen05 tensor cores
     if (fa_prefill_sm100_supported(pl.p, pl.p.kv_kind == 0)) return fa_prefill_sm100_launch(pl.p, bf, stream);
+    if (pl.decode_tma) {
+        const int drc = fa_decode_tma_launch(pl.p, bf, pl.grid, stream);
+        return drc || pl.p.n_splits == 1 ? drc : fa_combine_launch(pl, stream);
+    }
     if (a->d <= 64) return bf ? fa_launch<64, true>(pl, stream) : fa_launch<64, false>(pl, stream);
     if (a->d <= 128) return bf ? fa_launch<128, true>(pl, stream) : fa_launch<128, false>(pl, stream);
     return bf ? fa_launch<256, true>(pl, stream) : fa_launch<256, false>(pl, stream);
@@ -677,6 +714,10 @@ extern "C" int b200_flash_attn_paged(const B200FaArgs *a, const B200Page *pages,
         pl.p.part_lse = reinterpret_cast<float *>(ws + pre + pl.off_lse);
     }
     const bool bf = pl.bf16;
+    if (pl.decode_tma) {
+        const int drc = fa_decode_tma_launch(pl.p, bf, pl.grid, stream);
+        return drc || pl.p.n_splits == 1 ? drc : fa_combine_launch(pl, stream);
+    }
     if (a->d <= 64) return bf ? fa_launch<64, true>(pl, stream) : fa_launch<64, false>(pl, stream);
     if (a->d <= 128) return bf ? fa_launch<128, true>(pl, stream) : fa_launch<128, false>(pl, stream);
     return bf ? fa_launch<256, true>(pl, stream) : fa_launch<256, false>(pl, stream);

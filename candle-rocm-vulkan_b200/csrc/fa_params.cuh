@@ -3,6 +3,8 @@
 #pragma once
 #include "common.cuh"
 
+struct CUtensorMap_st;
+
 namespace b200 {
 
 struct FaParams {
@@ -29,5 +31,16 @@ struct FaParams {
 // prefill tiles on the 5th generation tensor cores (fa_prefill_sm100.cu)
 bool fa_prefill_sm100_supported(const FaParams &p, bool kv16);
 int fa_prefill_sm100_launch(const FaParams &p, bool bf16, cudaStream_t stream);
+
+// Tensor maps of K and V (boxes of 64 elements x `keys` keys, 128-byte swizzle; past the head dim and past the last key zeros
+// arrive). `order`: the coordinates' places of head, key and batch entry, two bits each, K in bits 0-5, V in bits 8-13. With
+// k == null only whether maps can describe the tensors. fa_prefill_sm100.cu.
+bool fa_kv_maps(const FaParams &p, bool bf16, uint32_t keys, CUtensorMap_st *k, CUtensorMap_st *v, uint32_t *order);
+
+// decode over 16-bit K / V by tensor copies (fa_decode_tma.cu): grid (1, hkv, b * n_splits)
+bool fa_decode_tma_takes(const FaParams &p, bool paged);
+int fa_decode_tma_launch(const FaParams &p, bool bf16, dim3 grid, cudaStream_t stream);
+int fa_decode_wait_status();
+int fa_decode_wait_clear();
 
 }  // namespace b200

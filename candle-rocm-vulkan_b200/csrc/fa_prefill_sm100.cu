@@ -1631,12 +1631,12 @@ static bool kv_dims(KvDims *m, const void *base, uint64_t nb, uint64_t hkv, uint
     }
     return true;
 }
-// boxes of 64 elements x 128 keys, 128-byte swizzle; elements past the head dim and keys past the end read as zeros
-static bool make_kv_map(CUtensorMap *m, const KvDims &k, const void *base, bool bf16, uint64_t d) {
+// boxes of 64 elements x `keys` keys, 128-byte swizzle; elements past the head dim and keys past the end read as zeros
+static bool make_kv_map(CUtensorMap *m, const KvDims &k, const void *base, bool bf16, uint64_t d, uint32_t keys) {
     const cuuint64_t dims[4] = {(cuuint64_t)d, k.size[0], k.size[1], k.size[2]};
     const cuuint64_t strides[3] = {k.stride[0], k.stride[1], k.stride[2]};
     cuuint32_t box[4] = {64, 1, 1, 1};
-    box[1 + ((k.order >> 2) & 3u)] = P3_BN;
+    box[1 + ((k.order >> 2) & 3u)] = keys;
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const EncodeTiledFn enc = encode_tiled_fn();
     return enc && enc(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr,
@@ -1680,6 +1680,14 @@ static bool kv_dims_of(const FaParams &p, KvDims *k, KvDims *v) {
     return kv_dims(k, p.k, nb, p.hkv, n, p.d, p.k_sb, p.k_sh, p.k_ss) && kv_dims(v, p.v, nb, p.hkv, n, p.d, p.v_sb, p.v_sh, p.v_ss);
 }
 
+bool fa_kv_maps(const FaParams &p, bool bf16, uint32_t keys, CUtensorMap *tm_k, CUtensorMap *tm_v, uint32_t *order) {
+    KvDims k, v;
+    if (!kv_dims_of(p, &k, &v)) return false;
+    if (!tm_k) return true;
+    *order = k.order | (v.order << 8);
+    return make_kv_map(tm_k, k, p.k, bf16, p.d, keys) && make_kv_map(tm_v, v, p.v, bf16, p.d, keys);
+}
+
 enum { PF_NONE = 0, PF_ROWS128, PF_ROWS256, PF_TMA };
 constexpr uint64_t P3_MIN_ROWS = 512;  // two items' worth of rows per kv head; below, 64-row tiles spread over more SMs
 static int fa_prefill_route(const FaParams &p, bool kv16) {
@@ -1690,12 +1698,11 @@ static int fa_prefill_route(const FaParams &p, bool kv16) {
     static const bool off = [] { const char *e = diag_env("B200_FA_NO_TCGEN05"); return e && *e == '1'; }();
     if (off) return PF_NONE;
     const uint64_t rows = (uint64_t)p.lq * p.group;
-    KvDims k, v;
     cuuint64_t qs[4];
     static const bool no_tma = [] { const char *e = diag_env("B200_FA_NO_TMA"); return e && *e == '1'; }();
     if (!no_tma && rows >= P3_MIN_ROWS && p.d <= 128 && (reinterpret_cast<uintptr_t>(p.o) & 15) == 0 && p.lk < (1u << 31) && rows < (1ull << 31) &&
         (rows + P3_ROWS - 1) / P3_ROWS * p.b * p.hkv < (1ull << 31) && q_strides(p, qs) &&
-        kv_dims_of(p, &k, &v))
+        fa_kv_maps(p, false, 0, nullptr, nullptr, nullptr))
         return PF_TMA;
     // tensors that no map describes: 16-byte chunks, head dim 128
     if (p.d != PF_D || rows < 4 * PF_BM) return PF_NONE;  // short chunks and decode stay on the mma.sync kernel
@@ -1727,11 +1734,10 @@ static int fa_prefill_tma_launch(const FaParams &p, cudaStream_t stream) {
     static thread_local bool done[16] = {};
     const int rc = pf_opt_in(fa_prefill_tma_kernel<HD, BF16>, P3<HD>::SMEM, done);
     if (rc) return rc;
-    KvDims k, v;
     CUtensorMap tm_k, tm_v, tm_q;
-    if (!kv_dims_of(p, &k, &v) || !make_kv_map(&tm_k, k, p.k, BF16, p.d) || !make_kv_map(&tm_v, v, p.v, BF16, p.d) || !make_q_map(&tm_q, p, BF16))
-        return set_error(B200_ERR_LAUNCH, "flash_attn (tcgen05 tiles): the driver refuses a tensor map");
     P3Grid gr;
+    if (!fa_kv_maps(p, BF16, P3_BN, &tm_k, &tm_v, &gr.tm_order) || !make_q_map(&tm_q, p, BF16))
+        return set_error(B200_ERR_LAUNCH, "flash_attn (tcgen05 tiles): the driver refuses a tensor map");
     const uint64_t rows = (uint64_t)p.lq * p.group, pair_bytes = std::max<uint64_t>((uint64_t)p.lk * p.d * 4, 1);
     gr.tiles = (uint32_t)((rows + P3_ROWS - 1) / P3_ROWS);
     gr.pairs = p.b * p.hkv;
@@ -1739,7 +1745,6 @@ static int fa_prefill_tma_launch(const FaParams &p, cudaStream_t stream) {
     gr.items = gr.tiles * gr.pairs;
     gr.group_log2 = 0;
     while ((1u << gr.group_log2) < p.group) ++gr.group_log2;
-    gr.tm_order = k.order | (v.order << 8);
     fa_prefill_tma_kernel<HD, BF16><<<gr.items, P3_THREADS, P3<HD>::SMEM, stream>>>(p, tm_k, tm_v, tm_q, gr);
     return check_launch("flash_attn (tcgen05 tiles)");
 }
@@ -1781,9 +1786,9 @@ int decode_wait_clear();
 extern "C" int b200_device_wait_status(void) {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_wait_failed, sizeof(int)) != cudaSuccess) return -1;
-    const int d = b200::decode_wait_status();
-    if (d < 0) return -1;
-    return (v != 0 || d != 0) ? 1 : 0;
+    const int d = b200::decode_wait_status(), f = b200::fa_decode_wait_status();
+    if (d < 0 || f < 0) return -1;
+    return (v != 0 || d != 0 || f != 0) ? 1 : 0;
 }
 
 // B200_ERR_DEVICE_WAIT when a bounded device-side wait has run out on the current device since the library was loaded
@@ -1794,7 +1799,7 @@ extern "C" int b200_device_wait_check(int clear) {
     if (st < 0) return set_error(B200_ERR_LAUNCH, "device_wait_check: the flag cannot be read (%s)", cudaGetErrorString(cudaGetLastError()));
     if (clear) {
         const int zero = 0;
-        if (cudaMemcpyToSymbol(g_wait_failed, &zero, sizeof(int)) != cudaSuccess || b200::decode_wait_clear() != 0)
+        if (cudaMemcpyToSymbol(g_wait_failed, &zero, sizeof(int)) != cudaSuccess || b200::decode_wait_clear() != 0 || b200::fa_decode_wait_clear() != 0)
             return set_error(B200_ERR_LAUNCH, "device_wait_check: the flag cannot be cleared");
     }
     if (st) return set_error(B200_ERR_DEVICE_WAIT, "a bounded device-side wait ran out: the outputs of the call that met it are incomplete");

@@ -405,6 +405,22 @@ def test_tensor_copy_tiles_at_their_edges(P, lq, lk, b, hq, hkv, d, wl, wr, dt):
     assert (out.double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dt] * want.norm()
 
 
+# decode by tensor copies: tiles of 16 and 32 keys over four warps, one split and many, 1 to 16 rows, head dims at and between
+# the buckets, windows that end a split's range, keys of another type than the queries
+@pytest.mark.parametrize("b,lq,lk,hq,hkv,d,wl,wr", [
+    (1, 1, 1, 1, 1, 64, -1, 0), (2, 1, 16, 4, 4, 128, -1, 0), (1, 1, 129, 16, 1, 128, -1, -1), (3, 2, 63, 8, 2, 72, -1, 0), (1, 16, 500, 1, 1, 8, 40, 0),
+    (2, 3, 3001, 10, 2, 64, 100, 2), (40, 1, 2000, 16, 4, 128, -1, 0), (1, 5, 3, 2, 2, 128, -1, 0)])
+@pytest.mark.parametrize("qdt,dt", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float16), (torch.float32, torch.bfloat16)])
+def test_decode_by_tensor_copies_at_its_edges(P, b, lq, lk, hq, hkv, d, wl, wr, qdt, dt):
+    g = torch.Generator(device="cuda:0").manual_seed(lk)
+    q = torch.randn((b, lq, hq, d), generator=g, device="cuda:0").to(qdt)
+    k, v = (torch.randn((b, lk, hkv, d), generator=g, device="cuda:0", dtype=dt) for _ in range(2))
+    out = P.flash_attn.flash_attn_with_config(q, k, v, cfg_of(P, d, wl, wr))
+    want = torch.stack([_plain(*x, 1.0 / np.sqrt(d), wl, wr) for x in zip(q.to(dt), k, v)])
+    # weights and output are each rounded once: half an ulp each at most, in the 2-norm
+    assert (out.double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dt] * want.norm()
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (2, 2, 64), (4, 4, 96)])
 def test_varlen_rows_beside_infinities(P, hq, hkv, d):
     """The last key tile of a sequence reaches into the next one: what is there, infinities and NaN included, has no part in it."""
