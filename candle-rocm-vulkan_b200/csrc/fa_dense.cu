@@ -493,6 +493,7 @@ struct FaPlan {
     size_t smem, ws_bytes, off_lse;
     bool bf16;  // mma operand type
     bool decode_tma;  // fa_decode_tma_kernel takes the call
+    bool prefill;     // the tiles of fa_prefill_sm100.cu do
 };
 
 // keys before every block of a paged call, and their total behind them: one block of threads, a running sum over
@@ -583,8 +584,8 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false) {
         }
     }
     p.n_splits = 1;
-    // long chunks run as whole tiles on the tcgen05 kernel and are never split along the keys
-    if (paged || !fa_prefill_sm100_supported(p, kv16)) p.n_splits = std::max(splits, 1u);
+    pl.prefill = !paged && !pl.decode_tma && fa_prefill_sm100_supported(p, kv16);
+    p.n_splits = pl.prefill ? fa_prefill_sm100_splits(p, (uint32_t)sms) : std::max(splits, 1u);
     if ((uint64_t)a->b * p.n_splits > 65535) return set_error(B200_ERR_UNSUPPORTED_SHAPE, "flash_attn: batch x splits too large");
     pl.grid = dim3(row_tiles, a->hkv, a->b * p.n_splits);
     const size_t rowb = (a->d <= 64 ? 64 : (a->d <= 128 ? 128 : 256)) * 2 + 16;
@@ -658,6 +659,8 @@ extern "C" int b200_flash_attn(const B200FaArgs *a, b200_stream_t stream_) {
     if (rc) return rc;
     if (a->total_q * a->hq == 0 || a->b == 0) return B200_OK;
     if (!a->q || !a->k || !a->v || !a->o) return set_error(B200_ERR_BAD_ARG, "flash_attn: null pointer");
+    // tcgen05 tiles: key splits are worth a workspace, not a refusal
+    if (pl.prefill && pl.ws_bytes && (!a->workspace || a->workspace_bytes < pl.ws_bytes)) pl.p.n_splits = 1, pl.ws_bytes = 0;
     if (pl.ws_bytes) {
         if (!a->workspace || a->workspace_bytes < pl.ws_bytes)
             return set_error(B200_ERR_WORKSPACE, "flash_attn: workspace of %zu bytes needed, %zu given", pl.ws_bytes,
@@ -667,8 +670,10 @@ extern "C" int b200_flash_attn(const B200FaArgs *a, b200_stream_t stream_) {
     }
     cudaStream_t stream = (cudaStream_t)stream_;
     const bool bf = pl.bf16;
-    // long prefill chunks: tiles on the tcgen05 tensor cores
-    if (fa_prefill_sm100_supported(pl.p, pl.p.kv_kind == 0)) return fa_prefill_sm100_launch(pl.p, bf, stream);
+    if (pl.prefill) {  // tiles on the tcgen05 tensor cores
+        const int prc = fa_prefill_sm100_launch(pl.p, bf, stream);
+        return prc || pl.p.n_splits == 1 ? prc : fa_combine_launch(pl, stream);
+    }
     if (pl.decode_tma) {
         const int drc = fa_decode_tma_launch(pl.p, bf, pl.grid, stream);
         return drc || pl.p.n_splits == 1 ? drc : fa_combine_launch(pl, stream);

@@ -30,6 +30,7 @@ struct FaParams {
 
 // prefill tiles on the 5th generation tensor cores (fa_prefill_sm100.cu)
 bool fa_prefill_sm100_supported(const FaParams &p, bool kv16);
+uint32_t fa_prefill_sm100_splits(const FaParams &p, uint32_t sms);  // key splits (part_o, part_lse, then fa_combine_kernel)
 int fa_prefill_sm100_launch(const FaParams &p, bool bf16, cudaStream_t stream);
 
 // Tensor maps of K and V (boxes of 64 elements x `keys` keys, 128-byte swizzle; past the head dim and past the last key zeros

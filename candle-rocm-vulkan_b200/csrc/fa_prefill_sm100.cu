@@ -992,7 +992,7 @@ struct P3 {
     static_assert(COUNT * 8 <= 464, "barriers");  // then the answer (464), item numbers (480), tensor memory (496), give-up flag (504)
 };
 
-// The grid's work: items = (batch entries x kv heads) x row tiles. The pairs are taken `hpc` at a time (their keys and
+// The grid's work: items = (batch entries x kv heads) x row tiles x key splits (p.n_splits). The pairs are taken `hpc` at a time (their keys and
 // values stay in L2 together), inside such a chunk the row tiles with the most keys first.
 struct P3Grid {
     uint32_t tiles, pairs, hpc, items;
@@ -1001,10 +1001,10 @@ struct P3Grid {
 };
 
 struct P3Item {
-    uint32_t b, hk, row0, R, gl;
+    uint32_t b, hk, row0, R, gl, split;
     uint64_t q0, k0;
     int lq, lk;
-    int t_lo, t_hi;  // the keys that some row of the item sees
+    int t_lo, t_hi;  // the keys that some row of the item sees, within the item's key split
     int ntiles;
 };
 // the keys [lo, hi) that row r sees
@@ -1016,6 +1016,11 @@ __device__ __forceinline__ void p3_range(const FaParams &p, const P3Item &it, ui
 }
 // work item n; false when it has no rows
 __device__ __forceinline__ bool p3_item(const FaParams &p, const P3Grid &gr, uint32_t n, P3Item &it) {
+    it.split = 0;
+    if (p.n_splits > 1) {
+        it.split = n % p.n_splits;
+        n /= p.n_splits;
+    }
     const uint32_t per = gr.hpc * gr.tiles, chunk = n / per, first = chunk * gr.hpc, width = min(gr.hpc, gr.pairs - first), m = n - chunk * per;
     const uint32_t rank = m / width, pair = first + (m - rank * width);
     it.b = pair / p.hkv;
@@ -1039,6 +1044,12 @@ __device__ __forceinline__ bool p3_item(const FaParams &p, const P3Grid &gr, uin
     p3_range(p, it, min(it.row0 + P3_ROWS, it.R) - 1, tmp, it.t_hi);
     it.t_hi = max(it.t_hi, it.t_lo);
     it.ntiles = (it.t_hi - it.t_lo + P3_BN - 1) / P3_BN;
+    if (p.n_splits > 1) {  // whole tiles
+        const int per = (it.ntiles + (int)p.n_splits - 1) / (int)p.n_splits, first = min((int)it.split * per, it.ntiles);
+        it.ntiles = min(per, it.ntiles - first);
+        it.t_lo += first * P3_BN;
+        it.t_hi = max(min(it.t_hi, it.t_lo + it.ntiles * P3_BN), it.t_lo);
+    }
     return true;
 }
 // the key tiles [t0, t1) of the item that some row of group g sees (empty: t0 == t1)
@@ -1049,6 +1060,8 @@ __device__ __forceinline__ void p3_group(const FaParams &p, const P3Item &it, in
     int lo, hi, tmp;
     p3_range(p, it, first, lo, tmp);
     p3_range(p, it, min(first + PF_BM, it.R) - 1, tmp, hi);
+    lo = max(lo, it.t_lo);
+    hi = min(hi, it.t_hi);
     if (hi <= lo) return;
     t0 = (lo - it.t_lo) / P3_BN;
     t1 = (hi - it.t_lo + P3_BN - 1) / P3_BN;
@@ -1411,12 +1424,12 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                 if (r < it.R) {
                     p3_range(p, it, r, lo, hi);
                     r_lo = lo - it.t_lo;
-                    r_hi = hi - it.t_lo;
+                    r_hi = min(hi, it.t_hi) - it.t_lo;
                 }
                 p3_range(p, it, min(g_row0 + PF_BM, it.R) - 1, lo, tmp);
                 p3_range(p, it, g_row0, tmp, hi);
                 lomax = lo - it.t_lo;
-                himin = g_row0 + PF_BM > it.R ? -1 : hi - it.t_lo;
+                himin = g_row0 + PF_BM > it.R ? -1 : min(hi, it.t_hi) - it.t_lo;
             }
             return true;
         };
@@ -1542,6 +1555,38 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
             // 64 elements of the warp's 32 rows at a time through shared memory, so that eight lanes write 128 bytes of a row
             // (a lane that writes its own row leaves every store in 32 lines)
             uint8_t *const stage = smem + C::SM_OUT + warp * 4096;
+            if (p.n_splits > 1) {
+                // a key split: f32 rows and the logarithm of the row's sum for fa_combine_kernel, 32 elements at a time
+                const uint64_t part = (uint64_t)cur.split * p.rows_total;
+                auto out_row = [&](uint32_t rr) { return (cur.q0 + (rr >> cur.gl)) * p.hq + (cur.hk << cur.gl) + (rr & ((1u << cur.gl) - 1)); };
+                const uint32_t r = cur.row0 + g * PF_BM + w4 * 32 + lane;
+                if (r < cur.R) p.part_lse[part + out_row(r)] = l > 0.0f ? mref * 0.6931471805599453f + logf(l) : -INFINITY;
+#pragma unroll 1
+                for (uint32_t c0 = 0; c0 < p.d; c0 += 32) {
+                    uint32_t o[32];
+                    if (any) {
+                        tc_ld32(o_col + c0, o);
+                        tc_wait_ld_for(o);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = 0u;
+                    }
+#pragma unroll
+                    for (int v4 = 0; v4 < 8; ++v4)
+                        *reinterpret_cast<float4 *>(stage + lane * 128 + ((v4 ^ (lane & 7)) << 4)) =
+                            make_float4(u2f(o[4 * v4]) * inv, u2f(o[4 * v4 + 1]) * inv, u2f(o[4 * v4 + 2]) * inv, u2f(o[4 * v4 + 3]) * inv);
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t row = i * 4 + (lane >> 3), c4 = lane & 7, rr = cur.row0 + g * PF_BM + w4 * 32 + row;
+                        const float4 w = *reinterpret_cast<const float4 *>(stage + row * 128 + ((c4 ^ (row & 7)) << 4));
+                        if (rr < cur.R && c0 + 4 * c4 < p.d) *reinterpret_cast<float4 *>(p.part_o + (part + out_row(rr)) * p.d + c0 + 4 * c4) = w;
+                    }
+                    __syncwarp();
+                }
+                tc_fence_before();
+                continue;
+            }
 #pragma unroll 1
             for (int hf = 0; hf < C::HALVES; ++hf) {
 #pragma unroll
@@ -1689,9 +1734,13 @@ bool fa_kv_maps(const FaParams &p, bool bf16, uint32_t keys, CUtensorMap *tm_k, 
 }
 
 enum { PF_NONE = 0, PF_ROWS128, PF_ROWS256, PF_TMA };
-constexpr uint64_t P3_MIN_ROWS = 512;  // two items' worth of rows per kv head; below, 64-row tiles spread over more SMs
+// More rows than a decode call has (up to 16 rows the keys are read by warps of their own: fa_decode_tma.cu). With 17 to 511 rows
+// a block's products run partly on rows that do not exist, and still beat the 64-row tiles of mma.sync: 60 tokens, 32 / 8 heads of
+// 128: 26 -> 10 us; 8 x 200 tokens, 16 heads of 128: 65 -> 13; 16 x 400 tokens, 16 heads of 64: 188 -> 38. One item per SM bounds the
+// small ones, so few items are split along the keys (fa_plan).
+constexpr uint64_t P3_MIN_ROWS = 17;
 static int fa_prefill_route(const FaParams &p, bool kv16) {
-    if (!kv16 || p.kv_kind != 0 || p.n_splits != 1) return PF_NONE;
+    if (!kv16 || p.kv_kind != 0) return PF_NONE;
     if (p.q_dtype != B200_F16 && p.q_dtype != B200_BF16) return PF_NONE;
     if (p.softcap > 0.0f || p.alibi != nullptr) return PF_NONE;
     if (!(p.scale * p.kd > 0.0f)) return PF_NONE;  // the row maximum is taken before the scale is applied
@@ -1715,6 +1764,14 @@ static int fa_prefill_route(const FaParams &p, bool kv16) {
     return rows >= 1024 ? PF_ROWS256 : PF_ROWS128;
 }
 bool fa_prefill_sm100_supported(const FaParams &p, bool kv16) { return fa_prefill_route(p, kv16) != PF_NONE; }
+uint32_t fa_prefill_sm100_splits(const FaParams &p, uint32_t sms) {
+    if (p.varlen || fa_prefill_route(p, p.kv_kind == 0) != PF_TMA) return 1;
+    // Where the items leave SMs idle: as many key splits as give each SM one, of at least four key tiles (about 8 us; a partial
+    // result and the combine grid cost 4)
+    // 256 query tokens over 8192 keys, 32 / 8 heads of 128: 145 -> 48 us; 300 over 12 000, 8 / 1 heads: 392 -> 30; 8 tokens x 2 over 4000 keys: 59 -> 24.
+    const uint64_t items = ((uint64_t)p.lq * p.group + P3_ROWS - 1) / P3_ROWS * p.b * p.hkv, keys = p.wl >= 0 ? std::min<uint64_t>(p.lk, (uint64_t)p.wl + P3_ROWS) : p.lk;
+    return (uint32_t)std::max<uint64_t>(std::min<uint64_t>(std::min<uint64_t>(sms / std::max<uint64_t>(items, 1), keys / (4 * P3_BN)), 64), 1);
+}
 
 // shared memory opt-in, once per kernel, thread and device
 template <typename K>
@@ -1742,7 +1799,7 @@ static int fa_prefill_tma_launch(const FaParams &p, cudaStream_t stream) {
     gr.tiles = (uint32_t)((rows + P3_ROWS - 1) / P3_ROWS);
     gr.pairs = p.b * p.hkv;
     gr.hpc = (uint32_t)std::min<uint64_t>(std::max<uint64_t>((64ull << 20) / pair_bytes, 1), gr.pairs);
-    gr.items = gr.tiles * gr.pairs;
+    gr.items = gr.tiles * gr.pairs * p.n_splits;
     gr.group_log2 = 0;
     while ((1u << gr.group_log2) < p.group) ++gr.group_log2;
     fa_prefill_tma_kernel<HD, BF16><<<gr.items, P3_THREADS, P3<HD>::SMEM, stream>>>(p, tm_k, tm_v, tm_q, gr);

@@ -421,6 +421,27 @@ def test_decode_by_tensor_copies_at_its_edges(P, b, lq, lk, hq, hkv, d, wl, wr, 
     assert (out.double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dt] * want.norm()
 
 
+# few work items: split along the keys (whole tiles, a last split that is short or empty, windows that leave splits without keys
+# for some rows, 17 rows and more), and the same call without a workspace, which goes unsplit
+@pytest.mark.parametrize("b,lq,lk,hq,hkv,d,wl,wr", [(1, 17, 2000, 1, 1, 64, -1, 0), (1, 33, 5000, 8, 1, 128, -1, 0), (2, 300, 4111, 8, 2, 72, 2500, 50),
+                                                    (1, 64, 6500, 32, 8, 128, -1, -1), (1, 1200, 3100, 1, 1, 128, -1, 0)])
+def test_key_splits_of_the_tensor_copy_tiles(P, b, lq, lk, hq, hkv, d, wl, wr):
+    import ctypes
+    g = torch.Generator(device="cuda:0").manual_seed(lk)
+    q, k, v = (torch.randn((b, n, h, d), generator=g, device="cuda:0", dtype=torch.bfloat16) for n, h in ((lq, hq), (lk, hkv), (lk, hkv)))
+    F, A = P.flash_attn, P._abi
+    a, out, keep = F._fa_args(q, k, v, cfg_of(P, d, wl, wr))
+    assert a.workspace_bytes > 0  # the splits' partial results
+    want = torch.stack([_plain(*x, 1.0 / np.sqrt(d), wl, wr) for x in zip(q, k, v)])
+    for bare in (False, True):
+        if bare:
+            a.workspace, a.workspace_bytes = None, 0
+        out.fill_(float("nan"))
+        A.check(A.lib().b200_flash_attn(ctypes.byref(a), 0))
+        torch.cuda.synchronize()
+        assert (out.double() - want).norm() <= 2.0 ** -8 * want.norm(), bare
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (2, 2, 64), (4, 4, 96)])
 def test_varlen_rows_beside_infinities(P, hq, hkv, d):
     """The last key tile of a sequence reaches into the next one: what is there, infinities and NaN included, has no part in it."""
