@@ -156,8 +156,8 @@ def lib():
         l.b200_tq_rotate.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint64, C.c_uint32, C.c_int, C.c_void_p]
         l.b200_tq_quantize.argtypes = [C.POINTER(TqQuantArgs), C.c_void_p]
         l.b200_tq_dequantize.argtypes = [C.POINTER(TqDequantArgs), C.c_void_p]
-        l.b200_kv_append.argtypes = [C.POINTER(KvAppendArgs), C.c_void_p]
-        l.b200_kv_unpack.argtypes = [C.POINTER(KvUnpackArgs), C.c_void_p]
+        l.b200_kv_append.argtypes = [C.c_void_p, C.c_void_p]  # a KvAppendArgs by reference, or its bytes
+        l.b200_kv_unpack.argtypes = [C.c_void_p, C.c_void_p]
         l.b200_tq_attention_workspace_bytes.argtypes = [C.POINTER(TqAttnArgs)]
         l.b200_tq_attention_workspace_bytes.restype = C.c_size_t
         l.b200_tq_attention.argtypes = [C.POINTER(TqAttnArgs), C.c_void_p]

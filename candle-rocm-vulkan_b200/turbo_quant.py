@@ -9,6 +9,7 @@ the C ABI (include/b200attn.h). There is no CPU path: tensors must live on a CUD
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from dataclasses import dataclass, field
 from typing import Optional, Tuple
 
@@ -72,8 +73,23 @@ def _dtype_id(t: torch.Tensor) -> int:
         raise ValueError(f"unsupported dtype {t.dtype} (f32, f16, bf16)") from None
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream's handle (without the Python object of torch.cuda.current_stream, a microsecond and a half)."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index if device.index is not None else torch.cuda.current_device())
+
+
+# The argument structures of the calls of a decode step, and of rows unpacked, as one `struct.pack` each, in the order of the header (0P: the
+# alignment of a nested structure): a third of the time that filling the ctypes structures field by field takes.
+_SIDE = "0PiiPiP"
+_APPEND_ARGS = struct.Struct("@PP3Q3QPP3Q3QPiIIIIi" + _SIDE + _SIDE + "IPII0P")
+_ATTN_ARGS = struct.Struct("@PPii3Q3QPP3Q3QPIPIIIIII" + _SIDE + _SIDE + "ffiiPIiPNPIiI0P")
+_UNPACK_ARGS = struct.Struct("@PP3Q3QPPIIIIiI" + _SIDE + _SIDE + "0P")
+assert _UNPACK_ARGS.size == C.sizeof(A.KvUnpackArgs) and _APPEND_ARGS.size == C.sizeof(A.KvAppendArgs) and _ATTN_ARGS.size == C.sizeof(A.TqAttnArgs)
 
 
 def _need_cuda(t: torch.Tensor, what: str):
@@ -162,6 +178,11 @@ class TurboQuantizer:
     def row_words(self) -> int:
         return self.layout.row_words
 
+    def side_fields(self):
+        """The fields of `side()`, for `struct.pack`."""
+        return (self.format.mode, self.format.bits, self.tab.data_ptr(), A.ROT_HADAMARD if self.rotation == "hadamard" else A.ROT_NONE,
+                self.signs.data_ptr() if self.signs is not None else 0)
+
     def side(self) -> A.QuantSide:
         return A.QuantSide(self.format.mode, self.format.bits, self.tab.data_ptr(),
                            A.ROT_HADAMARD if self.rotation == "hadamard" else A.ROT_NONE,
@@ -234,11 +255,15 @@ class TurboQuantizer:
             return self.quantize_rotated_rows(self.rotate(x))
         # the fused rotation comes with the append, which takes two tensors: one half of the rows each (an odd number of
         # rows: both write the same bytes of the middle one)
-        x = x.view(1, 1, rows, d)
-        out = torch.empty((1, 1, rows, self.layout.row_words), dtype=torch.int32, device=x.device)
-        half = (rows + 1) // 2
-        _kv_append(x[:, :, :half], x[:, :, rows - half:], out[:, :, :half], out[:, :, rows - half:], self, self, 0)
-        return out.view(rows, self.layout.row_words)
+        if x.stride(1) != 1:
+            x = x.contiguous()
+        words, step, half, side = self.layout.row_words, x.stride(0), (rows + 1) // 2, self.side_fields()
+        out = torch.empty((rows, words), dtype=torch.int32, device=x.device)
+        src, dst = x.data_ptr(), out.data_ptr()
+        A.check(A.lib().b200_kv_append(_APPEND_ARGS.pack(
+            src, src + (rows - half) * step * x.element_size(), 0, 0, step, 0, 0, step, dst, dst + (rows - half) * words * 4,
+            0, 0, words, 0, 0, words, 0, 0, 1, 1, half, d, _dtype_id(x), *side, *side, half, 0, 0, 0), _stream(x.device)))
+        return out
 
     def dequantize_rows(self, data: torch.Tensor) -> torch.Tensor:
         """`(rows, row_words)` -> `(rows, dim)` f32 in the original domain (turbo_quant.rs:250-270)."""
@@ -291,15 +316,15 @@ def _kv_append(k, v, k_cache, v_cache, kq: TurboQuantizer, vq: TurboQuantizer, p
     if v.stride(3) != 1:
         v = v.contiguous()
     pos_t = pos if isinstance(pos, torch.Tensor) else None
-    args = A.KvAppendArgs(
-        k.data_ptr(), v.data_ptr(), A.u64x3(*k.stride()[:3]), A.u64x3(*v.stride()[:3]),
-        k_cache.data_ptr(), v_cache.data_ptr(), A.u64x3(*k_cache.stride()[:3]), A.u64x3(*v_cache.stride()[:3]),
-        pos_t.data_ptr() if pos_t is not None else None, int(pos_add) if pos_t is not None else int(pos) + int(pos_add),
-        b, h, t, d, _dtype_id(k), kq.side(), vq.side(), min(k_cache.shape[2], v_cache.shape[2]),
-        status.data_ptr() if status is not None else None,
+    args = _APPEND_ARGS.pack(
+        k.data_ptr(), v.data_ptr(), *k.stride()[:3], *v.stride()[:3], k_cache.data_ptr(), v_cache.data_ptr(),
+        *k_cache.stride()[:3], *v_cache.stride()[:3],
+        pos_t.data_ptr() if pos_t is not None else 0, int(pos_add) if pos_t is not None else int(pos) + int(pos_add),
+        b, h, t, d, _dtype_id(k), *kq.side_fields(), *vq.side_fields(), min(k_cache.shape[2], v_cache.shape[2]),
+        status.data_ptr() if status is not None else 0,
         # B200_KV_AFTER_PREV: the stream's previous kernel neither reads the rows written here nor writes k, v or pos
         A.KV_AFTER_PREV if after_prev else 0, 0)
-    A.check(A.lib().b200_kv_append(C.byref(args), _stream(k.device)))
+    A.check(A.lib().b200_kv_append(args, _stream(k.device)))
 
 
 def _kv_unpack(k_rows, v_rows, kq: TurboQuantizer, vq: Optional[TurboQuantizer], t: int, dtype):
@@ -307,10 +332,11 @@ def _kv_unpack(k_rows, v_rows, kq: TurboQuantizer, vq: Optional[TurboQuantizer],
     b, h = k_rows.shape[:2]
     k = torch.empty((b, h, t, kq.dim), dtype=dtype, device=k_rows.device)
     v = torch.empty_like(k) if v_rows is not None else None
-    args = A.KvUnpackArgs(k_rows.data_ptr(), v_rows.data_ptr() if v is not None else None, A.u64x3(*k_rows.stride()[:3]),
-                          A.u64x3(*v_rows.stride()[:3]) if v is not None else A.u64x3(), k.data_ptr(), v.data_ptr() if v is not None else None,
-                          b, h, t, kq.dim, _dtype_id(k), 0, kq.side(), (vq or kq).side())
-    A.check(A.lib().b200_kv_unpack(C.byref(args), _stream(k.device)))
+    none = (0, 0, 0)
+    args = _UNPACK_ARGS.pack(k_rows.data_ptr(), v_rows.data_ptr() if v is not None else 0, *k_rows.stride()[:3],
+                             *(v_rows.stride()[:3] if v is not None else none), k.data_ptr(), v.data_ptr() if v is not None else 0,
+                             b, h, t, kq.dim, _dtype_id(k), 0, *kq.side_fields(), *(vq or kq).side_fields())
+    A.check(A.lib().b200_kv_unpack(args, _stream(k.device)))
     return k, v
 
 
@@ -320,7 +346,7 @@ _WORKSPACES = {}
 def _workspace(device, nbytes: int) -> torch.Tensor:
     """One growing scratch buffer per (device, stream): calls on one stream are ordered, so they
     can share it; the reference allocates the split buffers per call (accel.rs:190-199)."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
+    key = (device, _stream(device))
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
@@ -486,7 +512,7 @@ class PackedAttention:
 
     def run(self) -> torch.Tensor:
         self._dense.before()
-        rc = self._fn(self._ref, torch.cuda.current_stream(self.device).cuda_stream)
+        rc = self._fn(self._ref, _stream(self.device))
         if rc:
             A.check(rc)
         self._dense.after()
@@ -589,7 +615,7 @@ class PackedBlocksAttention:
 
     def run(self) -> torch.Tensor:
         self._dense.before()
-        rc = A.lib().b200_tq_attention(self._ref, torch.cuda.current_stream(self.device).cuda_stream)
+        rc = A.lib().b200_tq_attention(self._ref, _stream(self.device))
         if rc:
             A.check(rc)
         self._dense.after()
@@ -714,4 +740,30 @@ class TurboKvCache:
             from .flash_attn import flash_attn_bhsd
             k, v = self.keys_values()
             return flash_attn_bhsd(q, k.to(q.dtype), v.to(q.dtype), cfg)
-        return attention_packed(q, self.k, self.v, self.len, self.kq, self.vq, cfg)
+        kq, vq = self.kq, self.vq
+        if cfg.alibi_slopes is not None or kq.qjl is not None or kq.rotation == "dense" or vq.rotation == "dense":
+            return attention_packed(q, self.k, self.v, self.len, kq, vq, cfg)
+        # the same call as attention_packed, without the object of a prepared one
+        k, v, lk = self.k, self.v, self.len
+        (kb, _, kcap, kw), (vb, vh, vcap, vw) = k.shape, v.shape
+        if (kb != b or vb != b or vh != hkv or lk == 0 or min(kcap, vcap) < lk or d != self.dim or kw < kq.row_words() or vw < vq.row_words()
+                or k.stride(3) != 1 or v.stride(3) != 1):
+            return attention_packed(q, k, v, lk, kq, vq, cfg)  # says what does not match
+        _need_cuda(q, "q")
+        if q.stride(3) != 1:
+            q = q.contiguous()
+        out = torch.empty((b, hq, lq, d), dtype=q.dtype, device=q.device)
+        dt, wl, wr = _dtype_id(q), *cfg.window_i32()
+        args = A.TqAttnArgs.from_buffer_copy(_ATTN_ARGS.pack(
+            q.data_ptr(), out.data_ptr(), dt, dt, *q.stride()[:3], *out.stride()[:3], k.data_ptr(), v.data_ptr(), *k.stride()[:3], *v.stride()[:3],
+            0, 0, 0, b, lq, lk, hq, hkv, d, *kq.side_fields(), *vq.side_fields(), cfg.softmax_scale, cfg.softcap or 0.0, wl, wr, 0, 0, cfg.splits,
+            0, 0, 0, 0, 0, 0))
+        lib, ref = A.lib(), C.byref(args)
+        nbytes = lib.b200_tq_attention_workspace_bytes(ref)
+        if nbytes:
+            ws = _workspace(q.device, nbytes)
+            args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
+        rc = lib.b200_tq_attention(ref, _stream(q.device))  # nbytes 0: reports why the call cannot be planned
+        if rc:
+            A.check(rc)
+        return out

@@ -101,6 +101,32 @@ def test_python_constants_mirror_the_header(pkg):
     assert seen >= 10
 
 
+def test_packed_argument_structures_mirror_the_ctypes_ones(pkg):
+    """The two calls of a decode step pack their arguments with `struct`: every field lands where ctypes has it."""
+    A, T = pkg._abi, pkg.turbo_quant
+
+    def flat(cls):
+        for name, kind in cls._fields_:
+            if issubclass(kind, C.Structure):
+                yield from ((f"{name}.{n}", k, c) for n, k, c in flat(kind))
+            else:
+                yield name, kind, getattr(kind, "_length_", 1)
+
+    def at(obj, path):
+        for n in path.split("."):
+            obj = getattr(obj, n)
+        return obj
+
+    for packer, cls in ((T._APPEND_ARGS, A.KvAppendArgs), (T._UNPACK_ARGS, A.KvUnpackArgs), (T._ATTN_ARGS, A.TqAttnArgs)):
+        fields = list(flat(cls))
+        values = iter(range(1, 1000))
+        given = [[next(values) for _ in range(n)] for _, _, n in fields]
+        obj = cls.from_buffer_copy(packer.pack(*(x for g in given for x in g)))
+        for (name, _, n), want in zip(fields, given):
+            got = at(obj, name)
+            assert (list(got) if n > 1 else [got]) == want, name
+
+
 def test_row_layouts_and_errors(pkg, oracle):
     A = pkg._abi
     for mode in (0, 2, 3, 4, 5):
