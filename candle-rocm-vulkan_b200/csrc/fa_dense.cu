@@ -487,6 +487,44 @@ __global__ void __launch_bounds__(128) fa_combine_kernel(const float *__restrict
     }
 }
 
+// q, k and v of other types as 16-bit tensors (token-major, contiguous) for the tcgen05 tiles: f32 rounded to nearest and E4M3
+// widened, as fa_dense_kernel does on the way into shared memory. One launch: grid.y = q, k, v; eight elements per thread.
+struct CastSide {
+    const void *src;
+    uint16_t *dst;
+    uint64_t s_b, s_s, s_h;  // elements
+    uint32_t l, h, kind;     // kind as FaParams::kv_kind
+};
+struct CastParams {
+    CastSide side[3];
+    uint32_t d8;
+};
+template <bool BF16>
+__global__ void __launch_bounds__(256) fa_cast_kernel(const CastParams p, uint32_t b) {
+    const CastSide &c = p.side[blockIdx.y];
+    const uint64_t n = (uint64_t)b * c.l * c.h * p.d8;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t row = i / p.d8, tok = row / c.h;
+        const uint32_t e = (uint32_t)(i - row * p.d8) * 8, h = (uint32_t)(row - tok * c.h), t = (uint32_t)(tok % c.l);
+        const uint64_t at = tok / c.l * c.s_b + t * c.s_s + h * c.s_h + e;
+        uint32_t w[4];
+        if (c.kind == 2) {
+            const float *s = reinterpret_cast<const float *>(c.src) + at;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = pack2<BF16>(s[2 * k], s[2 * k + 1]);
+        } else if (c.kind == 1) {
+            const uint8_t *s = reinterpret_cast<const uint8_t *>(c.src) + at;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = pack2<BF16>(e4m3_to_f(s[2 * k]), e4m3_to_f(s[2 * k + 1]));
+        } else {
+            const uint16_t *s = reinterpret_cast<const uint16_t *>(c.src) + at;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = s[2 * k] | (uint32_t)s[2 * k + 1] << 16;
+        }
+        *reinterpret_cast<uint4 *>(c.dst + i * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
 struct FaPlan {
     FaParams p;
     dim3 grid;
@@ -494,6 +532,8 @@ struct FaPlan {
     bool bf16;  // mma operand type
     bool decode_tma;  // fa_decode_tma_kernel takes the call
     bool prefill;     // the tiles of fa_prefill_sm100.cu do
+    bool cast;        // they do, over 16-bit copies of q, k and v in the workspace (at cast_off)
+    size_t cast_off[3];
 };
 
 // keys before every block of a paged call, and their total behind them: one block of threads, a running sum over
@@ -519,7 +559,18 @@ __global__ void __launch_bounds__(256) fa_page_prefix_kernel(const B200Page *__r
     if (threadIdx.x == 0) pg_keys[n_pages] = base;
 }
 
-static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false) {
+// the call over 16-bit copies of its tensors
+static void fa_as_copies(FaParams &p, bool bf16, char *q, char *k, char *v, int out_dtype) {
+    p.q = q, p.k = k, p.v = v;
+    p.q_sh = p.k_sh = p.v_sh = p.d;
+    p.q_ss = (uint64_t)p.hq * p.d, p.k_ss = p.v_ss = (uint64_t)p.hkv * p.d;
+    p.q_sb = p.q_ss * p.lq, p.k_sb = p.v_sb = p.k_ss * p.lk;
+    p.q_dtype = bf16 ? B200_BF16 : B200_F16;
+    p.kv_kind = 0;
+    p.o_f32 = out_dtype == B200_F32;
+}
+
+static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false, bool may_copy = true) {
     if (!a) return set_error(B200_ERR_BAD_ARG, "flash_attn: null args");
     if (a->hkv == 0 || a->hq % a->hkv != 0)
         return set_error(B200_ERR_BAD_ARG, "flash-attn: %u query heads are not a multiple of %u kv heads", a->hq, a->hkv);
@@ -585,7 +636,21 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false) {
     }
     p.n_splits = 1;
     pl.prefill = !paged && !pl.decode_tma && fa_prefill_sm100_supported(p, kv16);
-    p.n_splits = pl.prefill ? fa_prefill_sm100_splits(p, (uint32_t)sms) : std::max(splits, 1u);
+    // f32 tensors and E4M3 keys: rounded (widened) once into the workspace, then the same tiles. From 64 rows on, where the products
+    // weigh more than the copy; up to 256 MB of copies. f32, us, before and now: 8 x 1000 tokens, 16 heads of 64, 478 -> 81; 2 x 2048, 32 / 8
+    // heads of 128, 1293 -> 113; 64 tokens over 4000 keys, 4 heads, 68 -> 29.
+    pl.cast = false;
+    const size_t copies = ((size_t)a->b * a->lq * a->hq + 2 * (size_t)a->b * a->lk * a->hkv) * a->d * 2 + 768;
+    if (may_copy && !paged && !pl.decode_tma && !pl.prefill && !a->varlen && rows >= 64 && a->d <= 128 && copies <= (256u << 20) && a->b && a->lk &&
+        (a->q_dtype == B200_F32 || fp8)) {
+        FaParams c = pl.p;
+        fa_as_copies(c, pl.bf16, reinterpret_cast<char *>(1024), reinterpret_cast<char *>(1024), reinterpret_cast<char *>(1024), a->q_dtype);
+        pl.cast = fa_prefill_sm100_supported(c, true);
+        if (pl.cast) {
+            p.n_splits = fa_prefill_sm100_splits(c, (uint32_t)sms);
+        }
+    }
+    if (!pl.cast) p.n_splits = pl.prefill ? fa_prefill_sm100_splits(p, (uint32_t)sms) : std::max(splits, 1u);
     if ((uint64_t)a->b * p.n_splits > 65535) return set_error(B200_ERR_UNSUPPORTED_SHAPE, "flash_attn: batch x splits too large");
     pl.grid = dim3(row_tiles, a->hkv, a->b * p.n_splits);
     const size_t rowb = (a->d <= 64 ? 64 : (a->d <= 128 ? 128 : 256)) * 2 + 16;
@@ -595,6 +660,16 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false) {
     const size_t part_o = p.n_splits > 1 ? (size_t)p.n_splits * p.rows_total * a->d * 4 : 0;
     pl.off_lse = (part_o + 255) / 256 * 256;
     pl.ws_bytes = p.n_splits > 1 ? pl.off_lse + (size_t)p.n_splits * p.rows_total * 4 : 0;
+    if (pl.cast) {
+        const size_t qn = (size_t)a->b * a->lq * a->hq * a->d * 2, kn = (size_t)a->b * a->lk * a->hkv * a->d * 2;
+        pl.cast_off[0] = (pl.ws_bytes + 255) / 256 * 256;
+        pl.cast_off[1] = pl.cast_off[0] + (qn + 255) / 256 * 256;
+        pl.cast_off[2] = pl.cast_off[1] + (kn + 255) / 256 * 256;
+        pl.ws_bytes = pl.cast_off[2] + kn;
+    }
+    // partial results and copies move in 16-byte pieces: the buffers start at the workspace's first 16-byte boundary (a paged
+    // call's workspace is aligned)
+    if (!paged && pl.ws_bytes) pl.ws_bytes += 16;
     return B200_OK;
 }
 
@@ -659,17 +734,38 @@ extern "C" int b200_flash_attn(const B200FaArgs *a, b200_stream_t stream_) {
     if (rc) return rc;
     if (a->total_q * a->hq == 0 || a->b == 0) return B200_OK;
     if (!a->q || !a->k || !a->v || !a->o) return set_error(B200_ERR_BAD_ARG, "flash_attn: null pointer");
-    // tcgen05 tiles: key splits are worth a workspace, not a refusal
+    // tcgen05 tiles: key splits and copies are worth a workspace, not a refusal
+    if (pl.cast && (!a->workspace || a->workspace_bytes < pl.ws_bytes)) {
+        const int prc = fa_plan(a, pl, false, false);
+        if (prc) return prc;
+    }
     if (pl.prefill && pl.ws_bytes && (!a->workspace || a->workspace_bytes < pl.ws_bytes)) pl.p.n_splits = 1, pl.ws_bytes = 0;
+    char *const ws = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(a->workspace) + 15) & ~(uintptr_t)15);
     if (pl.ws_bytes) {
         if (!a->workspace || a->workspace_bytes < pl.ws_bytes)
             return set_error(B200_ERR_WORKSPACE, "flash_attn: workspace of %zu bytes needed, %zu given", pl.ws_bytes,
                              a->workspace ? a->workspace_bytes : (size_t)0);
-        pl.p.part_o = reinterpret_cast<float *>(a->workspace);
-        pl.p.part_lse = reinterpret_cast<float *>(reinterpret_cast<char *>(a->workspace) + pl.off_lse);
+        pl.p.part_o = reinterpret_cast<float *>(ws);
+        pl.p.part_lse = reinterpret_cast<float *>(ws + pl.off_lse);
     }
     cudaStream_t stream = (cudaStream_t)stream_;
     const bool bf = pl.bf16;
+    if (pl.cast) {
+        FaParams c = pl.p;
+        fa_as_copies(c, bf, ws + pl.cast_off[0], ws + pl.cast_off[1], ws + pl.cast_off[2], a->q_dtype);
+        const FaParams &p = pl.p;
+        const uint32_t qk = a->q_dtype == B200_F32 ? 2u : 0u, kk = (uint32_t)p.kv_kind;
+        const CastParams cp = {{{p.q, (uint16_t *)c.q, p.q_sb, p.q_ss, p.q_sh, p.lq, p.hq, qk},
+                                {p.k, (uint16_t *)c.k, p.k_sb, p.k_ss, p.k_sh, p.lk, p.hkv, kk},
+                                {p.v, (uint16_t *)c.v, p.v_sb, p.v_ss, p.v_sh, p.lk, p.hkv, kk}}, p.d / 8};
+        const uint64_t most = (uint64_t)p.b * std::max<uint64_t>((uint64_t)p.lq * p.hq, (uint64_t)p.lk * p.hkv) * cp.d8;
+        const dim3 grid((unsigned)std::min<uint64_t>((most + 255) / 256, 148ull * 8), 3);
+        if (bf) fa_cast_kernel<true><<<grid, 256, 0, stream>>>(cp, p.b);
+        else fa_cast_kernel<false><<<grid, 256, 0, stream>>>(cp, p.b);
+        int crc = check_launch("flash_attn (copies)");
+        if (!crc) crc = fa_prefill_sm100_launch(c, bf, stream);
+        return crc || c.n_splits == 1 ? crc : fa_combine_launch(pl, stream);
+    }
     if (pl.prefill) {  // tiles on the tcgen05 tensor cores
         const int prc = fa_prefill_sm100_launch(pl.p, bf, stream);
         return prc || pl.p.n_splits == 1 ? prc : fa_combine_launch(pl, stream);

@@ -1555,12 +1555,13 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
             // 64 elements of the warp's 32 rows at a time through shared memory, so that eight lanes write 128 bytes of a row
             // (a lane that writes its own row leaves every store in 32 lines)
             uint8_t *const stage = smem + C::SM_OUT + warp * 4096;
-            if (p.n_splits > 1) {
-                // a key split: f32 rows and the logarithm of the row's sum for fa_combine_kernel, 32 elements at a time
+            if (p.n_splits > 1 || p.o_f32) {
+                // f32 rows, 32 elements at a time: outputs, or a key split with the logarithm of the row's sum for fa_combine_kernel
+                float *const dst = p.n_splits > 1 ? p.part_o : reinterpret_cast<float *>(p.o);
                 const uint64_t part = (uint64_t)cur.split * p.rows_total;
                 auto out_row = [&](uint32_t rr) { return (cur.q0 + (rr >> cur.gl)) * p.hq + (cur.hk << cur.gl) + (rr & ((1u << cur.gl) - 1)); };
                 const uint32_t r = cur.row0 + g * PF_BM + w4 * 32 + lane;
-                if (r < cur.R) p.part_lse[part + out_row(r)] = l > 0.0f ? mref * 0.6931471805599453f + logf(l) : -INFINITY;
+                if (p.n_splits > 1 && r < cur.R) p.part_lse[part + out_row(r)] = l > 0.0f ? mref * 0.6931471805599453f + logf(l) : -INFINITY;
 #pragma unroll 1
                 for (uint32_t c0 = 0; c0 < p.d; c0 += 32) {
                     uint32_t o[32];
@@ -1580,7 +1581,7 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                     for (int i = 0; i < 8; ++i) {
                         const uint32_t row = i * 4 + (lane >> 3), c4 = lane & 7, rr = cur.row0 + g * PF_BM + w4 * 32 + row;
                         const float4 w = *reinterpret_cast<const float4 *>(stage + row * 128 + ((c4 ^ (row & 7)) << 4));
-                        if (rr < cur.R && c0 + 4 * c4 < p.d) *reinterpret_cast<float4 *>(p.part_o + (part + out_row(rr)) * p.d + c0 + 4 * c4) = w;
+                        if (rr < cur.R && c0 + 4 * c4 < p.d) *reinterpret_cast<float4 *>(dst + (part + out_row(rr)) * p.d + c0 + 4 * c4) = w;
                     }
                     __syncwarp();
                 }

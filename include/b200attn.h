@@ -445,6 +445,8 @@ typedef struct B200FaArgs {
     void *workspace;
     size_t workspace_bytes;
 } B200FaArgs;
+/* The workspace holds key splits' partial results and, for chunks of f32 or E4M3 tensors, 16-bit copies. A chunk on the
+ * tensor-copy tiles that is given less goes unsplit, one that needs copies takes the general kernel; the others are refused. */
 size_t b200_flash_attn_workspace_bytes(const B200FaArgs *args);
 int b200_flash_attn(const B200FaArgs *args, b200_stream_t stream);
 

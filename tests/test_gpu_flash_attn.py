@@ -442,6 +442,49 @@ def test_key_splits_of_the_tensor_copy_tiles(P, b, lq, lk, hq, hkv, d, wl, wr):
         assert (out.double() - want).norm() <= 2.0 ** -8 * want.norm(), bare
 
 
+@pytest.mark.parametrize("lq,hq,lk,dt", [(1, 4, 3000, torch.bfloat16), (64, 8, 4000, torch.bfloat16), (80, 2, 700, torch.float32)])
+def test_workspace_at_an_odd_address(P, lq, hq, lk, dt):
+    """Key splits and copies in a workspace that starts four bytes past a boundary: the same bits as in an aligned one."""
+    import ctypes
+    g = torch.Generator(device="cuda:0").manual_seed(lk)
+    q, k, v = (torch.randn((1, n, h, 128), generator=g, device="cuda:0", dtype=dt) for n, h in ((lq, hq), (lk, 1), (lk, 1)))
+    a, out, keep = P.flash_attn._fa_args(q, k, v, cfg_of(P, 128, -1, 0))
+    need = P._abi.lib().b200_flash_attn_workspace_bytes(ctypes.byref(a))
+    assert need > 0
+    buf, got = torch.empty(need + 8, dtype=torch.uint8, device="cuda:0"), []
+    for shift in (0, 4):
+        a.workspace, a.workspace_bytes = buf.data_ptr() + shift, need
+        P._abi.check(P._abi.lib().b200_flash_attn(ctypes.byref(a), 0))
+        torch.cuda.synchronize()
+        got.append(out.clone())
+    assert torch.equal(*got)
+
+
+# f32 tensors, E4M3 keys and keys of another type than the queries through 16-bit copies on the tensor-copy tiles: outputs of 16
+# bits and of 32, one split and several, strided views; and many rows without a workspace, which take the general kernel
+@pytest.mark.parametrize("qdt,kdt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, "fp8"), (torch.float32, "fp8")])
+@pytest.mark.parametrize("b,lq,lk,hq,hkv,d,wl,wr", [(2, 100, 100, 4, 4, 64, -1, 0), (1, 64, 2100, 4, 2, 128, -1, 0), (3, 70, 333, 6, 2, 72, 90, 4), (1, 513, 513, 16, 2, 40, -1, -1), (24, 70, 90, 8, 8, 64, -1, 0)])
+def test_other_types_on_the_tensor_copy_tiles(P, qdt, kdt, b, lq, lk, hq, hkv, d, wl, wr):
+    import ctypes
+    g = torch.Generator(device="cuda:0").manual_seed(lk + d)
+    q = torch.randn((b, hq, lq, d), generator=g, device="cuda:0").to(qdt).transpose(1, 2)
+    k, v = (torch.randn((b, hkv, lk, d), generator=g, device="cuda:0").to(torch.float8_e4m3fn if kdt == "fp8" else kdt).transpose(1, 2) for _ in range(2))
+    cfg = cfg_of(P, d, wl, wr, kd=0.5 if kdt == "fp8" else 1.0)
+    kind = torch.bfloat16 if qdt == torch.bfloat16 or kdt == torch.bfloat16 else torch.float16  # what the products run in
+    x, y, z = (t.to(torch.float32).to(kind) for t in (q, k, v))
+    want = torch.stack([_plain(*t, cfg.k_descale / np.sqrt(d), wl, wr) for t in zip(x, y, z)])
+    a, out, keep = P.flash_attn._fa_args(q, k, v, cfg)
+    for bare in (False, True):
+        if bare:
+            a.workspace, a.workspace_bytes = None, 0
+            if b < 24:
+                break  # the general kernel wants a workspace of its own for so few rows
+        P._abi.check(P._abi.lib().b200_flash_attn(ctypes.byref(a), 0))
+        torch.cuda.synchronize()
+        # weights and output are each rounded once: half an ulp each at most, in the 2-norm
+        assert (out.double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[kind] * want.norm(), bare
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (2, 2, 64), (4, 4, 96)])
 def test_varlen_rows_beside_infinities(P, hq, hkv, d):
     """The last key tile of a sequence reaches into the next one: what is there, infinities and NaN included, has no part in it."""
