@@ -844,10 +844,10 @@ def prefill_leg(env, steps, warmup):
             "roofline": {"bound": "tensor", "kernel": "fa_prefill_tma_kernel (attention alone)", "achieved": achieved,
                          "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "peak_source": kind + (f" x {world} GPUs" if world > 1 else ""),
                          "frac_of_sustained": achieved / (pk["bf16_tflops_sustained"] * world) if "bf16_tflops_sustained" in pk else None,
-                         # dram read + write of one launch at B = 1 (50.4 + 3.0 MB, part of q / k / v still in L2 from the
+                         # dram read + write of one launch at B = 1 (53.9 MB, part of q / k / v still in L2 from the
                          # call before), times the 4 batch entries of c3, whose blocks do not share data
-                         "traffic": 4 * 53_400_000 if world == 1 else None, "traffic_unit": "bytes per launch",
-                         "traffic_source": "ncu capture at B=1 scaled by 4, profiles/fa_prefill_sm100_kernel2_b1_s4096.md"},
+                         "traffic": 4 * 53_900_000 if world == 1 else None, "traffic_unit": "bytes per launch",
+                         "traffic_source": "ncu capture at B=1 scaled by 4, profiles/fa_prefill_tma_kernel_b1_s4096.md"},
             "cpu_baseline": cpu, "clocks": clocks}
     from baseline import ref_cuda as R
     if R.available() and world == 1:
