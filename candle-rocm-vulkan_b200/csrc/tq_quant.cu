@@ -349,6 +349,7 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
         if (threadIdx.x < 16) bound[threadIdx.x] = threadIdx.x < (1u << sp.cb) - 1u ? sp.tab[16 + threadIdx.x] : 0.0f;
         __syncthreads();
     }
+    const float b7 = bound[7], b3 = bound[3], b11 = bound[11];  // (codebook formats of four bits)
     after_prev_begin(p);
     for (uint32_t base = (blockIdx.x * Q128_WARPS + (threadIdx.x >> 5)) * Q128_RPW; base < rows; base += gridDim.x * Q128_WARPS * Q128_RPW) {
         bool live = base + (lane >> 3) < rows;  // a row past the end repeats the last one and stores nothing
@@ -422,20 +423,35 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
             }
             const float norm = __fsqrt_rn(__fadd_rn(v[0], v[1]));
             const float inv = norm > 0.0f ? __fdiv_rn(1.0f, norm) : 0.0f;
+            // A code is the number of boundaries that the element reaches: they ascend, so by halves (a NaN reaches none).
             const uint32_t cb = sp.cb;
             uint64_t w = 0;
+            if (cb == 4) {
+                // unrolled: the first two halves from registers, offsets in bytes (65 528 rows: 22.4 -> 13.1 us, rotated 30.7 -> 20.3)
+                uint32_t w4[2] = {0u, 0u};
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                // the number of boundaries that u reaches: they ascend, so by halves (a NaN reaches none)
-                const float u = __fmul_rn(x[k], inv);
-                uint32_t idx = 0;
-                for (uint32_t st = 1u << (cb - 1); st; st >>= 1) idx += u >= bound[idx + st - 1] ? st : 0u;
-                w |= (uint64_t)idx << (k * cb);
+                for (int k = 0; k < 16; ++k) {
+                    const float u = __fmul_rn(x[k], inv);
+                    const bool p8 = u >= b7;
+                    const bool p4 = u >= (p8 ? b11 : b3);
+                    uint32_t off = (p8 ? 32u : 0u) + (p4 ? 16u : 0u);
+                    const char *at = reinterpret_cast<const char *>(bound);
+                    off += u >= *reinterpret_cast<const float *>(at + off + 4) ? 8u : 0u;
+                    off += u >= *reinterpret_cast<const float *>(at + off) ? 4u : 0u;
+                    w4[k >> 3] |= (off >> 2) << (4 * (k & 7));
+                }
+                if (live) orow[2 * l8] = w4[0], orow[2 * l8 + 1] = w4[1];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const float u = __fmul_rn(x[k], inv);
+                    uint32_t idx = 0;
+                    for (uint32_t st = 1u << (cb - 1); st; st >>= 1) idx += u >= bound[idx + st - 1] ? st : 0u;
+                    w |= (uint64_t)idx << (k * cb);
+                }
             }
             if (live) {
-                if (cb == 4) {
-                    orow[2 * l8] = (uint32_t)w, orow[2 * l8 + 1] = (uint32_t)(w >> 32);
-                } else {
+                if (cb != 4) {
                     uint16_t *dst = reinterpret_cast<uint16_t *>(orow) + l8 * cb;  // 16 codes of cb bits
                     for (uint32_t i = 0; i < cb; ++i) dst[i] = (uint16_t)(w >> (16 * i));
                 }
