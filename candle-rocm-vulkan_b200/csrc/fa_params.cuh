@@ -26,7 +26,7 @@ struct FaParams {
     const B200Page *pages;
     const uint32_t *pg_keys;
     uint32_t n_pages;
-    uint32_t o_f32;  // fa_prefill_tma_kernel: outputs are f32 (q, k, v are 16-bit copies of other types)
+    uint32_t o_f32;  // outputs are f32 (q, k, v are 16-bit copies of other types); only fa_prefill_tma_kernel writes them
 };
 
 // prefill tiles on the 5th generation tensor cores (fa_prefill_sm100.cu)

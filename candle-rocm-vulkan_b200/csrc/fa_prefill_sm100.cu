@@ -1756,6 +1756,7 @@ static int fa_prefill_route(const FaParams &p, bool kv16) {
         return PF_TMA;
     // tensors that no map describes: 16-byte chunks, head dim 128
     if (p.d != PF_D || rows < 4 * PF_BM) return PF_NONE;  // short chunks and decode stay on the mma.sync kernel
+    if (p.o_f32) return PF_NONE;  // these two kernels store 16-bit rows only
     if ((reinterpret_cast<uintptr_t>(p.q) & 15) || ((p.q_sb | p.q_ss | p.q_sh) & 7)) return PF_NONE;
     static const long force = [] { const char *e = diag_env("B200_FA_TC_ROWS"); return e ? atol(e) : 0l; }();  // 128 or 256: tile height
     if (force == 128) return PF_ROWS128;

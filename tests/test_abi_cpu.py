@@ -194,6 +194,21 @@ def test_argument_errors_without_gpu(pkg):
     assert lib.b200_tq_attention_workspace_bytes(C.byref(args)) == 0
 
 
+def test_f32_outputs_only_where_the_tiles_write_them(pkg):
+    """Calls of f32 queries take 16-bit copies (and the workspace for them) where the tensor-copy tiles serve them: groups of a
+    power of two. Other groups stay on the general kernel, which writes f32 rows."""
+    A = pkg._abi
+    for hq, hkv, copied in ((32, 8, True), (24, 8, False), (28, 4, False), (12, 2, False), (6, 2, False)):
+        for kv in (A.F32, A.BF16, A.FP8):
+            a = A.FaArgs()
+            a.b, a.lq, a.lk, a.hq, a.hkv, a.d, a.total_q = 8, 600, 600, hq, hkv, 128, 8 * 600  # enough rows to go unsplit
+            a.q_strides, a.k_strides, a.v_strides = (A.u64x3(600 * h * 128, h * 128, 128) for h in (hq, hkv, hkv))
+            a.q_dtype, a.kv_dtype, a.scale, a.k_descale, a.v_descale, a.wl, a.wr = A.F32, kv, 0.1, 1.0, 1.0, -1, 0
+            copies = 8 * (600 * hq + 2 * 600 * hkv) * 128 * 2
+            need = A.lib().b200_flash_attn_workspace_bytes(C.byref(a))
+            assert need >= copies if copied else need == 0, (hq, hkv, kv)
+
+
 def test_paged_dense_attention_argument_errors_without_gpu(pkg):
     """The checks of the paged entry points run before anything touches the device (candle-nn/src/flash_attn.rs:650-689,
     candle-flash-attn/src/lib.rs:357-392)."""

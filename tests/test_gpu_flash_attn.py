@@ -485,6 +485,21 @@ def test_other_types_on_the_tensor_copy_tiles(P, qdt, kdt, b, lq, lk, hq, hkv, d
         assert (out.double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[kind] * want.norm(), bare
 
 
+@pytest.mark.parametrize("qdt,kdt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.float32, "fp8"), (torch.bfloat16, "fp8")])
+@pytest.mark.parametrize("hq,hkv,lq,lk", [(24, 8, 171, 171), (28, 4, 600, 600), (12, 2, 171, 500), (6, 2, 512, 600)])
+def test_other_types_in_groups_of_any_size(P, qdt, kdt, hq, hkv, lq, lk):
+    """Query groups that are no power of two, at the head dim and row counts of the 16-byte chunk tiles, which cannot write f32."""
+    g = torch.Generator(device="cuda:0").manual_seed(lq + hq)
+    q = torch.randn((1, lq, hq, 128), generator=g, device="cuda:0").to(qdt)
+    k, v = (torch.randn((1, lk, hkv, 128), generator=g, device="cuda:0").to(torch.float8_e4m3fn if kdt == "fp8" else kdt) for _ in range(2))
+    kind = torch.bfloat16 if qdt == torch.bfloat16 or kdt == torch.bfloat16 else torch.float16  # what the products run in
+    x, y, z = (t.to(torch.float32).to(kind) for t in (q, k, v))
+    out = P.flash_attn.flash_attn_with_config(q, k, v, cfg_of(P, 128, -1, 0))
+    want = _plain(x[0], y[0], z[0], 1.0 / np.sqrt(128), -1, 0)
+    # weights and output are each rounded once: half an ulp each at most, in the 2-norm
+    assert (out[0].double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[kind] * want.norm()
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (2, 2, 64), (4, 4, 96)])
 def test_varlen_rows_beside_infinities(P, hq, hkv, d):
     """The last key tile of a sequence reaches into the next one: what is there, infinities and NaN included, has no part in it."""
