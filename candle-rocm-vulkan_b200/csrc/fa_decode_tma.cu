@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 2) fa_decode_tma_kernel(const F
             const char *v_src = reinterpret_cast<const char *>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(vr), row));
             const bool in = k_src != nullptr && ch * 8 < D;
             const uint32_t at = dst + (ch >> 3) * C::HALF + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
-            const void *none = p.q;  // what is not copied reads as zeros
+            const void *none = p.pg_keys;  // what is not copied reads as zeros; a source is 16-byte aligned even then, and q need not be
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(in ? k_src + ch * 16 : none), "r"(in ? 16 : 0) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + C::TILE), "l"(in ? v_src + ch * 16 : none), "r"(in ? 16 : 0) : "memory");
         }

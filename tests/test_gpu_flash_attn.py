@@ -244,6 +244,20 @@ def test_many_blocks_read_in_place_equal_the_concatenated_call(P, dt, d, page, n
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("d,lq,qdt", [(72, 1, torch.bfloat16), (128, 4, torch.bfloat16), (40, 2, torch.float32)])
+def test_blocks_with_queries_at_any_address(P, d, lq, qdt):
+    """Decode over blocks with a ragged last tile (and head dims that leave chunks of a row uncopied), queries one element past a
+    16-byte boundary: the bits of the aligned call."""
+    b, hq, hkv = 2, 8, 2
+    g = torch.Generator(device="cuda:0").manual_seed(d)
+    blocks = [P.KvBlockRef(*(torch.randn((b, hkv, 64, d), generator=g, device="cuda:0", dtype=torch.bfloat16) for _ in range(2)), r) for r in (64, 37)]
+    q = torch.randn((b, hq, lq, d), generator=g, device="cuda:0").to(qdt)
+    odd = torch.empty(q.numel() + 1, dtype=qdt, device="cuda:0")[1:].view(q.shape).copy_(q)
+    assert odd.data_ptr() % 16 != 0
+    cfg = P.FlashAttnConfig(d ** -0.5).causal()
+    assert torch.equal(P.flash_attn.flash_attn_blocks(odd, blocks, cfg), P.flash_attn.flash_attn_blocks(q, blocks, cfg))
+
+
 def test_paged_varlen_equals_varlen_on_gathered_pages(P):
     torch.manual_seed(9)
     hq, hkv, d, page, nblk = 8, 2, 128, 16, 40
