@@ -1745,12 +1745,13 @@ static int fa_prefill_route(const FaParams &p, bool kv16) {
     if (p.q_dtype != B200_F16 && p.q_dtype != B200_BF16) return PF_NONE;
     if (p.softcap > 0.0f || p.alibi != nullptr) return PF_NONE;
     if (!(p.scale * p.kd > 0.0f)) return PF_NONE;  // the row maximum is taken before the scale is applied
+    if (reinterpret_cast<uintptr_t>(p.o) & 15) return PF_NONE;  // rows are stored in 16-byte pieces
     static const bool off = [] { const char *e = diag_env("B200_FA_NO_TCGEN05"); return e && *e == '1'; }();
     if (off) return PF_NONE;
     const uint64_t rows = (uint64_t)p.lq * p.group;
     cuuint64_t qs[4];
     static const bool no_tma = [] { const char *e = diag_env("B200_FA_NO_TMA"); return e && *e == '1'; }();
-    if (!no_tma && rows >= P3_MIN_ROWS && p.d <= 128 && (reinterpret_cast<uintptr_t>(p.o) & 15) == 0 && p.lk < (1u << 31) && rows < (1ull << 31) &&
+    if (!no_tma && rows >= P3_MIN_ROWS && p.d <= 128 && p.lk < (1u << 31) && rows < (1ull << 31) &&
         (rows + P3_ROWS - 1) / P3_ROWS * p.b * p.hkv < (1ull << 31) && q_strides(p, qs) &&
         fa_kv_maps(p, false, 0, nullptr, nullptr, nullptr))
         return PF_TMA;

@@ -209,6 +209,19 @@ def test_f32_outputs_only_where_the_tiles_write_them(pkg):
             assert need >= copies if copied else need == 0, (hq, hkv, kv)
 
 
+def test_outputs_off_a_boundary_stay_on_the_general_kernel(pkg):
+    """The tcgen05 tiles store rows in 16-byte pieces: an output that starts elsewhere takes the general kernel, which splits
+    a call of this size along the keys (a workspace; the tiles would ask for none)."""
+    A = pkg._abi
+    for hq, kv, o, need in ((4, A.BF16, 4096, False), (4, A.BF16, 4096 + 8, True), (3, A.BF16, 4096 + 8, True), (3, A.FP8, 4096 + 8, True)):
+        a = A.FaArgs()
+        a.b, a.lq, a.lk, a.hq, a.hkv, a.d, a.total_q, a.o = 1, 512, 512, hq, 1, 128, 512, o
+        a.q_strides, a.k_strides, a.v_strides = (A.u64x3(512 * h * 128, h * 128, 128) for h in (hq, 1, 1))
+        a.q_dtype, a.kv_dtype, a.scale, a.k_descale, a.v_descale, a.wl, a.wr = A.BF16, kv, 0.1, 1.0, 1.0, -1, 0
+        got = A.lib().b200_flash_attn_workspace_bytes(C.byref(a))
+        assert (got >= 2 * 512 * hq * 129 * 4) == need, (hq, kv, o, got)
+
+
 def test_paged_dense_attention_argument_errors_without_gpu(pkg):
     """The checks of the paged entry points run before anything touches the device (candle-nn/src/flash_attn.rs:650-689,
     candle-flash-attn/src/lib.rs:357-392)."""

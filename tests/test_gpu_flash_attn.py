@@ -514,6 +514,25 @@ def test_other_types_in_groups_of_any_size(P, qdt, kdt, hq, hkv, lq, lk):
     assert (out[0].double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[kind] * want.norm()
 
 
+@pytest.mark.parametrize("hq,kdt", [(4, torch.bfloat16), (3, torch.bfloat16), (3, "fp8"), (4, "fp8")])
+def test_outputs_off_a_boundary(P, hq, kdt):
+    """An output buffer that starts 8 bytes past a 16-byte boundary, through the C ABI, at a size of the tcgen05 tiles."""
+    import ctypes
+    g = torch.Generator(device="cuda:0").manual_seed(hq)
+    q = torch.randn((1, 512, hq, 128), generator=g, device="cuda:0", dtype=torch.bfloat16)
+    k, v = (torch.randn((1, 512, 1, 128), generator=g, device="cuda:0").to(torch.float8_e4m3fn if kdt == "fp8" else kdt) for _ in range(2))
+    a, out, keep = P.flash_attn._fa_args(q, k, v, cfg_of(P, 128, -1, 0))
+    buf = torch.zeros(out.numel() + 8, dtype=out.dtype, device="cuda:0")
+    a.o = buf.data_ptr() + 8
+    ws = torch.empty(P._abi.lib().b200_flash_attn_workspace_bytes(ctypes.byref(a)), dtype=torch.uint8, device="cuda:0")
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    P._abi.check(P._abi.lib().b200_flash_attn(ctypes.byref(a), 0))
+    torch.cuda.synchronize()
+    want = _plain(q[0], k[0].to(torch.bfloat16), v[0].to(torch.bfloat16), 1.0 / np.sqrt(128), -1, 0)
+    assert (buf[4:-4].view(want.shape).double() - want).norm() <= 2.0 ** -8 * want.norm()
+    assert not buf[:4].any() and not buf[-4:].any()
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (2, 2, 64), (4, 4, 96)])
 def test_varlen_rows_beside_infinities(P, hq, hkv, d):
     """The last key tile of a sequence reaches into the next one: what is there, infinities and NaN included, has no part in it."""
