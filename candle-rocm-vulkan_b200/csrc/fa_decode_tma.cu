@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 2) fa_decode_tma_kernel(const F
             *reinterpret_cast<float2 *>(p.part_o + prow * D + dd) = make_float2(o0 * inv, o1 * inv);
         }
     }
-    if (p.n_splits > 1 && ch == 0) p.part_lse[prow] = L > 0.0f ? M * FD_LN2 + logf(L) : -INFINITY;
+    if (p.n_splits > 1 && ch == 0) p.part_lse[prow] = L == 0.0f ? -INFINITY : M * FD_LN2 + logf(L);  // a NaN stays one
 }
 
 bool fa_decode_tma_takes(const FaParams &p, bool paged) {

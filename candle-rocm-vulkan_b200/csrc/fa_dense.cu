@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(FA_WARPS * 32) fa_dense_kernel(const FaParams 
             if (p.n_splits == 1) store_elem_rt(p.o, orow * D + dd, o * inv, p.q_dtype);
             else p.part_o[prow * D + dd] = o * inv;
         }
-        if (p.n_splits > 1 && ch == 0) p.part_lse[prow] = L > 0.0f ? M + logf(L) : -INFINITY;
+        if (p.n_splits > 1 && ch == 0) p.part_lse[prow] = L == 0.0f ? -INFINITY : M + logf(L);  // a NaN stays one
     } else {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -440,14 +440,15 @@ __global__ void __launch_bounds__(FA_WARPS * 32) fa_dense_kernel(const FaParams 
 #pragma unroll
             for (int n = 0; n < NT; ++n)
                 if ((uint32_t)8 * n < D) *reinterpret_cast<float2 *>(po + 8 * n + 2 * c) = make_float2(oacc[n][2 * e] * inv, oacc[n][2 * e + 1] * inv);
-            if (c == 0) p.part_lse[prow] = l[e] > 0.0f ? m[e] + logf(l[e]) : -INFINITY;
+            if (c == 0) p.part_lse[prow] = l[e] == 0.0f ? -INFINITY : m[e] + logf(l[e]);  // a NaN stays one
         }
     }
     }
 }
 
 // candle-core/kernels/flash_attn_impl.h:445-473. One warp per row: a lane has the weights of splits lane and lane + 32 (there are
-// 64 at most), and four neighbouring elements of the sums, four splits' loads on their way at a time. Launched as a
+// 64 at most), and four neighbouring elements of the sums, four splits' loads on their way at a time. A split without
+// a key has a log-sum of -inf and no part; one whose sum is a NaN has a NaN there, and with it the row. Launched as a
 // programmatic dependent of the kernel that writes the partial results, whose end it waits for.
 __global__ void __launch_bounds__(128) fa_combine_kernel(const float *__restrict__ part_o, const float *__restrict__ part_lse,
                                                         void *__restrict__ o, int o_dtype, uint64_t rows, uint32_t D, uint32_t n_splits) {
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(128) fa_combine_kernel(const float *__restrict
             }
             if (d < D)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) store_elem_rt(o, row * D + d + k, wsum > 0.0f ? a[k] / wsum : 0.0f, o_dtype);
+                for (int k = 0; k < 4; ++k) store_elem_rt(o, row * D + d + k, wsum == 0.0f ? 0.0f : a[k] / wsum, o_dtype);
         }
     }
 }

@@ -1561,7 +1561,7 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                 const uint64_t part = (uint64_t)cur.split * p.rows_total;
                 auto out_row = [&](uint32_t rr) { return (cur.q0 + (rr >> cur.gl)) * p.hq + (cur.hk << cur.gl) + (rr & ((1u << cur.gl) - 1)); };
                 const uint32_t r = cur.row0 + g * PF_BM + w4 * 32 + lane;
-                if (p.n_splits > 1 && r < cur.R) p.part_lse[part + out_row(r)] = l > 0.0f ? mref * 0.6931471805599453f + logf(l) : -INFINITY;
+                if (p.n_splits > 1 && r < cur.R) p.part_lse[part + out_row(r)] = l == 0.0f ? -INFINITY : mref * 0.6931471805599453f + logf(l);  // a NaN stays one
 #pragma unroll 1
                 for (uint32_t c0 = 0; c0 < p.d; c0 += 32) {
                     uint32_t o[32];

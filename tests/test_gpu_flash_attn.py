@@ -456,6 +456,28 @@ def test_key_splits_of_the_tensor_copy_tiles(P, b, lq, lk, hq, hkv, d, wl, wr):
         assert (out.double() - want).norm() <= 2.0 ** -8 * want.norm(), bare
 
 
+# split along the keys: decode by tensor copies, decode on the general kernel, few query rows on the tiles, the same over 16-bit copies
+@pytest.mark.parametrize("lq,lk,d,dt", [(2, 3000, 128, torch.bfloat16), (1, 3000, 256, torch.bfloat16), (64, 6500, 128, torch.bfloat16),
+                                        (70, 2100, 64, torch.float32), (40, 3000, 256, torch.float16)])
+def test_key_splits_keep_nan(P, lq, lk, d, dt):
+    """A NaN in a query row, or in a key of one split, gives NaN in the rows that see it and in no other, as in unsplit calls."""
+    g = torch.Generator(device="cuda:0").manual_seed(lk)
+    q, k, v = (torch.randn((1, n, h, d), generator=g, device="cuda:0").to(dt) for n, h in ((lq, 4), (lk, 2), (lk, 2)))
+    a, out, keep = P.flash_attn._fa_args(q, k, v, cfg_of(P, d, -1, 0))
+    assert a.workspace_bytes > 0
+    call = lambda: P.flash_attn.flash_attn_with_config(q, k, v, cfg_of(P, d, -1, 0))
+    q[0, lq - 1, 1, 3] = float("nan")
+    nan = call().isnan()
+    assert nan[0, lq - 1, 1].all() and nan.sum() == d
+    q[0, lq - 1, 1, 3] = 1.0
+    for key in (100, lk - 1):
+        old = k[0, key, 1, 5].clone()
+        k[0, key, 1, 5] = float("nan")
+        nan, first = call().isnan(), max(key - (lk - lq), 0)
+        assert nan[0, first:, 2:].all() and nan.sum() == (lq - first) * 2 * d, key
+        k[0, key, 1, 5] = old
+
+
 @pytest.mark.parametrize("lq,hq,lk,dt", [(1, 4, 3000, torch.bfloat16), (64, 8, 4000, torch.bfloat16), (80, 2, 700, torch.float32)])
 def test_workspace_at_an_odd_address(P, lq, hq, lk, dt):
     """Key splits and copies in a workspace that starts four bytes past a boundary: the same bits as in an aligned one."""
