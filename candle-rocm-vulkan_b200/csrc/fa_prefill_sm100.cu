@@ -1052,12 +1052,12 @@ __device__ __forceinline__ bool p3_item(const FaParams &p, const P3Grid &gr, uin
     }
     return true;
 }
-// the key tiles [t0, t1) of the item that some row of group g sees (empty: t0 == t1)
-__device__ __forceinline__ void p3_group(const FaParams &p, const P3Item &it, int g, int &t0, int &t1) {
-    t0 = t1 = 0;
+// the key tiles [t0, t1) of the item that some row of group g sees (empty: t0 == t1), and these keys [lo, hi)
+__device__ __forceinline__ void p3_group(const FaParams &p, const P3Item &it, int g, int &t0, int &t1, int &lo, int &hi) {
+    t0 = t1 = lo = hi = 0;
     const uint32_t first = it.row0 + g * PF_BM;
     if (first >= it.R || it.ntiles == 0) return;
-    int lo, hi, tmp;
+    int tmp;
     p3_range(p, it, first, lo, tmp);
     p3_range(p, it, min(first + PF_BM, it.R) - 1, tmp, hi);
     lo = max(lo, it.t_lo);
@@ -1065,6 +1065,13 @@ __device__ __forceinline__ void p3_group(const FaParams &p, const P3Item &it, in
     if (hi <= lo) return;
     t0 = (lo - it.t_lo) / P3_BN;
     t1 = (hi - it.t_lo + P3_BN - 1) / P3_BN;
+}
+// Weights of keys that a row does not see are zero, but zero times an infinity is not. So a group's products over V take only the
+// steps of 16 keys that hold some it sees, and where the item's keys end inside such a step the owner warp clears the rest of
+// it: true for the item's last tile, at key j0, if what follows is another key (masked for all rows of the item) or
+// another sequence; past the end of the tensor the copy brings zeros.
+__device__ __forceinline__ bool p3_clears(const FaParams &p, const P3Item &it, int j0) {
+    return (p.varlen || it.t_hi < it.lk) && j0 + P3_BN > it.t_hi && ((it.t_hi - j0) & 15) != 0;
 }
 __device__ __forceinline__ bool elect_one() {
     uint32_t e;
@@ -1169,6 +1176,7 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
         if (warp == P3_LOADER) {
             // ============================================================ loader
             uint32_t kv = 0, nq = 0;  // key tiles and Q tiles so far
+            uint32_t tail = 0, tail_n = 0;  // a bit per stage: its V tile lands on the tail's barrier; the parity of that barrier's last copy
             const uint64_t k_total = p.varlen ? p.cu_k[p.b] : 0;
             const char *kbase = reinterpret_cast<const char *>(p.k), *vbase = reinterpret_cast<const char *>(p.v);
             for (int k = 0, n; next_item(k, n); ++k) {
@@ -1218,6 +1226,7 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                         if (lane == 0) {
                             mbar_arrive(&bars[C::KF + st]);
                             mbar_arrive(&bars[C::VF + st]);
+                            tail &= ~(1u << st);
                         }
                         continue;
                     }
@@ -1232,10 +1241,11 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                         break;
                     }
                     if (lane == 0) {
-                        // past the end of the item's keys lie other sequences' rows: the owner warp clears them first
-                        const int full = p.varlen && j0 + P3_BN > it.t_hi ? C::VT + st : C::VF + st;
+                        const int full = p3_clears(p, it, j0) ? C::VT + st : C::VF + st;
                         mbar_expect_tx(&bars[full], C::T_BYTES);
                         load(&tm_v, (gr.tm_order >> 8) & 0x3fu, dv, (int)it.k0 + j0, bar0 + 8 * full);
+                        tail = full == C::VT + st ? tail | 1u << st : tail & ~(1u << st);
+                        if (full == C::VT + st) tail_n ^= 1u << st;
                     }
                     __syncwarp();
                 }
@@ -1248,14 +1258,14 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                     if (nq > 0) pf_wait_landed(bar0 + 8 * C::QF, (nq - 1) & 1);
                     for (uint32_t t = kv > NS ? kv - NS : 0; t < kv; ++t) {
                         pf_wait_landed(bar0 + 8 * (C::KF + t % NS), (t / NS) & 1);
-                        if (!p.varlen) pf_wait_landed(bar0 + 8 * (C::VF + t % NS), (t / NS) & 1);
+                        const uint32_t st = t % NS;
+                        if (tail >> st & 1u) pf_wait_landed(bar0 + 8 * (C::VT + st), (tail_n >> st & 1u) ^ 1u);
+                        else pf_wait_landed(bar0 + 8 * (C::VF + st), (t / NS) & 1);
                     }
-                    if (p.varlen)  // a V tile may land on the tail's barrier: a pause that outlasts any copy
-                        for (int i = 0; i < 64; ++i) __nanosleep(1000);
                 }
             }
         } else if (warp == P3_OWNER) {
-            // ============================================================ work items; rows behind the keys of an item (varlen)
+            // ============================================================ work items; rows behind the keys of an item
             // The grid has a block per item. A block starts with its own and then takes over blocks that have not started
             // (heaviest first), so that late items go where there is time; items without rows end here. It asks when the last
             // tile of an item has been requested: the answer comes while the tiles in flight are worked on (asked for at an item's
@@ -1296,15 +1306,14 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                 if (!(ok = p3_wait(bar0 + 8 * C::GO, (k - 1) & 1, abort_flag))) break;
                 take(ahead);
                 announce(k);
-                if (!ok || !p.varlen || it.ntiles == 0) continue;
+                if (!ok || it.ntiles == 0) continue;
                 kv += it.ntiles;
                 const int st = (kv - 1) % NS, j0 = it.t_lo + (it.ntiles - 1) * P3_BN;
-                if (j0 + P3_BN <= it.t_hi || it.k0 + j0 + P3_BN > k_total) continue;
-                // The tile reaches into the next sequence (or into keys that no row of the item sees). Their weights are zero,
-                // but zero times an infinity is not: the rows are cleared before V is announced.
+                if (!p3_clears(p, it, j0) || (p.varlen && it.k0 + j0 + P3_BN > k_total)) continue;
+                // cleared before V is announced
                 if (!(ok = p3_wait(bar0 + 8 * (C::VT + st), (parity >> st) & 1, abort_flag))) break;
                 parity ^= 1u << st;
-                for (int idx = (it.t_hi - j0) * 8 + lane; idx < P3_BN * 8; idx += 32)
+                for (int idx = (it.t_hi - j0) * 8 + lane; idx < (it.t_hi - j0 + 15) / 16 * 128; idx += 32)
 #pragma unroll
                     for (int hf = 0; hf < C::HALVES; ++hf)
                         *reinterpret_cast<uint4 *>(smem + C::SM_V + st * C::T_BYTES + hf * C::T_HALF + idx * 16) = make_uint4(0, 0, 0, 0);
@@ -1341,8 +1350,8 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                 P3Item it;
                 p3_item(p, gr, n, it);
                 if (it.ntiles == 0) continue;
-                int t0, t1;
-                p3_group(p, it, g, t0, t1);
+                int t0, t1, lo, hi;
+                p3_group(p, it, g, t0, t1, lo, hi);
                 if (!(ok = p3_wait(bar0 + 8 * C::QF, nq & 1, abort_flag))) break;
                 ++nq;
                 if (t0 == t1 && elect_one()) mbar_arrive(&bars[C::QE]);
@@ -1374,16 +1383,19 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t v_desc = tc_desc_sw128(sbase + C::SM_V + st * C::T_BYTES, C::T_HALF, 1024);
+                    const int j0 = it.t_lo + t * P3_BN, ks0 = t == t0 ? (lo - j0) / 16 : 0, ks1 = t == t1 - 1 ? (hi - j0 + 15) / 16 : 8;
                     if (elect_one()) {  // O_g += P_g(t) V(t): the first 96 keys while the others' exponentials run
 #pragma unroll
-                        for (int ks = 0; ks < 6; ++ks) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, (t > t0 || ks > 0) ? 1u : 0u);
+                        for (int ks = 0; ks < 6; ++ks)
+                            if (ks >= ks0 && ks < ks1) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, (t > t0 || ks > ks0) ? 1u : 0u);
                     }
                     __syncwarp();
                     if (!(ok = p3_wait(bar0 + 8 * (C::P1 + g), sc & 1, abort_flag))) break;
                     tc_fence_after();
                     if (elect_one()) {
 #pragma unroll
-                        for (int ks = 6; ks < 8; ++ks) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, 1u);
+                        for (int ks = 6; ks < 8; ++ks)
+                            if (ks >= ks0 && ks < ks1) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, (t > t0 || ks > ks0) ? 1u : 0u);
                         tc_commit(bar0 + 8 * (C::VE + st));
                         if (C::EARLY) tc_commit(bar0 + 8 * (C::PV + g));
                         if (t == t1 - 1) tc_commit(bar0 + 8 * (C::O + g));
@@ -1416,11 +1428,11 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
         auto begin = [&](int k) {
             if (!next_item(k, n)) return false;
             p3_item(p, gr, (uint32_t)n, it);
-            p3_group(p, it, g, t0, t1);
+            int lo, hi, tmp;
+            p3_group(p, it, g, t0, t1, lo, hi);
             const uint32_t g_row0 = it.row0 + g * PF_BM, r = g_row0 + w4 * 32 + lane;
             r_lo = r_hi = lomax = 0, himin = -1;
             if (t1 > t0) {
-                int lo, hi, tmp;
                 if (r < it.R) {
                     p3_range(p, it, r, lo, hi);
                     r_lo = lo - it.t_lo;

@@ -426,7 +426,10 @@ int b200_tq_attention_gather(const B200TqAttnArgs *args, const B200PeerGather *g
  * k / v (b, lk, hkv, d) with (batch, seq, head) element strides; varlen: q (total_q, hq, d) with
  * cu_q / cu_k u32 offsets (b + 1 entries), lq / lk the maxima. o: (token, head, d) contiguous.
  * Head dims: every multiple of 8 up to 256 (kernel_supported of candle-core/src/accel/attention.rs:283-290 takes any
- * d <= 256; others return B200_ERR_UNSUPPORTED_SHAPE and the caller's unfused path serves them). */
+ * d <= 256; others return B200_ERR_UNSUPPORTED_SHAPE and the caller's unfused path serves them).
+ * A masked key has weight zero in its row, which makes nothing of an infinite or NaN value where the row's tile holds that key:
+ * such a value reaches the rows that see it and, at most, those of the same tile of up to 128 packed query rows (256 in the
+ * 16-byte chunk tiles), never another tile's, another sequence's or rows past the end of a block. */
 typedef struct B200FaArgs {
     const void *q, *k, *v;
     void *o;

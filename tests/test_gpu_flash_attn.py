@@ -569,6 +569,28 @@ def test_varlen_rows_beside_infinities(P, hq, hkv, d):
         assert (out[a:e].double() - want).norm() <= 2.0 ** -8 * want.norm()
 
 
+# an item of the tiles is 256 packed rows: 64 tokens of a group of four, two groups of 32; token i sees the keys up to i + 100
+@pytest.mark.parametrize("wl,bad,rows", [(-1, slice(164, 300), slice(0, 64)), (-1, slice(144, 300), slice(0, 32)), (-1, slice(231, 232), slice(0, 128)),
+                                         (50, slice(0, 50), slice(0, 200)), (50, slice(0, 82), slice(32, 200)), (50, slice(82, 114), slice(64, 200))])
+@pytest.mark.parametrize("d,dt", [(128, torch.bfloat16), (64, torch.float16), (96, torch.bfloat16), (64, torch.float32)])
+def test_infinities_that_no_row_of_a_tile_sees(P, d, dt, wl, bad, rows):
+    """Fixed-length batches: values past the keys of a group of rows (rounded up to 16 keys), or in front of them, have no part in
+    these rows even if they are not finite; rows that do see them are not finite."""
+    g = torch.Generator(device="cuda:0").manual_seed(d)
+    q, k, v = (torch.randn((2, n, h, d), generator=g, device="cuda:0").to(dt) for n, h in ((200, 8), (300, 2), (300, 2)))
+    kind = torch.float16 if dt == torch.float32 else dt  # what the products run in
+    x, y, z = (t.to(kind) for t in (q, k, v))
+    want = torch.stack([_plain(*t, 1.0 / np.sqrt(d), wl, 0) for t in zip(x, y, z)])
+    v[:, bad][:, ::2], v[:, bad][:, 1::2] = float("inf"), float("nan")
+    out = P.flash_attn.flash_attn_with_config(q, k, v, cfg_of(P, d, wl, 0))
+    seen = torch.zeros((200, 300), dtype=torch.bool, device="cuda:0")
+    for i in range(200):
+        seen[i, 0 if wl < 0 else max(i + 100 - wl, 0):i + 101] = True
+    hit = seen[:, bad].any(1)
+    assert not hit[rows].any() and not out[:, hit].isfinite().any()
+    assert (out[:, rows].double() - want[:, rows]).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[kind] * want[:, rows].norm()
+
+
 def test_argument_errors(P):
     A = P._abi
     F = P.flash_attn
