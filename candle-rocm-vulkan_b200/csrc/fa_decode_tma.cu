@@ -359,7 +359,7 @@ static int launch(const FaParams &p, dim3 grid, cudaStream_t stream) {
     CUtensorMap tm_k, tm_v;
     uint32_t order = 0;
     if (PAGED) memset(&tm_k, 0, sizeof(tm_k)), memset(&tm_v, 0, sizeof(tm_v));
-    else if (!fa_kv_maps(p, BF16, FD<HD>::KEYS, &tm_k, &tm_v, &order)) return set_error(B200_ERR_LAUNCH, "flash_attn (decode): the driver refuses a tensor map");
+    else if (!fa_kv_maps(p, BF16, FD<HD>::KEYS, &tm_k, &tm_v, &order)) return FA_NO_MAP;
     static thread_local bool done[16] = {};
     int dev = 0;
     cudaGetDevice(&dev);

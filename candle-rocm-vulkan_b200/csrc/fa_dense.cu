@@ -571,7 +571,7 @@ static void fa_as_copies(FaParams &p, bool bf16, char *q, char *k, char *v, int 
     p.o_f32 = out_dtype == B200_F32;
 }
 
-static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false, bool may_copy = true) {
+static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false, bool may_copy = true, bool may_map = true) {
     if (!a) return set_error(B200_ERR_BAD_ARG, "flash_attn: null args");
     if (a->hkv == 0 || a->hq % a->hkv != 0)
         return set_error(B200_ERR_BAD_ARG, "flash-attn: %u query heads are not a multiple of %u kv heads", a->hq, a->hkv);
@@ -611,6 +611,7 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false, bool may
     p.alibi_bs = a->alibi_bstride; p.varlen = a->varlen;
     p.q_dtype = a->q_dtype;
     p.kv_kind = kv16 ? 0 : (fp8 ? 1 : 2);
+    p.no_maps = !may_map;
     pl.bf16 = kv16 ? a->kv_dtype == B200_BF16 : a->q_dtype == B200_BF16;
     p.rows_total = a->total_q * a->hq;
     const uint64_t rows = (uint64_t)a->lq * p.group;
@@ -719,6 +720,38 @@ static int fa_launch(const FaPlan &pl, cudaStream_t stream) {
     return fa_launch_as<HD, BF16, false>(pl, stream);
 }
 
+// launches the planned call; FA_NO_MAP: the driver refuses a tensor map (16-bit copies may have been written by then)
+static int fa_run(const B200FaArgs *a, const FaPlan &pl, char *ws, cudaStream_t stream) {
+    const bool bf = pl.bf16;
+    if (pl.cast) {
+        FaParams c = pl.p;
+        fa_as_copies(c, bf, ws + pl.cast_off[0], ws + pl.cast_off[1], ws + pl.cast_off[2], a->q_dtype);
+        const FaParams &p = pl.p;
+        const uint32_t qk = a->q_dtype == B200_F32 ? 2u : 0u, kk = (uint32_t)p.kv_kind;
+        const CastParams cp = {{{p.q, (uint16_t *)c.q, p.q_sb, p.q_ss, p.q_sh, p.lq, p.hq, qk},
+                                {p.k, (uint16_t *)c.k, p.k_sb, p.k_ss, p.k_sh, p.lk, p.hkv, kk},
+                                {p.v, (uint16_t *)c.v, p.v_sb, p.v_ss, p.v_sh, p.lk, p.hkv, kk}}, p.d / 8};
+        const uint64_t most = (uint64_t)p.b * std::max<uint64_t>((uint64_t)p.lq * p.hq, (uint64_t)p.lk * p.hkv) * cp.d8;
+        const dim3 grid((unsigned)std::min<uint64_t>((most + 255) / 256, 148ull * 8), 3);
+        if (bf) fa_cast_kernel<true><<<grid, 256, 0, stream>>>(cp, p.b);
+        else fa_cast_kernel<false><<<grid, 256, 0, stream>>>(cp, p.b);
+        int crc = check_launch("flash_attn (copies)");
+        if (!crc) crc = fa_prefill_sm100_launch(c, bf, stream);
+        return crc || c.n_splits == 1 ? crc : fa_combine_launch(pl, stream);
+    }
+    if (pl.prefill) {  // tiles on the tcgen05 tensor cores
+        const int prc = fa_prefill_sm100_launch(pl.p, bf, stream);
+        return prc || pl.p.n_splits == 1 ? prc : fa_combine_launch(pl, stream);
+    }
+    if (pl.decode_tma) {
+        const int drc = fa_decode_tma_launch(pl.p, bf, pl.grid, stream);
+        return drc || pl.p.n_splits == 1 ? drc : fa_combine_launch(pl, stream);
+    }
+    if (a->d <= 64) return bf ? fa_launch<64, true>(pl, stream) : fa_launch<64, false>(pl, stream);
+    if (a->d <= 128) return bf ? fa_launch<128, true>(pl, stream) : fa_launch<128, false>(pl, stream);
+    return bf ? fa_launch<256, true>(pl, stream) : fa_launch<256, false>(pl, stream);
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -750,34 +783,19 @@ extern "C" int b200_flash_attn(const B200FaArgs *a, b200_stream_t stream_) {
         pl.p.part_lse = reinterpret_cast<float *>(ws + pl.off_lse);
     }
     cudaStream_t stream = (cudaStream_t)stream_;
-    const bool bf = pl.bf16;
-    if (pl.cast) {
-        FaParams c = pl.p;
-        fa_as_copies(c, bf, ws + pl.cast_off[0], ws + pl.cast_off[1], ws + pl.cast_off[2], a->q_dtype);
-        const FaParams &p = pl.p;
-        const uint32_t qk = a->q_dtype == B200_F32 ? 2u : 0u, kk = (uint32_t)p.kv_kind;
-        const CastParams cp = {{{p.q, (uint16_t *)c.q, p.q_sb, p.q_ss, p.q_sh, p.lq, p.hq, qk},
-                                {p.k, (uint16_t *)c.k, p.k_sb, p.k_ss, p.k_sh, p.lk, p.hkv, kk},
-                                {p.v, (uint16_t *)c.v, p.v_sb, p.v_ss, p.v_sh, p.lk, p.hkv, kk}}, p.d / 8};
-        const uint64_t most = (uint64_t)p.b * std::max<uint64_t>((uint64_t)p.lq * p.hq, (uint64_t)p.lk * p.hkv) * cp.d8;
-        const dim3 grid((unsigned)std::min<uint64_t>((most + 255) / 256, 148ull * 8), 3);
-        if (bf) fa_cast_kernel<true><<<grid, 256, 0, stream>>>(cp, p.b);
-        else fa_cast_kernel<false><<<grid, 256, 0, stream>>>(cp, p.b);
-        int crc = check_launch("flash_attn (copies)");
-        if (!crc) crc = fa_prefill_sm100_launch(c, bf, stream);
-        return crc || c.n_splits == 1 ? crc : fa_combine_launch(pl, stream);
+    int lrc = fa_run(a, pl, ws, stream);
+    if (lrc != FA_NO_MAP) return lrc;
+    // the kernels that need no map, split along the keys if the workspace has room for their partial results
+    lrc = fa_plan(a, pl, false, false, false);
+    if (lrc) return lrc;
+    if (pl.ws_bytes && a->workspace && a->workspace_bytes >= pl.ws_bytes) {
+        pl.p.part_o = reinterpret_cast<float *>(ws);
+        pl.p.part_lse = reinterpret_cast<float *>(ws + pl.off_lse);
+    } else {
+        pl.p.n_splits = 1;
+        pl.grid.z = a->b;
     }
-    if (pl.prefill) {  // tiles on the tcgen05 tensor cores
-        const int prc = fa_prefill_sm100_launch(pl.p, bf, stream);
-        return prc || pl.p.n_splits == 1 ? prc : fa_combine_launch(pl, stream);
-    }
-    if (pl.decode_tma) {
-        const int drc = fa_decode_tma_launch(pl.p, bf, pl.grid, stream);
-        return drc || pl.p.n_splits == 1 ? drc : fa_combine_launch(pl, stream);
-    }
-    if (a->d <= 64) return bf ? fa_launch<64, true>(pl, stream) : fa_launch<64, false>(pl, stream);
-    if (a->d <= 128) return bf ? fa_launch<128, true>(pl, stream) : fa_launch<128, false>(pl, stream);
-    return bf ? fa_launch<256, true>(pl, stream) : fa_launch<256, false>(pl, stream);
+    return fa_run(a, pl, ws, stream);
 }
 
 // Decoding attention over the dense K / V of paged cache blocks, read where they are (candle-core/src/cuda_backend/

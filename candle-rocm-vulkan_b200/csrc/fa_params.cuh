@@ -26,12 +26,14 @@ struct FaParams {
     const B200Page *pages;
     const uint32_t *pg_keys;
     uint32_t n_pages;
+    uint32_t no_maps;  // the driver has refused a tensor map of this call's tensors: kernels that need none
     uint32_t o_f32;  // outputs are f32 (q, k, v are 16-bit copies of other types); only fa_prefill_tma_kernel writes them
 };
 
 // prefill tiles on the 5th generation tensor cores (fa_prefill_sm100.cu)
 bool fa_prefill_sm100_supported(const FaParams &p, bool kv16);
 uint32_t fa_prefill_sm100_splits(const FaParams &p, uint32_t sms);  // key splits (part_o, part_lse, then fa_combine_kernel)
+constexpr int FA_NO_MAP = 1;  // the launches below: nothing was launched, the driver refuses a tensor map
 int fa_prefill_sm100_launch(const FaParams &p, bool bf16, cudaStream_t stream);
 
 // Tensor maps of K and V (boxes of 64 elements x `keys` keys, 128-byte swizzle; past the head dim and past the last key zeros

@@ -1740,7 +1740,7 @@ static bool kv_dims_of(const FaParams &p, KvDims *k, KvDims *v) {
 
 bool fa_kv_maps(const FaParams &p, bool bf16, uint32_t keys, CUtensorMap *tm_k, CUtensorMap *tm_v, uint32_t *order) {
     KvDims k, v;
-    if (!kv_dims_of(p, &k, &v)) return false;
+    if (p.no_maps || !kv_dims_of(p, &k, &v)) return false;
     if (!tm_k) return true;
     *order = k.order | (v.order << 8);
     return make_kv_map(tm_k, k, p.k, bf16, p.d, keys) && make_kv_map(tm_v, v, p.v, bf16, p.d, keys);
@@ -1803,13 +1803,12 @@ static int pf_opt_in(K kern, uint32_t bytes, bool (&done)[16]) {
 
 template <int HD, bool BF16>
 static int fa_prefill_tma_launch(const FaParams &p, cudaStream_t stream) {
+    CUtensorMap tm_k, tm_v, tm_q;
+    P3Grid gr;
+    if (!fa_kv_maps(p, BF16, P3_BN, &tm_k, &tm_v, &gr.tm_order) || !make_q_map(&tm_q, p, BF16)) return FA_NO_MAP;
     static thread_local bool done[16] = {};
     const int rc = pf_opt_in(fa_prefill_tma_kernel<HD, BF16>, P3<HD>::SMEM, done);
     if (rc) return rc;
-    CUtensorMap tm_k, tm_v, tm_q;
-    P3Grid gr;
-    if (!fa_kv_maps(p, BF16, P3_BN, &tm_k, &tm_v, &gr.tm_order) || !make_q_map(&tm_q, p, BF16))
-        return set_error(B200_ERR_LAUNCH, "flash_attn (tcgen05 tiles): the driver refuses a tensor map");
     const uint64_t rows = (uint64_t)p.lq * p.group, pair_bytes = std::max<uint64_t>((uint64_t)p.lk * p.d * 4, 1);
     gr.tiles = (uint32_t)((rows + P3_ROWS - 1) / P3_ROWS);
     gr.pairs = p.b * p.hkv;

@@ -222,6 +222,26 @@ def test_outputs_off_a_boundary_stay_on_the_general_kernel(pkg):
         assert (got >= 2 * 512 * hq * 129 * 4) == need, (hq, kv, o, got)
 
 
+def test_without_tensor_maps_the_general_kernels_are_launched(pkg):
+    """Without a driver no tensor map can be encoded: a call that the map-based kernels would serve goes on to a kernel that needs
+    none (whose launch then fails here for want of a device), instead of failing over the map. Pointers are never read."""
+    import pytest
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip("for machines without a driver")
+    A = pkg._abi
+    for lq, d, dt in ((1, 128, A.BF16), (2, 64, A.F16), (40, 64, A.BF16), (600, 128, A.BF16)):
+        a = A.FaArgs()
+        a.q = a.k = a.v = a.o = a.workspace = 1 << 20
+        a.workspace_bytes = 1 << 30
+        a.b, a.lq, a.lk, a.hq, a.hkv, a.d, a.total_q = 1, lq, 700, 4, 2, d, lq
+        a.q_strides, a.k_strides, a.v_strides = (A.u64x3(n * h * d, h * d, d) for n, h in ((lq, 4), (700, 2), (700, 2)))
+        a.q_dtype = a.kv_dtype = dt
+        a.scale, a.k_descale, a.v_descale, a.wl, a.wr = 0.1, 1.0, 1.0, -1, 0
+        assert A.lib().b200_flash_attn(C.byref(a), None) == A.ERR_LAUNCH
+        assert b"map" not in A.lib().b200_last_error(), (lq, d, A.lib().b200_last_error())
+
+
 def test_paged_dense_attention_argument_errors_without_gpu(pkg):
     """The checks of the paged entry points run before anything touches the device (candle-nn/src/flash_attn.rs:650-689,
     candle-flash-attn/src/lib.rs:357-392)."""
