@@ -341,11 +341,17 @@ def _kv_unpack(k_rows, v_rows, kq: TurboQuantizer, vq: Optional[TurboQuantizer],
 
 
 _WORKSPACES = {}
+_WORKSPACE_KEPT = 32 << 20
 
 
 def _workspace(device, nbytes: int) -> torch.Tensor:
-    """One growing scratch buffer per (device, stream): calls on one stream are ordered, so they
-    can share it; the reference allocates the split buffers per call (accel.rs:190-199)."""
+    """Scratch for a call on the current stream. Up to _WORKSPACE_KEPT bytes it is one growing buffer per (device, stream): calls
+    on one stream are ordered, so they can share it (the reference allocates the split buffers per call, accel.rs:190-199).
+    Larger ones (16-bit copies of f32 tensors take up to 256 MB) come from torch's allocator and return to it after the call,
+    in the order of the stream. So does the scratch of a call that is being captured: it belongs to the graph's own pool,
+    where a shared buffer would be replaced by a later, larger one while the graph still writes to it."""
+    if nbytes > _WORKSPACE_KEPT or torch.cuda.is_current_stream_capturing():
+        return torch.empty((nbytes + 15) // 16 * 16, dtype=torch.uint8, device=device)
     key = (device, _stream(device))
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:

@@ -242,6 +242,21 @@ def test_without_tensor_maps_the_general_kernels_are_launched(pkg):
         assert b"map" not in A.lib().b200_last_error(), (lq, d, A.lib().b200_last_error())
 
 
+def test_shared_scratch_is_bounded_and_stays_out_of_graphs(pkg, monkeypatch):
+    import torch
+    TQ, dev, capturing = pkg.turbo_quant, torch.device("cpu"), [False]
+    monkeypatch.setattr(TQ, "_WORKSPACES", {})
+    monkeypatch.setattr(TQ, "_stream", lambda device: 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    small = TQ._workspace(dev, 1000)
+    assert TQ._workspace(dev, 2000) is small
+    capturing[0] = True
+    assert TQ._workspace(dev, 1000) is not small
+    capturing[0] = False
+    assert TQ._workspace(dev, 100 << 20).numel() >= 100 << 20  # a call over copies: served, not kept
+    assert sum(t.numel() for t in TQ._WORKSPACES.values()) <= 32 << 20
+
+
 def test_paged_dense_attention_argument_errors_without_gpu(pkg):
     """The checks of the paged entry points run before anything touches the device (candle-nn/src/flash_attn.rs:650-689,
     candle-flash-attn/src/lib.rs:357-392)."""

@@ -478,6 +478,27 @@ def test_key_splits_keep_nan(P, lq, lk, d, dt):
         k[0, key, 1, 5] = old
 
 
+def test_captured_chunk_keeps_its_scratch(P):
+    """A chunk that is split along the keys, captured in a graph; then a larger call on the capture stream, whose scratch replaces a
+    shared buffer, and new tensors in the memory that comes free: the graph still writes its own scratch alone."""
+    g = torch.Generator(device="cuda:0").manual_seed(5)
+    data = lambda lq, hq, lk: [torch.randn((1, n, h, 128), generator=g, device="cuda:0", dtype=torch.bfloat16) for n, h in ((lq, hq), (lk, 2), (lk, 2))]
+    call = lambda x: P.flash_attn.flash_attn_with_config(*x, cfg_of(P, 128, -1, 0))
+    small, large = data(40, 4, 3000), data(300, 8, 9000)
+    want, st, graph = call(small).clone(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        call(small)
+        with torch.cuda.graph(graph, stream=st):
+            out = call(small)
+        call(large)
+        others = [torch.full((1 << 20,), 7, dtype=torch.uint8, device="cuda:0") for _ in range(8)]
+        out.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and all(bool((t == 7).all()) for t in others)
+
+
 @pytest.mark.parametrize("lq,hq,lk,dt", [(1, 4, 3000, torch.bfloat16), (64, 8, 4000, torch.bfloat16), (80, 2, 700, torch.float32)])
 def test_workspace_at_an_odd_address(P, lq, hq, lk, dt):
     """Key splits and copies in a workspace that starts four bytes past a boundary: the same bits as in an aligned one."""
