@@ -1352,6 +1352,9 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                 if (it.ntiles == 0) continue;
                 int t0, t1, lo, hi;
                 p3_group(p, it, g, t0, t1, lo, hi);
+                // the steps of 16 keys that O_g += P_g V takes: all eight, but the first tile starts at the one in the low four bits and the
+                // last ends before the one above them
+                const int steps = (((lo - it.t_lo) >> 4) - 8 * t0) | (((hi - it.t_lo + 15) >> 4) - 8 * (t1 - 1)) << 4;
                 if (!(ok = p3_wait(bar0 + 8 * C::QF, nq & 1, abort_flag))) break;
                 ++nq;
                 if (t0 == t1 && elect_one()) mbar_arrive(&bars[C::QE]);
@@ -1379,23 +1382,34 @@ __global__ void __launch_bounds__(P3_THREADS, 1) fa_prefill_tma_kernel(const FaP
                         if (!ok) break;
                         scores(sn, t + 1 == t1 - 1);
                     }
+                    const uint64_t v_desc = tc_desc_sw128(sbase + C::SM_V + st * C::T_BYTES, C::T_HALF, 1024);
+                    const bool whole = (t != t0 || (steps & 15) == 0) && (t != t1 - 1 || steps >> 4 == 8);
+                    auto some = [&](int from, int to) {  // a tile of which steps are left out
+                        const int ks0 = t == t0 ? steps & 15 : 0, ks1 = t == t1 - 1 ? steps >> 4 : 8;
+#pragma unroll 1
+                        for (int ks = max(from, ks0); ks < min(to, ks1); ++ks) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 128), IPV, t > t0 || ks > ks0 ? 1u : 0u);
+                    };
                     ok = p3_wait(bar0 + 8 * (C::VF + st), ph, abort_flag) && p3_wait(bar0 + 8 * (C::P0 + g), sc & 1, abort_flag);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint64_t v_desc = tc_desc_sw128(sbase + C::SM_V + st * C::T_BYTES, C::T_HALF, 1024);
-                    const int j0 = it.t_lo + t * P3_BN, ks0 = t == t0 ? (lo - j0) / 16 : 0, ks1 = t == t1 - 1 ? (hi - j0 + 15) / 16 : 8;
                     if (elect_one()) {  // O_g += P_g(t) V(t): the first 96 keys while the others' exponentials run
+                        if (whole) {
 #pragma unroll
-                        for (int ks = 0; ks < 6; ++ks)
-                            if (ks >= ks0 && ks < ks1) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, (t > t0 || ks > ks0) ? 1u : 0u);
+                            for (int ks = 0; ks < 6; ++ks) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, (t > t0 || ks > 0) ? 1u : 0u);
+                        } else {
+                            some(0, 6);
+                        }
                     }
                     __syncwarp();
                     if (!(ok = p3_wait(bar0 + 8 * (C::P1 + g), sc & 1, abort_flag))) break;
                     tc_fence_after();
                     if (elect_one()) {
+                        if (whole) {
 #pragma unroll
-                        for (int ks = 6; ks < 8; ++ks)
-                            if (ks >= ks0 && ks < ks1) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, (t > t0 || ks > ks0) ? 1u : 0u);
+                            for (int ks = 6; ks < 8; ++ks) tc_mma_ts(o_t, p_t + ks * 8, v_desc + (uint64_t)(ks * 2048 >> 4), IPV, 1u);
+                        } else {
+                            some(6, 8);
+                        }
                         tc_commit(bar0 + 8 * (C::VE + st));
                         if (C::EARLY) tc_commit(bar0 + 8 * (C::PV + g));
                         if (t == t1 - 1) tc_commit(bar0 + 8 * (C::O + g));
