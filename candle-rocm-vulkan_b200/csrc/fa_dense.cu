@@ -568,6 +568,7 @@ static void fa_as_copies(FaParams &p, bool bf16, char *q, char *k, char *v, int 
     p.q_sb = p.q_ss * p.lq, p.k_sb = p.v_sb = p.k_ss * p.lk;
     p.q_dtype = bf16 ? B200_BF16 : B200_F16;
     p.kv_kind = 0;
+    p.copies = 1;
     p.o_f32 = out_dtype == B200_F32;
 }
 

@@ -27,7 +27,8 @@ struct FaParams {
     const uint32_t *pg_keys;
     uint32_t n_pages;
     uint32_t no_maps;  // the driver has refused a tensor map of this call's tensors: kernels that need none
-    uint32_t o_f32;  // outputs are f32 (q, k, v are 16-bit copies of other types); only fa_prefill_tma_kernel writes them
+    uint32_t copies;  // q, k and v are 16-bit copies of the call's tensors
+    uint32_t o_f32;  // outputs are f32 (over copies); only fa_prefill_tma_kernel writes them
 };
 
 // prefill tiles on the 5th generation tensor cores (fa_prefill_sm100.cu)

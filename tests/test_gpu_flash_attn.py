@@ -590,6 +590,23 @@ def test_varlen_rows_beside_infinities(P, hq, hkv, d):
         assert (out[a:e].double() - want).norm() <= 2.0 ** -8 * want.norm()
 
 
+@pytest.mark.parametrize("lq,d,dt", [(300, 64, torch.float16), (300, 64, torch.bfloat16), (300, 96, torch.float16), (100, 128, torch.bfloat16),
+                                     (600, 128, torch.float32), (300, 64, torch.float32)])
+def test_the_largest_weight_is_one(P, lq, d, dt):
+    """One key of the second tile has the only value, and a score of up to 2^7.9 times the others'. Its weight is the largest, 1, which
+    16 bits hold exactly, so the output is rounded once (f32: not at all). Against a maximum that lags, the weight itself is
+    rounded too, and the error exceeds half an ulp in the 2-norm (1.25 of it in f16, 1.11 in bf16)."""
+    g = torch.Generator(device="cuda:0").manual_seed(d)
+    q, k, v = (torch.zeros((1, n, 1, d), device="cuda:0", dtype=dt) for n in (lq, 256, 256))
+    q[0, :, 0, 0] = ((torch.rand(lq, generator=g, device="cuda:0") * 7.4 + 0.5) * np.log(2) * np.sqrt(d)).to(dt)
+    k[0, 200, 0, 0] = 1
+    v[0, 200, 0] = torch.randn(d, generator=g, device="cuda:0").to(dt)
+    x, y, z = (t.to(torch.float16 if dt == torch.float32 else dt) for t in (q, k, v))
+    out = P.flash_attn.flash_attn_with_config(q, k, v, cfg_of(P, d))
+    want = _plain(x[0], y[0], z[0], 1.0 / np.sqrt(d), -1, -1)
+    assert (out[0].double() - want).norm() <= {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12, torch.float32: 2.0 ** -18}[dt] * want.norm()
+
+
 # an item of the tiles is 256 packed rows: 64 tokens of a group of four, two groups of 32; token i sees the keys up to i + 100
 @pytest.mark.parametrize("wl,bad,rows", [(-1, slice(164, 300), slice(0, 64)), (-1, slice(144, 300), slice(0, 32)), (-1, slice(231, 232), slice(0, 128)),
                                          (50, slice(0, 50), slice(0, 200)), (50, slice(0, 82), slice(32, 200)), (50, slice(82, 114), slice(64, 200))])
