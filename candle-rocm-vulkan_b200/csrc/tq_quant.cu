@@ -337,7 +337,9 @@ __device__ __forceinline__ void load16(const char *src, int l8, float (&x)[16]) 
 // n / d for n < 2^31 with the invariants of fastdiv_init
 __device__ __forceinline__ uint32_t fastdiv(uint32_t n, uint32_t mul, uint32_t shr) { return (__umulhi(n, mul) + n) >> shr; }
 
-template <int DT>
+// CODES: a side of the call is in a codebook format. Without, their code is left out: its registers and its prologue cost the block-scaled
+// formats 0.1 us of the 1.8 of a few rows.
+template <int DT, bool CODES>
 __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const QuantParams p) {
     const QuantSideParams &sp = p.side[blockIdx.y];
     const int lane = threadIdx.x & 31, l8 = lane & 7;
@@ -345,11 +347,12 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
     const uint32_t mode = sp.mode;
     // codebook formats: the boundaries between neighbouring codes, ascending; 15 words in 15 banks, so no two lanes collide
     __shared__ float bound[16];
-    if (mode <= B200_TURBO_PROD) {
+    float b7 = 0.0f, b3 = 0.0f, b11 = 0.0f;  // (codebook formats of four bits)
+    if (CODES && mode <= B200_TURBO_PROD) {
         if (threadIdx.x < 16) bound[threadIdx.x] = threadIdx.x < (1u << sp.cb) - 1u ? sp.tab[16 + threadIdx.x] : 0.0f;
         __syncthreads();
+        b7 = bound[7], b3 = bound[3], b11 = bound[11];
     }
-    const float b7 = bound[7], b3 = bound[3], b11 = bound[11];  // (codebook formats of four bits)
     after_prev_begin(p);
     for (uint32_t base = (blockIdx.x * Q128_WARPS + (threadIdx.x >> 5)) * Q128_RPW; base < rows; base += gridDim.x * Q128_WARPS * Q128_RPW) {
         bool live = base + (lane >> 3) < rows;  // a row past the end repeats the last one and stores nothing
@@ -400,7 +403,7 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
             for (int k = 0; k < 16; ++k) x[k] *= s;
         }
 
-        if (mode <= B200_TURBO_PROD) {
+        if (CODES && mode <= B200_TURBO_PROD) {
             // Sum of squares in the order of the reference's 128 lanes (red[t] += red[t + s], s = 64 ... 1): index bits 6, 5, 4
             // are the row's lanes, and each step leaves half of the residues with either lane (residue bit 3 with lane bit 2,
             // and so on); bits 3, 2, 1 then lie across the lanes, bit 0 in the register.
@@ -817,6 +820,10 @@ static bool rows128_takes(const QuantParams &p, int sides) {
     const uint64_t vec = p.src_dtype == B200_F32 ? 3 : 7;  // elements per 16 bytes - 1
     for (int s = 0; s < sides; ++s) {
         const QuantSideParams &sp = p.side[s];
+        // The search for codes of one to three bits is a chain of loads per element: few rows go faster with a warp each (three bits, f32
+        // rows of keys and values, us, a warp per row and here: 26 rows 3.8, 4.7; 337 rows 3.4, 4.0; 912 rows 4.6, 4.8; two
+        // bits, 1 208 rows 3.9, 3.8; three bits, 6 124 rows 14.3, 7.6).
+        if (sp.mode <= B200_TURBO_PROD && sp.cb != 4 && (uint64_t)p.nb * p.nh * p.nt * sides < 2048) return false;
         if (((uintptr_t)sp.src & 15) || (sp.s_b & vec) || (sp.s_h & vec) || (sp.s_t & vec)) return false;
         if (sp.rot == B200_ROT_HADAMARD && ((uintptr_t)sp.signs & 15)) return false;
         // NVFP4 code words are stored in pairs
@@ -842,26 +849,32 @@ static int launch_maybe_after_prev(void (*kern)(const QuantParams), dim3 grid, d
     return check_launch("tq_quantize");
 }
 
+template <bool CODES>
+static int launch_rows128(const QuantParams &p, int sides, cudaStream_t stream) {
+    QuantParams q = p;
+    fastdiv_init(p.nt, q.nt_mul, q.nt_shr);
+    fastdiv_init(p.nh, q.nh_mul, q.nh_shr);
+    const uint64_t rows = (uint64_t)p.nb * p.nh * p.nt, per_block = Q128_WARPS * Q128_RPW;
+    // as many blocks as are resident at once, shared by the sides
+    static const int resident = [] {
+        int per_sm = 4, sms = 148, dev = 0;
+        cudaGetDevice(&dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quant_rows128_kernel<B200_BF16, CODES>, Q128_WARPS * 32, 0);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        return std::max(per_sm, 1) * std::max(sms, 1);
+    }();
+    const dim3 grid((unsigned)std::min<uint64_t>((rows + per_block - 1) / per_block, (uint64_t)std::max(resident / sides, 1)), sides), block(Q128_WARPS * 32);
+    if (p.src_dtype == B200_F32) return launch_maybe_after_prev(quant_rows128_kernel<B200_F32, CODES>, grid, block, stream, q);
+    if (p.src_dtype == B200_F16) return launch_maybe_after_prev(quant_rows128_kernel<B200_F16, CODES>, grid, block, stream, q);
+    return launch_maybe_after_prev(quant_rows128_kernel<B200_BF16, CODES>, grid, block, stream, q);
+}
+
 static int launch_quant(const QuantParams &p, int sides, cudaStream_t stream) {
     const uint64_t rows = (uint64_t)p.nb * p.nh * p.nt;
     if (rows == 0) return B200_OK;
     if (rows128_takes(p, sides)) {
-        QuantParams q = p;
-        fastdiv_init(p.nt, q.nt_mul, q.nt_shr);
-        fastdiv_init(p.nh, q.nh_mul, q.nh_shr);
-        const uint64_t per_block = Q128_WARPS * Q128_RPW;
-        // as many blocks as are resident at once, shared by the sides
-        static const int resident = [] {
-            int per_sm = 4, sms = 148, dev = 0;
-            cudaGetDevice(&dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quant_rows128_kernel<B200_BF16>, Q128_WARPS * 32, 0);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            return std::max(per_sm, 1) * std::max(sms, 1);
-        }();
-        const dim3 grid((unsigned)std::min<uint64_t>((rows + per_block - 1) / per_block, (uint64_t)std::max(resident / sides, 1)), sides), block(Q128_WARPS * 32);
-        if (p.src_dtype == B200_F32) return launch_maybe_after_prev(quant_rows128_kernel<B200_F32>, grid, block, stream, q);
-        if (p.src_dtype == B200_F16) return launch_maybe_after_prev(quant_rows128_kernel<B200_F16>, grid, block, stream, q);
-        return launch_maybe_after_prev(quant_rows128_kernel<B200_BF16>, grid, block, stream, q);
+        const bool codes = p.side[0].mode <= B200_TURBO_PROD || (sides > 1 && p.side[1].mode <= B200_TURBO_PROD);
+        return codes ? launch_rows128<true>(p, sides, stream) : launch_rows128<false>(p, sides, stream);
     }
     const unsigned gx = (unsigned)std::min<uint64_t>((rows + QW - 1) / QW, 148ull * 64);
     const dim3 grid(gx, sides), block(QW * 32);

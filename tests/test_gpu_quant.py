@@ -293,3 +293,20 @@ def test_codebook_rows_of_128_on_both_kernels(name):
         odd = torch.empty(a.numel() + 1, dtype=dt, device="cuda:0")[1:].view(a.shape)
         odd.copy_(a)
         assert torch.equal(q.quantize_rotated_rows(a), q.quantize_rotated_rows(odd)), dt
+
+
+@pytest.mark.parametrize("name", ["turbo1", "turbo2", "turbo3"])
+@pytest.mark.parametrize("rotation", ["none", "hadamard"])
+def test_codebook_rows_at_once_and_in_pieces(P, name, rotation):
+    """Few rows of one to three bits are packed by a warp each, many by eight lanes each: the same bytes, zero rows, infinities
+    and NaN included."""
+    f = P.QuantFormat.parse(name)
+    g = torch.Generator(device="cuda:0").manual_seed(3)
+    k, v = (torch.randn((1, 2, 1500, 128), generator=g, device="cuda:0", dtype=torch.bfloat16) for _ in range(2))
+    k[0, 0, 5] = 0.0
+    k[0, 0, 6, 9], k[0, 1, 700, 100], v[0, 0, 1499, 0] = float("inf"), float("nan"), -float("inf")
+    caches = [P.TurboKvCache(f, f, 128, rotation, 42, 1500) for _ in range(2)]
+    caches[0].append(k, v)
+    for at in range(0, 1500, 100):
+        caches[1].append(k[:, :, at:at + 100], v[:, :, at:at + 100])
+    assert torch.equal(caches[0].k, caches[1].k) and torch.equal(caches[0].v, caches[1].v)
