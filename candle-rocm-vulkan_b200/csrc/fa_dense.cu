@@ -623,8 +623,9 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false, bool may
     const uint64_t ctas = (uint64_t)row_tiles * a->hkv * std::max<uint32_t>(a->b, 1);
     pl.decode_tma = fa_decode_tma_takes(p, paged);
     uint32_t splits = 1;
-    if (ctas < 2ull * sms && a->lk > 2 * FA_BN) {
-        const uint64_t by_occ = (2ull * sms + ctas - 1) / ctas, by_keys = (a->lk + 4 * FA_BN - 1) / (4 * FA_BN);
+    // fa_decode_tma_kernel: as many splits as its two blocks per SM take at once (136 blocks in three splits were a wave and a third)
+    if ((pl.decode_tma ? 2 * ctas <= 2ull * sms : ctas < 2ull * sms) && a->lk > 2 * FA_BN) {
+        const uint64_t by_occ = pl.decode_tma ? 2ull * sms / ctas : (2ull * sms + ctas - 1) / ctas, by_keys = (a->lk + 4 * FA_BN - 1) / (4 * FA_BN);
         splits = (uint32_t)std::min<uint64_t>(std::min(by_occ, by_keys), 64);
     } else if (rows <= 16 && a->lk >= 16 * FA_BN) {
         // decode with enough blocks to fill the device: up to four key splits where they make the blocks a better fit to
