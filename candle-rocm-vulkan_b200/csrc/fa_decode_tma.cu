@@ -17,6 +17,7 @@
 // walked the splits one dependent load at a time.
 //
 // Every wait is bounded; one that runs out raises the flag that b200_device_wait_status reads.
+#include <algorithm>
 #include <cuda.h>
 
 #include "common.cuh"
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 2) fa_decode_tma_kernel(const F
                 float x = s[n][i] * sc2;
                 if (!full) {
                     const int j = j0 + 8 * n + 2 * c + (i & 1);
-                    if (!plain) {
+                    if (!plain && (e == 0 || R > 8)) {  // (rows 8 to 15 of a call that has none need no soft cap)
                         x = s[n][i] * sc;
                         if (p.softcap > 0.0f) x = p.softcap * tanhf(x / p.softcap);
                         if (slope[e] != 0.0f) x -= slope[e] * fabsf((float)(r_pos[e] - j));
@@ -349,7 +350,19 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 2) fa_decode_tma_kernel(const F
     if (p.n_splits > 1 && ch == 0) p.part_lse[prow] = L == 0.0f ? -INFINITY : M * FD_LN2 + logf(L);  // a NaN stays one
 }
 
-bool fa_decode_tma_takes(const FaParams &p, bool paged) {
+bool fa_decode_tma_takes(const FaParams &p, bool paged, uint32_t sms) {
+    const uint64_t rows = (uint64_t)p.lq * p.group, blocks = (uint64_t)p.b * p.hkv;
+    const uint64_t keys = p.wl >= 0 ? std::min<uint64_t>(p.lk, (uint64_t)p.wl + p.lq) : p.lk;
+    // A soft cap costs more than the copies: where the tiles of 32 keys leave a warp more of a few keys than its share, the general
+    // kernel's four warps of 16 keys are ahead (us, there and here: up to eight rows, 20 keys 6.3, 6.7; 9 to 16 rows, 11 keys 8.3, 9.7;
+    // 132 keys 11.3, 12.4; eight rows, 126 keys 9.5, 8.5).
+    if ((p.softcap > 0.0f || p.alibi) && p.d <= 64 && keys <= (rows > 8 ? 192u : 64u)) return false;
+    // The general kernel has four blocks per SM up to head dim 64 and three up to 128, this one two. Calls over few keys that are one
+    // wave there and two here are ahead there (us, there and here: 432 blocks, 1 row, 58 keys of 64: 6.5, 9.2; 384 blocks, 4 rows,
+    // 108 keys 8.6, 10.4, but 468 blocks, 2 rows, 252 keys 13.5, 12.1; 16 rows: 327 blocks, 558 keys of 64 20.1, 22.1; 416 blocks,
+    // 34 keys of 128 16.6, 19.9; 390 blocks, 428 keys of 96 27.4, 32.0; 8 rows: 440 blocks, 52 keys of 96 11.5, 15.4; 432 blocks, 384 keys of 128 24.4, 26.4;
+    // 336 blocks, 665 keys 39.7, 42.0; 4 rows, 424 blocks, 681 keys of 96: equal).
+    if (blocks > 2ull * sms && blocks <= (p.d <= 64 ? 4ull : 3ull) * sms && keys <= (rows <= 8 && p.d <= 64 ? 192u : 704u)) return false;
     return p.kv_kind == 0 && !p.varlen && p.d <= 128 && p.lk > 0 && p.lk < (1u << 31) && (uint64_t)p.lq * p.group <= 16 &&
            (paged || fa_kv_maps(p, false, 0, nullptr, nullptr, nullptr));
 }

@@ -621,7 +621,7 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false, bool may
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint64_t ctas = (uint64_t)row_tiles * a->hkv * std::max<uint32_t>(a->b, 1);
-    pl.decode_tma = fa_decode_tma_takes(p, paged);
+    pl.decode_tma = fa_decode_tma_takes(p, paged, (uint32_t)sms);
     uint32_t splits = 1;
     // fa_decode_tma_kernel: as many splits as its two blocks per SM take at once (136 blocks in three splits were a wave and a third)
     if ((pl.decode_tma ? 2 * ctas <= 2ull * sms : ctas < 2ull * sms) && a->lk > 2 * FA_BN) {

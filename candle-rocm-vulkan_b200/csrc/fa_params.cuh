@@ -43,7 +43,7 @@ int fa_prefill_sm100_launch(const FaParams &p, bool bf16, cudaStream_t stream);
 bool fa_kv_maps(const FaParams &p, bool bf16, uint32_t keys, CUtensorMap_st *k, CUtensorMap_st *v, uint32_t *order);
 
 // decode over 16-bit K / V by tensor copies (fa_decode_tma.cu): grid (1, hkv, b * n_splits)
-bool fa_decode_tma_takes(const FaParams &p, bool paged);
+bool fa_decode_tma_takes(const FaParams &p, bool paged, uint32_t sms);
 int fa_decode_tma_launch(const FaParams &p, bool bf16, dim3 grid, cudaStream_t stream);
 int fa_decode_wait_status();
 int fa_decode_wait_clear();

@@ -435,6 +435,33 @@ def test_decode_by_tensor_copies_at_its_edges(P, b, lq, lk, hq, hkv, d, wl, wr, 
     assert (out.double() - want).norm() <= 2 * {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dt] * want.norm()
 
 
+# soft-capped decode: up to eight rows and more, at and beside the number of keys where the general kernel takes over
+@pytest.mark.parametrize("lq,hq,hkv,lk,d", [(1, 4, 4, 11, 64), (1, 8, 1, 300, 96), (2, 8, 1, 11, 64), (1, 4, 4, 65, 64), (2, 8, 1, 192, 64), (2, 8, 1, 193, 64), (3, 6, 2, 129, 128)])
+def test_soft_capped_decode(P, lq, hq, hkv, lk, d):
+    g = torch.Generator(device="cuda:0").manual_seed(lk)
+    q, k, v = (torch.randn((2, n, h, d), generator=g, device="cuda:0", dtype=torch.bfloat16) for n, h in ((lq, hq), (lk, hkv), (lk, hkv)))
+    out = P.flash_attn.flash_attn_with_config(q, k, v, cfg_of(P, d, -1, 0, softcap=1.5))
+    kk, vv = (t.double().transpose(1, 2).repeat_interleave(hq // hkv, 1) for t in (k, v))
+    s = 1.5 * torch.tanh((q.double().transpose(1, 2) @ kk.transpose(2, 3)) * d ** -0.5 / 1.5)
+    s.masked_fill_(torch.arange(lk, device="cuda:0")[None] > torch.arange(lq, device="cuda:0")[:, None] + lk - lq, -torch.inf)
+    want = (torch.softmax(s, -1) @ vv).transpose(1, 2)
+    # weights and output are each rounded once: half an ulp each at most, in the 2-norm
+    assert (out.double() - want).norm() <= 2 * 2.0 ** -9 * want.norm()
+
+
+# more blocks than the tensor-copy kernel takes at once, few keys: at and beside the numbers where the general kernel takes over
+@pytest.mark.parametrize("b,lq,lk,hq,hkv,d,wl", [(100, 1, 192, 12, 3, 64, -1), (100, 1, 193, 12, 3, 64, -1), (150, 2, 704, 16, 2, 72, -1), (150, 2, 705, 16, 2, 72, -1),
+                                                 (75, 1, 900, 4, 4, 40, 100), (149, 1, 50, 8, 4, 64, -1),
+                                                 (50, 1, 704, 16, 8, 128, -1), (50, 1, 705, 16, 8, 128, -1)])
+def test_decode_of_many_short_sequences(P, b, lq, lk, hq, hkv, d, wl):
+    g = torch.Generator(device="cuda:0").manual_seed(lk)
+    q, k, v = (torch.randn((b, n, h, d), generator=g, device="cuda:0", dtype=torch.bfloat16) for n, h in ((lq, hq), (lk, hkv), (lk, hkv)))
+    out = P.flash_attn.flash_attn_with_config(q, k, v, cfg_of(P, d, wl, 0))
+    want = torch.stack([_plain(*x, 1.0 / np.sqrt(d), wl, 0) for x in zip(q, k, v)])
+    # weights and output are each rounded once: half an ulp each at most, in the 2-norm
+    assert (out.double() - want).norm() <= 2 * 2.0 ** -9 * want.norm()
+
+
 # few work items: split along the keys (whole tiles, a last split that is short or empty, windows that leave splits without keys
 # for some rows, 17 rows and more), and the same call without a workspace, which goes unsplit
 @pytest.mark.parametrize("b,lq,lk,hq,hkv,d,wl,wr", [(1, 17, 2000, 1, 1, 64, -1, 0), (1, 33, 5000, 8, 1, 128, -1, 0), (2, 300, 4111, 8, 2, 72, 2500, 50),
