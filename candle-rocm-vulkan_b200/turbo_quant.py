@@ -74,6 +74,7 @@ def _dtype_id(t: torch.Tensor) -> int:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", torch.cuda.is_current_stream_capturing)
 
 
 def _stream(device) -> int:
@@ -344,15 +345,15 @@ _WORKSPACES = {}
 _WORKSPACE_KEPT = 32 << 20
 
 
-def _workspace(device, nbytes: int) -> torch.Tensor:
+def _workspace(device, nbytes: int, stream: Optional[int] = None) -> torch.Tensor:
     """Scratch for a call on the current stream. Up to _WORKSPACE_KEPT bytes it is one growing buffer per (device, stream): calls
     on one stream are ordered, so they can share it (the reference allocates the split buffers per call, accel.rs:190-199).
     Larger ones (16-bit copies of f32 tensors take up to 256 MB) come from torch's allocator and return to it after the call,
     in the order of the stream. So does the scratch of a call that is being captured: it belongs to the graph's own pool,
     where a shared buffer would be replaced by a later, larger one while the graph still writes to it."""
-    if nbytes > _WORKSPACE_KEPT or torch.cuda.is_current_stream_capturing():
+    if nbytes > _WORKSPACE_KEPT or _capturing():
         return torch.empty((nbytes + 15) // 16 * 16, dtype=torch.uint8, device=device)
-    key = (device, _stream(device))
+    key = (device, _stream(device) if stream is None else stream)
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
@@ -764,12 +765,12 @@ class TurboKvCache:
             q.data_ptr(), out.data_ptr(), dt, dt, *q.stride()[:3], *out.stride()[:3], k.data_ptr(), v.data_ptr(), *k.stride()[:3], *v.stride()[:3],
             0, 0, 0, b, lq, lk, hq, hkv, d, *kq.side_fields(), *vq.side_fields(), cfg.softmax_scale, cfg.softcap or 0.0, wl, wr, 0, 0, cfg.splits,
             0, 0, 0, 0, 0, 0))
-        lib, ref = A.lib(), C.byref(args)
+        lib, ref, stream = A.lib(), C.byref(args), _stream(q.device)
         nbytes = lib.b200_tq_attention_workspace_bytes(ref)
         if nbytes:
-            ws = _workspace(q.device, nbytes)
+            ws = _workspace(q.device, nbytes, stream)
             args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
-        rc = lib.b200_tq_attention(ref, _stream(q.device))  # nbytes 0: reports why the call cannot be planned
+        rc = lib.b200_tq_attention(ref, stream)  # nbytes 0: reports why the call cannot be planned
         if rc:
             A.check(rc)
         return out

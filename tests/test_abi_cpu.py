@@ -247,7 +247,7 @@ def test_shared_scratch_is_bounded_and_stays_out_of_graphs(pkg, monkeypatch):
     TQ, dev, capturing = pkg.turbo_quant, torch.device("cpu"), [False]
     monkeypatch.setattr(TQ, "_WORKSPACES", {})
     monkeypatch.setattr(TQ, "_stream", lambda device: 0)
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    monkeypatch.setattr(TQ, "_capturing", lambda: capturing[0])
     small = TQ._workspace(dev, 1000)
     assert TQ._workspace(dev, 2000) is small
     capturing[0] = True
