@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import _abi as A
-from .turbo_quant import FlashAttnConfig, TurboQuantizer, _dtype_id, _need_cuda, _stream, _workspace
+from .turbo_quant import FlashAttnConfig, TurboQuantizer, _call_workspace, _dtype_id, _need_cuda, _stream
 
 _FP8 = getattr(torch, "float8_e4m3fn", None)
 
@@ -93,7 +93,7 @@ def _fa_args(q, k, v, cfg: FlashAttnConfig, cu_q=None, cu_k=None, max_q=0, max_k
     a.alibi, a.alibi_bstride = (alibi.data_ptr() if alibi is not None else None), abs_
     a.varlen, a.total_q = int(varlen), total_q
     nbytes = A.lib().b200_flash_attn_workspace_bytes(C.byref(a))
-    ws = _workspace(q.device, nbytes) if nbytes else None
+    ws = _call_workspace(q.device, nbytes) if nbytes else None
     a.workspace, a.workspace_bytes = (ws.data_ptr(), ws.numel()) if ws is not None else (None, 0)
     keep = (q, k, v, cu_q, cu_k, alibi, ws)
     return a, out, keep
@@ -249,7 +249,7 @@ def flash_attn_blocks(q, blocks, cfg: FlashAttnConfig) -> torch.Tensor:
     nbytes = A.lib().b200_flash_attn_paged_workspace_bytes(C.byref(a), len(live))
     if nbytes == 0:
         A.check(A.lib().b200_flash_attn_paged(C.byref(a), pages.data_ptr(), len(live), _stream(q.device)))  # raises with the reason
-    ws = _workspace(q.device, nbytes)
+    ws = _call_workspace(q.device, nbytes)
     a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
     A.check(A.lib().b200_flash_attn_paged(C.byref(a), pages.data_ptr(), len(live), _stream(q.device)))
     return out.transpose(1, 2)

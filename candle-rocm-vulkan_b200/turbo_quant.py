@@ -342,23 +342,36 @@ def _kv_unpack(k_rows, v_rows, kq: TurboQuantizer, vq: Optional[TurboQuantizer],
 
 
 _WORKSPACES = {}
+_WORKSPACES_OUTGROWN = []
 _WORKSPACE_KEPT = 32 << 20
 
 
 def _workspace(device, nbytes: int, stream: Optional[int] = None) -> torch.Tensor:
     """Scratch for a call on the current stream. Up to _WORKSPACE_KEPT bytes it is one growing buffer per (device, stream): calls
     on one stream are ordered, so they can share it (the reference allocates the split buffers per call, accel.rs:190-199).
-    Larger ones (16-bit copies of f32 tensors take up to 256 MB) come from torch's allocator and return to it after the call,
-    in the order of the stream. So does the scratch of a call that is being captured: it belongs to the graph's own pool,
-    where a shared buffer would be replaced by a later, larger one while the graph still writes to it."""
-    if nbytes > _WORKSPACE_KEPT or _capturing():
-        return torch.empty((nbytes + 15) // 16 * 16, dtype=torch.uint8, device=device)
+    A graph may have captured the address of a buffer that has become too small, so these stay; sizes double, which makes
+    them one more _WORKSPACE_KEPT in all. Larger requests (16-bit copies of f32 tensors take up to 256 MB) come from torch's
+    allocator and return to it after the call, in the order of the stream."""
+    nbytes = (nbytes + 15) // 16 * 16
+    if nbytes > _WORKSPACE_KEPT:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
     key = (device, _stream(device) if stream is None else stream)
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+        if ws is not None:
+            _WORKSPACES_OUTGROWN.append(ws)
+        size = 1 << 20
+        while size < nbytes:
+            size *= 2
+        ws = torch.empty(size, dtype=torch.uint8, device=device)
         _WORKSPACES[key] = ws
     return ws
+
+
+def _call_workspace(device, nbytes: int) -> torch.Tensor:
+    """The same for calls over dense tensors, but a call that is being captured has scratch of its own, in its graph's memory pool:
+    two graphs captured on one stream may run side by side."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device) if _capturing() else _workspace(device, nbytes)
 
 
 class OutputGather:

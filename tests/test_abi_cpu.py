@@ -242,19 +242,23 @@ def test_without_tensor_maps_the_general_kernels_are_launched(pkg):
         assert b"map" not in A.lib().b200_last_error(), (lq, d, A.lib().b200_last_error())
 
 
-def test_shared_scratch_is_bounded_and_stays_out_of_graphs(pkg, monkeypatch):
+def test_shared_scratch_is_bounded_and_outlives_graphs(pkg, monkeypatch):
     import torch
-    TQ, dev, capturing = pkg.turbo_quant, torch.device("cpu"), [False]
+    TQ, dev, capturing, old = pkg.turbo_quant, torch.device("cpu"), [False], []
     monkeypatch.setattr(TQ, "_WORKSPACES", {})
+    monkeypatch.setattr(TQ, "_WORKSPACES_OUTGROWN", old)
     monkeypatch.setattr(TQ, "_stream", lambda device: 0)
     monkeypatch.setattr(TQ, "_capturing", lambda: capturing[0])
     small = TQ._workspace(dev, 1000)
-    assert TQ._workspace(dev, 2000) is small
+    assert TQ._workspace(dev, 2000) is small and TQ._call_workspace(dev, 2000) is small
     capturing[0] = True
-    assert TQ._workspace(dev, 1000) is not small
+    assert TQ._call_workspace(dev, 1000) is not small
     capturing[0] = False
+    for mb in (2, 3, 5, 9, 20, 32):
+        assert TQ._workspace(dev, mb << 20).numel() >= mb << 20
+    assert old[0] is small  # a graph may hold its address
     assert TQ._workspace(dev, 100 << 20).numel() >= 100 << 20  # a call over copies: served, not kept
-    assert sum(t.numel() for t in TQ._WORKSPACES.values()) <= 32 << 20
+    assert sum(t.numel() for t in [*TQ._WORKSPACES.values(), *old]) <= 64 << 20
 
 
 def test_paged_dense_attention_argument_errors_without_gpu(pkg):
