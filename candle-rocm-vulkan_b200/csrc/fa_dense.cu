@@ -641,8 +641,8 @@ static int fa_plan(const B200FaArgs *a, FaPlan &pl, bool paged = false, bool may
     p.n_splits = 1;
     pl.prefill = !paged && !pl.decode_tma && fa_prefill_sm100_supported(p, kv16);
     // f32 tensors and E4M3 keys: rounded (widened) once into the workspace, then the same tiles. From 64 rows on, where the products
-    // weigh more than the copy; up to 256 MB of copies. f32, us, before and now: 8 x 1000 tokens, 16 heads of 64, 478 -> 81; 2 x 2048, 32 / 8
-    // heads of 128, 1293 -> 113; 64 tokens over 4000 keys, 4 heads, 68 -> 29.
+    // weigh more than the copy; up to 256 MB of copies. f32, us, before and now: 8 x 1000 tokens, 16 heads of 64, 478 -> 85; 2 x 2048, 32 / 8
+    // heads of 128, 1293 -> 120; 64 tokens over 4000 keys, 4 heads, 68 -> 29.
     pl.cast = false;
     const size_t copies = ((size_t)a->b * a->lq * a->hq + 2 * (size_t)a->b * a->lk * a->hkv) * a->d * 2 + 768;
     if (may_copy && !paged && !pl.decode_tma && !pl.prefill && !a->varlen && rows >= 64 && a->d <= 128 && copies <= (256u << 20) && a->b && a->lk &&
@@ -861,8 +861,9 @@ static std::atomic<unsigned> g_fork_next{0};
 extern "C" int b200_fa_prefill_append(const B200FaArgs *fa, const B200KvAppendArgs *append, b200_stream_t stream_) {
     // The attention reads the uncompressed k / v and is bound by the tensor core; the cache write reads the same
     // tensors once more and is bound by memory. They do not depend on one another, so the cache write runs on an
-    // auxiliary stream beside the attention (its blocks fit into the registers and shared memory the attention blocks
-    // leave free) and joins the caller's stream at the end. Both orderings are expressed with events, so the call
+    // auxiliary stream and joins the caller's stream at the end. An attention block of the tcgen05 tiles has nearly all of its SM's
+    // registers and shared memory, so the write's blocks run on SMs that the attention leaves idle and at its end (44 us
+    // behind the attention of 4 x 4096 tokens over 8 kv heads of 128, NVFP4 rows). Both orderings are expressed with events, so the call
     // can be captured in a CUDA graph.
     cudaStream_t stream = (cudaStream_t)stream_;
     int dev = 0;
@@ -889,7 +890,7 @@ extern "C" int b200_fa_prefill_append(const B200FaArgs *fa, const B200KvAppendAr
     }
     if (cudaEventRecord(f->fork, stream) != cudaSuccess || cudaStreamWaitEvent(f->aux, f->fork, 0) != cudaSuccess)
         return set_error(B200_ERR_LAUNCH, "fa_prefill_append: fork: %s", cudaGetErrorString(cudaGetLastError()));
-    // the attention first: its blocks (one per SM) take their place, the blocks of the cache write fill in beside them
+    // the attention first: its blocks (one per SM) take their place, the blocks of the cache write what is left
     const int rc_attn = b200_flash_attn(fa, stream_);
     const int rc_append = b200_kv_append(append, (b200_stream_t)f->aux);
     // join in any case, so that the auxiliary stream never outlives the call in the caller's ordering

@@ -966,8 +966,8 @@ __global__ void __launch_bounds__(P2_THREADS, 1) fa_prefill_sm100_kernel2(const 
 //     scores are formed while the last one's rows leave, and no SM waits for a heavy item that came last.
 // Measured (us, causal unless said; before: two threads per row, a block per item; head dims other than 128 on mma.sync,
 // sequences of different lengths by 16-byte chunks): B 4, 4096 tokens, 32 / 8 heads of 128: 690 -> 502 (1 094 TFLOP/s); B 1,
-// 16 384 tokens: 2 031 -> 1 785 (1 232); 8 x 1000 tokens, 16 heads of 64, no mask: 416 -> 77; 4 x 4096, 16 heads of 64: 1 410 ->
-// 220; 2 x 2048, 16 / 4 heads of 96: 417 -> 48; 12 sequences of 100-2960: 654 -> 354. At 16 384 tokens a tile of 256 x 128 takes
+// 16 384 tokens: 2 031 -> 1 785 (1 232); 8 x 1000 tokens, 16 heads of 64, no mask: 416 -> 81; 4 x 4096, 16 heads of 64: 1 410 ->
+// 237; 2 x 2048, 16 / 4 heads of 96: 417 -> 52; 12 sequences of 100-2960: 654 -> 354. At 16 384 tokens a tile of 256 x 128 takes
 // 3 100 cycles (the power limit holds the clock near 1.55 GHz), of which a group spends 1 500 in its exponentials and 1 250
 // waiting for its next scores: eight 128 x 128 x 16 products with both operands in shared memory take 840 cycles, not 512.
 // Taken back: a polynomial for some of the exponentials (on the multiply-add pipe; degree 5, f32 accurate) made every size
@@ -1779,7 +1779,7 @@ bool fa_kv_maps(const FaParams &p, bool bf16, uint32_t keys, CUtensorMap *tm_k, 
 enum { PF_NONE = 0, PF_ROWS128, PF_ROWS256, PF_TMA };
 // More rows than a decode call has (up to 16 rows the keys are read by warps of their own: fa_decode_tma.cu). With 17 to 511 rows
 // a block's products run partly on rows that do not exist, and still beat the 64-row tiles of mma.sync: 60 tokens, 32 / 8 heads of
-// 128: 26 -> 10 us; 8 x 200 tokens, 16 heads of 128: 65 -> 13; 16 x 400 tokens, 16 heads of 64: 188 -> 38. One item per SM bounds the
+// 128: 26 -> 10 us; 8 x 200 tokens, 16 heads of 128: 65 -> 13; 16 x 400 tokens, 16 heads of 64: 188 -> 41. One item per SM bounds the
 // small ones, so few items are split along the keys (fa_plan).
 constexpr uint64_t P3_MIN_ROWS = 17;
 static int fa_prefill_route(const FaParams &p, bool kv16) {

@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint32_t *__res
 // The chain it stands for (dequant_rows_kernel, hadamard_rows_kernel, a cast; in f32, with a copy in front when the rows
 // are not back to back) moves ten times the bytes in three or four launches. Values are the chain's, bit for bit: the same
 // roundings in the same order, butterflies from index bit 0 up. Measured: keys and values of 8192 x 8 cached MXFP8 rows, rotated, for a chunk of 1024 query tokens: the
-// call 414 -> 173 us (141 of them the attention); 65 528 TurboQuant-4 rows packed and unpacked 250 -> 56 us (with the codebook
+// call 414 -> 173 us (141 of them the attention); 65 528 TurboQuant-4 rows packed and unpacked 250 -> 37 us (with the codebook
 // formats in quant_rows128_kernel, and each row packed once instead of twice).
 // ---------------------------------------------------------------------------------------------
 struct UnpackSide {
