@@ -9,7 +9,7 @@
 
 namespace b200 {
 
-template <int KM, int VM, int HD, bool NAT, bool PAGED>
+template <int KM, int VM, int HD, bool NAT, bool PAGED, int NH>
 int launch_decode(const DecodeParams &p, dim3 grid, size_t smem, cudaStream_t stream);
 template <int KM, int VM, int HD, bool NAT>
 int launch_decode_pair(const DecodeParams &p, dim3 grid, size_t smem, cudaStream_t stream);
@@ -23,6 +23,7 @@ struct DecodePlan {
     int hd_idx;
     uint32_t workers;  // warps (or pairs of warps) that share the tiles
     bool pair;       // the kernel whose workers are pairs of warps (4-bit formats)
+    bool wide;       // columns of 16 query rows
     bool nat;        // rows packed back to back on both sides: the instantiation with compile-time row strides
     bool in_kernel;  // the decode grid merges the segments itself (arrival counters), no combine grid
 };
@@ -63,7 +64,8 @@ static int fill_decode_side(DecodeSide &s, const B200QuantSide &q, uint32_t d, c
 }
 
 // paged: the plan of a call whose rows are read in the blocks of its page table (the tensor-core kernel walks the table)
-static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false) {
+// narrow: columns of eight query rows, whatever the shape (a workspace that is too small for the wider ones)
+static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false, bool narrow = false) {
     if (!a) return set_error(B200_ERR_BAD_ARG, "tq_attention: null args");
     if (a->hkv == 0 || a->hq % a->hkv != 0)
         return set_error(B200_ERR_BAD_ARG, "tq_attention: %u query heads are not a multiple of %u kv heads", a->hq, a->hkv);
@@ -102,7 +104,17 @@ static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false
     p.b = a->b; p.lq = a->lq; p.lk = a->lk; p.hq = a->hq; p.hkv = a->hkv; p.d = a->d;
     p.group = a->hq / a->hkv;
     p.rows_per_kv = p.group * a->lq;
-    p.packs = (p.rows_per_kv + PACK - 1) / PACK;
+    // More than eight query rows per kv head: columns of 16, whose two groups of eight rows share the decoded keys and values.
+    // A tile of such a column costs 1.1 times one of eight rows, and two thirds as many warps work on them: worth it where it
+    // (nearly) halves the columns, and where every worker has a few tiles (us, columns of 8 -> 16: 16 rows, 64 sequences of 512 to
+    // 8192 MXFP4 keys 163 -> 140, 32 of 8192 MXFP8 keys 213 -> 140; 24 rows, 8 x 4000 MXFP8 keys of 64: 41 -> 44; 32 rows,
+    // one sequence of 4000 keys: 31 -> 35). For keys and values in one format, head dims 64 and 128; the kernel whose workers
+    // are pairs of warps has no such form.
+    const uint32_t packs8 = (p.rows_per_kv + PACK - 1) / PACK, packs16 = (p.rows_per_kv + 2 * PACK - 1) / (2 * PACK);
+    pl.wide = !narrow && 5 * packs16 < 3 * packs8 && a->kq.mode == a->vq.mode && a->d <= 128 && (paged || !pair_formats(a->kq.mode, a->vq.mode)) &&
+              (uint64_t)a->b * a->hkv * packs16 * ((a->lk + WK - 1) / WK) >= 3ull * decode_blocks(2) * DW * sm_count_cached();
+    p.pack_rows = pl.wide ? 2 * PACK : PACK;
+    p.packs = (p.rows_per_kv + p.pack_rows - 1) / p.pack_rows;
     p.scale = a->scale;
     p.softcap = a->softcap;
     p.wl = a->wl;
@@ -129,7 +141,7 @@ static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false
     for (int ns = 2; ns <= NS_MAX; ++ns) {
         const size_t sm = fixed + DW * ns * stage;
         if (sm > 227 * 1024) break;
-        const int fit = (int)std::min<size_t>(B200_DECODE_MIN_BLOCKS, (228 * 1024) / (sm + 1024));
+        const int fit = (int)std::min<size_t>(decode_blocks(pl.wide ? 2 : 1), (228 * 1024) / (sm + 1024));
         if (fit < 1) break;
         const size_t flight = (size_t)fit * DW * (ns - 1) * stage;
         if (flight > best || (flight == best && fit > bps)) {
@@ -199,6 +211,20 @@ static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false
     p.prefetch = (p.after_prev && (a->flags & B200_TQ_INPUTS_FINAL)) ? 1u : 0u;
     p.out_free = (p.after_prev && (a->flags & B200_TQ_OUTPUTS_FREE)) ? 1u : 0u;
     p.fresh_rows = std::min<uint32_t>(a->fresh_rows, 0x7fffffffu);
+    // Parts of the work by place (tq_decode.cuh), for a full grid of the kernel whose workers are warps with three blocks per SM:
+    // the times that the places' blocks took with equal shares, inverted. Ragged MXFP4, 64 sequences: 100.4 us with equal shares,
+    // 96.9 with these (before the other changes of the call's ends). Two blocks per SM (columns of 16 rows) end within 2 % of one
+    // another: 154.9 with equal shares, 158.3 with parts of 130 and 126. In a chain of calls that do not wait for one another
+    // the blocks of a call take the places of the last one as these come free.
+    p.place_workers = 0;
+    if (!pl.pair && a->splits <= 0 && !p.out_free && bps == 3 && pl.blocks == (uint32_t)(sm_count_cached() * bps)) {
+        p.place_workers = (uint32_t)(sm_count_cached() * DW);
+        p.place_end[0] = 92;
+        p.place_end[1] = 177;
+        p.place_end[2] = 256;
+    }
+    // rows of all sequences (at their longest, or as far as the cache goes) against the 126 MB of L2; packs of query rows read them again
+    p.stream = p.packs == 1 && (uint64_t)a->b * a->hkv * lk * (p.k_ss + p.v_ss) * 4 > (64ull << 20) ? 1u : 0u;
     pl.nat = !paged && p.k_ss == (uint64_t)kl.row_words && p.v_ss == (uint64_t)vl.row_words && a->kq.mode == a->vq.mode && a->d == 128;
     if (pl.nat) {
         // the native-row kernels read a lane's codes with 8- or 16-byte loads where the row length allows: every
@@ -210,7 +236,7 @@ static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false
     p.pages = paged ? a->pages : nullptr;
     p.n_pages = paged ? a->n_pages : 0u;
     pl.in_kernel = merges_itself(pl.blocks, wpb);
-    const size_t prow = std::min<size_t>(PACK, p.rows_per_kv);
+    const size_t prow = std::min<size_t>(p.pack_rows, p.rows_per_kv);
     const size_t slots = ((size_t)pl.workers + ncols) * prow;
     const size_t part_o = slots * a->d * 4;
     const size_t part_l = slots * 4;
@@ -234,21 +260,32 @@ static int dispatch_hd(const DecodePlan &pl, dim3 grid, cudaStream_t stream) {
             }
         }
     }
+    if constexpr (KM == VM && !pair_formats(KM, VM)) {
+        if (pl.wide) {
+            if (pl.hd_idx == 0) return launch_decode<KM, VM, 64, false, false, 2>(pl.p, grid, pl.smem, stream);
+            if (pl.nat) return launch_decode<KM, VM, 128, true, false, 2>(pl.p, grid, pl.smem, stream);
+            return launch_decode<KM, VM, 128, false, false, 2>(pl.p, grid, pl.smem, stream);
+        }
+    }
     if constexpr (KM == VM)
-        if (pl.nat && pl.hd_idx == 1) return launch_decode<KM, VM, 128, true, false>(pl.p, grid, pl.smem, stream);
+        if (pl.nat && pl.hd_idx == 1) return launch_decode<KM, VM, 128, true, false, 1>(pl.p, grid, pl.smem, stream);
     switch (pl.hd_idx) {
-    case 0: return launch_decode<KM, VM, 64, false, false>(pl.p, grid, pl.smem, stream);
-    case 1: return launch_decode<KM, VM, 128, false, false>(pl.p, grid, pl.smem, stream);
-    default: return launch_decode<KM, VM, 256, false, false>(pl.p, grid, pl.smem, stream);
+    case 0: return launch_decode<KM, VM, 64, false, false, 1>(pl.p, grid, pl.smem, stream);
+    case 1: return launch_decode<KM, VM, 128, false, false, 1>(pl.p, grid, pl.smem, stream);
+    default: return launch_decode<KM, VM, 256, false, false, 1>(pl.p, grid, pl.smem, stream);
     }
 }
 
 template <int KM>
 static int dispatch_paged(const DecodePlan &pl, dim3 grid, cudaStream_t stream) {
+    if (pl.wide) {
+        if (pl.hd_idx == 0) return launch_decode<KM, KM, 64, false, true, 2>(pl.p, grid, pl.smem, stream);
+        return launch_decode<KM, KM, 128, false, true, 2>(pl.p, grid, pl.smem, stream);
+    }
     switch (pl.hd_idx) {
-    case 0: return launch_decode<KM, KM, 64, false, true>(pl.p, grid, pl.smem, stream);
-    case 1: return launch_decode<KM, KM, 128, false, true>(pl.p, grid, pl.smem, stream);
-    default: return launch_decode<KM, KM, 256, false, true>(pl.p, grid, pl.smem, stream);
+    case 0: return launch_decode<KM, KM, 64, false, true, 1>(pl.p, grid, pl.smem, stream);
+    case 1: return launch_decode<KM, KM, 128, false, true, 1>(pl.p, grid, pl.smem, stream);
+    default: return launch_decode<KM, KM, 256, false, true, 1>(pl.p, grid, pl.smem, stream);
     }
 }
 
@@ -260,7 +297,10 @@ static int dispatch_v(const DecodePlan &pl, dim3 grid, cudaStream_t stream) {
     if constexpr (pair_formats(KM, KM)) {
         if (pl.pair) return launch_decode_pair<KM, KM, 128, true>(pl.p, grid, pl.smem, stream);
     }
-    return launch_decode<KM, KM, 128, true, false>(pl.p, grid, pl.smem, stream);
+    if constexpr (!pair_formats(KM, KM)) {
+        if (pl.wide) return launch_decode<KM, KM, 128, true, false, 2>(pl.p, grid, pl.smem, stream);
+    }
+    return launch_decode<KM, KM, 128, true, false, 1>(pl.p, grid, pl.smem, stream);
 #else
     switch (pl.p.v.mode) {
     case B200_TURBO_MSE: return dispatch_hd<KM, B200_TURBO_MSE>(pl, grid, stream);
@@ -477,7 +517,7 @@ static bool paged_fast_plan(const B200TqAttnArgs *a, PagedFast &f) {
 // that kernel. Workspace: the keys and tiles before every block (written by a one-block kernel in front of the
 // attention), then the attention's own.
 static size_t paged_prefix_bytes(uint32_t n_pages) { return ((size_t)(n_pages + 1) * 8 + 255) / 256 * 256; }
-static bool paged_direct_plan(const B200TqAttnArgs *a, DecodePlan &pl) {
+static bool paged_direct_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool narrow = false) {
     static const bool off = diag_env("B200_PAGED_NO_WALK") != nullptr;  // diagnostic: paged rows on the compaction / general paths
     if (off || !a || !a->pages || a->n_pages == 0 || a->lk == 0 || a->b == 0 || a->kq.mode != a->vq.mode) return false;
     if (a->flags & B200_TQ_IN_PLACE) return false;  // the caller asked for the general kernel
@@ -485,13 +525,14 @@ static bool paged_direct_plan(const B200TqAttnArgs *a, DecodePlan &pl) {
     t.flags &= ~(B200_TQ_AFTER_PREV | B200_TQ_INPUTS_FINAL);  // the prefix kernel of the call runs right before the attention
     if (tq_generic_takes(&t) && (a->d != 64 && a->d != 128 && a->d != 256)) return false;
     if (a->kq.mode == B200_TURBO_MSE && (a->kq.bits != 4 || a->vq.bits != 4)) return false;
-    return make_plan(&t, pl, true) == B200_OK;
+    return make_plan(&t, pl, true, narrow) == B200_OK;
 }
 
-extern "C" size_t b200_tq_attention_workspace_bytes(const B200TqAttnArgs *a) {
+// what a call asks for; narrow: the least that its tensor-core kernel runs with (columns of eight query rows)
+static size_t workspace_need(const B200TqAttnArgs *a, bool narrow) {
     {
         DecodePlan pl;
-        if (paged_direct_plan(a, pl)) return paged_prefix_bytes(a->n_pages) + pl.ws_bytes;
+        if (paged_direct_plan(a, pl, narrow)) return paged_prefix_bytes(a->n_pages) + pl.ws_bytes;
     }
     {
         // paged rows: with this much workspace the blocks are compacted into it and the tensor-core kernel runs; with
@@ -501,9 +542,11 @@ extern "C" size_t b200_tq_attention_workspace_bytes(const B200TqAttnArgs *a) {
     }
     if (tq_generic_takes(a)) return tq_generic_workspace_bytes(a);
     DecodePlan pl;
-    if (make_plan(a, pl)) return 0;
+    if (make_plan(a, pl, false, narrow)) return 0;
     return pl.ws_bytes;
 }
+
+extern "C" size_t b200_tq_attention_workspace_bytes(const B200TqAttnArgs *a) { return workspace_need(a, false); }
 
 // set by b200_tq_attention_gather around its call of b200_tq_attention (same thread)
 static thread_local const B200PeerGather *tl_gather = nullptr;
@@ -516,15 +559,21 @@ extern "C" int b200_tq_attention(const B200TqAttnArgs *a, b200_stream_t stream_)
         DecodePlan pl;
         if (paged_direct_plan(a, pl)) {
             const size_t pre = paged_prefix_bytes(a->n_pages);
+            // a workspace that only the columns of eight rows fit
+            if (pl.wide && a->workspace_bytes < pre + pl.ws_bytes) paged_direct_plan(a, pl, true);
             if (a->workspace && a->workspace_bytes >= pre + pl.ws_bytes && !(reinterpret_cast<uintptr_t>(a->workspace) & 15) &&
                 (uint64_t)a->b * a->hq * a->lq != 0 && a->q && a->out) {
                 char *ws = reinterpret_cast<char *>(a->workspace);
                 uint32_t *pg_keys = reinterpret_cast<uint32_t *>(ws), *pg_tiles = pg_keys + (a->n_pages + 1);
+                pl.p.pg_keys = pg_keys;
+                pl.p.pg_tiles = pg_tiles;
+                if (a->n_pages <= PG_BUILD) {
+                    pl.p.pg_build = 1;  // the blocks of the attention work the sums out themselves
+                    return run_plan(a, pl, ws + pre, a->workspace_bytes - pre, (cudaStream_t)stream_);
+                }
                 tq_page_prefix_kernel<<<1, 256, 0, (cudaStream_t)stream_>>>(a->pages, a->n_pages, pg_keys, pg_tiles);
                 const int rc = check_launch("tq_page_prefix");
                 if (rc) return rc;
-                pl.p.pg_keys = pg_keys;
-                pl.p.pg_tiles = pg_tiles;
                 pl.p.after_prev = 1;  // launched as the prefix kernel's programmatic dependent (the paged kernel waits at its start)
                 return run_plan(a, pl, ws + pre, a->workspace_bytes - pre, (cudaStream_t)stream_);
             }
@@ -555,7 +604,8 @@ extern "C" int b200_tq_attention(const B200TqAttnArgs *a, b200_stream_t stream_)
         return tq_generic_launch(a, (cudaStream_t)stream_);
     }
     DecodePlan pl;
-    const int rc = make_plan(a, pl);
+    int rc = make_plan(a, pl);
+    if (rc == B200_OK && pl.wide && a->workspace_bytes < pl.ws_bytes) rc = make_plan(a, pl, false, true);  // a workspace that only the columns of eight rows fit
     if (rc) return rc;
     if ((uint64_t)a->b * a->hq * a->lq == 0) return B200_OK;
     if (!a->k_rows || !a->v_rows) return set_error(B200_ERR_BAD_ARG, "tq_attention: null pointer");
@@ -662,6 +712,7 @@ extern "C" int b200_tq_attention_static(const B200TqAttnArgs *a, b200_stream_t s
     args.workspace = nullptr;
     args.workspace_bytes = 0;
     size_t need = b200_tq_attention_workspace_bytes(&args);
+    if (need > (size_t)B200_STATIC_SCRATCH_BYTES) need = workspace_need(&args, true);
     const bool in_place = args.pages != nullptr && need > (size_t)B200_STATIC_SCRATCH_BYTES;  // too large to compact: read in place
     if (in_place) need = 16;
     if (need > (size_t)B200_STATIC_SCRATCH_BYTES)

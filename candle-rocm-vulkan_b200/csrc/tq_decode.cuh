@@ -43,9 +43,11 @@ constexpr int WK = 32;        // keys per warp tile
 #ifndef B200_DECODE_MIN_BLOCKS
 #define B200_DECODE_MIN_BLOCKS 3
 #endif
+// blocks per SM of the kernel with `nh` groups of eight query rows per column
+__host__ __device__ constexpr int decode_blocks(int nh) { return nh == 1 ? B200_DECODE_MIN_BLOCKS : 2; }
 constexpr int NS_MAX = 3;     // stages per warp (fewer when the rows are large)
 constexpr float MAX_SLACK = 8.0f;  // log2 of how far a score may exceed the running maximum before it moves
-constexpr int PACK = 8;       // query rows per block
+constexpr int PACK = 8;       // query rows of one product (a column holds PACK or 2 PACK, see DecodeParams::pack_rows)
 #ifndef B200_DECODE_COL_COST
 #define B200_DECODE_COL_COST 4  // cost of starting a column, in tiles, in the split of the work between the workers
 #endif
@@ -77,18 +79,23 @@ struct DecodeParams {
     int32_t kv_len_add;     // added to every entry of kv_len
     uint32_t b, lq, lk, hq, hkv, d, group;
     uint32_t rows_per_kv, packs;
+    uint32_t pack_rows;  // query rows of a column: PACK, or 2 PACK (tq_decode_kernel with two halves)
     DecodeSide k, v;
     float scale, softcap;
     int32_t wl, wr;
     const float *alibi;
     uint32_t alibi_bs;
-    float *part_o;     // [slot][rows][d], slot = worker + column, rows = min(PACK, query rows per kv head)
+    float *part_o;     // [slot][rows][d], slot = worker + column, rows = min(pack_rows, query rows per kv head)
     float *part_lse;   // [slot][rows]
     int32_t *meta;     // [column] (first slot, number of segments)
     int32_t *status;
     uint32_t k_stage_bytes, v_stage_bytes;
     uint32_t ns;       // stages per warp
     uint32_t rows_cap;      // rows that exist in every (batch, head) slab of both caches (0 = only the visible ones)
+    // shares by place: workers of the blocks that start together, one per SM (0: all shares are equal), and the ends of their
+    // places' parts of the work in 1/256
+    uint32_t place_workers, place_end[3];
+    uint32_t stream;        // the rows do not stay in L2 (CopySide::policy)
     uint32_t col_cost;      // cost of starting a column, in tiles, for the split of the work between the warps
     uint32_t qstage_bytes;  // query staging for the rotation (0 without it)
     uint32_t after_prev;    // launched as a programmatic dependent of the stream's previous kernel
@@ -106,9 +113,11 @@ struct DecodeParams {
     uint32_t *ctr;
     int32_t *lib_status;    // library-wide flag: set when a bounded wait of a kernel of this call runs out
     // paged rows (null: dense rows): the block table, and for every block the keys and the 32-key tiles of the
-    // blocks before it (n_pages + 1 entries each, written by tq_page_prefix_kernel right before this grid)
+    // blocks before it (n_pages + 1 entries each, written by tq_page_prefix_kernel right before this grid, or, pg_build, by
+    // every block of this grid for itself, all of them the same words)
     const B200Page *pages;
     uint32_t n_pages;
+    uint32_t pg_build;
     const uint32_t *pg_keys, *pg_tiles;
 };
 
@@ -327,6 +336,32 @@ __device__ __forceinline__ uint32_t page_of_key(const DecodeParams &p, uint32_t 
     }
     return lo;
 }
+// The keys and tiles before every block of a table of at most PG_BUILD blocks, by one warp. A kernel of its own in front costs
+// 2 us and its launch, this half a microsecond in every block (16 x 4000 keys in 8 blocks: 46 -> 44.5 us).
+constexpr uint32_t PG_BUILD = 127;
+__device__ __forceinline__ void page_prefix(const DecodeParams &p, int lane) {
+    uint32_t *keys = const_cast<uint32_t *>(p.pg_keys), *tiles = const_cast<uint32_t *>(p.pg_tiles);
+    uint32_t r[4], base_k = 0, base_t = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r[k] = 32u * k + lane < p.n_pages ? p.pages[32 * k + lane].rows : 0u;
+#pragma unroll 1
+    for (uint32_t k = 0; 32 * k <= p.n_pages; ++k) {
+        const uint32_t n = k == 0 ? r[0] : (k == 1 ? r[1] : (k == 2 ? r[2] : r[3])), t = (n + WK - 1) / WK;
+        uint32_t ik = n, it = t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(0xffffffffu, ik, o), c = __shfl_up_sync(0xffffffffu, it, o);
+            if (lane >= o) ik += a, it += c;
+        }
+        const uint32_t i = 32 * k + lane;
+        if (i <= p.n_pages) {
+            keys[i] = base_k + ik - n;
+            tiles[i] = base_t + it - t;
+        }
+        base_k += __shfl_sync(0xffffffffu, ik, 31);
+        base_t += __shfl_sync(0xffffffffu, it, 31);
+    }
+}
 // the block that holds tile T of the table's list (< the total number of tiles)
 __device__ __forceinline__ uint32_t page_of_tile(const DecodeParams &p, uint32_t T) {
     uint32_t lo = 0, hi = p.n_pages;
@@ -342,14 +377,11 @@ __device__ __forceinline__ Column make_column(const DecodeParams &p, uint32_t b)
     Column c;
     c.lk = p.kv_len ? min(max(p.kv_len[b] + p.kv_len_add, 0), (int)p.lk) : (int)p.lk;
     if (p.pages) c.lk = (int)min((uint32_t)c.lk, p.pg_keys[p.n_pages]);  // never more keys than the blocks hold
-    // union of the rows' ranges: first query token gives the lowest, the last the highest key
-    const long long pos0 = (long long)c.lk - (long long)p.lq, pos1 = (long long)c.lk - 1;
-    long long lo = p.wl >= 0 ? max(pos0 - p.wl, 0ll) : 0ll;
-    long long hi = p.wr >= 0 ? min(pos1 + p.wr + 1, (long long)c.lk) : (long long)c.lk;
-    lo = min(lo, (long long)c.lk);
-    hi = max(hi, lo);
-    c.lo = (int)lo;
-    c.hi = (int)hi;
+    // union of the rows' ranges: the first query token (position lk - lq) gives the lowest key, the last one (lk - 1) sees all from
+    // there on, whatever the right window
+    const int pos0 = c.lk - (int)p.lq;
+    c.lo = p.wl >= 0 && pos0 > p.wl ? min(pos0 - p.wl, c.lk) : 0;
+    c.hi = c.lk;
     c.t_lo = 0;
     if (p.pages == nullptr) {
         c.tiles = (c.hi - c.lo + WK - 1) / WK;
@@ -363,9 +395,55 @@ __device__ __forceinline__ Column make_column(const DecodeParams &p, uint32_t b)
     return c;
 }
 
-// worker that owns cost position x when `total` is shared by `nw` workers (worker i starts at floor(i total / nw))
-__device__ __forceinline__ uint32_t owner_of(uint64_t x, uint64_t total, uint32_t nw) {
-    return (uint32_t)(((x + 1) * nw - 1) / total);
+// What a worker does once, before its first tile and after its last, runs from a cold instruction cache: in a call of a few
+// tiles per worker that is most of its time (one sequence of 2048 FP8 keys: 12 of 18 thousand cycles), and it goes with the
+// number of instructions. So the arithmetic of the shares is in 32 bits where the call's cost positions fit (a 64-bit division
+// is a hundred instructions), and in 64 bits, out of line, where they do not.
+static __device__ __noinline__ uint64_t div64(uint64_t a, uint64_t b) { return a / b; }
+
+// The shares. Three blocks of four warps live on an SM, and its schedulers serve the warps that came first: with equal shares
+// the blocks of the first place were done after 72 us of a ragged MXFP4 call, those of the second after 77 and of the third
+// after 83 (83, 83 and 87 with a slower merge and these parts). So where a worker has many tiles, the places' shares differ (the
+// host gives the parts, see make_plan).
+constexpr uint32_t PLACE_MIN = 16;  // cost positions per worker from which the shares go by place
+struct Places {
+    uint64_t total;
+    uint32_t nw, n;      // workers, workers per place
+    bool by_place;
+};
+__device__ __forceinline__ Places places_of(const DecodeParams &p, uint64_t total, uint32_t nw) {
+    const bool by = p.place_workers != 0 && total >= (uint64_t)PLACE_MIN * nw;
+    return {total, nw, by ? p.place_workers : nw, by};
+}
+// the part [lo, lo + width) of the cost positions that place `k` works on
+__device__ __forceinline__ void place_part(const DecodeParams &p, const Places &pl, uint32_t k, uint64_t &lo, uint64_t &width) {
+    lo = k == 0 ? 0 : (pl.total * p.place_end[k - 1]) >> 8;
+    width = (pl.by_place ? (pl.total * p.place_end[k]) >> 8 : pl.total) - lo;
+}
+// first cost position of worker i (i == nw: the end); workers < 2^16
+__device__ __forceinline__ uint64_t share_start(const DecodeParams &p, const Places &pl, uint32_t i) {
+    uint32_t k = 0;
+    if (pl.by_place) k = (i >= pl.n && pl.n < pl.nw ? 1u : 0u) + (i >= 2 * pl.n && 2 * pl.n < pl.nw ? 1u : 0u);
+    uint64_t lo, width;
+    place_part(p, pl, k, lo, width);
+    i -= k * pl.n;
+    if (B200_LIKELY((pl.total >> 32) == 0)) {
+        const uint32_t q = (uint32_t)width / pl.n, r = (uint32_t)width - q * pl.n;
+        return lo + (uint64_t)q * i + r * i / pl.n;  // r < n, i <= n
+    }
+    return lo + div64(width * i, pl.n);
+}
+// the worker that owns cost position x
+__device__ __forceinline__ uint32_t owner_of(const DecodeParams &p, const Places &pl, uint64_t x) {
+    uint32_t k = 0;
+    uint64_t lo, width;
+    place_part(p, pl, 0, lo, width);
+    while (x >= lo + width) place_part(p, pl, ++k, lo, width);
+    const uint64_t n = (x - lo + 1) * pl.n - 1;
+    // n < 2^48, width < 2^32: the quotient, below 2^16, is at least 2^-32 away from an integer that it does not reach, and a
+    // double next to it less than 2^-37
+    if (B200_LIKELY((pl.total >> 32) == 0)) return k * pl.n + (uint32_t)((double)n / (double)(uint32_t)width);
+    return k * pl.n + (uint32_t)div64(n, width);
 }
 
 // A worker's share is a list of segments: tiles [t0, t1) of column y of batch entry b.
@@ -377,6 +455,10 @@ struct Segment {
     uint64_t x;  // cost position of tile t0
     Column col;
 };
+
+// kv head and pack of query rows of column y (most calls have one pack per kv head: no division)
+__device__ __forceinline__ uint32_t head_of(const DecodeParams &p, uint32_t y) { return p.packs == 1 ? y : y / p.packs; }
+__device__ __forceinline__ uint32_t pack_of(const DecodeParams &p, uint32_t y) { return p.packs == 1 ? 0u : y % p.packs; }
 
 // next segment of the share that ends at x_end; false when the share is exhausted
 __device__ __forceinline__ bool next_segment(Segment &s, const DecodeParams &p, uint32_t ny, uint64_t x_end) {
@@ -412,7 +494,7 @@ __host__ __device__ constexpr uint32_t stage_part_bytes(uint32_t row_bytes) { re
 // Output offset (elements) of row rr of column (b, y), and its index among the rows of the call in
 // (batch, head, token) order; false for a row that the pack does not have.
 __device__ __forceinline__ bool row_addr(const DecodeParams &p, uint32_t b, uint32_t y, uint32_t rr, size_t &obase, size_t &grow) {
-    const uint32_t hk = y / p.packs, pack = y % p.packs, r = pack * PACK + rr;
+    const uint32_t hk = head_of(p, y), r = pack_of(p, y) * p.pack_rows + rr;
     if (r >= p.rows_per_kv) return false;
     const uint32_t i = p.lq == 1 ? 0u : r / p.group, h = hk * p.group + (p.lq == 1 ? r : r % p.group);
     obase = (size_t)b * p.o_sb + (size_t)h * p.o_sh + (size_t)i * p.o_ss;
@@ -535,68 +617,70 @@ __device__ __forceinline__ void finish_row(const DecodeParams &p, size_t obase, 
 }
 
 // Merge of all rows of one column by one warp, inside the decode grid (the last worker of the column to arrive).
-// Eight lanes share a row (lane l: row l / 8 of a group of four rows, elements [(l % 8) HD / 8, +HD / 8)), so four
-// rows are merged side by side and the partial rows of two segments are in flight per lane: a group of rows costs two
-// or three trips to L2 instead of a few per row. `slot0`: the first segment's slot; consecutive segments are
-// consecutive slots. Rotated values are rotated back in registers.
+// Eight lanes share a row (lane l: row l / 8 of a group of four rows, elements [(l % 8) HD / 8, +HD / 8)). The log-sum-exps
+// of eight segments (one per lane of a row) and the row's first MS partials are asked for together, the next MS while these are
+// added up: four rows cost one trip to L2 per MS segments, at the end of the call's slowest workers. The code is short and takes few
+// registers on purpose: it runs from a cold instruction cache (lane = 1/32 of a row, four segments of four rows in flight: 21
+// thousand cycles for 4.4 segments, this form 4.5, a form that reads the log-sum-exps per segment 8.5), and a larger one also costs
+// the loop over the tiles its registers (MS = 4: TurboQuant-4, 32 x 32768 keys, 55.8 -> 70 us). `slot0`: the first segment's slot;
+// consecutive segments are consecutive slots. Rotated values are rotated back in registers.
 template <int HD>
 __device__ __forceinline__ void merge_column(const DecodeParams &p, uint32_t b, uint32_t y, size_t slot0, int ns, uint32_t prow, size_t g_base,
                                              int lane) {
-    constexpr int LPR = 8, EL = HD / LPR;  // lanes per row, elements of a row per lane
-    const uint32_t q = (uint32_t)lane % LPR;
+    constexpr int LPR = 8, EL = HD / LPR, MS = 2;  // lanes per row, elements of a row per lane, segments at a time
+    const int q = lane % LPR;
     const size_t seg_stride = (size_t)prow * HD;
+#pragma unroll 1
     for (uint32_t rbase = 0; rbase < prow; rbase += 32 / LPR) {
-        const uint32_t rr = rbase + (uint32_t)lane / LPR;
-        size_t obase = 0, grow = 0;
-        const bool live = rr < prow && row_addr(p, b, y, rr, obase, grow);
-        const float *pl = p.part_lse + slot0 * prow + rr;
-        const float *po = p.part_o + (slot0 * prow + rr) * HD + q * EL;
-        float acc[EL];
+        const uint32_t rr = rbase + (uint32_t)lane / LPR, rl = min(rr, prow - 1);  // rows past the last one are merged with it and not stored
+        const float *pl = p.part_lse + slot0 * prow + rl;
+        const float *po = p.part_o + (slot0 * prow + rl) * HD + q * EL;
+        float4 v[MS][EL / 4];
+        float e = q < ns ? __ldcg(pl + (size_t)q * prow) : -INFINITY, mx = e, wsum = 0.0f, acc[EL];
+#pragma unroll
+        for (int j = 0; j < MS; ++j)
+#pragma unroll
+            for (int k = 0; k < EL / 4; ++k) v[j][k] = __ldcg(reinterpret_cast<const float4 *>(po + min(j, ns - 1) * seg_stride) + k);
 #pragma unroll
         for (int k = 0; k < EL; ++k) acc[k] = 0.0f;
-        if (live) {
-            // the first two segments' rows are requested before the log-sum-exps are looked at
-            float4 pre[2][EL / 4];
+#pragma unroll 1
+        for (int s = q + LPR; s < ns; s += LPR) mx = fmaxf(mx, __ldcg(pl + (size_t)s * prow));
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+        for (int o = 1; o < LPR; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        float w = e == -INFINITY ? 0.0f : expf(e - mx);  // of segment s0 / 8 * 8 + q
+#pragma unroll 1
+        for (int s0 = 0;;) {
 #pragma unroll
-                for (int k = 0; k < EL / 4; ++k)
-                    pre[j][k] = j < ns ? __ldcg(reinterpret_cast<const float4 *>(po + (size_t)j * seg_stride) + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            float mx = -INFINITY;
-#pragma unroll 8
-            for (int s0 = 0; s0 < ns; ++s0) mx = fmaxf(mx, __ldcg(pl + (size_t)s0 * prow));
-            float wsum = 0.0f;
-            for (int s0 = 0; s0 < ns; s0 += 2) {
-                float w[2];
+            for (int j = 0; j < MS; ++j) {
+                if (s0 + j >= ns) break;
+                const float wj = __shfl_sync(0xffffffffu, w, (lane & ~(LPR - 1)) | ((s0 + j) & (LPR - 1)));
+                wsum += wj;
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const float e = s0 + j < ns ? __ldcg(pl + (size_t)(s0 + j) * prow) : -INFINITY;
-                    w[j] = e == -INFINITY ? 0.0f : expf(e - mx);
-                    wsum += w[j];
+                for (int k = 0; k < EL / 4; ++k) {
+                    acc[4 * k] = fmaf(wj, v[j][k].x, acc[4 * k]);
+                    acc[4 * k + 1] = fmaf(wj, v[j][k].y, acc[4 * k + 1]);
+                    acc[4 * k + 2] = fmaf(wj, v[j][k].z, acc[4 * k + 2]);
+                    acc[4 * k + 3] = fmaf(wj, v[j][k].w, acc[4 * k + 3]);
                 }
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int k = 0; k < EL / 4; ++k) {
-                        acc[4 * k] = fmaf(w[j], pre[j][k].x, acc[4 * k]);
-                        acc[4 * k + 1] = fmaf(w[j], pre[j][k].y, acc[4 * k + 1]);
-                        acc[4 * k + 2] = fmaf(w[j], pre[j][k].z, acc[4 * k + 2]);
-                        acc[4 * k + 3] = fmaf(w[j], pre[j][k].w, acc[4 * k + 3]);
-                    }
-                // the next two segments
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int k = 0; k < EL / 4; ++k)
-                        if (s0 + 2 + j < ns) pre[j][k] = __ldcg(reinterpret_cast<const float4 *>(po + (size_t)(s0 + 2 + j) * seg_stride) + k);
             }
-            const float inv = wsum > 0.0f ? 1.0f / wsum : 0.0f;
+            s0 += MS;
+            if (s0 >= ns) break;
 #pragma unroll
-            for (int k = 0; k < EL; ++k) acc[k] *= inv;
+            for (int j = 0; j < MS; ++j)
+#pragma unroll
+                for (int k = 0; k < EL / 4; ++k) v[j][k] = __ldcg(reinterpret_cast<const float4 *>(po + min(s0 + j, ns - 1) * seg_stride) + k);
+            if ((s0 & (LPR - 1)) == 0) {
+                e = s0 + q < ns ? __ldcg(pl + (size_t)(s0 + q) * prow) : -INFINITY;
+                w = e == -INFINITY ? 0.0f : expf(e - mx);
+            }
         }
+        const float inv = wsum > 0.0f ? 1.0f / wsum : 0.0f;
+#pragma unroll
+        for (int k = 0; k < EL; ++k) acc[k] *= inv;
         // rotate back: the eight lanes of a row are consecutive (part = lane % 8)
-        if (p.v.rot == B200_ROT_HADAMARD) hadamard_back_parts<EL>(acc, lane, 1, 2, 4, p.v.signs, (int)(q * EL));
-        if (live) {
+        if (p.v.rot == B200_ROT_HADAMARD) hadamard_back_parts<EL>(acc, lane, 1, 2, 4, p.v.signs, q * EL);
+        size_t obase = 0, grow = 0;
+        if (rr < prow && row_addr(p, b, y, rr, obase, grow)) {
             store_row_piece<EL>(p.out, obase + q * EL, acc, p.out_dtype);
             // the same row into every rank's gathered buffer: plain stores through the peer mappings
             for (uint32_t pr = 0; pr < p.world; ++pr) store_row_piece<EL>(p.peer_bufs[pr], g_base + grow * HD + q * EL, acc, p.out_dtype);
@@ -745,19 +829,19 @@ __device__ __forceinline__ bool softmax_masked(const float (&sr)[2][4], const fl
     return moved;
 }
 
-// Query rows of pack `pack` of kv head `hk` of batch entry `b` as the B fragments of K Q^T: row g of the pack for the
+// Query rows row0 ... row0 + 7 of kv head `hk` of batch entry `b` as the B fragments of K Q^T: row row0 + g for the
 // lanes of quad row g, rotated with the key signs when the cache is rotated (through the warp's staging rows), then
 // normalized by a power of two and rounded to f16. Per k-step the four contraction slots of a lane are the
 // consecutive dims dbase(s) ... + 3, so the four lanes of a quad hold the whole row between them. qs[e]: the score
 // scale of row 2c + e (softmax scale times the power of two taken out), qs2[e] the same in the log2 domain.
 template <int KM, int HD>
-__device__ __forceinline__ void load_query(const DecodeParams &p, uint32_t b, uint32_t hk, uint32_t pack, float *qstage, int lane,
+__device__ __forceinline__ void load_query(const DecodeParams &p, uint32_t b, uint32_t hk, uint32_t row0, float *qstage, int lane,
                                            uint32_t (&qb0)[HD / 16], uint32_t (&qb1)[HD / 16], float (&qs)[2], float (&qs2)[2]) {
     constexpr int STEPS = HD / 16;
     constexpr bool KMX = fmt_is_mx(KM);
     const int g = lane >> 2, c = lane & 3;
     const uint32_t G = p.group, R = p.rows_per_kv;
-    const uint32_t r = pack * PACK + g;
+    const uint32_t r = row0 + g;
     float qv[STEPS][4];
     if (HD <= 128 && p.k.rot == B200_ROT_HADAMARD) {
         // Rotation in registers. The four lanes of quad row g hold row g between them, each the HD / 4 elements that its
@@ -828,7 +912,7 @@ __device__ __forceinline__ void load_query(const DecodeParams &p, uint32_t b, ui
     } else if (p.k.rot == B200_ROT_HADAMARD) {
         __syncwarp();
         for (int idx = lane; idx < PACK * HD; idx += 32) {
-            const uint32_t rr = idx / HD, dd = idx % HD, r2 = pack * PACK + rr;
+            const uint32_t rr = idx / HD, dd = idx % HD, r2 = row0 + rr;
             float v = 0.0f;
             if (r2 < R) {
                 const uint32_t i = p.lq == 1 ? 0u : r2 / G, h = hk * G + (p.lq == 1 ? r2 : r2 % G);
@@ -971,14 +1055,15 @@ __device__ __forceinline__ void tile_meta(uint32_t kr, uint32_t vr, uint32_t met
 }
 
 // Scores of keys g and g + 8 of the 16 keys at `ka` (the lane's first code byte of key g; rows krb bytes apart)
-// against the query rows 2c, 2c + 1: sr[2 k + e] = key g + 8 k, row 2c + e. `mrow`: the f32 key scales of key g
+// against the query rows 2c, 2c + 1 of each group: sr[h][u][2 k + e] = key g + 8 k, row 8 h + 2c + e. `mrow`: the f32 key scales of key g
 // (per-key scalars of the tile), qb0 / qb1: the query fragments.
 // AL: what the rows' addresses in shared memory are known to be multiples of (bytes).
 // PERM: the tile's keys are dealt to the lanes in another order (perm_key below): the lane's second key is 2 rows
 // after its first instead of 8.
-template <int KM, int HD, bool WIDE = false, int AL = 4, bool PERM = false>
-__device__ __forceinline__ void k_scores16(uint32_t ka, uint32_t krb, uint32_t mrow, const uint32_t (&qb0)[HD / 16], const uint32_t (&qb1)[HD / 16],
-                                           uint32_t lut_k, uint32_t plane_k, int c, float (&sr)[4]) {
+// NH: groups of eight query rows; the keys are decoded once for all of them.
+template <int KM, int HD, bool WIDE = false, int AL = 4, bool PERM = false, int NH = 1>
+__device__ __forceinline__ void k_scores16(uint32_t ka, uint32_t krb, uint32_t mrow, const uint32_t (&qb0)[NH][HD / 16], const uint32_t (&qb1)[NH][HD / 16],
+                                           uint32_t lut_k, uint32_t plane_k, int c, float (&sr)[NH][2][4], int u) {
     constexpr int STEPS = HD / 16;
     constexpr bool K4 = fmt_is4(KM), KMX = fmt_is_mx(KM);
     constexpr int KMW = kmeta_words(KM, HD);
@@ -1001,29 +1086,39 @@ __device__ __forceinline__ void k_scores16(uint32_t ka, uint32_t krb, uint32_t m
         }
 #pragma unroll
         for (int bk = 0; bk < NBK; ++bk) {
-            float acc[4];
+            float acc[NH][4];
             if constexpr (K4) {
                 const uint32_t x0 = lds32(ka + 16 * bk), x8 = lds32(ka8 + 16 * bk);
                 uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
                 cvt_e2m1x8_f16x2(x0, a0, a1, a2, a3);
                 cvt_e2m1x8_f16x2(x8, b0, b1, b2, b3);
-                mma_f16_16816_z(acc, a0, b0, a1, b1, qb0[2 * bk], qb1[2 * bk]);
-                mma_f16_16816(acc, a2, b2, a3, b3, qb0[2 * bk + 1], qb1[2 * bk + 1]);
+#pragma unroll
+                for (int h = 0; h < NH; ++h) {
+                    mma_f16_16816_z(acc[h], a0, b0, a1, b1, qb0[h][2 * bk], qb1[h][2 * bk]);
+                    mma_f16_16816(acc[h], a2, b2, a3, b3, qb0[h][2 * bk + 1], qb1[h][2 * bk + 1]);
+                }
             } else {
                 const uint32_t x0 = lds32(ka + 32 * bk), x8 = lds32(ka8 + 32 * bk);
                 const uint32_t y0 = lds32(ka + 32 * bk + 4), y8 = lds32(ka8 + 32 * bk + 4);
-                mma_f16_16816_z(acc, cvt_e4m3x2_f16x2(x0), cvt_e4m3x2_f16x2(x8), cvt_e4m3x2_hi_f16x2(x0),
-                                cvt_e4m3x2_hi_f16x2(x8), qb0[2 * bk], qb1[2 * bk]);
-                mma_f16_16816(acc, cvt_e4m3x2_f16x2(y0), cvt_e4m3x2_f16x2(y8), cvt_e4m3x2_hi_f16x2(y0),
-                              cvt_e4m3x2_hi_f16x2(y8), qb0[2 * bk + 1], qb1[2 * bk + 1]);
+                const uint32_t a0 = cvt_e4m3x2_f16x2(x0), b0 = cvt_e4m3x2_f16x2(x8), a1 = cvt_e4m3x2_hi_f16x2(x0), b1 = cvt_e4m3x2_hi_f16x2(x8);
+                const uint32_t a2 = cvt_e4m3x2_f16x2(y0), b2 = cvt_e4m3x2_f16x2(y8), a3 = cvt_e4m3x2_hi_f16x2(y0), b3 = cvt_e4m3x2_hi_f16x2(y8);
+#pragma unroll
+                for (int h = 0; h < NH; ++h) {
+                    mma_f16_16816_z(acc[h], a0, b0, a1, b1, qb0[h][2 * bk], qb1[h][2 * bk]);
+                    mma_f16_16816(acc[h], a2, b2, a3, b3, qb0[h][2 * bk + 1], qb1[h][2 * bk + 1]);
+                }
             }
-            if (bk == 0) {
-                sr[0] = acc[0] * ks0[0]; sr[1] = acc[1] * ks0[0]; sr[2] = acc[2] * ks8[0]; sr[3] = acc[3] * ks8[0];
-            } else {
-                sr[0] = fmaf(acc[0], ks0[bk], sr[0]);
-                sr[1] = fmaf(acc[1], ks0[bk], sr[1]);
-                sr[2] = fmaf(acc[2], ks8[bk], sr[2]);
-                sr[3] = fmaf(acc[3], ks8[bk], sr[3]);
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                float(&s)[4] = sr[h][u];
+                if (bk == 0) {
+                    s[0] = acc[h][0] * ks0[0]; s[1] = acc[h][1] * ks0[0]; s[2] = acc[h][2] * ks8[0]; s[3] = acc[h][3] * ks8[0];
+                } else {
+                    s[0] = fmaf(acc[h][0], ks0[bk], s[0]);
+                    s[1] = fmaf(acc[h][1], ks0[bk], s[1]);
+                    s[2] = fmaf(acc[h][2], ks8[bk], s[2]);
+                    s[3] = fmaf(acc[h][3], ks8[bk], s[3]);
+                }
             }
         }
     } else {
@@ -1065,9 +1160,12 @@ __device__ __forceinline__ void k_scores16(uint32_t ka, uint32_t krb, uint32_t m
                     a0 = hmul2_u32(a0, s0); a1 = hmul2_u32(a1, s0); a2 = hmul2_u32(a2, s0); a3 = hmul2_u32(a3, s0);
                     b0 = hmul2_u32(b0, s8); b1 = hmul2_u32(b1, s8); b2 = hmul2_u32(b2, s8); b3 = hmul2_u32(b3, s8);
                 }
-                if (w == 0) mma_f16_16816_z(sr, a0, b0, a1, b1, qb0[0], qb1[0]);
-                else mma_f16_16816(sr, a0, b0, a1, b1, qb0[2 * w], qb1[2 * w]);
-                mma_f16_16816(sr, a2, b2, a3, b3, qb0[2 * w + 1], qb1[2 * w + 1]);
+#pragma unroll
+                for (int h = 0; h < NH; ++h) {
+                    if (w == 0) mma_f16_16816_z(sr[h][u], a0, b0, a1, b1, qb0[h][0], qb1[h][0]);
+                    else mma_f16_16816(sr[h][u], a0, b0, a1, b1, qb0[h][2 * w], qb1[h][2 * w]);
+                    mma_f16_16816(sr[h][u], a2, b2, a3, b3, qb0[h][2 * w + 1], qb1[h][2 * w + 1]);
+                }
             }
         } else {
             uint32_t xs0[STEPS], xs8[STEPS];  // the lane's chunk of a row: HD / 4 bytes at a multiple of HD / 4
@@ -1076,25 +1174,28 @@ __device__ __forceinline__ void k_scores16(uint32_t ka, uint32_t krb, uint32_t m
 #pragma unroll
             for (int s = 0; s < STEPS; ++s) {
                 const uint32_t x0 = xs0[s], x8 = xs8[s];
-                if (s == 0)
-                    mma_f16_16816_z(sr, cvt_e4m3x2_f16x2(x0), cvt_e4m3x2_f16x2(x8), cvt_e4m3x2_hi_f16x2(x0),
-                                    cvt_e4m3x2_hi_f16x2(x8), qb0[0], qb1[0]);
-                else
-                    mma_f16_16816(sr, cvt_e4m3x2_f16x2(x0), cvt_e4m3x2_f16x2(x8), cvt_e4m3x2_hi_f16x2(x0),
-                                  cvt_e4m3x2_hi_f16x2(x8), qb0[s], qb1[s]);
+                const uint32_t a0 = cvt_e4m3x2_f16x2(x0), b0 = cvt_e4m3x2_f16x2(x8), a1 = cvt_e4m3x2_hi_f16x2(x0), b1 = cvt_e4m3x2_hi_f16x2(x8);
+#pragma unroll
+                for (int h = 0; h < NH; ++h) {
+                    if (s == 0) mma_f16_16816_z(sr[h][u], a0, b0, a1, b1, qb0[h][0], qb1[h][0]);
+                    else mma_f16_16816(sr[h][u], a0, b0, a1, b1, qb0[h][s], qb1[h][s]);
+                }
             }
         }
         const float kp0 = u2f(lds32(mrow)), kp8 = u2f(lds32(mrow + (PERM ? 2 : 8) * 4));
-        sr[0] *= kp0; sr[1] *= kp0; sr[2] *= kp8; sr[3] *= kp8;
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+            sr[h][u][0] *= kp0; sr[h][u][1] *= kp0; sr[h][u][2] *= kp8; sr[h][u][3] *= kp8;
+        }
     }
 }
 
 // O^T += V^T P^T for the 16 keys at `va` (the lane's first code byte of key 2c; rows vrb bytes apart): keys 2c, 2c+1 |
 // 2c+8, 2c+9, dims [g HD/8, (g+1) HD/8). `vsc_row`: the f16 block scales of the keys 2c, 2c + 1 (+ 16 bytes: 2c + 8,
-// 2c + 9), pb0 / pb1: the weights as B fragments.
+// 2c + 9), pb[h][2 u], pb[h][2 u + 1]: the weights of query rows 8 h ... as B fragments.
 // PERM: the lane's four keys are four consecutive rows from `va` on (perm_key below) instead of 2c, 2c + 1, 2c + 8, 2c + 9.
-template <int VM, int HD, bool WIDE = false, int AL = 4, bool PERM = false>
-__device__ __forceinline__ void v_accum16(uint32_t va, uint32_t vrb, uint32_t vsc_row, uint32_t pb0, uint32_t pb1, float (&oacc)[HD / 16][4],
+template <int VM, int HD, bool WIDE = false, int AL = 4, bool PERM = false, int NH = 1>
+__device__ __forceinline__ void v_accum16(uint32_t va, uint32_t vrb, uint32_t vsc_row, const uint32_t (&pb)[NH][4], int u, float (&oacc)[NH][HD / 16][4],
                                           uint32_t lut_v, uint32_t plane_v, int g) {
     constexpr bool V4 = fmt_is4(VM);
     constexpr int NBV = vsc_blocks(VM, HD);
@@ -1138,7 +1239,9 @@ __device__ __forceinline__ void v_accum16(uint32_t va, uint32_t vrb, uint32_t vs
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) mma_f16_16816(oacc[4 * w + i], l0[i], h0[i], l1[i], h1[i], pb0, pb1);
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int h = 0; h < NH; ++h) mma_f16_16816(oacc[h][4 * w + i], l0[i], h0[i], l1[i], h1[i], pb[h][2 * u], pb[h][2 * u + 1]);
         } else {
             const uint32_t ta0 = __byte_perm(xa, xb, 0x5140), ta1 = __byte_perm(xa, xb, 0x7362);
             const uint32_t tb0 = __byte_perm(xc, xd, 0x5140), tb1 = __byte_perm(xc, xd, 0x7362);
@@ -1152,8 +1255,11 @@ __device__ __forceinline__ void v_accum16(uint32_t va, uint32_t vrb, uint32_t vs
                 l0 = hmul2_u32(l0, sa); h0 = hmul2_u32(h0, sa); l2 = hmul2_u32(l2, sa); h2 = hmul2_u32(h2, sa);
                 l1 = hmul2_u32(l1, sb); h1 = hmul2_u32(h1, sb); l3 = hmul2_u32(l3, sb); h3 = hmul2_u32(h3, sb);
             }
-            mma_f16_16816(oacc[2 * w], l0, h0, l1, h1, pb0, pb1);
-            mma_f16_16816(oacc[2 * w + 1], l2, h2, l3, h3, pb0, pb1);
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                mma_f16_16816(oacc[h][2 * w], l0, h0, l1, h1, pb[h][2 * u], pb[h][2 * u + 1]);
+                mma_f16_16816(oacc[h][2 * w + 1], l2, h2, l3, h3, pb[h][2 * u], pb[h][2 * u + 1]);
+            }
         }
     }
 }
@@ -1218,14 +1324,15 @@ __device__ __forceinline__ Share worker_share(const DecodeParams &p, uint32_t ny
     sh.has_work = wid < sh.nw;
     sh.x_end = 0;
     if (!sh.has_work) return sh;
-    const uint64_t x_begin = total * wid / sh.nw;
-    sh.x_end = total * (wid + 1) / sh.nw;
+    const Places pl = places_of(p, total, sh.nw);
+    const uint64_t x_begin = share_start(p, pl, wid);
+    sh.x_end = share_start(p, pl, wid + 1);
     // batch entry that holds cost position x_begin, and the position of its first column
     uint32_t b0 = 0;
     uint64_t b0_start = 0;
     if (p.kv_len == nullptr) {
         const uint64_t per_b = batch_cost(0);
-        b0 = (uint32_t)(x_begin / per_b);
+        b0 = (total >> 32) == 0 ? (uint32_t)x_begin / (uint32_t)per_b : (uint32_t)div64(x_begin, per_b);
         b0_start = (uint64_t)b0 * per_b;
     } else if (few) {
         bool found = false;
@@ -1266,9 +1373,9 @@ __device__ __forceinline__ Share worker_share(const DecodeParams &p, uint32_t ny
     seg.b = b0;
     seg.col = make_column(p, b0);
     const uint32_t tb = (uint32_t)seg.col.tiles;
-    const uint64_t rem = x_begin - b0_start;
-    seg.y = (uint32_t)(rem / (tb + cc));
-    const uint32_t in_col = (uint32_t)(rem % (tb + cc));
+    const uint32_t rem = (uint32_t)(x_begin - b0_start);  // one entry's positions fit 32 bits (batch_cost)
+    seg.y = rem / (tb + cc);
+    const uint32_t in_col = rem - seg.y * (tb + cc);
     seg.t0 = in_col > cc ? in_col - cc : 0u;
     seg.x = b0_start + (uint64_t)seg.y * (tb + cc) + cc + seg.t0;
     if (seg.x >= sh.x_end) sh.has_work = false;  // the share lies inside a set up gap: no tile
@@ -1298,7 +1405,7 @@ struct Worker {
     size_t g_base;    // and the offset of this rank's rows in the step's slot of every rank's buffer
 
     __device__ __forceinline__ Worker(const DecodeParams &p_, int lane_, uint32_t wid_, uint32_t nw_grid_, uint32_t ny_, const Share &sh)
-        : p(p_), lane(lane_), wid(wid_), nw_grid(nw_grid_), ny(ny_), ncols(p_.b * ny_), prow(min((uint32_t)PACK, p_.rows_per_kv)),
+        : p(p_), lane(lane_), wid(wid_), nw_grid(nw_grid_), ny(ny_), ncols(p_.b * ny_), prow(min(p_.pack_rows, p_.rows_per_kv)),
           total(sh.total), nw(sh.nw), waited(false), g_step(0), g_base(0) {}
 
     __device__ __forceinline__ void prev_done() {
@@ -1357,63 +1464,72 @@ struct Worker {
         }
     }
 
-    // The end of a segment: oacc holds the unnormalized output rows 2c, 2c + 1 (dims [g HD/8, (g + 1) HD/8)) of the
+    // The end of a segment: oacc[h] holds the unnormalized output rows 8 h + 2c, + 1 (dims [g HD/8, (g + 1) HD/8)) of the
     // segment's keys, M / lsum their running maxima (log2 domain) and normalizers, summed over the warp. A column
     // that this worker covers alone is stored straight from the registers; otherwise the normalized partial result
     // and its log-sum-exp go to the workspace and the worker counts itself on the column's arrival counter: the last
     // to arrive merges the column. Without arrival counters the combine grid merges. Rotated values are rotated back in
     // registers, wherever a row is finished.
-    template <int HD>
-    __device__ __forceinline__ void finish_segment(const Segment &seg, const float (&oacc)[HD / 16][4], const float (&M)[2], const float (&lsum)[2]) {
+    template <int HD, int NH>
+    __device__ __forceinline__ void finish_segment(const Segment &seg, const float (&oacc)[NH][HD / 16][4], const float (&M)[NH][2], const float (&lsum)[NH][2]) {
         constexpr int STEPS = HD / 16;
         const int g = lane >> 2, c = lane & 3;
-        const uint32_t R = p.rows_per_kv, pack = seg.y % p.packs;
+        const uint32_t R = p.rows_per_kv, pack = pack_of(p, seg.y);
         if (!p.out_free) prev_done();
         const uint32_t colidx = seg.b * ny + seg.y;
-        const float inv0 = lsum[0] > 0.0f ? 1.0f / lsum[0] : 0.0f, inv1 = lsum[1] > 0.0f ? 1.0f / lsum[1] : 0.0f;
-        const uint32_t rr0 = 2 * c, rr1 = 2 * c + 1;
-        const bool w0 = rr0 < prow && pack * PACK + rr0 < R, w1 = rr1 < prow && pack * PACK + rr1 < R;
         // the column's segments are the workers first .. last (consecutive, every one of them owns a tile of it)
         const uint64_t x_col = seg.x - seg.t0;  // cost position of the column's first tile
-        const uint32_t first = seg.t0 == 0 ? wid : owner_of(x_col, total, nw);
-        const uint32_t last = seg.t1 == (uint32_t)seg.col.tiles ? wid : owner_of(x_col + seg.col.tiles - 1, total, nw);
+        const uint32_t first = seg.t0 == 0 ? wid : owner_of(p, places_of(p, total, nw), x_col);
+        const uint32_t last = seg.t1 == (uint32_t)seg.col.tiles ? wid : owner_of(p, places_of(p, total, nw), x_col + seg.col.tiles - 1);
         const uint32_t nseg = last - first + 1;
         if (p.ctr && nseg == 1) {
             // the whole column in this worker's registers
-            float o0[HD / 8], o1[HD / 8];
 #pragma unroll
-            for (int mt = 0; mt < STEPS; ++mt) {
-                o0[2 * mt] = oacc[mt][0] * inv0; o0[2 * mt + 1] = oacc[mt][2] * inv0;
-                o1[2 * mt] = oacc[mt][1] * inv1; o1[2 * mt + 1] = oacc[mt][3] * inv1;
-            }
-            if (p.v.rot == B200_ROT_HADAMARD) {
-                // rows 2c and 2c + 1, each spread over the eight lanes g = 0..7 of this c (part = lane >> 2)
-                hadamard_back_parts<HD / 8>(o0, lane, 4, 8, 16, p.v.signs, g * (HD / 8));
-                hadamard_back_parts<HD / 8>(o1, lane, 4, 8, 16, p.v.signs, g * (HD / 8));
-            }
-            size_t obase, grow;
-            if (w0 && row_addr(p, seg.b, seg.y, rr0, obase, grow)) {
-                store_row_piece<HD / 8>(p.out, obase + g * (HD / 8), o0, p.out_dtype);
-                for (uint32_t pr = 0; pr < p.world; ++pr) store_row_piece<HD / 8>(p.peer_bufs[pr], g_base + grow * HD + g * (HD / 8), o0, p.out_dtype);
-            }
-            if (w1 && row_addr(p, seg.b, seg.y, rr1, obase, grow)) {
-                store_row_piece<HD / 8>(p.out, obase + g * (HD / 8), o1, p.out_dtype);
-                for (uint32_t pr = 0; pr < p.world; ++pr) store_row_piece<HD / 8>(p.peer_bufs[pr], g_base + grow * HD + g * (HD / 8), o1, p.out_dtype);
+            for (int h = 0; h < NH; ++h) {
+                const float inv0 = lsum[h][0] > 0.0f ? 1.0f / lsum[h][0] : 0.0f, inv1 = lsum[h][1] > 0.0f ? 1.0f / lsum[h][1] : 0.0f;
+                const uint32_t rr0 = PACK * h + 2 * c, rr1 = rr0 + 1;
+                const bool w0 = rr0 < prow && pack * p.pack_rows + rr0 < R, w1 = rr1 < prow && pack * p.pack_rows + rr1 < R;
+                float o0[HD / 8], o1[HD / 8];
+#pragma unroll
+                for (int mt = 0; mt < STEPS; ++mt) {
+                    o0[2 * mt] = oacc[h][mt][0] * inv0; o0[2 * mt + 1] = oacc[h][mt][2] * inv0;
+                    o1[2 * mt] = oacc[h][mt][1] * inv1; o1[2 * mt + 1] = oacc[h][mt][3] * inv1;
+                }
+                if (p.v.rot == B200_ROT_HADAMARD) {
+                    // rows 2c and 2c + 1, each spread over the eight lanes g = 0..7 of this c (part = lane >> 2)
+                    hadamard_back_parts<HD / 8>(o0, lane, 4, 8, 16, p.v.signs, g * (HD / 8));
+                    hadamard_back_parts<HD / 8>(o1, lane, 4, 8, 16, p.v.signs, g * (HD / 8));
+                }
+                size_t obase, grow;
+                if (w0 && row_addr(p, seg.b, seg.y, rr0, obase, grow)) {
+                    store_row_piece<HD / 8>(p.out, obase + g * (HD / 8), o0, p.out_dtype);
+                    for (uint32_t pr = 0; pr < p.world; ++pr) store_row_piece<HD / 8>(p.peer_bufs[pr], g_base + grow * HD + g * (HD / 8), o0, p.out_dtype);
+                }
+                if (w1 && row_addr(p, seg.b, seg.y, rr1, obase, grow)) {
+                    store_row_piece<HD / 8>(p.out, obase + g * (HD / 8), o1, p.out_dtype);
+                    for (uint32_t pr = 0; pr < p.world; ++pr) store_row_piece<HD / 8>(p.peer_bufs[pr], g_base + grow * HD + g * (HD / 8), o1, p.out_dtype);
+                }
             }
             column_done();
             return;
         }
         const size_t slot = (size_t)wid + colidx;
-        float *po0 = p.part_o + (slot * prow + rr0) * HD + g * (HD / 8);
-        float *po1 = p.part_o + (slot * prow + rr1) * HD + g * (HD / 8);
 #pragma unroll
-        for (int mt = 0; mt < STEPS; ++mt) {
-            if (w0) *reinterpret_cast<float2 *>(po0 + 2 * mt) = make_float2(oacc[mt][0] * inv0, oacc[mt][2] * inv0);
-            if (w1) *reinterpret_cast<float2 *>(po1 + 2 * mt) = make_float2(oacc[mt][1] * inv1, oacc[mt][3] * inv1);
-        }
-        if (g == 0) {
-            if (w0) p.part_lse[slot * prow + rr0] = lsum[0] > 0.0f ? M[0] * LN2 + logf(lsum[0]) : -INFINITY;
-            if (w1) p.part_lse[slot * prow + rr1] = lsum[1] > 0.0f ? M[1] * LN2 + logf(lsum[1]) : -INFINITY;
+        for (int h = 0; h < NH; ++h) {
+            const float inv0 = lsum[h][0] > 0.0f ? 1.0f / lsum[h][0] : 0.0f, inv1 = lsum[h][1] > 0.0f ? 1.0f / lsum[h][1] : 0.0f;
+            const uint32_t rr0 = PACK * h + 2 * c, rr1 = rr0 + 1;
+            const bool w0 = rr0 < prow && pack * p.pack_rows + rr0 < R, w1 = rr1 < prow && pack * p.pack_rows + rr1 < R;
+            float *po0 = p.part_o + (slot * prow + rr0) * HD + g * (HD / 8);
+            float *po1 = p.part_o + (slot * prow + rr1) * HD + g * (HD / 8);
+#pragma unroll
+            for (int mt = 0; mt < STEPS; ++mt) {
+                if (w0) *reinterpret_cast<float2 *>(po0 + 2 * mt) = make_float2(oacc[h][mt][0] * inv0, oacc[h][mt][2] * inv0);
+                if (w1) *reinterpret_cast<float2 *>(po1 + 2 * mt) = make_float2(oacc[h][mt][1] * inv1, oacc[h][mt][3] * inv1);
+            }
+            if (g == 0) {
+                if (w0) p.part_lse[slot * prow + rr0] = lsum[h][0] > 0.0f ? M[h][0] * LN2 + logf(lsum[h][0]) : -INFINITY;
+                if (w1) p.part_lse[slot * prow + rr1] = lsum[h][1] > 0.0f ? M[h][1] * LN2 + logf(lsum[h][1]) : -INFINITY;
+            }
         }
         if (p.ctr) {
             // count this segment; the last of the column's workers to get here merges them all
@@ -1456,11 +1572,20 @@ struct CopySide {
     uint32_t pg, off, pg_rows, k_cap, v_cap;
     uintptr_t pk, pv;
 
+    uint64_t pol;  // cache policy of the copies
+
+    // Rows that a call reads once and that do not fit L2 together leave first: otherwise they push the call's own code, its queries
+    // and partial results out (a merge of 4.4 partial results took 22 instead of 7 thousand cycles).
+    __device__ __forceinline__ void policy(const DecodeParams &p) {
+        if (p.stream) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+        else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+    }
+
     // per-segment constants
     __device__ __forceinline__ void enter(const DecodeParams &p, uint32_t krb, uint32_t vrb) {
         left = (int)(iseg.t1 - iseg.t0);
         simple = left - (iseg.t1 == (uint32_t)iseg.col.tiles ? 1 : 0);
-        const uint32_t hk = iseg.y / p.packs;
+        const uint32_t hk = head_of(p, iseg.y);
         key = iseg.col.lo + (int)iseg.t0 * WK;
         const uintptr_t ka = reinterpret_cast<uintptr_t>(p.k_rows + (size_t)iseg.b * p.k_sb + (size_t)hk * p.k_sh) + (uintptr_t)(uint32_t)key * krb;
         const uintptr_t va = reinterpret_cast<uintptr_t>(p.v_rows + (size_t)iseg.b * p.v_sb + (size_t)hk * p.v_sh) + (uintptr_t)(uint32_t)key * vrb;
@@ -1473,6 +1598,7 @@ struct CopySide {
     }
 
     __device__ __forceinline__ void start(const DecodeParams &p, const Segment &seg, uint32_t krb, uint32_t vrb) {
+        policy(p);
         iseg = seg;
         more = true;
         enter(p, krb, vrb);
@@ -1481,7 +1607,7 @@ struct CopySide {
     // ---- paged rows: a tile's source is (block, row in the block) instead of rows + key * stride
     __device__ __forceinline__ void load_page(const DecodeParams &p, uint32_t krb, uint32_t vrb) {
         const B200Page pgd = p.pages[pg];
-        const uint32_t hk = iseg.y / p.packs;
+        const uint32_t hk = head_of(p, iseg.y);
         pg_rows = pgd.rows;
         k_cap = pgd.k_cap;
         v_cap = pgd.v_cap;
@@ -1497,6 +1623,7 @@ struct CopySide {
         load_page(p, krb, vrb);
     }
     __device__ __forceinline__ void start_paged(const DecodeParams &p, const Segment &seg, uint32_t krb, uint32_t vrb) {
+        policy(p);
         iseg = seg;
         more = true;
         enter_paged(p, krb, vrb);
@@ -1532,12 +1659,12 @@ struct CopySide {
         if (lane == 0) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kbt + vbt) : "memory");
             if (kbt)
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(st), "l"(k0), "r"(kbt),
-                             "r"(bar)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(st), "l"(k0), "r"(kbt),
+                             "r"(bar), "l"(pol)
                              : "memory");
             if (vbt)
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(st + k_stage_bytes),
-                             "l"(v0), "r"(vbt), "r"(bar)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(st + k_stage_bytes),
+                             "l"(v0), "r"(vbt), "r"(bar), "l"(pol)
                              : "memory");
         }
         off += WK;
@@ -1564,11 +1691,11 @@ struct CopySide {
             --simple;
             if (lane == 0) {
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kb + vb) : "memory");
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(st), "l"(k),
-                             "r"(kb), "r"(bar)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(st), "l"(k),
+                             "r"(kb), "r"(bar), "l"(pol)
                              : "memory");
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(st + k_stage_bytes),
-                             "l"(v), "r"(vb), "r"(bar)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(st + k_stage_bytes),
+                             "l"(v), "r"(vb), "r"(bar), "l"(pol)
                              : "memory");
             }
         } else {
@@ -1596,13 +1723,13 @@ struct CopySide {
             if (lane == 0) {
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kbt + vbt) : "memory");
                 if (kbt)
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(st), "l"(k),
-                                 "r"(kbt), "r"(bar)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(st), "l"(k),
+                                 "r"(kbt), "r"(bar), "l"(pol)
                                  : "memory");
                 if (vbt)
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
                                      st + k_stage_bytes),
-                                 "l"(v), "r"(vbt), "r"(bar)
+                                 "l"(v), "r"(vbt), "r"(bar), "l"(pol)
                                  : "memory");
             }
         }
@@ -1635,15 +1762,11 @@ __device__ __forceinline__ bool stage_wait(uint32_t bar, uint32_t par) {
 
 // Visible keys of row r of a column's rows (ordered by token), bottom-right aligned masks
 __device__ __forceinline__ void row_range(const DecodeParams &p, const Column &col, uint32_t r, int &lo, int &hi, int &pos) {
-    const long long i = p.lq == 1 ? 0 : r / p.group;
-    const long long ps = i + (long long)col.lk - (long long)p.lq;
-    long long l = p.wl >= 0 ? max(ps - p.wl, 0ll) : 0ll;
-    long long h = p.wr >= 0 ? min(ps + p.wr + 1, (long long)col.lk) : (long long)col.lk;
-    l = min(l, (long long)col.lk);
-    h = max(h, l);
-    lo = (int)l;
-    hi = (int)h;
-    pos = (int)max(min(ps, 2147483647ll), -2147483647ll);
+    const int ps = (p.lq == 1 ? 0 : (int)(r / p.group)) + col.lk - (int)p.lq;
+    lo = p.wl >= 0 && ps > p.wl ? min(ps - p.wl, col.lk) : 0;
+    hi = p.wr >= 0 && ps < col.lk - 1 - p.wr ? ps + p.wr + 1 : col.lk;
+    hi = max(hi, lo);
+    pos = ps;
 }
 
 // Scores of a tile -> weights: vm from the tile's per-key scalars, plain or masked softmax. Returns whether the
@@ -1660,7 +1783,7 @@ struct SegMask {
 __host__ __device__ constexpr int perm_key(int g) { return (g & 1) + 8 * ((g >> 1) & 1) + 4 * (g >> 2); }
 
 template <bool PERM = false>
-__device__ __forceinline__ bool tile_softmax(const DecodeParams &p, const Segment &seg, const SegMask &sm, int key0, int nkeys, uint32_t vmeta_g,
+__device__ __forceinline__ bool tile_softmax(const DecodeParams &p, const Segment &seg, const SegMask &sm, uint32_t row0, int key0, int nkeys, uint32_t vmeta_g,
                                              const float (&sr)[2][4], const float (&qs)[2], const float (&qs2)[2], float (&M)[2], float (&lsum)[2],
                                              uint32_t (&pb)[4], float (&al)[2], int lane) {
     const int g = lane >> 2, c = lane & 3;
@@ -1669,11 +1792,11 @@ __device__ __forceinline__ bool tile_softmax(const DecodeParams &p, const Segmen
     for (int k = 0; k < 4; ++k) vm[k] = lds64f(vmeta_g + (PERM ? 16 * (k & 1) + 128 * (k >> 1) : k * 64));
     if (B200_LIKELY(sm.plain && nkeys == WK && key0 >= sm.LOmax && key0 + WK <= sm.HImin)) return softmax_plain(sr, vm, qs2, M, lsum, pb, al);
     // masks, soft-capping, ALiBi: the two query rows whose scores this lane holds (columns 2c, 2c + 1)
-    const uint32_t hk = seg.y / p.packs, pack = seg.y % p.packs, G = p.group;
+    const uint32_t hk = head_of(p, seg.y), G = p.group;
     RowMask rm;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-        const uint32_t r = pack * PACK + 2 * c + e;
+        const uint32_t r = row0 + 2 * c + e;
         rm.lo[e] = rm.hi[e] = rm.pos[e] = 0;
         rm.slope[e] = 0.0f;
         if (r < p.rows_per_kv) {
@@ -1688,11 +1811,11 @@ __device__ __forceinline__ bool tile_softmax(const DecodeParams &p, const Segmen
 __device__ __forceinline__ SegMask segment_mask(const DecodeParams &p, const Segment &seg) {
     // rows are ordered by token: the last row of the pack has the highest lower bound, the first the lowest upper bound
     SegMask sm;
-    const uint32_t pack = seg.y % p.packs;
+    const uint32_t pack = pack_of(p, seg.y);
     int lo, hi, pos;
-    row_range(p, seg.col, min(pack * PACK + PACK, p.rows_per_kv) - 1, lo, hi, pos);
+    row_range(p, seg.col, min((pack + 1) * p.pack_rows, p.rows_per_kv) - 1, lo, hi, pos);
     sm.LOmax = lo;
-    row_range(p, seg.col, pack * PACK, lo, hi, pos);
+    row_range(p, seg.col, pack * p.pack_rows, lo, hi, pos);
     sm.HImin = hi;
     sm.plain = p.softcap <= 0.0f && p.alibi == nullptr;
     return sm;
@@ -1727,8 +1850,11 @@ __device__ __forceinline__ void load_codebooks(const DecodeParams &p, uint32_t l
 // ---------------------------------------------------------------------------------------------
 // PAGED: the rows live in the blocks of a page table; tiles are cut at the blocks' ends, the copy side leaves a
 // description of every tile beside its stage, and the row strides are those of the call (NAT is not combined with it).
-template <int KM, int VM, int HD, bool NAT, bool PAGED = false>
-__global__ void __launch_bounds__(DW * 32, B200_DECODE_MIN_BLOCKS) tq_decode_kernel(const DecodeParams p) {
+// NH: groups of eight query rows of a column (1 or 2). With more than eight rows per kv head (several query tokens, or a wide
+// group) two groups share every decoded key and value: the decoding is most of a tile's instructions. Twice the accumulators
+// and query fragments take a block per SM less (two blocks of 255 registers instead of three of 168).
+template <int KM, int VM, int HD, bool NAT, bool PAGED = false, int NH = 1>
+__global__ void __launch_bounds__(DW * 32, decode_blocks(NH)) tq_decode_kernel(const DecodeParams p) {
     constexpr int STEPS = HD / 16;          // k-steps of K Q^T == m-tiles of the output
     constexpr bool K4 = fmt_is4(KM), V4 = fmt_is4(VM);
     constexpr bool KMX = fmt_is_mx(KM);     // block-wise accumulation, contraction order A
@@ -1757,13 +1883,16 @@ __global__ void __launch_bounds__(DW * 32, B200_DECODE_MIN_BLOCKS) tq_decode_ker
         for (int i = 0; i < DW * NS_MAX; ++i) mbar_init(&bars[i], 1);
         mbar_fence_init();
     }
+    if constexpr (PAGED) {
+        if (p.pg_build && warp == 1) page_prefix(p, lane);
+    }
     load_codebooks<KM, VM>(p, lut_k, lut_v, plane_k, tid, DW * 32);
     __syncthreads();
     // the next kernel of the stream may be scheduled from here on (a combine grid, or the next attention launched as
     // a programmatic dependent); it waits for this grid's completion itself before it touches memory
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    // paged rows: the kernel that wrote the table's prefix sums is the stream's previous kernel, and this grid was
+    // paged rows: where a kernel wrote the table's prefix sums it is the stream's previous kernel, and this grid was
     // launched as its programmatic dependent (its launch latency is hidden): the sums are read from here on
     if constexpr (PAGED) asm volatile("griddepcontrol.wait;" ::: "memory");
     const Share sh = worker_share(p, ny, wid, nw_grid, lane);
@@ -1785,9 +1914,8 @@ __global__ void __launch_bounds__(DW * 32, B200_DECODE_MIN_BLOCKS) tq_decode_ker
     const uint32_t wdesc_s = sbase + FIXED_SMEM + DW * META + p.qstage_bytes + (uint32_t)DW * NS * stage_bytes + (uint32_t)warp * NS_MAX * 16;
     bool wait_failed = false;
 
-    // Filling the ring. With the caller's word that the inputs are final (prefetch) all stages are asked for right away.
-    // Otherwise the first tile alone, and the other stages once the first query rows are loaded: with every worker of
-    // the grid asking for all its stages at once, the first tiles would arrive behind 26 MB of later ones.
+    // All stages are asked for right away: the first tiles land a little later than alone, but the code that asks is fetched
+    // once (ragged MXFP4 call: 92.7 -> 91.3 us; 64 x 2 query tokens, 64 heads: 139.6 -> 138.5).
     CopySide cs;
     if constexpr (PAGED) cs.start_paged(p, sh.seg, krb, vrb);
     else cs.start(p, sh.seg, krb, vrb);
@@ -1795,12 +1923,8 @@ __global__ void __launch_bounds__(DW * 32, B200_DECODE_MIN_BLOCKS) tq_decode_ker
         if constexpr (PAGED) cs.tile_paged(wk, st, bar, desc, krb, vrb, k_stage_bytes, sh.x_end);
         else cs.tile(wk, st, bar, krb, vrb, k_stage_bytes, sh.x_end);
     };
-    int primed = 0;
-    auto prime = [&](int upto) {
-        for (; primed < upto && cs.left > 0; ++primed)
-            copy_tile(wstage_s + (uint32_t)primed * stage_bytes, wbar_s + 8u * (uint32_t)primed, wdesc_s + 16u * (uint32_t)primed);
-    };
-    prime(p.prefetch ? NS : 1);
+    for (int i = 0; i < NS && cs.left > 0; ++i)
+        copy_tile(wstage_s + (uint32_t)i * stage_bytes, wbar_s + 8u * (uint32_t)i, wdesc_s + 16u * (uint32_t)i);
 
     // ------------------------------------------------------------------ the compute side
     // lane offsets inside a tile: K rows g (and g + 8), V rows 2c (and 2c + 1, 2c + 8, 2c + 9)
@@ -1811,26 +1935,30 @@ __global__ void __launch_bounds__(DW * 32, B200_DECODE_MIN_BLOCKS) tq_decode_ker
     int c_stage = 0;
     uint32_t par = 0;  // parity to wait for on the current stage: flips every time the ring wraps
 
-    uint32_t qb0[STEPS], qb1[STEPS];
-    float qs[2], qs2[2];
-    float oacc[STEPS][4];
+    uint32_t qb0[NH][STEPS], qb1[NH][STEPS];
+    float qs[NH][2], qs2[NH][2];
+    float oacc[NH][STEPS][4];
 
     Segment seg = sh.seg;
     bool more = true;
     while (more) {
         // ================================================================ segment set up
-        const uint32_t hk = seg.y / p.packs, pack = seg.y % p.packs;
+        const uint32_t hk = head_of(p, seg.y), row0 = pack_of(p, seg.y) * (PACK * NH);
         const Column &col = seg.col;
         const SegMask sm = segment_mask(p, seg);
         // running maxima (log2 domain, value scale folded in) and partial normalizers of rows 2c, 2c + 1
-        float M[2] = {-1e30f, -1e30f}, lsum[2] = {0.0f, 0.0f};
+        float M[NH][2], lsum[NH][2];
 #pragma unroll
-        for (int mt = 0; mt < STEPS; ++mt) oacc[mt][0] = oacc[mt][1] = oacc[mt][2] = oacc[mt][3] = 0.0f;
+        for (int h = 0; h < NH; ++h) {
+            M[h][0] = M[h][1] = -1e30f;
+            lsum[h][0] = lsum[h][1] = 0.0f;
+#pragma unroll
+            for (int mt = 0; mt < STEPS; ++mt) oacc[h][mt][0] = oacc[h][mt][1] = oacc[h][mt][2] = oacc[h][mt][3] = 0.0f;
+        }
 
         if (!wait_failed) {
-            load_query<KM, HD>(p, seg.b, hk, pack, qstage, lane, qb0, qb1, qs, qs2);
-            // the other stages of the ring (first segment only)
-            prime(NS);
+#pragma unroll
+            for (int h = 0; h < NH; ++h) load_query<KM, HD>(p, seg.b, hk, row0 + PACK * h, qstage, lane, qb0[h], qb1[h], qs[h], qs2[h]);
 
             // ============================================================ the tiles of the segment
             const int n_t = (int)(seg.t1 - seg.t0);
@@ -1867,25 +1995,28 @@ __global__ void __launch_bounds__(DW * 32, B200_DECODE_MIN_BLOCKS) tq_decode_ker
                 if (B200_UNLIKELY(nkeys < WK)) clear_stale_rows(st_s + tk_off, st_s + k_stage_bytes + tv_off, nkeys, krb, vrb, lane);
                 // ---- per-key scalars of the tile, lane = key
                 tile_meta<KM, VM, HD>(st_s + kr_off, st_s + vr_off, meta_s, vmeta_s, vsc_s, lane);
-                // ---- scores of the 32 keys: sr[u][2 k + e] = key 16 u + g + 8 k, row 2c + e
-                float sr[2][4];
-                k_scores16<KM, HD, false, KAL>(st_s + kt_off, krb, mrow_g, qb0, qb1, lut_k, plane_k, c, sr[0]);
-                k_scores16<KM, HD, false, KAL>(st_s + kt_off + 16 * krb, krb, mrow_g + 16 * KMW * 4, qb0, qb1, lut_k, plane_k, c, sr[1]);
+                // ---- scores of the 32 keys: sr[h][u][2 k + e] = key 16 u + g + 8 k, row 8 h + 2c + e
+                float sr[NH][2][4];
+                k_scores16<KM, HD, false, KAL, false, NH>(st_s + kt_off, krb, mrow_g, qb0, qb1, lut_k, plane_k, c, sr, 0);
+                k_scores16<KM, HD, false, KAL, false, NH>(st_s + kt_off + 16 * krb, krb, mrow_g + 16 * KMW * 4, qb0, qb1, lut_k, plane_k, c, sr, 1);
                 // ---- online softmax
-                uint32_t pb[4];
-                float al[2];
-                if (B200_UNLIKELY(tile_softmax(p, seg, sm, key0, nkeys, vmeta_g, sr, qs, qs2, M, lsum, pb, al, lane))) {
+                uint32_t pb[NH][4];
 #pragma unroll
-                    for (int mt = 0; mt < STEPS; ++mt) {
-                        oacc[mt][0] *= al[0];
-                        oacc[mt][1] *= al[1];
-                        oacc[mt][2] *= al[0];
-                        oacc[mt][3] *= al[1];
+                for (int h = 0; h < NH; ++h) {
+                    float al[2];
+                    if (B200_UNLIKELY(tile_softmax(p, seg, sm, row0 + PACK * h, key0, nkeys, vmeta_g, sr[h], qs[h], qs2[h], M[h], lsum[h], pb[h], al, lane))) {
+#pragma unroll
+                        for (int mt = 0; mt < STEPS; ++mt) {
+                            oacc[h][mt][0] *= al[0];
+                            oacc[h][mt][1] *= al[1];
+                            oacc[h][mt][2] *= al[0];
+                            oacc[h][mt][3] *= al[1];
+                        }
                     }
                 }
                 // ---- O^T += V^T P^T
-                v_accum16<VM, HD, false, VAL>(st_s + vt_off, vrb, vsc_c, pb[0], pb[1], oacc, lut_v, plane_v, g);
-                v_accum16<VM, HD, false, VAL>(st_s + vt_off + 16 * vrb, vrb, vsc_c + 32, pb[2], pb[3], oacc, lut_v, plane_v, g);
+                v_accum16<VM, HD, false, VAL, false, NH>(st_s + vt_off, vrb, vsc_c, pb, 0, oacc, lut_v, plane_v, g);
+                v_accum16<VM, HD, false, VAL, false, NH>(st_s + vt_off + 16 * vrb, vrb, vsc_c + 32, pb, 1, oacc, lut_v, plane_v, g);
                 // the stage was read (and possibly patched) through the generic proxy: order that before the
                 // bulk copy of the next tile into it
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1904,11 +2035,13 @@ __global__ void __launch_bounds__(DW * 32, B200_DECODE_MIN_BLOCKS) tq_decode_ker
 
         // ================================================================ this warp's partial result of the column
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
-            lsum[0] += __shfl_xor_sync(0xffffffffu, lsum[0], o);
-            lsum[1] += __shfl_xor_sync(0xffffffffu, lsum[1], o);
-        }
-        wk.finish_segment<HD>(seg, oacc, M, lsum);
+        for (int h = 0; h < NH; ++h)
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                lsum[h][0] += __shfl_xor_sync(0xffffffffu, lsum[h][0], o);
+                lsum[h][1] += __shfl_xor_sync(0xffffffffu, lsum[h][1], o);
+            }
+        wk.finish_segment<HD, NH>(seg, oacc, M, lsum);
         more = next_segment(seg, p, ny, sh.x_end);
     }
     wk.zero_columns<HD>(true);
@@ -2033,7 +2166,7 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
         const uint32_t kg = PERM ? (uint32_t)perm_key(g) : (uint32_t)g;  // the key (of 16) behind the lane's row g
         const uint32_t k_lane = kg * krb + (KMX ? (K4 ? 4u * c : 8u * c) : (K4 ? c * (HD / 8) : c * (HD / 4)));
         const uint32_t mrow_g = meta_s + kg * KMW * 4, vmeta_g = vmeta_s + kg * 8;
-        uint32_t qb0[STEPS], qb1[STEPS];
+        uint32_t qb0[1][STEPS], qb1[1][STEPS];
         float qs[2], qs2[2];
         // a free slot for message `msgs`: the values' warp has taken message msgs - PQ
         auto slot_wait = [&]() -> bool {
@@ -2046,11 +2179,11 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
             ++msgs;
         };
         while (more && !wait_failed) {
-            const uint32_t hk = seg.y / p.packs, pack = seg.y % p.packs;
+            const uint32_t hk = head_of(p, seg.y), row0 = pack_of(p, seg.y) * PACK;
             const Column &col = seg.col;
             const SegMask sm = segment_mask(p, seg);
             float M[2] = {-1e30f, -1e30f}, lsum[2] = {0.0f, 0.0f};
-            load_query<KM, HD>(p, seg.b, hk, pack, qstage, lane, qb0, qb1, qs, qs2);
+            load_query<KM, HD>(p, seg.b, hk, row0, qstage, lane, qb0[0], qb1[0], qs, qs2);
             const int n_t = (int)(seg.t1 - seg.t0);
             int key0 = col.lo + (int)seg.t0 * WK;
             const uint32_t koff = (uint32_t)((reinterpret_cast<uintptr_t>(p.k_rows + (size_t)seg.b * p.k_sb + (size_t)hk * p.k_sh) + (uintptr_t)(uint32_t)key0 * krb) & 15u);
@@ -2066,12 +2199,12 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
                 const int nkeys = min(WK, col.hi - key0);
                 if (nkeys < WK) clear_stale_rows(st_s + koff, st_s + k_stage_bytes + voff, nkeys, krb, vrb, lane);
                 tile_meta<KM, VM, HD>(st_s + kr_off, st_s + vr_off, meta_s, vmeta_s, msg_s + 784, lane);
-                float sr[2][4];
-                k_scores16<KM, HD, WIDE, KAL, PERM>(st_s + kt_off, krb, mrow_g, qb0, qb1, lut_k, plane_k, c, sr[0]);
-                k_scores16<KM, HD, WIDE, KAL, PERM>(st_s + kt_off + 16 * krb, krb, mrow_g + 16 * KMW * 4, qb0, qb1, lut_k, plane_k, c, sr[1]);
+                float sr[1][2][4];
+                k_scores16<KM, HD, WIDE, KAL, PERM>(st_s + kt_off, krb, mrow_g, qb0, qb1, lut_k, plane_k, c, sr, 0);
+                k_scores16<KM, HD, WIDE, KAL, PERM>(st_s + kt_off + 16 * krb, krb, mrow_g + 16 * KMW * 4, qb0, qb1, lut_k, plane_k, c, sr, 1);
                 uint32_t pb[4];
                 float al[2];
-                const bool moved = tile_softmax<PERM>(p, seg, sm, key0, nkeys, vmeta_g, sr, qs, qs2, M, lsum, pb, al, lane);
+                const bool moved = tile_softmax<PERM>(p, seg, sm, row0, key0, nkeys, vmeta_g, sr[0], qs, qs2, M, lsum, pb, al, lane);
                 asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(msg_s + lane * 16), "r"(pb[0]), "r"(pb[1]), "r"(pb[2]), "r"(pb[3]) : "memory");
                 if (moved) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(msg_s + 512 + lane * 8), "f"(al[0]), "f"(al[1]) : "memory");
                 if (lane == 0) sts32(msg_s + 768, moved ? 1u : 0u);
@@ -2105,7 +2238,7 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
     } else {
         // ============================================================== the values' warp
         const uint32_t v_lane = (PERM ? (uint32_t)perm_key(2 * c) : 2u * c) * vrb + (V4 ? g * (HD / 16) : g * (HD / 8));
-        float oacc[STEPS][4];
+        float oacc[1][STEPS][4];
         CopySide cs;
         cs.start(p, sh.seg, krb, vrb);
         for (int i = 0; i < NS && cs.left > 0; ++i)
@@ -2117,11 +2250,11 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
             ++msgs;
         };
         while (more) {
-            const uint32_t hk = seg.y / p.packs;
+            const uint32_t hk = head_of(p, seg.y);
             const Column &col = seg.col;
-            float M[2] = {-1e30f, -1e30f}, lsum[2] = {0.0f, 0.0f};
+            float M[1][2] = {{-1e30f, -1e30f}}, lsum[1][2] = {{0.0f, 0.0f}};
 #pragma unroll
-            for (int mt = 0; mt < STEPS; ++mt) oacc[mt][0] = oacc[mt][1] = oacc[mt][2] = oacc[mt][3] = 0.0f;
+            for (int mt = 0; mt < STEPS; ++mt) oacc[0][mt][0] = oacc[0][mt][1] = oacc[0][mt][2] = oacc[0][mt][3] = 0.0f;
             if (!wait_failed) {
                 const int n_t = (int)(seg.t1 - seg.t0);
                 const int key0 = col.lo + (int)seg.t0 * WK;
@@ -2140,17 +2273,17 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
                         const float2 al = lds64f(msg_s + 512 + lane * 8);
 #pragma unroll
                         for (int mt = 0; mt < STEPS; ++mt) {
-                            oacc[mt][0] *= al.x;
-                            oacc[mt][1] *= al.y;
-                            oacc[mt][2] *= al.x;
-                            oacc[mt][3] *= al.y;
+                            oacc[0][mt][0] *= al.x;
+                            oacc[0][mt][1] *= al.y;
+                            oacc[0][mt][2] *= al.x;
+                            oacc[0][mt][3] *= al.y;
                         }
                     }
-                    uint32_t pb[4];
-                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(pb[0]), "=r"(pb[1]), "=r"(pb[2]), "=r"(pb[3]) : "r"(msg_s + lane * 16));
+                    uint32_t pb[1][4];
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(pb[0][0]), "=r"(pb[0][1]), "=r"(pb[0][2]), "=r"(pb[0][3]) : "r"(msg_s + lane * 16));
                     const uint32_t vsc_c = msg_s + 784 + 4 * c;
-                    v_accum16<VM, HD, WIDE, VAL, PERM>(st_s + vt_off, vrb, vsc_c, pb[0], pb[1], oacc, lut_v, plane_v, g);
-                    v_accum16<VM, HD, WIDE, VAL, PERM>(st_s + vt_off + 16 * vrb, vrb, vsc_c + 32, pb[2], pb[3], oacc, lut_v, plane_v, g);
+                    v_accum16<VM, HD, WIDE, VAL, PERM>(st_s + vt_off, vrb, vsc_c, pb, 0, oacc, lut_v, plane_v, g);
+                    v_accum16<VM, HD, WIDE, VAL, PERM>(st_s + vt_off + 16 * vrb, vrb, vsc_c + 32, pb, 1, oacc, lut_v, plane_v, g);
                     // the stage was read through the generic proxy (by both warps: the keys' warp before it sent the
                     // message): order that before the bulk copy of the next tile into it
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -2168,7 +2301,7 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
                 if (!wait_failed) {
                     if (msg_wait()) {
                         const float4 ml = lds128f(queue_s + (msgs % PQ) * MSG + lane * 16);
-                        M[0] = ml.x; M[1] = ml.y; lsum[0] = ml.z; lsum[1] = ml.w;
+                        M[0][0] = ml.x; M[0][1] = ml.y; lsum[0][0] = ml.z; lsum[0][1] = ml.w;
                         msg_done();
                     } else {
                         wait_failed = true;
@@ -2178,9 +2311,9 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
             }
             if (wait_failed) {
                 // void outputs (the status says so); the segment is still counted, so that no column waits for it
-                lsum[0] = lsum[1] = 0.0f;
+                lsum[0][0] = lsum[0][1] = 0.0f;
             }
-            wk.finish_segment<HD>(seg, oacc, M, lsum);
+            wk.finish_segment<HD, 1>(seg, oacc, M, lsum);
             more = next_segment(seg, p, ny, sh.x_end);
         }
         wk.zero_columns<HD>(true);
@@ -2205,7 +2338,7 @@ __global__ void __launch_bounds__(128) tq_combine_kernel(const DecodeParams p) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t rows = (size_t)p.b * p.hq * p.lq;
     const uint32_t ny = p.hkv * p.packs;
-    const uint32_t prow = min((uint32_t)PACK, p.rows_per_kv);
+    const uint32_t prow = min(p.pack_rows, p.rows_per_kv);
     // launched with programmatic stream serialization: wait here until the decode grid has finished
     // and its partial results are visible
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -2217,11 +2350,11 @@ __global__ void __launch_bounds__(128) tq_combine_kernel(const DecodeParams p) {
     const uint32_t g_step = p.world ? *reinterpret_cast<volatile uint32_t *>(p.step) + 1u : 0u;
     const size_t g_base = p.world ? ((size_t)(g_step & 1u) * p.world + p.rank) * rows * HD : 0;
     for (size_t row = blockIdx.x; row < rows; row += gridDim.x) {
-        const uint32_t i = (uint32_t)(row % p.lq);
-        const uint32_t h = (uint32_t)((row / p.lq) % p.hq);
-        const uint32_t b = (uint32_t)(row / ((size_t)p.lq * p.hq));
+        // 32 bits: 2^32 output rows do not fit the device
+        const uint32_t t = p.lq == 1 ? (uint32_t)row : (uint32_t)row / p.lq, i = (uint32_t)row - t * p.lq;
+        const uint32_t b = t / p.hq, h = t - b * p.hq;
         const uint32_t hk = h / p.group, r = i * p.group + h % p.group;
-        const uint32_t y = hk * p.packs + r / PACK, rr = r % PACK;
+        const uint32_t y = hk * p.packs + r / p.pack_rows, rr = r % p.pack_rows;
         const size_t obase = b * p.o_sb + h * p.o_sh + i * p.o_ss;
         if (make_column(p, b).tiles == 0) {  // the same for the whole block
             if (warp == 0) {
@@ -2323,7 +2456,7 @@ __global__ void __launch_bounds__(128) tq_combine_rows_kernel(const DecodeParams
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t rows = (size_t)p.b * p.hq * p.lq;
     const uint32_t ny = p.hkv * p.packs;
-    const uint32_t prow = min((uint32_t)PACK, p.rows_per_kv);
+    const uint32_t prow = min(p.pack_rows, p.rows_per_kv);
     // launched with programmatic stream serialization: wait here until the decode grid has finished
     // and its partial results are visible
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -2335,11 +2468,11 @@ __global__ void __launch_bounds__(128) tq_combine_rows_kernel(const DecodeParams
     const uint32_t g_step = p.world ? *reinterpret_cast<volatile uint32_t *>(p.step) + 1u : 0u;
     const size_t g_base = p.world ? ((size_t)(g_step & 1u) * p.world + p.rank) * rows * HD : 0;
     for (size_t row = (size_t)blockIdx.x * CW + warp; row < rows; row += (size_t)gridDim.x * CW) {
-        const uint32_t i = (uint32_t)(row % p.lq);
-        const uint32_t h = (uint32_t)((row / p.lq) % p.hq);
-        const uint32_t b = (uint32_t)(row / ((size_t)p.lq * p.hq));
+        // 32 bits: 2^32 output rows do not fit the device
+        const uint32_t t = p.lq == 1 ? (uint32_t)row : (uint32_t)row / p.lq, i = (uint32_t)row - t * p.lq;
+        const uint32_t b = t / p.hq, h = t - b * p.hq;
         const uint32_t hk = h / p.group, r = i * p.group + h % p.group;
-        const uint32_t y = hk * p.packs + r / PACK, rr = r % PACK;
+        const uint32_t y = hk * p.packs + r / p.pack_rows, rr = r % p.pack_rows;
         const size_t obase = b * p.o_sb + h * p.o_sh + i * p.o_ss;
         const size_t col = (size_t)b * ny + y;
         float acc[EPL];
