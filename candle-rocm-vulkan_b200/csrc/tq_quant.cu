@@ -334,6 +334,57 @@ __device__ __forceinline__ void load16(const char *src, int l8, float (&x)[16]) 
     }
 }
 
+// Butterflies of a row of 16 LPR elements (lane ll of the row: elements 16 ll ..., index bits 0-3 in the registers, the rest across
+// the lanes), bit 0 first, two elements per instruction: a - c as c * -1 + a and the lanes' y +- x as x * +-1 + y, whose products
+// are exact, so every sum is the one that an addition rounds. 72 instructions and 16 shuffles a lane bit against 160 and 16.
+__device__ __forceinline__ uint64_t pair2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpair2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+template <int LPR>
+__device__ __forceinline__ void butterflies16(float (&x)[16], int lane) {
+    uint64_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = pair2(__fadd_rn(x[2 * k], x[2 * k + 1]), __fsub_rn(x[2 * k], x[2 * k + 1]));
+    const uint64_t neg = pair2(-1.0f, -1.0f);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (!(k & o)) {
+                const uint64_t a = v[k], c = v[k | o];
+                v[k] = add2(a, c);
+                v[k | o] = fma2(c, neg, a);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < LPR; o <<= 1) {
+        const float sg = (lane & o) ? -1.0f : 1.0f;
+        const uint64_t sg2 = pair2(sg, sg);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float lo, hi;
+            unpair2(v[k], lo, hi);
+            v[k] = fma2(v[k], sg2, pair2(__shfl_xor_sync(0xffffffffu, lo, o), __shfl_xor_sync(0xffffffffu, hi, o)));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) unpair2(v[k], x[2 * k], x[2 * k + 1]);
+}
+
 // n / d for n < 2^31 with the invariants of fastdiv_init
 __device__ __forceinline__ uint32_t fastdiv(uint32_t n, uint32_t mul, uint32_t shr) { return (__umulhi(n, mul) + n) >> shr; }
 
@@ -372,32 +423,13 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
         load16<DT>(src, l8, x);
 
         if (sp.rot == B200_ROT_HADAMARD) {
-            // element index bits 0-3 across the registers, bits 4-6 across the lanes: the butterflies run in the same
-            // order (bit 0 first) as in quant_rows_kernel
+            // the butterflies run in the same order (bit 0 first) as in quant_rows_kernel
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float4 sg = __ldg(reinterpret_cast<const float4 *>(sp.signs) + 4 * l8 + q);
                 x[4 * q] *= sg.x, x[4 * q + 1] *= sg.y, x[4 * q + 2] *= sg.z, x[4 * q + 3] *= sg.w;
             }
-#pragma unroll
-            for (int o = 1; o < 16; o <<= 1) {
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    if (!(k & o)) {
-                        const float a = x[k], c = x[k | o];
-                        x[k] = a + c;
-                        x[k | o] = a - c;
-                    }
-                }
-            }
-#pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const float y = __shfl_xor_sync(0xffffffffu, x[k], o);
-                    x[k] = (lane & o) ? y - x[k] : x[k] + y;
-                }
-            }
+            butterflies16<8>(x, lane);
             const float s = 1.0f / sqrtf(128.0f);
 #pragma unroll
             for (int k = 0; k < 16; ++k) x[k] *= s;
@@ -578,7 +610,8 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint32_t *__res
 // are not back to back) moves ten times the bytes in three or four launches. Values are the chain's, bit for bit: the same
 // roundings in the same order, butterflies from index bit 0 up. Measured: keys and values of 8192 x 8 cached MXFP8 rows, rotated, for a chunk of 1024 query tokens: the
 // call 414 -> 173 us (141 of them the attention); 65 528 TurboQuant-4 rows packed and unpacked 250 -> 37 us (with the codebook
-// formats in quant_rows128_kernel, and each row packed once instead of twice).
+// formats in quant_rows128_kernel, and each row packed once instead of twice). Hardware conversions of the codes and butterflies
+// of two elements per instruction: 37.7 -> 36.4 (35 of them host time), the chunk 173.5 -> 172.
 // ---------------------------------------------------------------------------------------------
 struct UnpackSide {
     const uint32_t *src;
@@ -594,12 +627,15 @@ struct UnpackParams {
 };
 constexpr int UP_WARPS = 8;
 
+__device__ __forceinline__ void f16x2_to_f(uint32_t h, float &lo, float &hi) { lo = f16_bits_to_f((uint16_t)h), hi = f16_bits_to_f((uint16_t)(h >> 16)); }
+
 template <int LPR, int DT>
 __global__ void __launch_bounds__(UP_WARPS * 32) unpack_rows_kernel(const UnpackParams p) {
     constexpr int RPW = 32 / LPR, D = LPR * 16;
     const UnpackSide &sp = p.side[blockIdx.y];
     const int lane = threadIdx.x & 31, ll = lane % LPR;
     const uint32_t rows = p.nb * p.nh * p.nt, mode = sp.mode, cb = sp.cb;
+    const bool wide_signs = (reinterpret_cast<uintptr_t>(sp.signs) & 15u) == 0;
     __shared__ float tab[16];
     if (mode <= B200_TURBO_PROD) {
         if (threadIdx.x < 16) tab[threadIdx.x] = sp.tab[threadIdx.x];
@@ -618,10 +654,35 @@ __global__ void __launch_bounds__(UP_WARPS * 32) unpack_rows_kernel(const Unpack
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const uint32_t w = __ldg(r + 4 * ll + i);
+                // the hardware conversions, exact; a NaN code stays a NaN
+                float e[4];
+                f16x2_to_f(cvt_e4m3x2_f16x2(w), e[0], e[1]);
+                f16x2_to_f(cvt_e4m3x2_hi_f16x2(w), e[2], e[3]);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float e = e4m3_to_f((w >> (8 * k)) & 0xffu);
-                    x[4 * i + k] = __fmul_rn(rsc0, mode == B200_MXFP8 ? __fmul_rn(e, sc) : e);
+                for (int k = 0; k < 4; ++k) x[4 * i + k] = __fmul_rn(rsc0, mode == B200_MXFP8 ? __fmul_rn(e[k], sc) : e[k]);
+            }
+        } else if (cb == 4) {
+            const uint32_t w[2] = {__ldg(r + 2 * ll), __ldg(r + 2 * ll + 1)};
+            if (mode <= B200_TURBO_PROD) {
+                const char *at = reinterpret_cast<const char *>(tab);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const uint32_t v = w[k >> 3], sh = 4 * (k & 7), off = (sh < 2 ? v << 2 : v >> (sh - 2)) & 60u;
+                    x[k] = __fmul_rn(rsc0, *reinterpret_cast<const float *>(at + off));
+                }
+            } else {
+                const float sc = mode == B200_MXFP4 ? e8m0_to_f(__ldg(aux + ll / 2)) : e4m3_to_f(__ldg(aux + ll));
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    uint32_t h[4];
+                    cvt_e2m1x8_f16x2(w[i], h[0], h[1], h[2], h[3]);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        float lo, hi;
+                        f16x2_to_f(h[k], lo, hi);
+                        x[8 * i + 2 * k] = __fmul_rn(rsc0, __fmul_rn(lo, sc));
+                        x[8 * i + 2 * k + 1] = __fmul_rn(rsc0, __fmul_rn(hi, sc));
+                    }
                 }
             }
         } else {
@@ -631,39 +692,24 @@ __global__ void __launch_bounds__(UP_WARPS * 32) unpack_rows_kernel(const Unpack
             if (sh + 16u * cb > 32u) w |= (uint64_t)__ldg(r + (bit0 >> 5) + 1) << 32;
             w >>= sh;
             const uint32_t mask = (1u << cb) - 1u;
-            if (mode <= B200_TURBO_PROD) {
 #pragma unroll
-                for (int k = 0; k < 16; ++k) x[k] = __fmul_rn(rsc0, tab[(uint32_t)(w >> (k * cb)) & mask]);
-            } else {
-                const float sc = mode == B200_MXFP4 ? e8m0_to_f(__ldg(aux + ll / 2)) : e4m3_to_f(__ldg(aux + ll));
-#pragma unroll
-                for (int k = 0; k < 16; ++k) x[k] = __fmul_rn(rsc0, __fmul_rn(fp4_to_f((uint32_t)(w >> (4 * k)) & 15u), sc));
-            }
+            for (int k = 0; k < 16; ++k) x[k] = __fmul_rn(rsc0, tab[(uint32_t)(w >> (k * cb)) & mask]);  // codebooks of one to three bits
         }
         if (sp.rot == B200_ROT_HADAMARD) {
             // x = diag(s) H y / sqrt(D)
-#pragma unroll
-            for (int o = 1; o < 16; o <<= 1) {
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    if (!(k & o)) {
-                        const float a = x[k], c = x[k | o];
-                        x[k] = __fadd_rn(a, c);
-                        x[k | o] = __fsub_rn(a, c);
-                    }
-                }
-            }
-#pragma unroll
-            for (int o = 1; o < LPR; o <<= 1) {
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const float y = __shfl_xor_sync(0xffffffffu, x[k], o);
-                    x[k] = (lane & o) ? __fsub_rn(y, x[k]) : __fadd_rn(x[k], y);
-                }
-            }
+            butterflies16<LPR>(x, lane);
             const float s = 1.0f / sqrtf((float)D);
 #pragma unroll
-            for (int k = 0; k < 16; ++k) x[k] = __fmul_rn(__fmul_rn(x[k], s), __ldg(sp.signs + 16 * ll + k));
+            for (int q = 0; q < 4; ++q) {
+                const float *at = sp.signs + 16 * ll + 4 * q;
+                float4 sg;
+                if (wide_signs) sg = __ldg(reinterpret_cast<const float4 *>(at));
+                else sg = make_float4(__ldg(at), __ldg(at + 1), __ldg(at + 2), __ldg(at + 3));
+                x[4 * q] = __fmul_rn(__fmul_rn(x[4 * q], s), sg.x);
+                x[4 * q + 1] = __fmul_rn(__fmul_rn(x[4 * q + 1], s), sg.y);
+                x[4 * q + 2] = __fmul_rn(__fmul_rn(x[4 * q + 2], s), sg.z);
+                x[4 * q + 3] = __fmul_rn(__fmul_rn(x[4 * q + 3], s), sg.w);
+            }
         }
         if (!live) continue;
         char *dst = reinterpret_cast<char *>(sp.dst) + ((uint64_t)row * D + 16 * ll) * dtype_size(DT);
