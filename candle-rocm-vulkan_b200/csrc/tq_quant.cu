@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(QW * 32) quant_rows_kernel(const QuantParams p
 }
 
 // ---------------------------------------------------------------------------------------------
-// Rows of 128 elements. Eight lanes share a row (four rows per warp): lane l of the eight owns
+// Rows of 64, 128 and 256 elements. At 128 eight lanes share a row (four rows per warp): lane l of the eight owns
 // elements 16 l .. 16 l + 15 (two or four 16-byte loads), which is exactly one NVFP4 scale block and half an MX block, so the
 // block arithmetic runs once per 16 elements, the row maximum is three shuffles, and a lane's codes are already the 8 or
 // 16 bytes of the row that it stores. The codes come from the hardware conversions (cvt.rn.satfinite.e2m1x2 /
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(QW * 32) quant_rows_kernel(const QuantParams p
 // explicitly. Maxima do not depend on the order of the reduction, every division is IEEE, so rows are bit-identical to
 // quant_rows_kernel's. Row -> (batch entry, head, token) uses multiply-high division by the launch's invariants.
 // ---------------------------------------------------------------------------------------------
-constexpr int Q128_WARPS = 8, Q128_RPW = 4;  // warps per block, rows per warp
+constexpr int Q128_WARPS = 8;  // warps per block
 
 // one value -> its e4m3 code
 __device__ __forceinline__ uint32_t e4m3_hw(float f) {
@@ -390,10 +390,13 @@ __device__ __forceinline__ uint32_t fastdiv(uint32_t n, uint32_t mul, uint32_t s
 
 // CODES: a side of the call is in a codebook format. Without, their code is left out: its registers and its prologue cost the block-scaled
 // formats 0.1 us of the 1.8 of a few rows.
-template <int DT, bool CODES>
+// LPR: lanes that share a row, 16 elements each: rows of 64, 128 or 256 elements. TurboQuant-4 rows packed and unpacked, with a warp per
+// row for the packing and like this: 64 000 rows of 64 elements 72 -> 36 us, 32 000 of 256 57 -> 28 (host time from there on).
+template <int DT, bool CODES, int LPR>
 __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const QuantParams p) {
     const QuantSideParams &sp = p.side[blockIdx.y];
-    const int lane = threadIdx.x & 31, l8 = lane & 7;
+    constexpr int RPW = 32 / LPR;
+    const int lane = threadIdx.x & 31, l8 = lane % LPR;
     const uint32_t rows = p.nb * p.nh * p.nt;
     const uint32_t mode = sp.mode;
     // codebook formats: the boundaries between neighbouring codes, ascending; 15 words in 15 banks, so no two lanes collide
@@ -405,9 +408,9 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
         b7 = bound[7], b3 = bound[3], b11 = bound[11];
     }
     after_prev_begin(p);
-    for (uint32_t base = (blockIdx.x * Q128_WARPS + (threadIdx.x >> 5)) * Q128_RPW; base < rows; base += gridDim.x * Q128_WARPS * Q128_RPW) {
-        bool live = base + (lane >> 3) < rows;  // a row past the end repeats the last one and stores nothing
-        const uint32_t row = live ? base + (lane >> 3) : rows - 1;
+    for (uint32_t base = (blockIdx.x * Q128_WARPS + (threadIdx.x >> 5)) * RPW; base < rows; base += gridDim.x * Q128_WARPS * RPW) {
+        bool live = base + lane / LPR < rows;  // a row past the end repeats the last one and stores nothing
+        const uint32_t row = live ? base + lane / LPR : rows - 1;
         const uint32_t bh = fastdiv(row, p.nt_mul, p.nt_shr), t = row - bh * p.nt, b = fastdiv(bh, p.nh_mul, p.nh_shr), h = bh - b * p.nh;
         const char *src = reinterpret_cast<const char *>(sp.src) + (b * sp.s_b + h * sp.s_h + t * sp.s_t) * (uint64_t)dtype_size(DT);
         int64_t pos = (sp.pos ? (int64_t)sp.pos[b] + sp.pos0 : (int64_t)sp.pos0) + (int64_t)t;
@@ -429,21 +432,21 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
                 const float4 sg = __ldg(reinterpret_cast<const float4 *>(sp.signs) + 4 * l8 + q);
                 x[4 * q] *= sg.x, x[4 * q + 1] *= sg.y, x[4 * q + 2] *= sg.z, x[4 * q + 3] *= sg.w;
             }
-            butterflies16<8>(x, lane);
-            const float s = 1.0f / sqrtf(128.0f);
+            butterflies16<LPR>(x, lane);
+            const float s = 1.0f / sqrtf(16.0f * LPR);
 #pragma unroll
             for (int k = 0; k < 16; ++k) x[k] *= s;
         }
 
         if (CODES && mode <= B200_TURBO_PROD) {
-            // Sum of squares in the order of the reference's 128 lanes (red[t] += red[t + s], s = 64 ... 1): index bits 6, 5, 4
-            // are the row's lanes, and each step leaves half of the residues with either lane (residue bit 3 with lane bit 2,
-            // and so on); bits 3, 2, 1 then lie across the lanes, bit 0 in the register.
+            // Sum of squares in the order of the reference's 128 lanes (a lane adds j = t, t + 128; red[t] += red[t + s], s = 64 ... 1): the
+            // index bits from 4 up are the row's lanes, and each step leaves half of the residues with either lane (residue bit 3
+            // with the highest lane bit, and so on); those bits of the residues then lie across the lanes, the rest in the registers.
             float v[16];
 #pragma unroll
             for (int k = 0; k < 16; ++k) v[k] = __fmul_rn(x[k], x[k]);
 #pragma unroll
-            for (int o = 4, n = 8; o > 0; o >>= 1, n >>= 1) {
+            for (int o = LPR / 2, n = 8; o > 0; o >>= 1, n >>= 1) {
                 const bool up = l8 & o;
 #pragma unroll
                 for (int k = 0; k < n; ++k) {
@@ -452,11 +455,14 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
                 }
             }
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) {
-                v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
-                v[1] = __fadd_rn(v[1], __shfl_xor_sync(0xffffffffu, v[1], o));
-            }
-            const float norm = __fsqrt_rn(__fadd_rn(v[0], v[1]));
+            for (int o = LPR / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < 16 / LPR; ++k) v[k] = __fadd_rn(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+#pragma unroll
+            for (int n = 8 / LPR; n > 0; n >>= 1)
+#pragma unroll
+                for (int k = 0; k < n; ++k) v[k] = __fadd_rn(v[k], v[k + n]);
+            const float norm = __fsqrt_rn(v[0]);
             const float inv = norm > 0.0f ? __fdiv_rn(1.0f, norm) : 0.0f;
             // A code is the number of boundaries that the element reaches: they ascend, so by halves (a NaN reaches none).
             const uint32_t cb = sp.cb;
@@ -490,7 +496,7 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
                     uint16_t *dst = reinterpret_cast<uint16_t *>(orow) + l8 * cb;  // 16 codes of cb bits
                     for (uint32_t i = 0; i < cb; ++i) dst[i] = (uint16_t)(w >> (16 * i));
                 }
-                for (int i = l8; i < sp.aux_words; i += 8) orow[sp.code_words + i] = 0u;
+                for (int i = l8; i < sp.aux_words; i += LPR) orow[sp.code_words + i] = 0u;
                 if (l8 < 2) orow[sp.code_words + sp.aux_words + l8] = l8 ? 0u : f2u(norm);
             }
             continue;
@@ -508,11 +514,10 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
         float rsc0 = 1.0f;
         uint32_t cw;  // words of codes before the scales
         if (mode == B200_NVFP4) {
-            cw = 16;
+            cw = 2 * LPR;
             float am = fmaxf(0.0f, bm);
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 4));
+#pragma unroll
+            for (int o = 1; o < LPR; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
             const float g = am > 0.0f ? __fdiv_rn(am, 2688.0f) : 1.0f;
             rsc0 = g;
             const uint32_t scode = e4m3_hw(__fdiv_rn(__fdiv_rn(bm, 6.0f), g));  // the lane's 16 elements are one scale block
@@ -523,15 +528,15 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
                 else fp4x16_div<false>(x, eff, w);
             }
             if (live) {
-                *reinterpret_cast<uint2 *>(orow + 2 * l8) = make_uint2(w[0], w[1]);
-                reinterpret_cast<uint8_t *>(orow + 16)[l8] = (uint8_t)scode;
+                if (LPR == 8) *reinterpret_cast<uint2 *>(orow + 2 * l8) = make_uint2(w[0], w[1]);
+                else orow[2 * l8] = w[0], orow[2 * l8 + 1] = w[1];  // rows of 11 words: 4-byte alignment only
+                reinterpret_cast<uint8_t *>(orow + 2 * LPR)[l8] = (uint8_t)scode;
             }
         } else if (mode == B200_FP8_ROW) {
-            cw = 32;
+            cw = 4 * LPR;
             float am = fmaxf(0.0f, bm);
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-            am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 4));
+#pragma unroll
+            for (int o = 1; o < LPR; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
             const float s = am > 0.0f ? __fdiv_rn(am, 448.0f) : 1.0f;
             rsc0 = s;
             uint32_t w[4];
@@ -547,7 +552,7 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
             const uint32_t code = mx_scale_code(bm, mode == B200_MXFP4 ? 2 : 8);
             const float s = e8m0_recip(code);  // the divisor is a power of two: multiply by its reciprocal, same bits
             if (mode == B200_MXFP4) {
-                cw = 16;
+                cw = 2 * LPR;
                 uint32_t w[2] = {0u, 0u};
                 if (code != 0) {
                     if (special) fp4x16_div<true, true>(x, s, w);
@@ -555,7 +560,7 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
                 }
                 if (live) orow[2 * l8] = w[0], orow[2 * l8 + 1] = w[1];  // rows of 19 words: 4-byte alignment only
             } else {
-                cw = 32;
+                cw = 4 * LPR;
                 uint32_t w[4] = {0u, 0u, 0u, 0u};
                 if (code != 0) {
                     if (special) e4m3x16_div<true, true>(x, s, w);
@@ -567,6 +572,7 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
                 }
             }
             if (live && (l8 & 1) == 0) reinterpret_cast<uint8_t *>(orow + cw)[l8 >> 1] = (uint8_t)code;
+            if (LPR == 4 && live && (l8 & 1)) reinterpret_cast<uint8_t *>(orow + cw)[2 + (l8 >> 1)] = 0;  // the rest of the scales' word
         }
         if (live && l8 < 2) orow[cw + (uint32_t)sp.aux_words + l8] = l8 ? 0u : f2u(rsc0);
     }
@@ -862,7 +868,7 @@ static void fastdiv_init(uint32_t d, uint32_t &mul, uint32_t &shr) {
 // rows of 128 elements whose source rows can be read as 16-byte vectors
 static bool rows128_takes(const QuantParams &p, int sides) {
     static const bool off = diag_env("B200_QUANT_GENERIC") != nullptr;
-    if (off || p.d != 128 || (uint64_t)p.nb * p.nh * p.nt >= 0x7fffff00ull) return false;
+    if (off || (p.d != 64 && p.d != 128 && p.d != 256) || (uint64_t)p.nb * p.nh * p.nt >= 0x7fffff00ull) return false;
     const uint64_t vec = p.src_dtype == B200_F32 ? 3 : 7;  // elements per 16 bytes - 1
     for (int s = 0; s < sides; ++s) {
         const QuantSideParams &sp = p.side[s];
@@ -873,7 +879,7 @@ static bool rows128_takes(const QuantParams &p, int sides) {
         if (((uintptr_t)sp.src & 15) || (sp.s_b & vec) || (sp.s_h & vec) || (sp.s_t & vec)) return false;
         if (sp.rot == B200_ROT_HADAMARD && ((uintptr_t)sp.signs & 15)) return false;
         // NVFP4 code words are stored in pairs
-        if (sp.mode == B200_NVFP4 && (((uintptr_t)sp.dst & 7) || (sp.c_b & 1) || (sp.c_h & 1) || (sp.c_t & 1))) return false;
+        if (p.d == 128 && sp.mode == B200_NVFP4 && (((uintptr_t)sp.dst & 7) || (sp.c_b & 1) || (sp.c_h & 1) || (sp.c_t & 1))) return false;
     }
     return true;
 }
@@ -895,24 +901,24 @@ static int launch_maybe_after_prev(void (*kern)(const QuantParams), dim3 grid, d
     return check_launch("tq_quantize");
 }
 
-template <bool CODES>
+template <bool CODES, int LPR>
 static int launch_rows128(const QuantParams &p, int sides, cudaStream_t stream) {
     QuantParams q = p;
     fastdiv_init(p.nt, q.nt_mul, q.nt_shr);
     fastdiv_init(p.nh, q.nh_mul, q.nh_shr);
-    const uint64_t rows = (uint64_t)p.nb * p.nh * p.nt, per_block = Q128_WARPS * Q128_RPW;
+    const uint64_t rows = (uint64_t)p.nb * p.nh * p.nt, per_block = Q128_WARPS * (32 / LPR);
     // as many blocks as are resident at once, shared by the sides
     static const int resident = [] {
         int per_sm = 4, sms = 148, dev = 0;
         cudaGetDevice(&dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quant_rows128_kernel<B200_BF16, CODES>, Q128_WARPS * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quant_rows128_kernel<B200_BF16, CODES, LPR>, Q128_WARPS * 32, 0);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         return std::max(per_sm, 1) * std::max(sms, 1);
     }();
     const dim3 grid((unsigned)std::min<uint64_t>((rows + per_block - 1) / per_block, (uint64_t)std::max(resident / sides, 1)), sides), block(Q128_WARPS * 32);
-    if (p.src_dtype == B200_F32) return launch_maybe_after_prev(quant_rows128_kernel<B200_F32, CODES>, grid, block, stream, q);
-    if (p.src_dtype == B200_F16) return launch_maybe_after_prev(quant_rows128_kernel<B200_F16, CODES>, grid, block, stream, q);
-    return launch_maybe_after_prev(quant_rows128_kernel<B200_BF16, CODES>, grid, block, stream, q);
+    if (p.src_dtype == B200_F32) return launch_maybe_after_prev(quant_rows128_kernel<B200_F32, CODES, LPR>, grid, block, stream, q);
+    if (p.src_dtype == B200_F16) return launch_maybe_after_prev(quant_rows128_kernel<B200_F16, CODES, LPR>, grid, block, stream, q);
+    return launch_maybe_after_prev(quant_rows128_kernel<B200_BF16, CODES, LPR>, grid, block, stream, q);
 }
 
 static int launch_quant(const QuantParams &p, int sides, cudaStream_t stream) {
@@ -920,7 +926,9 @@ static int launch_quant(const QuantParams &p, int sides, cudaStream_t stream) {
     if (rows == 0) return B200_OK;
     if (rows128_takes(p, sides)) {
         const bool codes = p.side[0].mode <= B200_TURBO_PROD || (sides > 1 && p.side[1].mode <= B200_TURBO_PROD);
-        return codes ? launch_rows128<true>(p, sides, stream) : launch_rows128<false>(p, sides, stream);
+        if (p.d == 64) return codes ? launch_rows128<true, 4>(p, sides, stream) : launch_rows128<false, 4>(p, sides, stream);
+        if (p.d == 256) return codes ? launch_rows128<true, 16>(p, sides, stream) : launch_rows128<false, 16>(p, sides, stream);
+        return codes ? launch_rows128<true, 8>(p, sides, stream) : launch_rows128<false, 8>(p, sides, stream);
     }
     const unsigned gx = (unsigned)std::min<uint64_t>((rows + QW - 1) / QW, 148ull * 64);
     const dim3 grid(gx, sides), block(QW * 32);
