@@ -106,13 +106,13 @@ static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false
     p.rows_per_kv = p.group * a->lq;
     // More than eight query rows per kv head: columns of 16, whose two groups of eight rows share the decoded keys and values.
     // A tile of such a column costs 1.1 times one of eight rows, and two thirds as many warps work on them: worth it where it
-    // (nearly) halves the columns, and where every worker has a few tiles (us, columns of 8 -> 16: 16 rows, 64 sequences of 512 to
-    // 8192 MXFP4 keys 163 -> 140, 32 of 8192 MXFP8 keys 213 -> 140; 24 rows, 8 x 4000 MXFP8 keys of 64: 41 -> 44; 32 rows,
-    // one sequence of 4000 keys: 31 -> 35). For keys and values in one format, head dims 64 and 128; the kernel whose workers
+    // (nearly) halves the columns, and where every worker has six tiles (us, columns of 8 -> 16: 16 rows, 64 sequences of 512 to
+    // 8192 MXFP4 keys 163 -> 127, 32 of 8192 MXFP8 keys 213 -> 123; 24 rows, 8 x 4000 MXFP8 keys of 64: 41 -> 44; 32 rows,
+    // one sequence of 4000 keys: 31 -> 35; 12 rows, 5 x 4000 MXFP8 keys, four tiles a worker: 36.9 -> 39.0). For keys and values in one format, head dims 64 and 128; the kernel whose workers
     // are pairs of warps has no such form.
     const uint32_t packs8 = (p.rows_per_kv + PACK - 1) / PACK, packs16 = (p.rows_per_kv + 2 * PACK - 1) / (2 * PACK);
     pl.wide = !narrow && 5 * packs16 < 3 * packs8 && a->kq.mode == a->vq.mode && a->d <= 128 && (paged || !pair_formats(a->kq.mode, a->vq.mode)) &&
-              (uint64_t)a->b * a->hkv * packs16 * ((a->lk + WK - 1) / WK) >= 3ull * decode_blocks(2) * DW * sm_count_cached();
+              (uint64_t)a->b * a->hkv * packs16 * ((a->lk + WK - 1) / WK) >= 6ull * decode_blocks(2) * DW * sm_count_cached();
     p.pack_rows = pl.wide ? 2 * PACK : PACK;
     p.packs = (p.rows_per_kv + p.pack_rows - 1) / p.pack_rows;
     p.scale = a->scale;
