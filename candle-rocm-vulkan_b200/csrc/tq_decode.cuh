@@ -113,12 +113,13 @@ struct DecodeParams {
     uint32_t *ctr;
     int32_t *lib_status;    // library-wide flag: set when a bounded wait of a kernel of this call runs out
     // paged rows (null: dense rows): the block table, and for every block the keys and the 32-key tiles of the
-    // blocks before it (n_pages + 1 entries each, written by tq_page_prefix_kernel right before this grid, or, pg_build, by
-    // every block of this grid for itself, all of them the same words)
+    // blocks before it (n_pages + 1 entries each, written by tq_page_prefix_kernel right before this grid). pg_build: every
+    // block works the sums out in its own shared memory, pg_sums bytes from the start, and block 0 leaves them at pg_keys /
+    // pg_tiles for the combine grid; nothing in this grid reads those.
     const B200Page *pages;
     uint32_t n_pages;
-    uint32_t pg_build;
-    const uint32_t *pg_keys, *pg_tiles;
+    uint32_t pg_build, pg_sums;
+    uint32_t *pg_keys, *pg_tiles;
 };
 
 __host__ __device__ constexpr bool fmt_is4(int m) { return m == B200_MXFP4 || m == B200_NVFP4 || m == B200_TURBO_MSE; }
@@ -327,20 +328,23 @@ struct Column {
 // Paged rows: tiles never straddle blocks (as the reference's windows never do, candle-core/kernels/
 // flash_attn_impl.h:135-151): block g holds ceil(rows_g / WK) tiles, the last one short. The block that holds key
 // position `key` (< the total number of keys): the last g with pg_keys[g] <= key.
-__device__ __forceinline__ uint32_t page_of_key(const DecodeParams &p, uint32_t key) {
-    uint32_t lo = 0, hi = p.n_pages;  // invariant: pg_keys[lo] <= key < pg_keys[hi]
+struct PageSums {
+    const uint32_t *keys, *tiles;  // of the blocks before each block; null for dense rows
+};
+__device__ __forceinline__ uint32_t page_of_key(const DecodeParams &p, const PageSums &ps, uint32_t key) {
+    uint32_t lo = 0, hi = p.n_pages;  // invariant: keys[lo] <= key < keys[hi]
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (p.pg_keys[mid] <= key) lo = mid;
+        if (ps.keys[mid] <= key) lo = mid;
         else hi = mid;
     }
     return lo;
 }
-// The keys and tiles before every block of a table of at most PG_BUILD blocks, by one warp. A kernel of its own in front costs
-// 2 us and its launch, this half a microsecond in every block (16 x 4000 keys in 8 blocks: 46 -> 44.5 us).
+// The keys and tiles before every block of a table of at most PG_BUILD blocks, by one warp, into the block's shared memory and
+// (`copy`) to pg_keys / pg_tiles. A kernel of its own in front costs 2 us and its launch, this half a microsecond in every block.
 constexpr uint32_t PG_BUILD = 127;
-__device__ __forceinline__ void page_prefix(const DecodeParams &p, int lane) {
-    uint32_t *keys = const_cast<uint32_t *>(p.pg_keys), *tiles = const_cast<uint32_t *>(p.pg_tiles);
+constexpr uint32_t PG_SUMS_BYTES = 2 * (PG_BUILD + 1) * 4;
+__device__ __forceinline__ void page_prefix(const DecodeParams &p, uint32_t *keys, uint32_t *tiles, bool copy, int lane) {
     uint32_t r[4], base_k = 0, base_t = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) r[k] = 32u * k + lane < p.n_pages ? p.pages[32 * k + lane].rows : 0u;
@@ -357,26 +361,27 @@ __device__ __forceinline__ void page_prefix(const DecodeParams &p, int lane) {
         if (i <= p.n_pages) {
             keys[i] = base_k + ik - n;
             tiles[i] = base_t + it - t;
+            if (copy) p.pg_keys[i] = base_k + ik - n, p.pg_tiles[i] = base_t + it - t;
         }
         base_k += __shfl_sync(0xffffffffu, ik, 31);
         base_t += __shfl_sync(0xffffffffu, it, 31);
     }
 }
 // the block that holds tile T of the table's list (< the total number of tiles)
-__device__ __forceinline__ uint32_t page_of_tile(const DecodeParams &p, uint32_t T) {
+__device__ __forceinline__ uint32_t page_of_tile(const DecodeParams &p, const PageSums &ps, uint32_t T) {
     uint32_t lo = 0, hi = p.n_pages;
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (p.pg_tiles[mid] <= T) lo = mid;
+        if (ps.tiles[mid] <= T) lo = mid;
         else hi = mid;
     }
     return lo;
 }
 
-__device__ __forceinline__ Column make_column(const DecodeParams &p, uint32_t b) {
+__device__ __forceinline__ Column make_column(const DecodeParams &p, const PageSums &ps, uint32_t b) {
     Column c;
     c.lk = p.kv_len ? min(max(p.kv_len[b] + p.kv_len_add, 0), (int)p.lk) : (int)p.lk;
-    if (p.pages) c.lk = (int)min((uint32_t)c.lk, p.pg_keys[p.n_pages]);  // never more keys than the blocks hold
+    if (p.pages) c.lk = (int)min((uint32_t)c.lk, ps.keys[p.n_pages]);  // never more keys than the blocks hold
     // union of the rows' ranges: the first query token (position lk - lq) gives the lowest key, the last one (lk - 1) sees all from
     // there on, whatever the right window
     const int pos0 = c.lk - (int)p.lq;
@@ -386,9 +391,9 @@ __device__ __forceinline__ Column make_column(const DecodeParams &p, uint32_t b)
     if (p.pages == nullptr) {
         c.tiles = (c.hi - c.lo + WK - 1) / WK;
     } else if (c.hi > c.lo) {
-        const uint32_t g0 = page_of_key(p, (uint32_t)c.lo), g1 = page_of_key(p, (uint32_t)c.hi - 1);
-        c.t_lo = p.pg_tiles[g0] + ((uint32_t)c.lo - p.pg_keys[g0]) / WK;
-        c.tiles = (int)(p.pg_tiles[g1] + ((uint32_t)c.hi - 1 - p.pg_keys[g1]) / WK + 1 - c.t_lo);
+        const uint32_t g0 = page_of_key(p, ps, (uint32_t)c.lo), g1 = page_of_key(p, ps, (uint32_t)c.hi - 1);
+        c.t_lo = ps.tiles[g0] + ((uint32_t)c.lo - ps.keys[g0]) / WK;
+        c.tiles = (int)(ps.tiles[g1] + ((uint32_t)c.hi - 1 - ps.keys[g1]) / WK + 1 - c.t_lo);
     } else {
         c.tiles = 0;
     }
@@ -461,7 +466,7 @@ __device__ __forceinline__ uint32_t head_of(const DecodeParams &p, uint32_t y) {
 __device__ __forceinline__ uint32_t pack_of(const DecodeParams &p, uint32_t y) { return p.packs == 1 ? 0u : y % p.packs; }
 
 // next segment of the share that ends at x_end; false when the share is exhausted
-__device__ __forceinline__ bool next_segment(Segment &s, const DecodeParams &p, uint32_t ny, uint64_t x_end) {
+__device__ __forceinline__ bool next_segment(Segment &s, const DecodeParams &p, const PageSums &ps, uint32_t ny, uint64_t x_end) {
     if (s.t1 < (uint32_t)s.col.tiles) return false;  // the share ended inside the column
     const uint64_t x = s.x + (s.t1 - s.t0) + p.col_cost;
     if (x >= x_end) return false;
@@ -469,7 +474,7 @@ __device__ __forceinline__ bool next_segment(Segment &s, const DecodeParams &p, 
         s.y = 0;
         do {
             if (++s.b >= p.b) return false;
-            s.col = make_column(p, s.b);
+            s.col = make_column(p, ps, s.b);
         } while (s.col.tiles == 0);
     }
     s.x = x;
@@ -1278,11 +1283,11 @@ struct Share {
 // Computed by every worker (warp) from the lengths alone. Never more workers than cost positions: every worker
 // between the owners of two tiles of a column then owns a tile of that column itself, so a column's segments are
 // the consecutive workers first owner .. last owner.
-__device__ __forceinline__ Share worker_share(const DecodeParams &p, uint32_t ny, uint32_t wid, uint32_t nw_grid, int lane) {
+__device__ __forceinline__ Share worker_share(const DecodeParams &p, const PageSums &ps, uint32_t ny, uint32_t wid, uint32_t nw_grid, int lane) {
     Share sh;
     const uint32_t cc = p.col_cost;
     auto batch_cost = [&](uint32_t bb) -> uint32_t {
-        const uint32_t t = (uint32_t)make_column(p, bb).tiles;
+        const uint32_t t = (uint32_t)make_column(p, ps, bb).tiles;
         return t ? (t + cc) * ny : 0u;
     };
     uint64_t total = 0;
@@ -1371,7 +1376,7 @@ __device__ __forceinline__ Share worker_share(const DecodeParams &p, uint32_t ny
     // snaps to the column's first tile)
     Segment &seg = sh.seg;
     seg.b = b0;
-    seg.col = make_column(p, b0);
+    seg.col = make_column(p, ps, b0);
     const uint32_t tb = (uint32_t)seg.col.tiles;
     const uint32_t rem = (uint32_t)(x_begin - b0_start);  // one entry's positions fit 32 bits (batch_cost)
     seg.y = rem / (tb + cc);
@@ -1396,6 +1401,7 @@ __device__ __forceinline__ Share worker_share(const DecodeParams &p, uint32_t ny
 // finish, and only the rows it must not read yet (the last fresh_rows of a sequence) and all stores wait.
 struct Worker {
     const DecodeParams &p;
+    const PageSums &ps;
     int lane;
     uint32_t wid, nw_grid, ny, ncols, prow;
     uint64_t total;
@@ -1404,8 +1410,8 @@ struct Worker {
     uint32_t g_step;  // gathered outputs: this step's number, read once the previous kernel is done
     size_t g_base;    // and the offset of this rank's rows in the step's slot of every rank's buffer
 
-    __device__ __forceinline__ Worker(const DecodeParams &p_, int lane_, uint32_t wid_, uint32_t nw_grid_, uint32_t ny_, const Share &sh)
-        : p(p_), lane(lane_), wid(wid_), nw_grid(nw_grid_), ny(ny_), ncols(p_.b * ny_), prow(min(p_.pack_rows, p_.rows_per_kv)),
+    __device__ __forceinline__ Worker(const DecodeParams &p_, const PageSums &ps_, int lane_, uint32_t wid_, uint32_t nw_grid_, uint32_t ny_, const Share &sh)
+        : p(p_), ps(ps_), lane(lane_), wid(wid_), nw_grid(nw_grid_), ny(ny_), ncols(p_.b * ny_), prow(min(p_.pack_rows, p_.rows_per_kv)),
           total(sh.total), nw(sh.nw), waited(false), g_step(0), g_base(0) {}
 
     __device__ __forceinline__ void prev_done() {
@@ -1449,7 +1455,7 @@ struct Worker {
         if (!p.out_free) prev_done();
         for (uint32_t col = wid; col < ncols; col += nw_grid) {
             const uint32_t b = col / ny, y = col - b * ny;
-            if (make_column(p, b).tiles != 0) continue;
+            if (make_column(p, ps, b).tiles != 0) continue;
             float z[HD / 32];
 #pragma unroll
             for (int k = 0; k < HD / 32; ++k) z[k] = 0.0f;
@@ -1615,18 +1621,18 @@ struct CopySide {
         pk = reinterpret_cast<uintptr_t>(pgd.k) + ((uintptr_t)iseg.b * p.hkv + hk) * pgd.k_cap * krb;
         pv = reinterpret_cast<uintptr_t>(pgd.v) + ((uintptr_t)iseg.b * p.hkv + hk) * pgd.v_cap * vrb;
     }
-    __device__ __forceinline__ void enter_paged(const DecodeParams &p, uint32_t krb, uint32_t vrb) {
+    __device__ __forceinline__ void enter_paged(const DecodeParams &p, const PageSums &ps, uint32_t krb, uint32_t vrb) {
         left = (int)(iseg.t1 - iseg.t0);
         const uint32_t T = iseg.col.t_lo + iseg.t0;
-        pg = page_of_tile(p, T);
-        off = (T - p.pg_tiles[pg]) * WK;
+        pg = page_of_tile(p, ps, T);
+        off = (T - ps.tiles[pg]) * WK;
         load_page(p, krb, vrb);
     }
-    __device__ __forceinline__ void start_paged(const DecodeParams &p, const Segment &seg, uint32_t krb, uint32_t vrb) {
+    __device__ __forceinline__ void start_paged(const DecodeParams &p, const PageSums &ps, const Segment &seg, uint32_t krb, uint32_t vrb) {
         policy(p);
         iseg = seg;
         more = true;
-        enter_paged(p, krb, vrb);
+        enter_paged(p, ps, krb, vrb);
     }
     // Copies the next tile into stage `st` and leaves its description (offsets of the first row inside the copies, first
     // key, number of keys) at `desc` for the compute side.
@@ -1634,7 +1640,7 @@ struct CopySide {
                                                uint64_t x_end) {
         const DecodeParams &p = w.p;
         const int lane = w.lane;
-        const int key0 = (int)(p.pg_keys[pg] + off);
+        const int key0 = (int)(w.ps.keys[pg] + off);
         const int nkeys = min(min(WK, (int)(pg_rows - off)), iseg.col.hi - key0);
         if (!w.waited && key0 + nkeys > iseg.col.lk - (int)p.fresh_rows) w.prev_done();
         const uintptr_t ka = pk + (uintptr_t)off * krb, va = pv + (uintptr_t)off * vrb;
@@ -1670,8 +1676,8 @@ struct CopySide {
         off += WK;
         if (--left == 0) {
             if (more) {
-                more = next_segment(iseg, p, w.ny, x_end);
-                if (more) enter_paged(p, krb, vrb);
+                more = next_segment(iseg, p, w.ps, w.ny, x_end);
+                if (more) enter_paged(p, w.ps, krb, vrb);
             }
         } else if (off >= pg_rows) {
             // the next block that holds rows (there is one: tiles are left in this column)
@@ -1738,7 +1744,7 @@ struct CopySide {
         v += (uintptr_t)WK * vrb;
         key += WK;
         if (B200_UNLIKELY(--left == 0 && more)) {
-            more = next_segment(iseg, p, w.ny, x_end);
+            more = next_segment(iseg, p, w.ps, w.ny, x_end);
             if (more) enter(p, krb, vrb);
         }
     }
@@ -1883,8 +1889,14 @@ __global__ void __launch_bounds__(DW * 32, decode_blocks(NH)) tq_decode_kernel(c
         for (int i = 0; i < DW * NS_MAX; ++i) mbar_init(&bars[i], 1);
         mbar_fence_init();
     }
+    PageSums ps = {nullptr, nullptr};
     if constexpr (PAGED) {
-        if (p.pg_build && warp == 1) page_prefix(p, lane);
+        ps = {p.pg_keys, p.pg_tiles};
+        if (p.pg_build) {
+            uint32_t *sums = reinterpret_cast<uint32_t *>(smem + p.pg_sums);
+            if (warp == 1) page_prefix(p, sums, sums + PG_BUILD + 1, blockIdx.x == 0, lane);
+            ps = {sums, sums + PG_BUILD + 1};
+        }
     }
     load_codebooks<KM, VM>(p, lut_k, lut_v, plane_k, tid, DW * 32);
     __syncthreads();
@@ -1895,8 +1907,8 @@ __global__ void __launch_bounds__(DW * 32, decode_blocks(NH)) tq_decode_kernel(c
     // paged rows: where a kernel wrote the table's prefix sums it is the stream's previous kernel, and this grid was
     // launched as its programmatic dependent (its launch latency is hidden): the sums are read from here on
     if constexpr (PAGED) asm volatile("griddepcontrol.wait;" ::: "memory");
-    const Share sh = worker_share(p, ny, wid, nw_grid, lane);
-    Worker wk(p, lane, wid, nw_grid, ny, sh);
+    const Share sh = worker_share(p, ps, ny, wid, nw_grid, lane);
+    Worker wk(p, ps, lane, wid, nw_grid, ny, sh);
     if (PAGED || !p.prefetch) wk.prev_done();
     if (!sh.has_work) {
         wk.zero_columns<HD>(false);
@@ -1917,7 +1929,7 @@ __global__ void __launch_bounds__(DW * 32, decode_blocks(NH)) tq_decode_kernel(c
     // All stages are asked for right away: the first tiles land a little later than alone, but the code that asks is fetched
     // once (ragged MXFP4 call: 92.7 -> 91.3 us; 64 x 2 query tokens, 64 heads: 139.6 -> 138.5).
     CopySide cs;
-    if constexpr (PAGED) cs.start_paged(p, sh.seg, krb, vrb);
+    if constexpr (PAGED) cs.start_paged(p, ps, sh.seg, krb, vrb);
     else cs.start(p, sh.seg, krb, vrb);
     auto copy_tile = [&](uint32_t st, uint32_t bar, uint32_t desc) {
         if constexpr (PAGED) cs.tile_paged(wk, st, bar, desc, krb, vrb, k_stage_bytes, sh.x_end);
@@ -2042,7 +2054,7 @@ __global__ void __launch_bounds__(DW * 32, decode_blocks(NH)) tq_decode_kernel(c
                 lsum[h][1] += __shfl_xor_sync(0xffffffffu, lsum[h][1], o);
             }
         wk.finish_segment<HD, NH>(seg, oacc, M, lsum);
-        more = next_segment(seg, p, ny, sh.x_end);
+        more = next_segment(seg, p, ps, ny, sh.x_end);
     }
     wk.zero_columns<HD>(true);
     if (wait_failed) {
@@ -2131,9 +2143,10 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+    const PageSums ps = {nullptr, nullptr};
     // both warps of a pair work out the pair's share
-    const Share sh = worker_share(p, ny, wid, nw_grid, lane);
-    Worker wk(p, lane, wid, nw_grid, ny, sh);
+    const Share sh = worker_share(p, ps, ny, wid, nw_grid, lane);
+    Worker wk(p, ps, lane, wid, nw_grid, ny, sh);
     if (!p.prefetch) wk.prev_done();
     if (!sh.has_work) {
         if (!keys_side) wk.zero_columns<HD>(false);
@@ -2233,7 +2246,7 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
                          "f"(lsum[1])
                          : "memory");
             slot_send();
-            more = next_segment(seg, p, ny, sh.x_end);
+            more = next_segment(seg, p, ps, ny, sh.x_end);
         }
     } else {
         // ============================================================== the values' warp
@@ -2314,7 +2327,7 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
                 lsum[0][0] = lsum[0][1] = 0.0f;
             }
             wk.finish_segment<HD, 1>(seg, oacc, M, lsum);
-            more = next_segment(seg, p, ny, sh.x_end);
+            more = next_segment(seg, p, ps, ny, sh.x_end);
         }
         wk.zero_columns<HD>(true);
     }
@@ -2356,7 +2369,7 @@ __global__ void __launch_bounds__(128) tq_combine_kernel(const DecodeParams p) {
         const uint32_t hk = h / p.group, r = i * p.group + h % p.group;
         const uint32_t y = hk * p.packs + r / p.pack_rows, rr = r % p.pack_rows;
         const size_t obase = b * p.o_sb + h * p.o_sh + i * p.o_ss;
-        if (make_column(p, b).tiles == 0) {  // the same for the whole block
+        if (make_column(p, {p.pg_keys, p.pg_tiles}, b).tiles == 0) {  // the same for the whole block
             if (warp == 0) {
 #pragma unroll
                 for (int k = 0; k < EPL; ++k) store_elem_rt(p.out, obase + lane + 32 * k, 0.0f, p.out_dtype);
@@ -2476,7 +2489,7 @@ __global__ void __launch_bounds__(128) tq_combine_rows_kernel(const DecodeParams
         const size_t obase = b * p.o_sb + h * p.o_sh + i * p.o_ss;
         const size_t col = (size_t)b * ny + y;
         float acc[EPL];
-        const bool any = make_column(p, b).tiles != 0;  // otherwise nothing was written for the row: zeros
+        const bool any = make_column(p, {p.pg_keys, p.pg_tiles}, b).tiles != 0;  // otherwise nothing was written for the row: zeros
         if (any) {
             const int2 fm = *reinterpret_cast<const int2 *>(p.meta + 2 * col);
             const size_t slot0 = (size_t)fm.x * prow + rr;

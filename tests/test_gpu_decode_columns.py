@@ -90,7 +90,8 @@ def test_wide_columns_over_blocks(P, rows_of_a_block):
 
 @pytest.mark.parametrize("pages", [1, 31, 32, 127, 128, 300])
 def test_prefix_sums_of_the_block_table(P, pages):
-    """Up to 127 blocks the attention's own blocks work the sums out, above a kernel in front does; odd fill levels, empty blocks."""
+    """Up to 127 blocks the attention's own blocks work the sums out, each for itself, above a kernel in front does; odd fill levels, empty
+    blocks. Either way one copy in global memory, at the start of the workspace, is the combine grid's."""
     b, hq, hkv, d, f = 2, 8, 2, 128, (2, 4)
     g = torch.Generator(device="cuda:0").manual_seed(pages)
     kq, vq = P.TurboQuantizer(fmt(P, *f), d, "none", 42), P.TurboQuantizer(fmt(P, *f), d, "none", 44)
@@ -106,7 +107,11 @@ def test_prefix_sums_of_the_block_table(P, pages):
     for lq in (1, 4):
         q = torch.randn((b, hq, lq, d), generator=g, device="cuda:0")
         lens = torch.tensor([lk, max(1, lk - 9)], dtype=torch.int32, device="cuda:0")
-        got = P.attention_packed_blocks(q, blocks, kq, vq, c, kv_len=lens)
+        call = P.PackedBlocksAttention(q, blocks, kq, vq, c, kv_len=lens)
+        got = call.run()
+        tiles = [(n + 31) // 32 for n in fills]
+        sums = [sum(fills[:i]) for i in range(pages + 1)] + [sum(tiles[:i]) for i in range(pages + 1)]
+        assert words(call._keep[-1][: 8 * (pages + 1)]).tolist() == sums
         want = P.attention_packed(q, torch.cat(ks, 2).contiguous(), torch.cat(vs, 2).contiguous(), lens, kq, vq, c)
         assert_close(got.cpu().numpy(), want.cpu().numpy(), 1e-3, 1e-3, f"{pages} blocks, {lq} query tokens")
 
