@@ -211,18 +211,6 @@ static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false
     p.prefetch = (p.after_prev && (a->flags & B200_TQ_INPUTS_FINAL)) ? 1u : 0u;
     p.out_free = (p.after_prev && (a->flags & B200_TQ_OUTPUTS_FREE)) ? 1u : 0u;
     p.fresh_rows = std::min<uint32_t>(a->fresh_rows, 0x7fffffffu);
-    // Parts of the work by place (tq_decode.cuh), for a full grid of the kernel whose workers are warps with three blocks per SM:
-    // the times that the places' blocks took with equal shares, inverted. Ragged MXFP4, 64 sequences: 100.4 us with equal shares,
-    // 96.9 with these (before the other changes of the call's ends). Two blocks per SM (columns of 16 rows) end within 2 % of one
-    // another: 154.9 with equal shares, 158.3 with parts of 130 and 126. In a chain of calls that do not wait for one another
-    // the blocks of a call take the places of the last one as these come free.
-    p.place_workers = 0;
-    if (!pl.pair && a->splits <= 0 && !p.out_free && bps == 3 && pl.blocks == (uint32_t)(sm_count_cached() * bps)) {
-        p.place_workers = (uint32_t)(sm_count_cached() * DW);
-        p.place_end[0] = 92;
-        p.place_end[1] = 177;
-        p.place_end[2] = 256;
-    }
     // rows of all sequences (at their longest, or as far as the cache goes) against the 126 MB of L2; packs of query rows read them again
     p.stream = p.packs == 1 && (uint64_t)a->b * a->hkv * lk * (p.k_ss + p.v_ss) * 4 > (64ull << 20) ? 1u : 0u;
     pl.nat = !paged && p.k_ss == (uint64_t)kl.row_words && p.v_ss == (uint64_t)vl.row_words && a->kq.mode == a->vq.mode && a->d == 128;

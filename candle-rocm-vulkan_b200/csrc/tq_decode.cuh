@@ -92,9 +92,6 @@ struct DecodeParams {
     uint32_t k_stage_bytes, v_stage_bytes;
     uint32_t ns;       // stages per warp
     uint32_t rows_cap;      // rows that exist in every (batch, head) slab of both caches (0 = only the visible ones)
-    // shares by place: workers of the blocks that start together, one per SM (0: all shares are equal), and the ends of their
-    // places' parts of the work in 1/256
-    uint32_t place_workers, place_end[3];
     uint32_t stream;        // the rows do not stay in L2 (CopySide::policy)
     uint32_t col_cost;      // cost of starting a column, in tiles, for the split of the work between the warps
     uint32_t qstage_bytes;  // query staging for the rotation (0 without it)
@@ -406,49 +403,24 @@ __device__ __forceinline__ Column make_column(const DecodeParams &p, const PageS
 // is a hundred instructions), and in 64 bits, out of line, where they do not.
 static __device__ __noinline__ uint64_t div64(uint64_t a, uint64_t b) { return a / b; }
 
-// The shares. Three blocks of four warps live on an SM, and its schedulers serve the warps that came first: with equal shares
-// the blocks of the first place were done after 72 us of a ragged MXFP4 call, those of the second after 77 and of the third
-// after 83 (83, 83 and 87 with a slower merge and these parts). So where a worker has many tiles, the places' shares differ (the
-// host gives the parts, see make_plan).
-constexpr uint32_t PLACE_MIN = 16;  // cost positions per worker from which the shares go by place
-struct Places {
-    uint64_t total;
-    uint32_t nw, n;      // workers, workers per place
-    bool by_place;
-};
-__device__ __forceinline__ Places places_of(const DecodeParams &p, uint64_t total, uint32_t nw) {
-    const bool by = p.place_workers != 0 && total >= (uint64_t)PLACE_MIN * nw;
-    return {total, nw, by ? p.place_workers : nw, by};
-}
-// the part [lo, lo + width) of the cost positions that place `k` works on
-__device__ __forceinline__ void place_part(const DecodeParams &p, const Places &pl, uint32_t k, uint64_t &lo, uint64_t &width) {
-    lo = k == 0 ? 0 : (pl.total * p.place_end[k - 1]) >> 8;
-    width = (pl.by_place ? (pl.total * p.place_end[k]) >> 8 : pl.total) - lo;
-}
-// first cost position of worker i (i == nw: the end); workers < 2^16
-__device__ __forceinline__ uint64_t share_start(const DecodeParams &p, const Places &pl, uint32_t i) {
-    uint32_t k = 0;
-    if (pl.by_place) k = (i >= pl.n && pl.n < pl.nw ? 1u : 0u) + (i >= 2 * pl.n && 2 * pl.n < pl.nw ? 1u : 0u);
-    uint64_t lo, width;
-    place_part(p, pl, k, lo, width);
-    i -= k * pl.n;
-    if (B200_LIKELY((pl.total >> 32) == 0)) {
-        const uint32_t q = (uint32_t)width / pl.n, r = (uint32_t)width - q * pl.n;
-        return lo + (uint64_t)q * i + r * i / pl.n;  // r < n, i <= n
+// The shares are equal: worker i of nw starts at floor(i total / nw). Parts by the order in which an SM's three blocks started
+// (92 : 85 : 79, the inverse of the times they took in one call) were slower or equal: ragged MXFP4 84.9 against 84.0 us, NVFP4 89.8
+// against 88.2, FP8 of head dim 64 63.5 against 61.8.
+// First cost position of worker i (i == nw: the end); workers < 2^16
+__device__ __forceinline__ uint64_t share_start(uint64_t total, uint32_t nw, uint32_t i) {
+    if (B200_LIKELY((total >> 32) == 0)) {
+        const uint32_t q = (uint32_t)total / nw, r = (uint32_t)total - q * nw;
+        return (uint64_t)q * i + r * i / nw;  // r < nw, i <= nw
     }
-    return lo + div64(width * i, pl.n);
+    return div64(total * i, nw);
 }
 // the worker that owns cost position x
-__device__ __forceinline__ uint32_t owner_of(const DecodeParams &p, const Places &pl, uint64_t x) {
-    uint32_t k = 0;
-    uint64_t lo, width;
-    place_part(p, pl, 0, lo, width);
-    while (x >= lo + width) place_part(p, pl, ++k, lo, width);
-    const uint64_t n = (x - lo + 1) * pl.n - 1;
-    // n < 2^48, width < 2^32: the quotient, below 2^16, is at least 2^-32 away from an integer that it does not reach, and a
+__device__ __forceinline__ uint32_t owner_of(uint64_t x, uint64_t total, uint32_t nw) {
+    const uint64_t n = (x + 1) * nw - 1;
+    // n < 2^48, total < 2^32: the quotient, below 2^16, is at least 2^-32 away from an integer that it does not reach, and a
     // double next to it less than 2^-37
-    if (B200_LIKELY((pl.total >> 32) == 0)) return k * pl.n + (uint32_t)((double)n / (double)(uint32_t)width);
-    return k * pl.n + (uint32_t)div64(n, width);
+    if (B200_LIKELY((total >> 32) == 0)) return (uint32_t)((double)n / (double)(uint32_t)total);
+    return (uint32_t)div64(n, total);
 }
 
 // A worker's share is a list of segments: tiles [t0, t1) of column y of batch entry b.
@@ -1329,9 +1301,8 @@ __device__ __forceinline__ Share worker_share(const DecodeParams &p, const PageS
     sh.has_work = wid < sh.nw;
     sh.x_end = 0;
     if (!sh.has_work) return sh;
-    const Places pl = places_of(p, total, sh.nw);
-    const uint64_t x_begin = share_start(p, pl, wid);
-    sh.x_end = share_start(p, pl, wid + 1);
+    const uint64_t x_begin = share_start(total, sh.nw, wid);
+    sh.x_end = share_start(total, sh.nw, wid + 1);
     // batch entry that holds cost position x_begin, and the position of its first column
     uint32_t b0 = 0;
     uint64_t b0_start = 0;
@@ -1485,8 +1456,8 @@ struct Worker {
         const uint32_t colidx = seg.b * ny + seg.y;
         // the column's segments are the workers first .. last (consecutive, every one of them owns a tile of it)
         const uint64_t x_col = seg.x - seg.t0;  // cost position of the column's first tile
-        const uint32_t first = seg.t0 == 0 ? wid : owner_of(p, places_of(p, total, nw), x_col);
-        const uint32_t last = seg.t1 == (uint32_t)seg.col.tiles ? wid : owner_of(p, places_of(p, total, nw), x_col + seg.col.tiles - 1);
+        const uint32_t first = seg.t0 == 0 ? wid : owner_of(x_col, total, nw);
+        const uint32_t last = seg.t1 == (uint32_t)seg.col.tiles ? wid : owner_of(x_col + seg.col.tiles - 1, total, nw);
         const uint32_t nseg = last - first + 1;
         if (p.ctr && nseg == 1) {
             // the whole column in this worker's registers

@@ -119,11 +119,11 @@ def test_prefix_sums_of_the_block_table(P, pages):
 @pytest.mark.parametrize("rotation", ["none", "hadamard"])
 @pytest.mark.parametrize("b,lk", [(24, 9000), (1, 70000), (200, 700)])
 def test_shares_and_merges_of_large_calls(P, rotation, b, lk):
-    """Shares by place (16 cost positions per worker and more), columns of few and of many segments, rows that leave L2 first."""
+    """Many tiles per worker, columns of few and of many segments, rows that leave L2 first."""
     f, hq, hkv, d = (2, 4), 16, 8, 128
     q, k, v, kq, vq = case(P, f, b, hq, hkv, 1, lk, d, 7, rotation)
     lens = torch.tensor([max(1, lk - (lk // 3) * (i % 3)) for i in range(b)], dtype=torch.int32, device="cuda:0")
     c = P.FlashAttnConfig(d ** -0.5).causal()
     got = P.attention_packed(q, k, v, lens, kq, vq, c)
-    one = P.attention_packed(q, k, v, lens, kq, vq, P.FlashAttnConfig(d ** -0.5, splits=1).causal())  # equal shares, one per column
-    assert_close(got.cpu().numpy(), one.cpu().numpy(), 1e-3, 1e-3, "shares by place against one share per column")
+    one = P.attention_packed(q, k, v, lens, kq, vq, P.FlashAttnConfig(d ** -0.5, splits=1).causal())  # one share per column
+    assert_close(got.cpu().numpy(), one.cpu().numpy(), 1e-3, 1e-3, "shares of the work against one share per column")
