@@ -63,9 +63,34 @@ static int fill_decode_side(DecodeSide &s, const B200QuantSide &q, uint32_t d, c
     return B200_OK;
 }
 
+// More than eight query rows per kv head: whether columns of 16, whose two groups of eight rows share the decoded keys and values, are
+// the faster ones (keys and values in one format, head dims 64 and 128; the kernel whose workers are pairs of warps has no such form).
+// A tile of such a column costs 1.1 to 1.3 times one of eight rows and two thirds as many warps work on them, so every worker needs enough
+// tiles: six, nine where a code is four bits and its conversion one instruction, a third more at head dim 64. Columns that many workers
+// share end in the merge of twice the rows: 40 tiles more for each partial result of a column. Short columns side by side over one kv
+// head's rows gain little from one decoding: 18 tiles more per column. us, columns of 8 -> 16 rows, tiles per worker, 8 kv heads:
+//   MXFP4, 16 rows, 16 sequences: 1480 keys (5) 32.7 -> 33.1, 2664 (9) 41.2 -> 41.0, 4144 (14) 53.3 -> 47.7, 8880 (30) 90.1 -> 73.7
+//   FP8, 16 rows, 16 sequences: 1480 keys 34.9 -> 36.2, 2072 (7) 39.0 -> 36.9, 4144 63.8 -> 48.8, 8880 115.6 -> 74.0
+//   one sequence (8 columns), 16 rows: MXFP4 42 624 keys (9) 45.1 -> 49.6, 66 304 (14) 57.0 -> 55.9; FP8 33 152 (7) 40.9 -> 47.8,
+//   52 096 (11) 52.0 -> 52.1
+//   32 rows, 64 sequences (1024 columns): MXFP4 518 keys (14) 71.2 -> 79.8, 740 (20) 85.8 -> 86.1, 1110 (30) 103.3 -> 91.0
+//   TurboQuant-4 in blocks of a page table, 16 rows, 16 sequences of 2000 keys (7) 52.7 -> 47.1
+// Lengths in device memory: lk is only their bound, and what a call loses where they are far below it is worst in few columns (one FP8
+// sequence of 8192 keys in a larger cache, 16 rows: 26 -> 37; 16 sequences of 512 keys: 23 -> 28, of 100: 17 -> 25), so the partial
+// results count four times.
+static bool wide_columns_pay(const B200TqAttnArgs *a, uint32_t packs16, bool paged) {
+    const uint64_t visible = a->wl >= 0 ? std::min<uint64_t>(a->lk, (uint64_t)a->wl + a->lq) : a->lk;
+    const uint64_t cols = std::max<uint64_t>((uint64_t)a->b * a->hkv * packs16, 1), tiles = cols * ((visible + WK - 1) / WK);
+    const uint64_t workers = (uint64_t)decode_blocks(2) * DW * sm_count_cached();
+    const uint64_t share = (a->kq.mode == B200_MXFP4 || a->kq.mode == B200_NVFP4 ? 9 : 6) * workers;
+    return tiles >= (a->d == 64 ? share * 4 / 3 : share) + (packs16 > 1 ? 18 * cols : 0) + (a->kv_len_dev && !paged ? 160 : 40) * workers / cols;
+}
+
 // paged: the plan of a call whose rows are read in the blocks of its page table (the tensor-core kernel walks the table)
 // narrow: columns of eight query rows, whatever the shape (a workspace that is too small for the wider ones)
-static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false, bool narrow = false) {
+// wide: columns of 16 query rows where there is such a form, whatever the lengths (the size that workspaces are asked for)
+enum class Columns { by_rule, narrow, wide };
+static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false, Columns columns = Columns::by_rule) {
     if (!a) return set_error(B200_ERR_BAD_ARG, "tq_attention: null args");
     if (a->hkv == 0 || a->hq % a->hkv != 0)
         return set_error(B200_ERR_BAD_ARG, "tq_attention: %u query heads are not a multiple of %u kv heads", a->hq, a->hkv);
@@ -104,15 +129,9 @@ static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false
     p.b = a->b; p.lq = a->lq; p.lk = a->lk; p.hq = a->hq; p.hkv = a->hkv; p.d = a->d;
     p.group = a->hq / a->hkv;
     p.rows_per_kv = p.group * a->lq;
-    // More than eight query rows per kv head: columns of 16, whose two groups of eight rows share the decoded keys and values.
-    // A tile of such a column costs 1.1 times one of eight rows, and two thirds as many warps work on them: worth it where it
-    // (nearly) halves the columns, and where every worker has six tiles (us, columns of 8 -> 16: 16 rows, 64 sequences of 512 to
-    // 8192 MXFP4 keys 163 -> 127, 32 of 8192 MXFP8 keys 213 -> 123; 24 rows, 8 x 4000 MXFP8 keys of 64: 41 -> 44; 32 rows,
-    // one sequence of 4000 keys: 31 -> 35; 12 rows, 5 x 4000 MXFP8 keys, four tiles a worker: 36.9 -> 39.0). For keys and values in one format, head dims 64 and 128; the kernel whose workers
-    // are pairs of warps has no such form.
     const uint32_t packs8 = (p.rows_per_kv + PACK - 1) / PACK, packs16 = (p.rows_per_kv + 2 * PACK - 1) / (2 * PACK);
-    pl.wide = !narrow && 5 * packs16 < 3 * packs8 && a->kq.mode == a->vq.mode && a->d <= 128 && (paged || !pair_formats(a->kq.mode, a->vq.mode)) &&
-              (uint64_t)a->b * a->hkv * packs16 * ((a->lk + WK - 1) / WK) >= 6ull * decode_blocks(2) * DW * sm_count_cached();
+    pl.wide = columns != Columns::narrow && 5 * packs16 < 3 * packs8 && a->kq.mode == a->vq.mode && a->d <= 128 &&
+              (paged || !pair_formats(a->kq.mode, a->vq.mode)) && (columns == Columns::wide || wide_columns_pay(a, packs16, paged));
     p.pack_rows = pl.wide ? 2 * PACK : PACK;
     p.packs = (p.rows_per_kv + p.pack_rows - 1) / p.pack_rows;
     p.scale = a->scale;
@@ -505,7 +524,7 @@ static bool paged_fast_plan(const B200TqAttnArgs *a, PagedFast &f) {
 // that kernel. Workspace: the keys and tiles before every block (written by a one-block kernel in front of the
 // attention), then the attention's own.
 static size_t paged_prefix_bytes(uint32_t n_pages) { return ((size_t)(n_pages + 1) * 8 + 255) / 256 * 256; }
-static bool paged_direct_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool narrow = false) {
+static bool paged_direct_plan(const B200TqAttnArgs *a, DecodePlan &pl, Columns columns = Columns::by_rule) {
     static const bool off = diag_env("B200_PAGED_NO_WALK") != nullptr;  // diagnostic: paged rows on the compaction / general paths
     if (off || !a || !a->pages || a->n_pages == 0 || a->lk == 0 || a->b == 0 || a->kq.mode != a->vq.mode) return false;
     if (a->flags & B200_TQ_IN_PLACE) return false;  // the caller asked for the general kernel
@@ -513,14 +532,13 @@ static bool paged_direct_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool narr
     t.flags &= ~(B200_TQ_AFTER_PREV | B200_TQ_INPUTS_FINAL);  // the prefix kernel of the call runs right before the attention
     if (tq_generic_takes(&t) && (a->d != 64 && a->d != 128 && a->d != 256)) return false;
     if (a->kq.mode == B200_TURBO_MSE && (a->kq.bits != 4 || a->vq.bits != 4)) return false;
-    return make_plan(&t, pl, true, narrow) == B200_OK;
+    return make_plan(&t, pl, true, columns) == B200_OK;
 }
 
-// what a call asks for; narrow: the least that its tensor-core kernel runs with (columns of eight query rows)
-static size_t workspace_need(const B200TqAttnArgs *a, bool narrow) {
+static size_t workspace_need(const B200TqAttnArgs *a, Columns columns) {
     {
         DecodePlan pl;
-        if (paged_direct_plan(a, pl, narrow)) return paged_prefix_bytes(a->n_pages) + pl.ws_bytes;
+        if (paged_direct_plan(a, pl, columns)) return paged_prefix_bytes(a->n_pages) + pl.ws_bytes;
     }
     {
         // paged rows: with this much workspace the blocks are compacted into it and the tensor-core kernel runs; with
@@ -530,11 +548,17 @@ static size_t workspace_need(const B200TqAttnArgs *a, bool narrow) {
     }
     if (tq_generic_takes(a)) return tq_generic_workspace_bytes(a);
     DecodePlan pl;
-    if (make_plan(a, pl, false, narrow)) return 0;
+    if (make_plan(a, pl, false, columns)) return 0;
     return pl.ws_bytes;
 }
+// what a call asks for: enough for the columns of 16 query rows where they may come to be the rule's choice, so that a workspace lasts
+// while the sequences grow
+static size_t workspace_ask(const B200TqAttnArgs *a) {
+    const size_t need = workspace_need(a, Columns::by_rule);
+    return need ? std::max(need, workspace_need(a, Columns::wide)) : 0;
+}
 
-extern "C" size_t b200_tq_attention_workspace_bytes(const B200TqAttnArgs *a) { return workspace_need(a, false); }
+extern "C" size_t b200_tq_attention_workspace_bytes(const B200TqAttnArgs *a) { return a && a->hkv && a->hq / a->hkv * (uint64_t)a->lq > PACK ? workspace_ask(a) : workspace_need(a, Columns::by_rule); }
 
 // set by b200_tq_attention_gather around its call of b200_tq_attention (same thread)
 static thread_local const B200PeerGather *tl_gather = nullptr;
@@ -548,7 +572,7 @@ extern "C" int b200_tq_attention(const B200TqAttnArgs *a, b200_stream_t stream_)
         if (paged_direct_plan(a, pl)) {
             const size_t pre = paged_prefix_bytes(a->n_pages);
             // a workspace that only the columns of eight rows fit
-            if (pl.wide && a->workspace_bytes < pre + pl.ws_bytes) paged_direct_plan(a, pl, true);
+            if (pl.wide && a->workspace_bytes < pre + pl.ws_bytes) paged_direct_plan(a, pl, Columns::narrow);
             if (a->workspace && a->workspace_bytes >= pre + pl.ws_bytes && !(reinterpret_cast<uintptr_t>(a->workspace) & 15) &&
                 (uint64_t)a->b * a->hq * a->lq != 0 && a->q && a->out) {
                 char *ws = reinterpret_cast<char *>(a->workspace);
@@ -599,7 +623,7 @@ extern "C" int b200_tq_attention(const B200TqAttnArgs *a, b200_stream_t stream_)
     }
     DecodePlan pl;
     int rc = make_plan(a, pl);
-    if (rc == B200_OK && pl.wide && a->workspace_bytes < pl.ws_bytes) rc = make_plan(a, pl, false, true);  // a workspace that only the columns of eight rows fit
+    if (rc == B200_OK && pl.wide && a->workspace_bytes < pl.ws_bytes) rc = make_plan(a, pl, false, Columns::narrow);  // a workspace that only the columns of eight rows fit
     if (rc) return rc;
     if ((uint64_t)a->b * a->hq * a->lq == 0) return B200_OK;
     if (!a->k_rows || !a->v_rows) return set_error(B200_ERR_BAD_ARG, "tq_attention: null pointer");
@@ -706,7 +730,7 @@ extern "C" int b200_tq_attention_static(const B200TqAttnArgs *a, b200_stream_t s
     args.workspace = nullptr;
     args.workspace_bytes = 0;
     size_t need = b200_tq_attention_workspace_bytes(&args);
-    if (need > (size_t)B200_STATIC_SCRATCH_BYTES) need = workspace_need(&args, true);
+    if (need > (size_t)B200_STATIC_SCRATCH_BYTES) need = workspace_need(&args, Columns::narrow);
     const bool in_place = args.pages != nullptr && need > (size_t)B200_STATIC_SCRATCH_BYTES;  // too large to compact: read in place
     if (in_place) need = 16;
     if (need > (size_t)B200_STATIC_SCRATCH_BYTES)

@@ -373,8 +373,10 @@ int b200_tq_attention(const B200TqAttnArgs *args, b200_stream_t stream);
  * nothing: no cudaMalloc, cudaFree or allocating library routine.
  *
  * args->workspace and args->workspace_bytes are ignored; inputs and outputs are passed as usual.
- * A call whose b200_tq_attention_workspace_bytes() exceeds B200_STATIC_SCRATCH_BYTES is refused
- * with B200_ERR_WORKSPACE and a message that names both sizes (use b200_tq_attention then).
+ * b200_tq_attention_workspace_bytes() asks for what the call's fastest form takes. Where that exceeds
+ * B200_STATIC_SCRATCH_BYTES the call takes its smallest form (eight query rows per column; paged rows
+ * read in place). Where that one does not fit either, the call is refused with B200_ERR_WORKSPACE and a
+ * message that names both sizes (use b200_tq_attention then).
  * The first call on each device looks up the buffer's device address (with that device current)
  * and keeps it; make that first call before any stream capture begins on that device.
  * Every call on a device shares the one buffer, which keeps the previous call's contents. Nothing

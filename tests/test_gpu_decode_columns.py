@@ -1,6 +1,6 @@
 """Columns of 16 query rows of the decode kernels over packed rows.
 
-They run from 9 query rows per kv head on, where they halve the columns and every worker has six tiles; the same call with a
+They run from 9 query rows per kv head on, where they halve the columns and every worker has enough tiles; the same call with a
 workspace that only the columns of eight rows fit takes those. Both forms are held to one another (same f16 weights up to the
 reference maximum of a split, f32 sums: 1e-3 + 1e-3 |x|) and to the oracle for one batch entry."""
 import importlib.util
@@ -127,3 +127,43 @@ def test_shares_and_merges_of_large_calls(P, rotation, b, lk):
     got = P.attention_packed(q, k, v, lens, kq, vq, c)
     one = P.attention_packed(q, k, v, lens, kq, vq, P.FlashAttnConfig(d ** -0.5, splits=1).causal())  # one share per column
     assert_close(got.cpu().numpy(), one.cpu().numpy(), 1e-3, 1e-3, "shares of the work against one share per column")
+
+
+# ---- where the columns of 16 rows begin. A call of 16 and more rows asks for the workspace of its widest form; with 16 bytes less it takes
+# columns of eight, whose splits of the keys, and with them the last bits, are others.
+def tiles_per_worker(tiles):
+    return tiles * 8 * torch.cuda.get_device_properties(0).multi_processor_count  # two blocks of four workers per SM
+
+
+def both_forms(P, call):
+    got = call.run().clone()
+    call.args.workspace_bytes = P._abi.lib().b200_tq_attention_workspace_bytes(call._ref) - 16
+    return got, call.run().clone()
+
+
+RULE = [
+    # format, b, hq, hkv, lq, d, tiles per worker, window on the left, lengths in device memory, columns of 16 rows
+    ((2, 4), 8, 32, 8, 4, 128, 12.0, -1, False, True),
+    ((2, 4), 8, 32, 8, 4, 128, 8.0, -1, False, False),
+    ((5, 4), 8, 32, 8, 4, 128, 8.0, -1, False, True),
+    ((5, 4), 8, 32, 8, 4, 128, 5.0, -1, False, False),
+    ((2, 4), 8, 32, 8, 4, 64, 11.0, -1, False, False),
+    ((2, 4), 8, 32, 8, 4, 64, 15.0, -1, False, True),
+    ((5, 4), 1, 32, 8, 4, 128, 9.0, -1, False, False),  # eight columns that 148 workers share each
+    ((5, 4), 1, 32, 8, 4, 128, 13.0, -1, False, True),
+    ((5, 4), 1, 32, 8, 4, 128, 13.0, -1, True, False),  # ... of which the lengths may be a small part
+    ((5, 4), 1, 32, 8, 4, 128, 13.0, 300, False, False),  # a window: the tiles that it shows
+    ((4, 4), 64, 32, 8, 8, 128, 18.0, -1, False, False),  # two short columns per kv head
+    ((4, 4), 64, 32, 8, 8, 128, 26.0, -1, False, True),
+]
+
+
+@pytest.mark.parametrize("f,b,hq,hkv,lq,d,tiles,wl,dev,wide", RULE, ids=lambda x: str(x))
+def test_where_columns_of_16_rows_begin(P, f, b, hq, hkv, lq, d, tiles, wl, dev, wide):
+    lk = int(tiles_per_worker(tiles)) * 32 // (b * hkv * ((hq // hkv * lq + 15) // 16))
+    q, k, v, kq, vq = case(P, f, b, hq, hkv, lq, lk, d, 11)
+    c = P.FlashAttnConfig(d ** -0.5).window(None if wl < 0 else wl, 0)
+    lens = torch.full((b,), lk, dtype=torch.int32, device="cuda:0") if dev else lk
+    got, small = both_forms(P, P.PackedAttention(q, k, v, lens, kq, vq, c))
+    assert_close(got.cpu().numpy(), small.cpu().numpy(), 1e-3, 1e-3, "the two forms")
+    assert torch.equal(got, small) != wide
