@@ -230,8 +230,6 @@ static int make_plan(const B200TqAttnArgs *a, DecodePlan &pl, bool paged = false
     p.prefetch = (p.after_prev && (a->flags & B200_TQ_INPUTS_FINAL)) ? 1u : 0u;
     p.out_free = (p.after_prev && (a->flags & B200_TQ_OUTPUTS_FREE)) ? 1u : 0u;
     p.fresh_rows = std::min<uint32_t>(a->fresh_rows, 0x7fffffffu);
-    // packs of query rows read the rows again; how many rows there are the kernel sees from the lengths (CopySide::policy)
-    p.stream = p.packs == 1 ? 1u : 0u;
     pl.nat = !paged && p.k_ss == (uint64_t)kl.row_words && p.v_ss == (uint64_t)vl.row_words && a->kq.mode == a->vq.mode && a->d == 128;
     if (pl.nat) {
         // the native-row kernels read a lane's codes with 8- or 16-byte loads where the row length allows: every

@@ -92,7 +92,6 @@ struct DecodeParams {
     uint32_t k_stage_bytes, v_stage_bytes;
     uint32_t ns;       // stages per warp
     uint32_t rows_cap;      // rows that exist in every (batch, head) slab of both caches (0 = only the visible ones)
-    uint32_t stream;        // the rows may be too many to stay in L2 (CopySide::policy)
     uint32_t col_cost;      // cost of starting a column, in tiles, for the split of the work between the warps
     uint32_t qstage_bytes;  // query staging for the rotation (0 without it)
     uint32_t after_prev;    // launched as a programmatic dependent of the stream's previous kernel
@@ -1551,17 +1550,14 @@ struct CopySide {
 
     uint64_t pol;  // cache policy of the copies
 
-    // Rows that a call reads once and that take half of L2 (126 MB) or more leave first: otherwise they push the call's own code, its
-    // queries and partial results out (a merge of 4.4 partial results took 22 instead of 7 thousand cycles). By the visible rows, not
-    // the capacity. us, normal order -> this, two and six caches read in turn (between two passes of a model's layer lie the others): 74 MB
-    // TurboQuant-4 36.5 -> 35.5 and 36.8 -> 36.1, 78 MB MXFP4 34.8 -> 32.9 and 34.5 -> 32.9, 147 MB MXFP8 51.3 -> 41.8 and 50.4 -> 43.7,
-    // 319 MB MXFP4 83.0 -> 80.6 and 83.1 -> 80.8, from 570 MB on equal. Fewer rows lose hits: 37 MB TurboQuant-4 25.7 -> 26.9, 20 MB MXFP4
-    // 18.5 -> 20.5 (two caches). One cache read again at once: 70 MB FP8 25.5 -> 26.7, 147 MB MXFP8 51.1 -> 39.4, because a part survives.
-    static constexpr uint64_t STREAM_BYTES = 64ull << 20;
-    __device__ __forceinline__ void policy(const Worker &w, uint32_t krb, uint32_t vrb) {
-        const uint64_t setup = (uint64_t)w.ncols * w.p.col_cost;  // the rest of the call's cost is tiles (columns without keys cost nothing)
-        if (w.p.stream && w.total > setup && (w.total - setup) * (WK * (krb + vrb)) > STREAM_BYTES) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-        else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+    // Rows that a call reads once leave L2 first: otherwise they push the call's own code, its queries and partial results out (a merge of
+    // 4.4 partial results took 22 instead of 7 thousand cycles), and rows read again and again push one another out. Time against the normal
+    // order, geometric mean over the five formats and three shapes, one, three and twelve caches read in turn (between two passes of a
+    // model's layer lie the others): 12 MB of visible rows 1.00, 1.00, 0.99; 36 MB 1.00, 0.98, 0.98; 50 MB 1.00, 0.97, 0.98; 100 MB 0.92 with
+    // any number; 319 MB MXFP4 0.97; from 570 MB on equal. Of 500 single figures two lie above 1.015 (1.02 at 26 MB, 1.04 at 12).
+    __device__ __forceinline__ void policy(const DecodeParams &p) {
+        if (p.packs == 1) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+        else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));  // packs of query rows read the rows again
     }
 
     // per-segment constants
@@ -1580,11 +1576,11 @@ struct CopySide {
         vb = (voff + (uint32_t)WK * vrb + 15u) & ~15u;
     }
 
-    __device__ __forceinline__ void start(const Worker &w, const Segment &seg, uint32_t krb, uint32_t vrb) {
-        policy(w, krb, vrb);
+    __device__ __forceinline__ void start(const DecodeParams &p, const Segment &seg, uint32_t krb, uint32_t vrb) {
+        policy(p);
         iseg = seg;
         more = true;
-        enter(w.p, krb, vrb);
+        enter(p, krb, vrb);
     }
 
     // ---- paged rows: a tile's source is (block, row in the block) instead of rows + key * stride
@@ -1606,7 +1602,7 @@ struct CopySide {
         load_page(p, krb, vrb);
     }
     __device__ __forceinline__ void start_paged(const Worker &w, const Segment &seg, uint32_t krb, uint32_t vrb) {
-        policy(w, krb, vrb);
+        policy(w.p);
         iseg = seg;
         more = true;
         enter_paged(w.p, w.ps, krb, vrb);
@@ -1907,7 +1903,7 @@ __global__ void __launch_bounds__(DW * 32, decode_blocks(NH)) tq_decode_kernel(c
     // once (ragged MXFP4 call: 92.7 -> 91.3 us; 64 x 2 query tokens, 64 heads: 139.6 -> 138.5).
     CopySide cs;
     if constexpr (PAGED) cs.start_paged(wk, sh.seg, krb, vrb);
-    else cs.start(wk, sh.seg, krb, vrb);
+    else cs.start(p, sh.seg, krb, vrb);
     auto copy_tile = [&](uint32_t st, uint32_t bar, uint32_t desc) {
         if constexpr (PAGED) cs.tile_paged(wk, st, bar, desc, krb, vrb, k_stage_bytes, sh.x_end);
         else cs.tile(wk, st, bar, krb, vrb, k_stage_bytes, sh.x_end);
@@ -2230,7 +2226,7 @@ __global__ void __launch_bounds__(PW * 64, 2) tq_decode_pair_kernel(const Decode
         const uint32_t v_lane = (PERM ? (uint32_t)perm_key(2 * c) : 2u * c) * vrb + (V4 ? g * (HD / 16) : g * (HD / 8));
         float oacc[1][STEPS][4];
         CopySide cs;
-        cs.start(wk, sh.seg, krb, vrb);
+        cs.start(p, sh.seg, krb, vrb);
         for (int i = 0; i < NS && cs.left > 0; ++i)
             cs.tile(wk, wstage_s + (uint32_t)i * stage_bytes, wbar_s + 8u * (uint32_t)i, krb, vrb, k_stage_bytes, sh.x_end);
         auto msg_wait = [&]() -> bool { return stage_wait(qfull_s + 8u * (msgs % PQ), (msgs / PQ) & 1u); };
