@@ -553,10 +553,11 @@ static size_t workspace_need(const B200TqAttnArgs *a, Columns columns) {
 // while the sequences grow
 static size_t workspace_ask(const B200TqAttnArgs *a) {
     const size_t need = workspace_need(a, Columns::by_rule);
-    return need ? std::max(need, workspace_need(a, Columns::wide)) : 0;
+    const bool two_forms = need && a->hkv && (uint64_t)a->hq / a->hkv * a->lq > PACK;
+    return two_forms ? std::max(need, workspace_need(a, Columns::wide)) : need;
 }
 
-extern "C" size_t b200_tq_attention_workspace_bytes(const B200TqAttnArgs *a) { return a && a->hkv && a->hq / a->hkv * (uint64_t)a->lq > PACK ? workspace_ask(a) : workspace_need(a, Columns::by_rule); }
+extern "C" size_t b200_tq_attention_workspace_bytes(const B200TqAttnArgs *a) { return workspace_ask(a); }
 
 // set by b200_tq_attention_gather around its call of b200_tq_attention (same thread)
 static thread_local const B200PeerGather *tl_gather = nullptr;
@@ -577,11 +578,11 @@ extern "C" int b200_tq_attention(const B200TqAttnArgs *a, b200_stream_t stream_)
                 uint32_t *pg_keys = reinterpret_cast<uint32_t *>(ws), *pg_tiles = pg_keys + (a->n_pages + 1);
                 pl.p.pg_keys = pg_keys;
                 pl.p.pg_tiles = pg_tiles;
-                // Few blocks: the blocks of the attention work the sums out themselves (16 x 4000 keys in 8 blocks: 46 -> 44.5 us),
-                // where the kilobyte costs no resident block.
-                const size_t with = pl.smem + PG_SUMS_BYTES, per_sm = 228 * 1024;
-                if (a->n_pages <= PG_BUILD && with <= 227 * 1024 &&
-                    std::min<size_t>(per_sm / (with + 1024), decode_blocks(pl.wide ? 2 : 1)) == std::min<size_t>(per_sm / (pl.smem + 1024), decode_blocks(pl.wide ? 2 : 1))) {
+                // Few blocks: the blocks of the attention work the sums out themselves (us, a kernel in front -> this, 16 rows per kv head:
+                // MXFP4 16 x 4000 keys in 8 blocks 53.3 -> 51.8, FP8 1 x 7000 28.8 -> 27.1), where the kilobyte costs no resident block.
+                const size_t with = pl.smem + PG_SUMS_BYTES;
+                auto resident = [&](size_t smem) { return std::min<size_t>(228 * 1024 / (smem + 1024), decode_blocks(pl.wide ? 2 : 1)); };
+                if (a->n_pages <= PG_BUILD && with <= 227 * 1024 && resident(with) == resident(pl.smem)) {
                     pl.p.pg_build = 1;
                     pl.p.pg_sums = (uint32_t)pl.smem;
                     pl.smem = with;
@@ -621,7 +622,8 @@ extern "C" int b200_tq_attention(const B200TqAttnArgs *a, b200_stream_t stream_)
     }
     DecodePlan pl;
     int rc = make_plan(a, pl);
-    if (rc == B200_OK && pl.wide && a->workspace_bytes < pl.ws_bytes) rc = make_plan(a, pl, false, Columns::narrow);  // a workspace that only the columns of eight rows fit
+    // a workspace that only the columns of eight rows fit
+    if (rc == B200_OK && pl.wide && a->workspace_bytes < pl.ws_bytes) rc = make_plan(a, pl, false, Columns::narrow);
     if (rc) return rc;
     if ((uint64_t)a->b * a->hq * a->lq == 0) return B200_OK;
     if (!a->k_rows || !a->v_rows) return set_error(B200_ERR_BAD_ARG, "tq_attention: null pointer");

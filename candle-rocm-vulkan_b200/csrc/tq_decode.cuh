@@ -1,6 +1,6 @@
 // Decode attention over packed K/V rows (FP8, MXFP8, MXFP4, NVFP4, TurboQuant 4-bit): kernel body.
 //
-// Work split: the visible keys of every column (batch entry, kv head, pack of up to 8 query rows that
+// Work split: the visible keys of every column (batch entry, kv head, pack of up to 8 or 16 query rows that
 // share that kv head) are cut into 32-key tiles; the tiles of all columns form one list that the
 // warps of the persistent blocks share in cost order. Every warp is a worker of its own: it streams
 // its tiles through a private ring of shared memory stages filled by bulk copies (cp.async.bulk +
@@ -1899,8 +1899,9 @@ __global__ void __launch_bounds__(DW * 32, decode_blocks(NH)) tq_decode_kernel(c
     const uint32_t wdesc_s = sbase + FIXED_SMEM + DW * META + p.qstage_bytes + (uint32_t)DW * NS * stage_bytes + (uint32_t)warp * NS_MAX * 16;
     bool wait_failed = false;
 
-    // All stages are asked for right away: the first tiles land a little later than alone, but the code that asks is fetched
-    // once (ragged MXFP4 call: 92.7 -> 91.3 us; 64 x 2 query tokens, 64 heads: 139.6 -> 138.5).
+    // All stages are asked for right away: the first tiles land a little later than alone, but the code that asks is fetched once. Against
+    // the first tile alone and the others behind the first query rows: short calls 0.97 to 1.00 of the time (64 x 300 MXFP4 keys 18.6 ->
+    // 18.2 us, 200 x 100 27.8 -> 27.1), long ones equal within what two runs differ by.
     CopySide cs;
     if constexpr (PAGED) cs.start_paged(wk, sh.seg, krb, vrb);
     else cs.start(p, sh.seg, krb, vrb);

@@ -36,7 +36,7 @@ struct QuantParams {
     QuantSideParams side[2];
     uint32_t nb, nh, nt, d;
     int32_t src_dtype;
-    uint32_t nt_mul, nt_shr, nh_mul, nh_shr;  // fastdiv invariants of nt and nh (rows128 kernel)
+    uint32_t nt_mul, nt_shr, nh_mul, nh_shr;  // fastdiv invariants of nt and nh (rows16 kernel)
     uint32_t after_prev;  // launched as a programmatic dependent of the stream's previous kernel (B200_KV_AFTER_PREV)
 };
 
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(QW * 32) quant_rows_kernel(const QuantParams p
 // explicitly. Maxima do not depend on the order of the reduction, every division is IEEE, so rows are bit-identical to
 // quant_rows_kernel's. Row -> (batch entry, head, token) uses multiply-high division by the launch's invariants.
 // ---------------------------------------------------------------------------------------------
-constexpr int Q128_WARPS = 8;  // warps per block
+constexpr int Q16_WARPS = 8;  // warps per block
 
 // one value -> its e4m3 code
 __device__ __forceinline__ uint32_t e4m3_hw(float f) {
@@ -390,10 +390,12 @@ __device__ __forceinline__ uint32_t fastdiv(uint32_t n, uint32_t mul, uint32_t s
 
 // CODES: a side of the call is in a codebook format. Without, their code is left out: its registers and its prologue cost the block-scaled
 // formats 0.1 us of the 1.8 of a few rows.
-// LPR: lanes that share a row, 16 elements each: rows of 64, 128 or 256 elements. TurboQuant-4 rows packed and unpacked, with a warp per
-// row for the packing and like this: 64 000 rows of 64 elements 72 -> 36 us, 32 000 of 256 57 -> 28 (host time from there on).
+// LPR: lanes that share a row, 16 elements each: rows of 64, 128 or 256 elements. Against a warp per row (us, bf16 rows packed and
+// unpacked, device alone): 64 000 rows of 64 TurboQuant-4 rotated 66.8 -> 15.0, MXFP4 38.0 -> 8.7, FP8 38.7 -> 10.3; 32 000 of 256
+// TurboQuant-4 rotated 71.8 -> 33.6, NVFP4 54.1 -> 16.1. Few rows too (keys and values of 8 to 8000 rows, packed): MXFP4 of 64 elements 2.5 -> 1.6
+// at 8, 10.0 -> 2.3 at 8000; FP8 of 256 2.8 -> 2.2 and 12.6 -> 5.8; no format above 0.96 of its time.
 template <int DT, bool CODES, int LPR>
-__global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const QuantParams p) {
+__global__ void __launch_bounds__(Q16_WARPS * 32) quant_rows16_kernel(const QuantParams p) {
     const QuantSideParams &sp = p.side[blockIdx.y];
     constexpr int RPW = 32 / LPR;
     const int lane = threadIdx.x & 31, l8 = lane % LPR;
@@ -408,7 +410,7 @@ __global__ void __launch_bounds__(Q128_WARPS * 32) quant_rows128_kernel(const Qu
         b7 = bound[7], b3 = bound[3], b11 = bound[11];
     }
     after_prev_begin(p);
-    for (uint32_t base = (blockIdx.x * Q128_WARPS + (threadIdx.x >> 5)) * RPW; base < rows; base += gridDim.x * Q128_WARPS * RPW) {
+    for (uint32_t base = (blockIdx.x * Q16_WARPS + (threadIdx.x >> 5)) * RPW; base < rows; base += gridDim.x * Q16_WARPS * RPW) {
         bool live = base + lane / LPR < rows;  // a row past the end repeats the last one and stores nothing
         const uint32_t row = live ? base + lane / LPR : rows - 1;
         const uint32_t bh = fastdiv(row, p.nt_mul, p.nt_shr), t = row - bh * p.nt, b = fastdiv(bh, p.nh_mul, p.nh_shr), h = bh - b * p.nh;
@@ -611,13 +613,13 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint32_t *__res
 
 // ---------------------------------------------------------------------------------------------
 // Packed rows back to values in one pass: decode, rotate back, cast, store. LPR lanes share a row, each with 16 consecutive
-// elements (as in quant_rows128_kernel); grid.y: keys, values. Bound by memory: 65 528 rows of 72 bytes to bf16 move 21 MB.
+// elements (as in quant_rows16_kernel); grid.y: keys, values. Bound by memory: 65 528 rows of 72 bytes to bf16 move 21 MB.
 // The chain it stands for (dequant_rows_kernel, hadamard_rows_kernel, a cast; in f32, with a copy in front when the rows
 // are not back to back) moves ten times the bytes in three or four launches. Values are the chain's, bit for bit: the same
 // roundings in the same order, butterflies from index bit 0 up. Measured: keys and values of 8192 x 8 cached MXFP8 rows, rotated, for a chunk of 1024 query tokens: the
 // call 414 -> 173 us (141 of them the attention); 65 528 TurboQuant-4 rows packed and unpacked 250 -> 37 us (with the codebook
-// formats in quant_rows128_kernel, and each row packed once instead of twice). Hardware conversions of the codes and butterflies
-// of two elements per instruction: 37.7 -> 36.4 (35 of them host time), the chunk 173.5 -> 172.
+// formats in quant_rows16_kernel, and each row packed once instead of twice). Hardware conversions of the codes and butterflies of two
+// elements per instruction: 32.3 -> 31.8 of those on the device, the chunk 173.1 -> 171.4.
 // ---------------------------------------------------------------------------------------------
 struct UnpackSide {
     const uint32_t *src;
@@ -865,8 +867,8 @@ static void fastdiv_init(uint32_t d, uint32_t &mul, uint32_t &shr) {
     mul = (uint32_t)((((one << (32 + shr)) + d - 1) / d) - (one << 32));
 }
 
-// rows of 128 elements whose source rows can be read as 16-byte vectors
-static bool rows128_takes(const QuantParams &p, int sides) {
+// rows of 64, 128 and 256 elements whose source rows can be read as 16-byte vectors
+static bool rows16_takes(const QuantParams &p, int sides) {
     static const bool off = diag_env("B200_QUANT_GENERIC") != nullptr;
     if (off || (p.d != 64 && p.d != 128 && p.d != 256) || (uint64_t)p.nb * p.nh * p.nt >= 0x7fffff00ull) return false;
     const uint64_t vec = p.src_dtype == B200_F32 ? 3 : 7;  // elements per 16 bytes - 1
@@ -902,33 +904,33 @@ static int launch_maybe_after_prev(void (*kern)(const QuantParams), dim3 grid, d
 }
 
 template <bool CODES, int LPR>
-static int launch_rows128(const QuantParams &p, int sides, cudaStream_t stream) {
+static int launch_rows16(const QuantParams &p, int sides, cudaStream_t stream) {
     QuantParams q = p;
     fastdiv_init(p.nt, q.nt_mul, q.nt_shr);
     fastdiv_init(p.nh, q.nh_mul, q.nh_shr);
-    const uint64_t rows = (uint64_t)p.nb * p.nh * p.nt, per_block = Q128_WARPS * (32 / LPR);
+    const uint64_t rows = (uint64_t)p.nb * p.nh * p.nt, per_block = Q16_WARPS * (32 / LPR);
     // as many blocks as are resident at once, shared by the sides
     static const int resident = [] {
         int per_sm = 4, sms = 148, dev = 0;
         cudaGetDevice(&dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quant_rows128_kernel<B200_BF16, CODES, LPR>, Q128_WARPS * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quant_rows16_kernel<B200_BF16, CODES, LPR>, Q16_WARPS * 32, 0);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         return std::max(per_sm, 1) * std::max(sms, 1);
     }();
-    const dim3 grid((unsigned)std::min<uint64_t>((rows + per_block - 1) / per_block, (uint64_t)std::max(resident / sides, 1)), sides), block(Q128_WARPS * 32);
-    if (p.src_dtype == B200_F32) return launch_maybe_after_prev(quant_rows128_kernel<B200_F32, CODES, LPR>, grid, block, stream, q);
-    if (p.src_dtype == B200_F16) return launch_maybe_after_prev(quant_rows128_kernel<B200_F16, CODES, LPR>, grid, block, stream, q);
-    return launch_maybe_after_prev(quant_rows128_kernel<B200_BF16, CODES, LPR>, grid, block, stream, q);
+    const dim3 grid((unsigned)std::min<uint64_t>((rows + per_block - 1) / per_block, (uint64_t)std::max(resident / sides, 1)), sides), block(Q16_WARPS * 32);
+    if (p.src_dtype == B200_F32) return launch_maybe_after_prev(quant_rows16_kernel<B200_F32, CODES, LPR>, grid, block, stream, q);
+    if (p.src_dtype == B200_F16) return launch_maybe_after_prev(quant_rows16_kernel<B200_F16, CODES, LPR>, grid, block, stream, q);
+    return launch_maybe_after_prev(quant_rows16_kernel<B200_BF16, CODES, LPR>, grid, block, stream, q);
 }
 
 static int launch_quant(const QuantParams &p, int sides, cudaStream_t stream) {
     const uint64_t rows = (uint64_t)p.nb * p.nh * p.nt;
     if (rows == 0) return B200_OK;
-    if (rows128_takes(p, sides)) {
+    if (rows16_takes(p, sides)) {
         const bool codes = p.side[0].mode <= B200_TURBO_PROD || (sides > 1 && p.side[1].mode <= B200_TURBO_PROD);
-        if (p.d == 64) return codes ? launch_rows128<true, 4>(p, sides, stream) : launch_rows128<false, 4>(p, sides, stream);
-        if (p.d == 256) return codes ? launch_rows128<true, 16>(p, sides, stream) : launch_rows128<false, 16>(p, sides, stream);
-        return codes ? launch_rows128<true, 8>(p, sides, stream) : launch_rows128<false, 8>(p, sides, stream);
+        if (p.d == 64) return codes ? launch_rows16<true, 4>(p, sides, stream) : launch_rows16<false, 4>(p, sides, stream);
+        if (p.d == 256) return codes ? launch_rows16<true, 16>(p, sides, stream) : launch_rows16<false, 16>(p, sides, stream);
+        return codes ? launch_rows16<true, 8>(p, sides, stream) : launch_rows16<false, 8>(p, sides, stream);
     }
     const unsigned gx = (unsigned)std::min<uint64_t>((rows + QW - 1) / QW, 148ull * 64);
     const dim3 grid(gx, sides), block(QW * 32);

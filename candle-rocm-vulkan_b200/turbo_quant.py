@@ -743,7 +743,9 @@ class TurboKvCache:
 
     # query rows per kv head (tokens x heads of the group) from which a chunk of prefill over the cache goes through
     # the dequantized rows and the tensor-core prefill tiles instead of the decode kernel, which re-reads the packed
-    # rows once per pack of eight query rows
+    # rows once per pack of eight or sixteen query rows. us, decode kernel and tiles, rotated MXFP8, 512 rows: 1000 cached
+    # keys 45.9 and 45.9, 8000 122 and 59, 32 000 383 and 157; 256 rows: 32 and 46 (host time), 73 and 54, 211 and 133;
+    # 128 rows: 26 and 61, 49 and 61, 124 and 127. TurboQuant-4 and MXFP4 cross near the same rows
     PREFILL_ROWS = 512
 
     def attention(self, q: torch.Tensor, cfg: FlashAttnConfig) -> torch.Tensor:
