@@ -55,8 +55,6 @@ static int fill_decode_side(DecodeSide &s, const B200QuantSide &q, uint32_t d, c
         return set_error(B200_ERR_UNSUPPORTED_SHAPE, "tq_attention: only none / hadamard rotations are fused");
     }
     s.mode = q.mode;
-    s.code_words = l.code_words;
-    s.rsc_off = l.rsc_offset;
     s.rot = q.rotation;
     s.tab = q.tab;
     s.signs = q.signs;
@@ -583,7 +581,6 @@ extern "C" int b200_tq_attention(const B200TqAttnArgs *a, b200_stream_t stream_)
                 const size_t with = pl.smem + PG_SUMS_BYTES;
                 auto resident = [&](size_t smem) { return std::min<size_t>(228 * 1024 / (smem + 1024), decode_blocks(pl.wide ? 2 : 1)); };
                 if (a->n_pages <= PG_BUILD && with <= 227 * 1024 && resident(with) == resident(pl.smem)) {
-                    pl.p.pg_build = 1;
                     pl.p.pg_sums = (uint32_t)pl.smem;
                     pl.smem = with;
                     return run_plan(a, pl, ws + pre, a->workspace_bytes - pre, (cudaStream_t)stream_);

@@ -62,8 +62,7 @@ constexpr float LN2 = 0.6931471805599453f;
 #define B200_UNLIKELY(x) __builtin_expect(!!(x), 0)
 
 struct DecodeSide {
-    int32_t mode, code_words, rsc_off;
-    int32_t rot;
+    int32_t mode, rot;
     const float *tab;
     const float *signs;
 };
@@ -109,14 +108,19 @@ struct DecodeParams {
     uint32_t *ctr;
     int32_t *lib_status;    // library-wide flag: set when a bounded wait of a kernel of this call runs out
     // paged rows (null: dense rows): the block table, and for every block the keys and the 32-key tiles of the
-    // blocks before it (n_pages + 1 entries each, written by tq_page_prefix_kernel right before this grid). pg_build: every
+    // blocks before it (n_pages + 1 entries each, written by tq_page_prefix_kernel right before this grid). pg_sums not 0: every
     // block works the sums out in its own shared memory, pg_sums bytes from the start, and block 0 leaves them at pg_keys /
     // pg_tiles for the combine grid; nothing in this grid reads those.
     const B200Page *pages;
     uint32_t n_pages;
-    uint32_t pg_build, pg_sums;
+    uint32_t pg_sums;
     uint32_t *pg_keys, *pg_tiles;
+    uint32_t unused[10];
 };
+// The host's part of a launch depends on the arguments' size modulo 64 bytes: an empty kernel takes it 2.13 us with 480 bytes (2.05 as a
+// programmatic dependent), 2.45 with eight bytes more or less and 2.85 (2.4) with 440, 448, 464 or 512. Attention and combine grid of a
+// decode step over 2047 FP8 keys: 1.1 us of 24.
+static_assert(sizeof(DecodeParams) == 480, "pad the launch arguments to 32 bytes past a multiple of 64");
 
 __host__ __device__ constexpr bool fmt_is4(int m) { return m == B200_MXFP4 || m == B200_NVFP4 || m == B200_TURBO_MSE; }
 __host__ __device__ constexpr bool fmt_is_mx(int m) { return m == B200_MXFP4 || m == B200_MXFP8; }
@@ -1865,7 +1869,7 @@ __global__ void __launch_bounds__(DW * 32, decode_blocks(NH)) tq_decode_kernel(c
     PageSums ps = {nullptr, nullptr};
     if constexpr (PAGED) {
         ps = {p.pg_keys, p.pg_tiles};
-        if (p.pg_build) {
+        if (p.pg_sums) {
             uint32_t *sums = reinterpret_cast<uint32_t *>(smem + p.pg_sums);
             if (warp == 1) page_prefix(p, sums, sums + PG_BUILD + 1, blockIdx.x == 0, lane);
             ps = {sums, sums + PG_BUILD + 1};
